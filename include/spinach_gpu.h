@@ -86,6 +86,13 @@ typedef struct {
 #define SPX_FLAG_NO_FP32_CHECK 1   /* skip the FP64 check of an FP32 run */
 #define SPX_FLAG_NO_PROMOTE 2      /* report the check, never re-run in FP64 */
 
+/*
+ * Powder runs restrict themselves to the states that exchange signal with the
+ * coils: the connected components of the Liouvillian's pattern that hold both
+ * coil and initial-state entries, at most 512 states.  The FIDs do not depend
+ * on the others.  A run whose options set threads, cluster, chunk_steps or
+ * chunk_target takes the whole system in that shape.
+ */
 /* Statistics of the last spx_run_powder* call on a handle. */
 typedef struct {
     int64_t n_orientations;
@@ -119,7 +126,10 @@ typedef struct {
                                   the checked orientations' FIDs (0 when not measured) */
     int32_t promoted_fp64;     /* 1 if spx_run_powder found the FP32 error above the
                                   bar and returned an FP64 re-run instead */
-    int32_t reserved;
+    int32_t coupled_dim;       /* states that couple to the coils, if the run was restricted
+                                  to them (0: the whole system ran).  threads, cluster,
+                                  smem_bytes, nnz and ell_entries describe the whole
+                                  system and its launch shape either way */
     double fp32_powder_error;  /* the error those imply for the powder FID, two parts in
                                   quadrature: the checked orientations' running relative
                                   error weighted by the powder FID's intensity over time,

@@ -1,0 +1,1041 @@
+// Propagation of the states that couple to the detection states.
+//
+// The Liouvillian of a powder is block diagonal over the connected components
+// of its sparsity pattern (coherence orders and, in restricted bases, further
+// product states never mix), and an orientation's FID coil' exp(-1i L t) rho0
+// depends only on the components that hold coil entries and rho0 entries.
+// The engine finds those rows once per system (block_plan.h) and these kernels
+// run the same chunked Chebyshev expansion as kernels.cuh on them alone: 52 of
+// 1156 states for a seven-spin IK-0(3) system, 252 of 4096 for six spins, 144
+// of 2736 for the radical with ten protons.
+//
+// At these sizes a term's cost is latency and issue slots, not memory, so the
+// layout differs from kernels.cuh: one small CTA per orientation, many CTAs
+// per SM; every lane keeps its share of one row (values, columns, diagonal) in
+// registers for the whole orientation and only the state is read from shared
+// memory; a wide row is split over 2-32 neighbouring lanes, whose partial sums
+// meet in shuffles; the detection states are extra rows of the matrix, so a
+// term's product yields the moments too.  Spectral bounds and Bessel tables
+// are separate launches: the bounds of every orientation come first, and the
+// tables are shared by all orientations whose half-widths fall into the same
+// step of a geometric ladder (at most 32 tables instead of one per
+// orientation).
+#pragma once
+
+#include "kernels.cuh"
+
+namespace spx {
+
+constexpr int kBlockRows = 512;        // largest number of coupled states
+constexpr int kBlockLevels = 32;       // steps of the half-width ladder (Bessel tables)
+constexpr int kBlockMaxEntries = 24;   // entries of one lane
+
+// One layout of the rows on a CTA's lanes (device pointers).
+struct BlockLayout {
+    int n;                      // coupled states
+    int nv;                     // detection rows
+    int threads;                // lanes (the CTA of the FP64 kernel has two threads for each)
+    int ecap;                   // entries per lane
+    const int *lane_row;        // [threads] state row, n + v for detection row v, -1: none
+    const int *lane_part;       // [threads] lanes of the row | part index << 8
+    const int *warp_shape;      // [threads/32] entries per lane | shuffle rounds << 8
+    const int *src;             // [ecap][threads] ELL entry of the system, -1 none, -2-i: coil value i
+    const uint16_t *col;        // [ecap][threads] state row the entry reads
+    const int *row_src;         // [n] row of the system (sliced order)
+    const double2 *vval;        // entry values of the detection rows
+    const int *vchan;           // [nv] channel of a detection row
+    const int *vfac;            // [nv] 0: times 1, 1: times -1i (imaginary parts of a complex coil)
+};
+
+struct BlockRun {
+    int n_orient;
+    const double *alpha, *beta, *gamma;
+    int pick;                   // 0: orientation o of the grid; else orientation ((2 o + 1) pick) / (2 n_orient)
+    double dt;
+    int nsteps;
+    int Mcap;                   // largest chunk (steps)
+    double chunk_x;             // series argument of one chunk
+    int Kmax;                   // largest series
+    double tol;
+    int lanczos_its, safe_bounds;
+    // bounds and ladder
+    double *centre;             // [n_orient]
+    double *halfwidth;          // [n_orient]
+    unsigned long long *extent; // [2] largest half-width's bits, complement of the smallest's (zeroed)
+    int nlev;                   // ladder steps in use, 1..kBlockLevels
+    double *lev_half;           // [nlev]
+    int *lev_m, *lev_k, *lev_raw;   // [nlev] steps per chunk, table rows, series length before the cap
+    int *kcut;                  // [nlev][Mcap+1] terms a column needs
+    double *table;              // [nlev][Kmax][M+1] (2 - delta_k0) J_k(half j dt)
+    float *tablef;              // the same rounded to float, or null
+    double max_im_diag;
+    // states
+    const double2 *rho0;        // one initial state (read at row_src, or at the row itself when rho0_own)
+    const double2 *rho0s;       // or one per orientation, rho0_stride apart
+    size_t rho0_stride;
+    int rho0_own;
+    double2 *state_out;         // or null: [n_orient][n] the state after the last step
+    void *fids;                 // [n_orient][nchan][nsteps+1]; not written when nv == 0
+    int nchan;
+    double *saved;              // or null: every orientation's assembled L, in lane order (block_saved)
+    int *status, *kused, *mused;
+    long long *matvecs;
+};
+
+// FP32 entries of one lane: values as hi + lo floats, and the byte offset of
+// the state they multiply.
+template <bool CPLX, int ECAP> struct BlockEntries;
+template <int ECAP> struct BlockEntries<false, ECAP> {
+    float hi[ECAP], lo[ECAP];
+    int col[ECAP];
+    __device__ __forceinline__ void set(int i, double re, double) { split(re, hi[i], lo[i]); }
+    // (Y, L, P) += v * x: Y + L + P is the sum.  The product is exact inside the
+    // fused multiply-adds, so the low-order part L keeps the product's rounding
+    // as well as the sum's; P sums the products of the values' low parts.  Each
+    // of the three takes one dependent operation per entry.
+    __device__ __forceinline__ void mac(int i, f2x &Y, f2x &L, f2x &P, f2x X) const {
+        const f2x H = f2pk(hi[i], hi[i]);
+        const f2x S = fma2(H, X, Y);
+        L = add2(L, fma2(H, X, sub2(Y, S)));
+        Y = S;
+        P = fma2(f2pk(lo[i], lo[i]), X, P);
+    }
+    __device__ __forceinline__ void plain(int i, float2 &y, float2 x) const {
+        y.x = fmaf(hi[i], x.x, y.x);
+        y.y = fmaf(hi[i], x.y, y.y);
+    }
+    __device__ __forceinline__ float mag(int i) const { return fabsf(hi[i]); }
+};
+template <int ECAP> struct BlockEntries<true, ECAP> {
+    float rh[ECAP], ih[ECAP], rl[ECAP], il[ECAP];
+    int col[ECAP];
+    __device__ __forceinline__ void set(int i, double re, double im) {
+        split(re, rh[i], rl[i]);
+        split(im, ih[i], il[i]);
+    }
+    __device__ __forceinline__ void mac(int i, f2x &Y, f2x &L, f2x &P, f2x X) const {
+        const f2x XS = swap2(X);
+        const f2x H = f2pk(rh[i], rh[i]), G = f2pk(-ih[i], ih[i]);
+        const f2x S = fma2(H, X, Y);
+        L = add2(L, fma2(H, X, sub2(Y, S)));
+        Y = fma2(G, XS, S);
+        L = add2(L, fma2(G, XS, sub2(S, Y)));
+        P = fma2(f2pk(rl[i], rl[i]), X, P);
+        P = fma2(f2pk(-il[i], il[i]), XS, P);
+    }
+    __device__ __forceinline__ void plain(int i, float2 &y, float2 x) const {
+        y.x = fmaf(rh[i], x.x, fmaf(-ih[i], x.y, y.x));
+        y.y = fmaf(rh[i], x.y, fmaf(ih[i], x.x, y.y));
+    }
+    __device__ __forceinline__ float mag(int i) const { return sqrtf(rh[i] * rh[i] + ih[i] * ih[i]); }
+};
+// Barrier of one orientation's CTA; the warps reach it from different loops.
+static __device__ __forceinline__ void block_sync() { asm volatile("barrier.sync 0;" ::: "memory"); }
+static __device__ __forceinline__ void st_shared(uint32_t a, f2x v) {
+    asm volatile("st.shared.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+
+// What a lane knows about its row.
+struct BlockLane {
+    int row;                    // state row, n + v, or -1
+    int parts, part;            // lanes of the row, this lane's index among them
+    int ew, rounds;             // entries per lane and shuffle rounds of the warp
+    bool own;                   // holds the row's diagonal and state
+    bool state;                 // own and a state row (not a detection row)
+};
+static __device__ __forceinline__ BlockLane block_lane(const BlockLayout &B, int t) {
+    BlockLane l;
+    l.row = B.lane_row[t];
+    const int p = B.lane_part[t], w = B.warp_shape[t >> 5];
+    l.parts = p & 0xff;
+    l.part = p >> 8;
+    l.ew = w & 0xff;
+    l.rounds = w >> 8;
+    l.own = l.row >= 0 && l.part == 0;
+    l.state = l.own && l.row < B.n;
+    return l;
+}
+
+// One lane's entries of an orientation's L: FP64 sums over the value streams
+// (coef: the rotational coefficients), stream by stream, so that the loads of
+// all entries are in flight together; detection rows keep their values.
+// Entries i of the lane with i % NTH == TH (threads that share the lane).
+template <bool CPLX, int ECAP>
+static __device__ __forceinline__ void block_assemble(const DevSystem &sys, const BlockLayout &B, int ew, int t,
+                                                      const double *coef, double (&re)[ECAP], double (&im)[ECAP]) {
+    int src[ECAP];
+#pragma unroll
+    for (int i = 0; i < ECAP; ++i) {
+        src[i] = i < ew ? B.src[i * B.threads + t] : -1;
+        re[i] = im[i] = 0.0;
+    }
+    for (int s = 0; s < sys.nstreams; ++s) {
+        const double c = coef[sys.stream_coef[s]];
+        const double *vr = sys.ell_re + (size_t)s * sys.ell_len;
+        const double *vi = CPLX ? sys.ell_im + (size_t)s * sys.ell_len : nullptr;
+#pragma unroll
+        for (int i = 0; i < ECAP; ++i)
+            if (src[i] >= 0) {
+                re[i] = fma(c, vr[src[i]], re[i]);
+                if (CPLX) im[i] = fma(c, vi[src[i]], im[i]);
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < ECAP; ++i)
+        if (src[i] <= -2) {
+            const double2 v = B.vval[-2 - src[i]];
+            re[i] = v.x;
+            im[i] = v.y;
+        }
+}
+
+// Diagonal entry of system row r.
+static __device__ __forceinline__ double2 block_diagonal(const DevSystem &sys, int r, const double *coef) {
+    double2 dg = make_double2(0.0, 0.0);
+    for (int s = 0; s < sys.nstreams; ++s) {
+        const double c = coef[sys.stream_coef[s]];
+        const double2 d = sys.diag[(size_t)s * sys.n_pad + r];
+        dg.x = fma(c, d.x, dg.x);
+        dg.y = fma(c, d.y, dg.y);
+    }
+    return dg;
+}
+
+// Doubles of one orientation in BlockRun::saved: the lanes' entries, then
+// their diagonals.
+static __host__ __device__ inline size_t block_saved(int ecap, int threads, bool cplx) {
+    return (size_t)threads * ((cplx ? 2 : 1) * ecap + 2);
+}
+
+// Index in the grid of the run's orientation o.
+static __device__ __forceinline__ int block_grid_index(const BlockRun &R, int o) {
+    return R.pick ? (int)(((2 * (long long)o + 1) * R.pick) / (2 * (long long)R.n_orient)) : o;
+}
+
+// Rotational coefficients of the run's orientation o into coef (all threads call).
+static __device__ __forceinline__ void block_coefficients(const DevSystem &sys, const BlockRun &R, int o, double *coef) {
+    o = block_grid_index(R, o);
+    for (int t = threadIdx.x; t < sys.nterms; t += blockDim.x) {
+        double re, im;
+        wigner_element(sys.term_rkm[3 * t], sys.term_rkm[3 * t + 1], sys.term_rkm[3 * t + 2], R.alpha[o], R.beta[o],
+                       R.gamma[o], re, im);
+        coef[1 + 2 * t] = re;
+        coef[2 + 2 * t] = im;
+    }
+    if (threadIdx.x == 0) coef[0] = 1.0;
+    __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// Spectral bounds of every orientation: Gershgorin discs, and Lanczos on the
+// Hermitian part, in FP32 for both precisions (the interval is widened by the
+// Ritz residuals and 2% of its width, and the propagation watches the norm).
+// One reduction per Lanczos step: beta^2 = |w|^2 - alpha^2 with the matrix
+// taken about the middle of its discs, where alpha is no larger than the
+// spread.  The assembled L goes to R.saved for the FP32 propagation, which
+// runs on the same layout.
+// ---------------------------------------------------------------------------
+template <bool CPLX, int ECAP>
+__global__ void __launch_bounds__(kBlockRows, 1) block_bounds_kernel(const DevSystem sys, const BlockLayout B,
+                                                                     const BlockRun R) {
+    __shared__ double s_coef[kMaxCoef];
+    __shared__ float2 s_x[2][kBlockRows + 1];
+    __shared__ float2 s_part[2][kBlockRows / 32];
+    __shared__ double s_al[kMaxLanczos], s_be[kMaxLanczos];
+    const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const BlockLane l = block_lane(B, tid);
+    block_coefficients(sys, R, o, s_coef);
+    BlockEntries<CPLX, ECAP> E;
+    double2 dg = make_double2(0.0, 0.0);
+    {
+        double re[ECAP], im[ECAP];
+        block_assemble<CPLX, ECAP>(sys, B, l.ew, tid, s_coef, re, im);
+        if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef);
+        double *save = R.saved ? R.saved + (size_t)o * block_saved(B.ecap, B.threads, CPLX) : nullptr;
+#pragma unroll
+        for (int i = 0; i < ECAP; ++i) {
+            E.set(i, re[i], im[i]);
+            E.col[i] = i < l.ew ? B.col[i * B.threads + tid] * (int)sizeof(float2) : 0;
+            if (save && i < l.ew) {
+                save[(size_t)i * B.threads + tid] = re[i];
+                if (CPLX) save[(size_t)(B.ecap + i) * B.threads + tid] = im[i];
+            }
+        }
+        if (save) {
+            double *sd = save + (size_t)(CPLX ? 2 : 1) * B.ecap * B.threads;
+            sd[tid] = dg.x;
+            sd[B.threads + tid] = dg.y;
+        }
+    }
+    int par = 0;
+    // sums (op 0) or maxima (op 1) of both components over the CTA; the slots
+    // alternate, so one barrier each
+    auto reduce = [&](float2 v, int op) {
+#pragma unroll
+        for (int q = 16; q; q >>= 1) {
+            const float ux = __shfl_xor_sync(0xffffffffu, v.x, q), uy = __shfl_xor_sync(0xffffffffu, v.y, q);
+            v.x = op ? fmaxf(v.x, ux) : v.x + ux;
+            v.y = op ? fmaxf(v.y, uy) : v.y + uy;
+        }
+        if (nwarps == 1) return v;
+        if (lane == 0) s_part[par][warp] = v;
+        __syncthreads();
+        v = s_part[par][0];
+        for (int w = 1; w < nwarps; ++w) {
+            const float2 u = s_part[par][w];
+            v.x = op ? fmaxf(v.x, u.x) : v.x + u.x;
+            v.y = op ? fmaxf(v.y, u.y) : v.y + u.y;
+        }
+        par ^= 1;
+        return v;
+    };
+    auto join = [&](float v) {                                // sum over the parts of a row
+        for (int r = 0; r < l.rounds; ++r) {
+            const float u = __shfl_xor_sync(0xffffffffu, v, 1 << r);
+            if ((l.parts >> r) > 1) v += u;
+        }
+        return v;
+    };
+    float rad = 0.f;
+#pragma unroll
+    for (int i = 0; i < ECAP; ++i) rad += E.mag(i);
+    rad = join(rad);
+    // float sums: 4e-6 of the row covers their rounding
+    const float dgf = (float)dg.x, slack = 4e-6f * (fabsf(dgf) + rad);
+    const float2 g = reduce(l.state ? make_float2(dgf + rad + slack, -(dgf - rad - slack))
+                                    : make_float2(-CUDART_INF_F, -CUDART_INF_F), 1);
+    const double gmax = g.x, gmin = -g.y, mid = 0.5 * (gmax + gmin);
+    const float dre = (float)(dg.x - mid);
+
+    float2 q_cur = make_float2(0.f, 0.f), q_prev = q_cur;
+    if (l.state) q_cur.x = 1.0f + 0.37f * __sinf(1.7f * (float)l.row + 0.3f);
+    {
+        const float inv = rsqrtf(reduce(make_float2(q_cur.x * q_cur.x, 0.f), 0).x);
+        q_cur.x *= inv;
+    }
+    float beta_prev = 0.f;
+    int m_eff = 0;
+    const int lits = min(R.lanczos_its, min(kMaxLanczos, B.n));
+    const int slot = l.state ? l.row : kBlockRows;
+    for (int j = 0; j < lits; ++j) {
+        float2 *x = s_x[j & 1];
+        x[slot] = q_cur;
+        __syncthreads();
+        float2 y = make_float2(0.f, 0.f);
+        const char *xb = reinterpret_cast<const char *>(x);
+#pragma unroll
+        for (int i = 0; i < ECAP; ++i) E.plain(i, y, *reinterpret_cast<const float2 *>(xb + E.col[i]));
+        y.x = join(y.x);
+        y.y = join(y.y);
+        if (l.state) {
+            y.x += dre * q_cur.x - beta_prev * q_prev.x;
+            y.y += dre * q_cur.y - beta_prev * q_prev.y;
+        } else {
+            y = make_float2(0.f, 0.f);
+        }
+        const float2 sums = reduce(make_float2(q_cur.x * y.x + q_cur.y * y.y, y.x * y.x + y.y * y.y), 0);
+        const float alpha = sums.x, b2 = sums.y - alpha * alpha, beta = b2 > 0.f ? sqrtf(b2) : 0.f;
+        if (tid == 0) { s_al[j] = (double)alpha; s_be[j] = (double)beta; }
+        m_eff = j + 1;
+        if (!(b2 > 1e-6f * sums.y)) break;                   // invariant subspace, to the sums' rounding
+        const float inv = 1.f / beta;
+        q_prev = q_cur;
+        q_cur.x = (y.x - alpha * q_cur.x) * inv;
+        q_cur.y = (y.y - alpha * q_cur.y) * inv;
+        beta_prev = beta;
+    }
+    __syncthreads();
+    if (tid < 32) {
+        double tlo, thi;
+        tridiag_extremes_warp(s_al, s_be, m_eff, tlo, thi, lane);
+        const double bl = fabs(s_be[m_eff - 1]);
+        double rr = 0.0;
+        if (!R.safe_bounds && lane < 2) rr = bl * ritz_last_component(s_al, s_be, m_eff, lane == 0 ? thi : tlo);
+        const double rhi = __shfl_sync(0xffffffffu, rr, 0), rlo = __shfl_sync(0xffffffffu, rr, 1);
+        if (lane == 0) {
+            double hi = gmax, lo = gmin;
+            if (!R.safe_bounds) {
+                const double wid = thi - tlo;
+                hi = fmin(mid + thi + rhi + 0.02 * wid, gmax);
+                lo = fmax(mid + tlo - rlo - 0.02 * wid, gmin);
+                if (!(hi >= lo)) { hi = gmax; lo = gmin; }
+            }
+            const double scale = fmax(fabs(hi), fabs(lo));
+            const double half = fmax(0.5 * (hi - lo) * 1.01 + 1e-9 * scale, R.max_im_diag) + 1e-30;
+            R.centre[o] = 0.5 * (hi + lo);
+            R.halfwidth[o] = half;
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(half);   // half > 0
+            atomicMax(R.extent, bits);
+            atomicMax(R.extent + 1, ~bits);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Bessel tables of the ladder: step i has half-width hmax * exp(-i * step);
+// an orientation takes the last step that still covers its own half-width, so
+// it runs at most e^step more terms than with a table of its own (16 steps to
+// an octave: 2 % on average).  Grid (columns / 32, steps); only steps that an
+// orientation takes are tabulated.
+// ---------------------------------------------------------------------------
+static __device__ __noinline__ double ladder_half(const unsigned long long *extent, int nlev, int lev) {
+    const double hmax = __longlong_as_double((long long)extent[0]);
+    const double hmin = __longlong_as_double((long long)~extent[1]);
+    double step = 0.69314718055994531 / 16;
+    if (nlev > 1) step = fmax(step, log(hmax / hmin) / (nlev - 1));
+    return lev == 0 ? hmax : hmax * exp(-lev * step);
+}
+
+// Column j of a table (bessel_column of kernels.cuh in two passes: the
+// recurrence stores unnormalised values, then eight at a time are scaled, so
+// that their loads overlap), also rounded to float; returns the terms the
+// column needs: the last one above tol (with the growth e^{k lg} that Im L
+// allows), plus two.
+static __device__ int block_column(double *tab, float *tf, int M, int j, int K, double half, double dt, double lg,
+                                   double tol) {
+    const size_t ld = (size_t)(M + 1);
+    double *col = tab + j;
+    const double x = half * j * dt;
+    double inv = 1.0;
+    int kn = min(K, 3);                               // terms that are not zero
+    if (x < 1e-6) {
+        // twice the leading terms, scaled as below
+        col[0] = 1.0 - 0.25 * x * x;
+        if (K > 1) col[ld] = 0.5 * x;
+        if (K > 2) col[2 * ld] = 0.125 * x * x;
+    } else {
+        kn = min(K, series_terms(x, 0.0, 1e-40, K + 64) + 1);
+        const int base = max(kn, (int)ceil(x));
+        int kst = base + 20 + (int)sqrtf(160.f * base);
+        kst += kst & 1;
+        const double two_over_x = 2.0 / x;
+        const float ftx = (float)two_over_x;
+        float fjp1 = 0.f, fjk = 1e-30f;
+        int k = kst;
+        for (; k > kn; --k) {
+            const float fjm1 = ((float)k * ftx) * fjk - fjp1;
+            fjp1 = fjk;
+            fjk = fjm1;
+            if (fabsf(fjk) > 1e20f) { fjk *= 1e-20f; fjp1 *= 1e-20f; }
+        }
+        double jp1 = fjp1, jk = fjk, even = 0.0;
+        for (; k >= 1; --k) {
+            const double jm1 = (k * two_over_x) * jk - jp1;
+            jp1 = jk;
+            jk = jm1;                                 // J_{k-1}, unnormalised
+            if (k > 1 && (k & 1)) even += jk;
+            col[(size_t)(k - 1) * ld] = jk;
+        }
+        inv = 1.0 / (2.0 * even + jk);                // J_0 + 2 sum J_2k = 1
+    }
+    int last = 2;
+    const double two = 2.0 * inv;
+    for (int k0 = 0; k0 < K; k0 += 8) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = k0 + q < kn ? col[(size_t)(k0 + q) * ld] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int k = k0 + q;
+            if (k < K) {
+                v[q] *= k == 0 ? inv : two;
+                col[(size_t)k * ld] = v[q];
+                if (tf) tf[(size_t)k * ld + j] = (float)v[q];
+            }
+        }
+    }
+    double grow = exp((kn - 1) * lg);
+    const double shrink = exp(-lg);
+    for (int k = kn - 1; k >= 2; --k, grow *= shrink)
+        if (!(fabs(col[(size_t)k * ld]) * grow <= tol)) { last = k + 1; break; }
+    return min(last + 2, K);
+}
+
+static __global__ void __launch_bounds__(128) block_tables_kernel(const BlockRun R) {
+    const int lev = blockIdx.y, tid = threadIdx.x;
+    const double half = ladder_half(R.extent, R.nlev, lev);
+    const double next = lev + 1 < R.nlev ? ladder_half(R.extent, R.nlev, lev + 1) : 0.0;
+    __shared__ int s_k, s_raw;
+    if (tid == 0) s_k = 0;
+    __syncthreads();
+    for (int o = tid; o < R.n_orient; o += blockDim.x) {
+        const double h = R.halfwidth[o];
+        if (h <= half && !(h <= next)) { s_k = 1; break; }
+    }
+    __syncthreads();
+    const bool used = s_k != 0;
+    __syncthreads();
+    const double target = R.chunk_x / (half * R.dt);
+    // a chunk damps the state by at most e^2: the terms grow with Im L, and
+    // their sum loses the digits they gained
+    const double damped = R.max_im_diag > 0.0 ? floor(2.0 / (R.max_im_diag * R.dt)) : (double)R.Mcap;
+    const int M = min((int)fmax(1.0, fmin((double)R.Mcap, fmin(damped, floor(target)))), R.nsteps + 1);
+    const double lg = 2.0 * R.max_im_diag / half;
+    if (tid == 0) {
+        s_raw = used ? series_terms(half * M * R.dt, lg, R.tol, R.Kmax + 1) : 0;
+        s_k = used ? min(R.Kmax, max(2, s_raw) + 2) : 0;        // 0: no table
+        if (blockIdx.x == 0) {
+            R.lev_half[lev] = half;
+            R.lev_m[lev] = M;
+            R.lev_k[lev] = s_k;
+            R.lev_raw[lev] = s_raw;
+        }
+    }
+    __syncthreads();
+    const int j = blockIdx.x * 32 + tid;
+    if (!used || tid >= 32 || j > M) return;
+    const int K = s_k;
+    double *tab = R.table + (size_t)lev * R.Kmax * (R.Mcap + 1);
+    float *tf = R.tablef ? R.tablef + (size_t)lev * R.Kmax * (R.Mcap + 1) : nullptr;
+    const int kl = block_column(tab, tf, M, j, K, half, R.dt, lg, R.tol);
+    R.kcut[(size_t)lev * (R.Mcap + 1) + j] = kl;
+}
+
+// Dynamic shared memory of the propagation kernels.
+static __host__ __device__ inline size_t block_smem32(int Kmax, int Mcap, int nv, int threads) {
+    return 8 * ((size_t)(Kmax + 2) * (1 + nv) + (size_t)(Mcap + 1) + (size_t)(threads > Mcap ? threads : Mcap));
+}
+static __host__ __device__ inline size_t block_smem64(int Kmax, int Mcap, int nv, int lanes, int ecap, int n, bool cplx) {
+    const size_t rec = (size_t)(2 * lanes > Mcap ? 2 * lanes : Mcap);
+    return 16 * (rec + (size_t)(Mcap + 1) + (size_t)(Kmax + 2) * nv) + 8 * (size_t)(Kmax + 2) +
+           8 * (size_t)ecap * lanes * (cplx ? 2 : 1) + 8 * 4 * (size_t)(n + 1) + 2 * (size_t)ecap * lanes;
+}
+
+// (-1i)^k is this sign times 1 (even k) or -1i (odd k).
+static __device__ __forceinline__ double block_sign(int k) { return (k & 2) ? -1.0 : 1.0; }
+
+// (-1i) * t as a packed pair
+static __device__ __forceinline__ f2x turn2(f2x t) {
+    const float2 f = f2up(t);
+    return f2pk(f.y, -f.x);
+}
+
+// What a CTA knows of its orientation's series.
+struct BlockSeries {
+    double cen, half;
+    int M, K, nchunks, j_last;
+    size_t ld;                  // table row length
+    const double *tab;
+    const float *tabf;
+    const int *kcut;
+    bool ok;
+};
+// The ladder step of orientation o; a series longer than the table sets the
+// orientation's status and ok = false.
+static __device__ __forceinline__ BlockSeries block_series(const BlockRun &R, int o) {
+    BlockSeries S;
+    const double own = R.halfwidth[o];
+    int lev = 0;
+    while (lev + 1 < R.nlev && R.lev_half[lev + 1] >= own) ++lev;
+    S.cen = R.centre[o];
+    S.half = R.lev_half[lev];
+    S.M = R.lev_m[lev];
+    const int Kb = R.lev_k[lev];
+    const size_t at = (size_t)lev * R.Kmax * (R.Mcap + 1);
+    S.kcut = R.kcut + (size_t)lev * (R.Mcap + 1);
+    S.K = Kb > 0 ? S.kcut[S.M] : 0;
+    S.tab = R.table + at;
+    S.tabf = R.tablef ? R.tablef + at : nullptr;
+    S.ld = (size_t)(S.M + 1);
+    S.nchunks = (R.nsteps + S.M) / S.M;
+    S.j_last = R.nsteps - (S.nchunks - 1) * S.M;
+    S.ok = !(Kb == 0 || (R.lev_raw[lev] + 2 > R.Kmax && S.K >= Kb - 2));
+    if (!S.ok && threadIdx.x == 0) {
+        R.status[o] = kDevTableTooSmall;
+        R.kused[o] = R.Kmax + 1;
+        R.mused[o] = S.M;
+        R.matvecs[o] = 0;
+    }
+    return S;
+}
+
+// e^{-i c j dt}, j < M: one sine and cosine per thread, turned on by
+// blockDim.x steps at a time (FP64 transcendentals are slow here); the phases
+// of a whole and of the last chunk; and the growth of |t_k|^2 that Im L allows
+// over the last chunk's terms.
+template <class Vec>
+static __device__ __forceinline__ void block_phases(const BlockRun &R, const BlockSeries &S, Vec *phase, double2 *turn,
+                                                    float *allow) {
+    const int tid = threadIdx.x, nt = (int)blockDim.x;
+    if (tid < S.M) {
+        double sn, cs, rs = 0.0, rc = 1.0;
+        sincos(-S.cen * tid * R.dt, &sn, &cs);
+        if (S.M > nt) sincos(-S.cen * nt * R.dt, &rs, &rc);
+        for (int j = tid; j < S.M; j += nt) {
+            phase[j] = tovec(make_double2(cs, sn), Vec());
+            const double c2 = cs * rc - sn * rs;
+            sn = sn * rc + cs * rs;
+            cs = c2;
+        }
+    }
+    if (tid < 2) {
+        double sn, cs;
+        sincos(-S.cen * (tid == 0 ? S.M : S.j_last) * R.dt, &sn, &cs);
+        turn[tid] = make_double2(cs, sn);
+    }
+    if (tid == nt - 1) {
+        const float q = (float)(R.max_im_diag / S.half);
+        *allow = __expf(fminf(80.f, 2.f * S.K * __logf(q + sqrtf(1.f + q * q))));
+    }
+}
+
+// FID points of chunk a: f_j = e^{-i c j dt} sum_k J_k(s j dt) (-1i)^k mu_k.
+// tr: the table in the run's precision.  Every thread calls, after a barrier;
+// the caller's next barrier ends it.
+template <class Vec, class Real>
+static __device__ __forceinline__ void block_points(const BlockLayout &B, const BlockRun &R, const BlockSeries &S,
+                                                    const Real *tr, int a, int Kc, const Vec *s_mu, const Vec *s_phase,
+                                                    Vec *s_rec, Vec *fid_out) {
+    const int tid = threadIdx.x, nt = (int)blockDim.x, M = S.M;
+    const int np = min(M, R.nsteps + 1 - a * M);                // points of this chunk
+    const int parts = max(1, nt / M);
+    const int kper = ((Kc + parts - 1) / parts + 3) & ~3;
+    const size_t ld = S.ld;
+    for (int v = 0; v < B.nv; ++v) {
+        const Vec *mu = s_mu + (size_t)v * (R.Kmax + 2);
+        if (v > 0) __syncthreads();                              // s_rec reused
+        for (int jj = tid; jj < M * parts; jj += nt) {
+            const int j = jj % M, k0 = (jj / M) * kper, k1 = min(min(Kc, k0 + kper), S.kcut[j]);
+            Vec e = vzero<Vec>(), d = vzero<Vec>();              // even and odd terms
+            int k = k0;
+            // the table sits in L2: 16 loads in flight, then 4, then one
+            auto add = [&](auto nc) {
+                constexpr int N = decltype(nc)::value;
+                for (; k + N <= k1; k += N) {
+                    Real J[N];
+#pragma unroll
+                    for (int q = 0; q < N; ++q) J[q] = tr[(size_t)(k + q) * ld + j];
+#pragma unroll
+                    for (int q = 0; q < N; ++q) {
+                        const Vec m = mu[k + q];
+                        const Real b = (q & 2) ? -J[q] : J[q];
+                        Vec &t = (q & 1) ? d : e;
+                        t.x += b * m.x;
+                        t.y += b * m.y;
+                    }
+                }
+            };
+            add(std::integral_constant<int, 16>{});
+            add(std::integral_constant<int, 4>{});
+            for (; k < k1; ++k) {
+                const Real b = (Real)block_sign(k) * tr[(size_t)k * ld + j];
+                Vec &t = (k & 1) ? d : e;
+                t.x += b * mu[k].x;
+                t.y += b * mu[k].y;
+            }
+            Vec f;                                               // e - 1i d
+            f.x = e.x + d.y;
+            f.y = e.y - d.x;
+            s_rec[jj] = f;
+        }
+        __syncthreads();
+        Vec *out = fid_out + (size_t)B.vchan[v] * (R.nsteps + 1) + (size_t)a * M;
+        const bool first = v == 0 || B.vchan[v] != B.vchan[v - 1];
+        for (int j = tid; j < np; j += nt) {
+            Vec f = s_rec[j];
+            for (int q = 1; q < parts; ++q) { f.x += s_rec[q * M + j].x; f.y += s_rec[q * M + j].y; }
+            const Vec ph = s_phase[j];
+            Vec g;
+            g.x = ph.x * f.x - ph.y * f.y;
+            g.y = ph.x * f.y + ph.y * f.x;
+            if (B.vfac[v]) { const Real t = g.x; g.x = g.y; g.y = -t; }
+            if (!first) { g.x += out[j].x; g.y += out[j].y; }
+            out[j] = g;
+        }
+    }
+}
+
+// Calls f(entries per lane, shuffle rounds), both compile-time, with the
+// smallest instance that covers this warp (every count up to 8, then steps of
+// an eighth of the kernel's largest): straight-line code, so that a term's
+// loads all start before its sums (a loop that left after the warp's own entry
+// count waited 70 cycles for every entry).
+template <int ECAP, int EW = ECAP, class F>
+static __device__ __forceinline__ void block_dispatch(const BlockLane &l, F &&f) {
+    constexpr int step = ECAP <= 8 ? 1 : ECAP / 8;
+    if constexpr (EW == ECAP) {
+        if (l.rounds == 1) return f(std::integral_constant<int, ECAP>{}, std::integral_constant<int, 1>{});
+        if (l.rounds == 2) return f(std::integral_constant<int, ECAP>{}, std::integral_constant<int, 2>{});
+        if (l.rounds > 2) return f(std::integral_constant<int, ECAP>{}, std::integral_constant<int, 5>{});
+    }
+    if constexpr (EW > step) {
+        if (l.ew <= EW - step) return block_dispatch<ECAP, EW - step>(l, f);
+    }
+    f(std::integral_constant<int, EW>{}, std::integral_constant<int, 0>{});
+}
+
+// ---------------------------------------------------------------------------
+// Propagation, FP32: values in registers, (re, im) in packed f32x2 operations.
+// ---------------------------------------------------------------------------
+template <bool CPLX, int ECAP>
+__global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const DevSystem sys, const BlockLayout B,
+                                                                        const BlockRun R) {
+    __shared__ double s_coef[kMaxCoef];
+    __shared__ float2 s_x[2][kBlockRows + 1];
+    __shared__ float s_norm[2][kBlockRows / 32];
+    __shared__ double2 s_turn[2];
+    __shared__ float s_allow;
+    extern __shared__ __align__(16) unsigned char smem[];
+    float2 *s_b = reinterpret_cast<float2 *>(smem);          // chunk-end coefficients (b, b)
+    float2 *s_mu = s_b + (R.Kmax + 2);                        // moments, one row per detection row
+    float2 *s_phase = s_mu + (size_t)(R.Kmax + 2) * B.nv;
+    float2 *s_rec = s_phase + (R.Mcap + 1);
+    const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const BlockLane l = block_lane(B, tid);
+    const BlockSeries S = block_series(R, o);
+    if (!S.ok) return;
+    const int nsteps = R.nsteps, M = S.M;
+
+    // 2 L~ = 2 (L - c) / s: the recurrence is t_{k+1} = 2 L~ t_k - t_{k-1}
+    BlockEntries<CPLX, ECAP> E;
+    float dh = 0.f, dl = 0.f, di = 0.f;
+    {
+        const double scale = 2.0 / S.half;
+        double re[ECAP], im[ECAP];
+        double2 dg = make_double2(0.0, 0.0);
+        if (R.saved) {
+            const double *save = R.saved + (size_t)o * block_saved(B.ecap, B.threads, CPLX);
+#pragma unroll
+            for (int i = 0; i < ECAP; ++i) {
+                re[i] = i < l.ew ? save[(size_t)i * B.threads + tid] : 0.0;
+                im[i] = CPLX && i < l.ew ? save[(size_t)(B.ecap + i) * B.threads + tid] : 0.0;
+            }
+            save += (size_t)(CPLX ? 2 : 1) * B.ecap * B.threads;
+            dg = make_double2(save[tid], save[B.threads + tid]);
+        } else {
+            block_coefficients(sys, R, o, s_coef);
+            block_assemble<CPLX, ECAP>(sys, B, l.ew, tid, s_coef, re, im);
+            if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef);
+        }
+        const double sc = l.row < B.n ? scale : 1.0;          // detection rows keep their values
+#pragma unroll
+        for (int i = 0; i < ECAP; ++i) {
+            E.set(i, re[i] * sc, im[i] * sc);
+            E.col[i] = i < l.ew ? B.col[i * B.threads + tid] * (int)sizeof(float2) : 0;
+        }
+        if (l.state) {
+            split((dg.x - S.cen) * scale, dh, dl);
+            di = (float)(dg.y * scale);
+        }
+    }
+    auto coefficients = [&](int j, int Kc) {                  // of the state j steps into a chunk
+        for (int k = tid; k < Kc; k += blockDim.x) {
+            const float b = (float)(block_sign(k) * S.tab[k * S.ld + j]);
+            s_b[k] = make_float2(b, b);
+        }
+        if (tid < 2) s_b[Kc + tid] = make_float2(0.f, 0.f);
+    };
+    block_phases(R, S, s_phase, s_turn, &s_allow);
+    coefficients(M, S.K);
+
+    float2 st = make_float2(0.f, 0.f);
+    if (l.state) {
+        const double2 *r0 = R.rho0s ? R.rho0s + (size_t)block_grid_index(R, o) * R.rho0_stride : R.rho0;
+        st = tovec(r0[R.rho0_own ? l.row : B.row_src[l.row]], float2());
+    }
+    const float2 *mu_row = s_mu + (size_t)(l.row >= B.n ? l.row - B.n : 0) * (R.Kmax + 2);
+    float2 *fid_out = reinterpret_cast<float2 *>(R.fids) + (size_t)o * R.nchan * (nsteps + 1);
+    int status = kDevOk;
+    long long mv = 0;
+    int par = 0;
+    // squared norm of the state over the CTA (the slots alternate)
+    auto norm2 = [&](float2 v) {
+        float s = l.state ? v.x * v.x + v.y * v.y : 0.f;
+#pragma unroll
+        for (int q = 16; q; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
+        if (lane == 0) s_norm[par][warp] = s;
+        __syncthreads();
+        s = s_norm[par][0];
+        for (int w = 1; w < nwarps; ++w) s += s_norm[par][w];
+        par ^= 1;
+        return s;
+    };
+    float start_n2 = norm2(st);
+
+    const f2x DH = f2pk(dh, dh), DL = f2pk(dl, dl), DI = f2pk(-di, di);
+    const f2x NEG = l.state ? f2pk(-1.f, -1.f) : 0ull, HALF = l.state ? f2pk(0.5f, 0.5f) : f2pk(1.f, 1.f);
+    const char *x0 = reinterpret_cast<const char *>(&s_x[0][0]), *x1 = reinterpret_cast<const char *>(&s_x[1][0]);
+    for (int a = 0; a < S.nchunks; ++a) {
+        const bool last = a + 1 == S.nchunks;
+        const bool advance = !last || R.state_out != nullptr;
+        const int Kc = last ? min(S.K, S.kcut[S.j_last]) : S.K;
+        mv += Kc - 1;
+        if (last && advance) coefficients(S.j_last, Kc);
+        else if (last && tid < 2) s_b[Kc + tid] = make_float2(0.f, 0.f);
+        if (l.state) s_x[0][l.row] = st;
+        __syncthreads();
+        // Where this lane's result goes: a state row's into the other state
+        // buffer, a detection row's into its moments (one further each term),
+        // other lanes' nowhere.  ad[1] is for odd terms, ad[0] for even ones.
+        uint32_t ad[2], inc = 0;
+        if (l.state) {
+            ad[1] = smem_u32(&s_x[1][l.row]);
+            ad[0] = smem_u32(&s_x[0][l.row]);
+        } else if (l.own) {
+            ad[1] = smem_u32(mu_row);
+            ad[0] = ad[1] + 8;
+            inc = 16;
+        } else {
+            ad[0] = ad[1] = smem_u32(&s_x[0][kBlockRows]);
+        }
+        // ntp = -t_{k-2}, so that a row's sum starts from it without another operation
+        f2x tc = f2pk(st.x, st.y), ntp = 0ull;
+        f2x acc, accl;
+        {
+            const f2x b0 = reinterpret_cast<const f2x *>(s_b)[0];
+            acc = mul2(b0, tc);
+            accl = fma2(b0, tc, sub2(0ull, acc));
+        }
+        auto term = [&](auto ewc, auto rnc, auto oddc, const char *src, int k) {
+            constexpr int EW = decltype(ewc)::value, RND = decltype(rnc)::value;
+            constexpr bool ODD = decltype(oddc)::value;
+            const f2x b = reinterpret_cast<const f2x *>(s_b)[k];
+            f2x Y = fma2(DH, tc, ntp);
+            f2x Lw = fma2(DH, tc, sub2(ntp, Y));
+            f2x P = fma2(DI, swap2(tc), mul2(DL, tc));
+#pragma unroll
+            for (int i0 = 0; i0 < EW; i0 += 8) {
+                f2x X[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (i0 + i < EW) X[i] = *reinterpret_cast<const f2x *>(src + E.col[i0 + i]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (i0 + i < EW) E.mac(i0 + i, Y, Lw, P, X[i]);
+            }
+            Lw = add2(Lw, P);
+#pragma unroll
+            for (int r = 0; r < RND; ++r) {
+                f2x uy = __shfl_xor_sync(0xffffffffu, Y, 1 << r);
+                f2x ul = __shfl_xor_sync(0xffffffffu, Lw, 1 << r);
+                if ((l.parts >> r) <= 1) uy = ul = 0ull;
+                const f2x Sm = add2(Y, uy);
+                Lw = add2(add2(Lw, ul), add2(uy, sub2(Y, Sm)));
+                Y = Sm;
+            }
+            f2x T = add2(Y, Lw);
+            if (k == 1) T = mul2(T, HALF);
+            st_shared(ad[ODD], T);
+            ad[ODD] += inc;
+            block_sync();
+            const f2x V = ODD ? turn2(T) : T;
+            const f2x Sm = fma2(b, V, acc);
+            accl = add2(accl, fma2(b, V, sub2(acc, Sm)));
+            acc = Sm;
+            ntp = mul2(NEG, tc);
+            tc = T;
+        };
+        auto terms = [&](auto ewc, auto rnc) {
+            for (int k = 1; k <= Kc; k += 2) {
+                term(ewc, rnc, std::true_type{}, x0, k);
+                if (k + 1 <= Kc) term(ewc, rnc, std::false_type{}, x1, k + 1);
+            }
+        };
+        block_dispatch<ECAP>(l, terms);
+        const float2 fin = f2up(advance ? add2(acc, accl) : tc);
+        st = make_float2(0.f, 0.f);
+        if (l.state) {
+            st = fin;
+            if (advance) {
+                const double2 ph = s_turn[last ? 1 : 0];
+                st.x = (float)(ph.x * (double)fin.x - ph.y * (double)fin.y);
+                st.y = (float)(ph.y * (double)fin.x + ph.x * (double)fin.y);
+            }
+        }
+        if (B.nv > 0) block_points<float2, float>(B, R, S, S.tabf, a, Kc, s_mu, s_phase, s_rec, fid_out);
+        // a state that grew shows a violated spectral bound (a dissipative L
+        // can only shrink it); the norm's barrier also ends this chunk's reads
+        const float end_n2 = norm2(st);
+        if (!isfinite(end_n2)) status = kDevNonFinite;
+        else if (end_n2 > 16.f * start_n2 * (advance ? 1.f : s_allow) + 1e-30f) status = kDevDiverged;
+        if (status != kDevOk) break;
+        start_n2 = end_n2;
+    }
+    if (R.state_out && l.state) R.state_out[(size_t)o * B.n + l.row] = tod(st);
+    if (tid == 0) {
+        R.status[o] = status;
+        R.kused[o] = S.K;
+        R.mused[o] = M;
+        R.matvecs[o] = mv;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Propagation, FP64.  An FP64 instruction takes a warp 64 cycles here (2 lanes
+// of each of the SM's four FP64 units a cycle), so the terms are bound by the
+// FP64 instructions of a warp and nothing else: the real and imaginary parts
+// of a row sit in two lanes of different warps (thread t and t + lanes), which
+// halves a warp's instructions per term and spreads one orientation over the
+// four units; values and columns sit in shared memory, whose loads cost
+// nothing beside them, so that every warp runs just its own entries.
+// ---------------------------------------------------------------------------
+template <bool CPLX>
+__global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(const DevSystem sys, const BlockLayout B,
+                                                                              const BlockRun R) {
+    __shared__ double s_coef[kMaxCoef];
+    __shared__ double s_norm[2][2 * kBlockRows / 32];
+    __shared__ double2 s_turn[2];
+    __shared__ float s_allow;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int T = B.threads, n = B.n, xs = n + 1;
+    const size_t rec = (size_t)(2 * T > R.Mcap ? 2 * T : R.Mcap);
+    double2 *s_rec = reinterpret_cast<double2 *>(smem);
+    double2 *s_phase = s_rec + rec;
+    double2 *s_mu = s_phase + (R.Mcap + 1);
+    double *s_b = reinterpret_cast<double *>(s_mu + (size_t)(R.Kmax + 2) * B.nv);
+    double *s_x = s_b + (R.Kmax + 2);                         // [buffer][part][n + 1]
+    double *s_val = s_x + 4 * (size_t)xs;                     // [entry][lane], imaginary parts after
+    uint16_t *s_col = reinterpret_cast<uint16_t *>(s_val + (size_t)B.ecap * T * (CPLX ? 2 : 1));
+    const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const int part = tid >= T ? 1 : 0, t = tid - part * T;    // 0: real parts, 1: imaginary parts
+    const BlockLane l = block_lane(B, t);
+    const BlockSeries S = block_series(R, o);
+    if (!S.ok) return;
+    const int nsteps = R.nsteps, M = S.M;
+    const bool damped = R.max_im_diag > 0.0;
+
+    const double scale = 2.0 / S.half;
+    block_coefficients(sys, R, o, s_coef);
+    const double sc = l.row < n ? scale : 1.0;
+    for (int i = 4 * part; i < l.ew; i += 8) {                // the two threads of a lane take turns
+        double re[4], im[4];
+        BlockLayout Bi = B;
+        Bi.src = B.src + (size_t)i * T;
+        block_assemble<CPLX, 4>(sys, Bi, min(4, l.ew - i), t, s_coef, re, im);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (i + q < l.ew) {
+                s_val[(size_t)(i + q) * T + t] = re[q] * sc;
+                if (CPLX) s_val[(size_t)(B.ecap + i + q) * T + t] = im[q] * sc;
+                s_col[(size_t)(i + q) * T + t] = B.col[(size_t)(i + q) * T + t];
+            }
+    }
+    double dr = 0.0, dm = 0.0;                                // diagonal; the other part's factor
+    if (l.state) {
+        const double2 d = block_diagonal(sys, B.row_src[l.row], s_coef);
+        dr = (d.x - S.cen) * scale;
+        dm = (part ? d.y : -d.y) * scale;
+    }
+    auto coefficients = [&](int j, int Kc) {
+        for (int k = tid; k < Kc; k += blockDim.x) s_b[k] = block_sign(k) * S.tab[k * S.ld + j];
+        if (tid < 2) s_b[Kc + tid] = 0.0;
+    };
+    block_phases(R, S, s_phase, s_turn, &s_allow);
+    coefficients(M, S.K);
+    if (tid < 4) s_x[tid * xs + n] = 0.0;                     // read by lanes without a state row
+
+    double st = 0.0;
+    if (l.state) {
+        const double2 *r0 = R.rho0s ? R.rho0s + (size_t)block_grid_index(R, o) * R.rho0_stride : R.rho0;
+        const double2 v = r0[R.rho0_own ? l.row : B.row_src[l.row]];
+        st = part ? v.y : v.x;
+    }
+    double *mu_row = reinterpret_cast<double *>(s_mu + (size_t)(l.row >= n ? l.row - n : 0) * (R.Kmax + 2)) + part;
+    double2 *fid_out = reinterpret_cast<double2 *>(R.fids) + (size_t)o * R.nchan * (nsteps + 1);
+    int status = kDevOk;
+    long long mv = 0;
+    int par = 0;
+    auto norm2 = [&](double v) {
+        double s = v * v;
+#pragma unroll
+        for (int q = 16; q; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
+        if (lane == 0) s_norm[par][warp] = s;
+        __syncthreads();
+        s = s_norm[par][0];
+        for (int w = 1; w < nwarps; ++w) s += s_norm[par][w];
+        par ^= 1;
+        return s;
+    };
+    double start_n2 = norm2(st);
+
+    const int own = l.state ? l.row : n;                      // where the diagonal's other part is read
+    const double *val = s_val + t, *vim = s_val + (size_t)B.ecap * T + t;
+    const uint16_t *col = s_col + t;
+    for (int a = 0; a < S.nchunks; ++a) {
+        const bool last = a + 1 == S.nchunks;
+        const bool advance = !last || R.state_out != nullptr;
+        const int Kc = last ? min(S.K, S.kcut[S.j_last]) : S.K;
+        mv += Kc - 1;
+        if (last && advance) coefficients(S.j_last, Kc);
+        else if (last && tid < 2) s_b[Kc + tid] = 0.0;
+        if (l.state) s_x[part * xs + l.row] = st;
+        __syncthreads();
+        double tc = st, tp = 0.0, even = s_b[0] * st, odd = 0.0;
+        auto term = [&](int buf, int k, double &acc) {
+            const double *x = s_x + (2 * buf + part) * xs, *xo = s_x + (2 * buf + 1 - part) * xs;
+            double y = fma(dr, tc, -tp);
+            if (damped) y = fma(dm, xo[own], y);
+            int i = 0;
+            for (; i + 4 <= l.ew; i += 4) {
+                double v[4], w[4], X[4], Xo[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int c = col[(i + q) * T];
+                    v[q] = val[(i + q) * T];
+                    X[q] = x[c];
+                    if (CPLX) { w[q] = vim[(i + q) * T]; Xo[q] = xo[c]; }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    y = fma(v[q], X[q], y);
+                    if (CPLX) y = fma(part ? w[q] : -w[q], Xo[q], y);
+                }
+            }
+            for (; i < l.ew; ++i) {
+                const int c = col[i * T];
+                y = fma(val[i * T], x[c], y);
+                if (CPLX) y = fma(part ? vim[i * T] : -vim[i * T], xo[c], y);
+            }
+            for (int r = 0; r < l.rounds; ++r) {
+                const double u = __shfl_xor_sync(0xffffffffu, y, 1 << r);
+                if ((l.parts >> r) > 1) y += u;
+            }
+            tp = 0.0;
+            if (l.state) {
+                if (k == 1) y *= 0.5;
+                s_x[(2 * (buf ^ 1) + part) * xs + l.row] = y;
+                acc = fma(s_b[k], y, acc);
+                tp = tc;
+                tc = y;
+            } else if (l.own) {
+                mu_row[2 * (k - 1)] = y;
+            }
+            __syncthreads();
+        };
+        for (int k = 1; k <= Kc; k += 2) {
+            term(0, k, odd);
+            if (k + 1 <= Kc) term(1, k + 1, even);
+        }
+        // sum of the terms: even - 1i odd, then the centre's phase; the parts
+        // meet in the state buffers
+        st = tc;
+        if (advance) {
+            if (l.state) {
+                s_x[part * xs + l.row] = even;
+                s_x[(2 + part) * xs + l.row] = odd;
+            }
+            __syncthreads();
+            if (l.state) {
+                const double er = s_x[l.row], ei = s_x[xs + l.row], dr2 = s_x[2 * xs + l.row], di2 = s_x[3 * xs + l.row];
+                const double fr = er + di2, fi = ei - dr2;
+                const double2 ph = s_turn[last ? 1 : 0];
+                st = part ? fma(ph.y, fr, ph.x * fi) : fma(ph.x, fr, -ph.y * fi);
+            }
+        }
+        if (B.nv > 0) block_points<double2, double>(B, R, S, S.tab, a, Kc, s_mu, s_phase, s_rec, fid_out);
+        const double end_n2 = norm2(st);
+        if (!isfinite(end_n2)) status = kDevNonFinite;
+        else if (end_n2 > 16.0 * start_n2 * (advance ? 1.0 : (double)s_allow) + 1e-300) status = kDevDiverged;
+        if (status != kDevOk) break;
+        start_n2 = end_n2;
+    }
+    if (R.state_out && l.state) reinterpret_cast<double *>(R.state_out)[2 * ((size_t)o * n + l.row) + part] = st;
+    if (tid == 0) {
+        R.status[o] = status;
+        R.kused[o] = S.K;
+        R.mused[o] = M;
+        R.matvecs[o] = mv;
+    }
+}
+
+}  // namespace spx

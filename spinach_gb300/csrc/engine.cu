@@ -24,6 +24,8 @@
 #include <vector>
 
 #include "spinach_gpu.h"
+#include "block.cuh"
+#include "block_plan.h"
 #include "builder.h"
 #include "kernels.cuh"
 
@@ -73,6 +75,28 @@ struct Cplx {
     double re = 0.0, im = 0.0;
 };
 
+// Coupled states of a run (block.cuh): their rows and a few lane layouts per
+// precision, in one device allocation.
+struct BlockPlan {
+    bool ok = false;                 // false: the whole system runs (kernels.cuh)
+    int n = 0, nv = 0, maxchan = 0;
+    struct Layout {
+        spx::BlockLayout dev{};
+        spx::BlockCost cost;
+        int warps = 0, ecap = 0;
+    };
+    std::vector<Layout> layouts[2];  // FP32, FP64
+    DevBuf<unsigned char> mem;
+};
+
+// Device buffers of the kernels of block.cuh for one run.
+struct BlockBufs {
+    DevBuf<double> centre, lev_half, table, saved;
+    DevBuf<float> tablef;
+    DevBuf<unsigned long long> extent;
+    DevBuf<int> lev, kcut;           // lev: steps per chunk | table rows | series lengths
+};
+
 // A pulse superoperator as CSR rows in the sliced order, with its 1-norm.
 struct PulseOp {
     DevBuf<int> ptr, col;
@@ -116,6 +140,17 @@ struct spx_handle {
     DevBuf<double2> d_echo_val;
     int64_t n_states = 0;           // their count (0: one initial state for all)
     std::vector<int> row_of;        // sliced-ELL row of every basis state
+
+    // coupled states of the plain acquisition (rebuilt with the coils and the
+    // initial states) and what finding them takes
+    std::vector<uint16_t> ell_col_host;
+    std::vector<int> component;     // connected component of every row under L
+    std::vector<double2> rho0_host;             // sliced order
+    std::vector<int> coil_row_host, coil_chan_host;
+    std::vector<double2> coil_val_host;
+    std::vector<char> state_rows;   // rows with a non-zero per-orientation initial state
+    BlockPlan plan;
+    BlockBufs blk, chk_blk;
 
     // run buffers
     DevBuf<double> d_grid;       // alpha | beta | gamma | weight
@@ -184,6 +219,146 @@ void for_each_entry(const spx_csc *A, F f) {
     for (int64_t c = 0; c < A->n; ++c)
         for (int64_t p = A->colptr[c]; p < A->colptr[c + 1]; ++p)
             f(A->rowidx[p], c, Cplx{A->values[2 * p], A->values[2 * p + 1]});
+}
+
+// f(row, column, ELL entry) for every off-diagonal entry of the pattern (sliced order).
+template <class F>
+void for_each_coupling(const spx_handle *h, F f) {
+    for (int s = 0; s < h->nslices; ++s)
+        for (int e = h->slice_off_host[s]; e < h->slice_off_host[s + 1]; ++e) {
+            const int row = s * 32 + ((e - h->slice_off_host[s]) & 31), col = h->ell_col_host[e];
+            if (row < h->n && col != row) f(row, col, e);         // padding points at its own row
+        }
+}
+
+// The coupled states of a run: rows whose connected component holds both a
+// coil entry and a row with start[row].  component: labels under everything
+// that moves the state (L, and the pulses of a sequence).
+void build_plan(spx_handle *h, const std::vector<int> &component, const std::vector<char> &start, BlockPlan &plan) {
+    const int n = h->n;
+    plan.ok = false;
+    plan.n = plan.nv = 0;
+    plan.layouts[0].clear();
+    plan.layouts[1].clear();
+    std::vector<char> seen(n, 0), live(n, 0);
+    for (int r : h->coil_row_host) seen[component[r]] = 1;
+    for (int i = 0; i < n; ++i)
+        if (start[i] && seen[component[i]]) live[component[i]] = 1;
+    spx::BlockPattern P;
+    std::vector<int> own(n, -1);
+    for (int i = 0; i < n; ++i)
+        if (live[component[i]]) { own[i] = (int)P.rows.size(); P.rows.push_back(i); }
+    P.n = (int)P.rows.size();
+    if (P.n < 1 || P.n > spx::kBlockRows) return;
+    P.entries.resize(P.n);
+    for_each_coupling(h, [&](int r, int c, int e) {
+        if (own[r] >= 0) P.entries[own[r]].push_back({own[c], e});
+    });
+    // detection rows conj(coil): a complex coil on real values takes a row for
+    // its real and one for its imaginary parts (times -1i)
+    for (int ch = 0; ch < h->nchan; ++ch)
+        for (int im = 0; im < (h->cplx ? 1 : 2); ++im) {
+            std::vector<spx::BlockPattern::Entry> row;
+            for (size_t i = 0; i < h->coil_row_host.size(); ++i) {
+                const int r = own[h->coil_row_host[i]];
+                const double2 v = h->coil_val_host[i];
+                if (h->coil_chan_host[i] != ch || r < 0) continue;
+                if (!h->cplx && (im ? v.y : v.x) == 0.0) continue;
+                row.push_back({r, -2 - (int)(P.values.size() / 2)});
+                P.values.push_back(h->cplx || !im ? v.x : v.y);
+                P.values.push_back(h->cplx ? -v.y : 0.0);
+            }
+            if (im && row.empty()) continue;
+            P.entries.push_back(row);
+            P.vchan.push_back(ch);
+            P.vfac.push_back(im);
+            ++P.nv;
+        }
+    // layouts: the best warp count for a few grid sizes, each precision
+    std::vector<unsigned char> blob;
+    auto put = [&](const void *p, size_t bytes) {
+        const size_t at = (blob.size() + 15) & ~size_t(15);
+        blob.resize(at + std::max<size_t>(bytes, 16));
+        if (bytes) std::memcpy(blob.data() + at, p, bytes);
+        return at;
+    };
+    const size_t o_rows = put(P.rows.data(), P.rows.size() * sizeof(int));
+    const size_t o_val = put(P.values.data(), P.values.size() * sizeof(double));
+    const size_t o_chan = put(P.vchan.data(), P.vchan.size() * sizeof(int));
+    const size_t o_fac = put(P.vfac.data(), P.vfac.size() * sizeof(int));
+    struct At { size_t row, part, shape, src, col; };
+    std::vector<At> at[2];
+    for (int p = 0; p < 2; ++p) {
+        const int ecap_max = p == 1 ? 32 : h->cplx ? 16 : spx::kBlockMaxEntries;
+        int widest = 1;
+        for (auto &r : P.entries) widest = std::max(widest, (int)r.size());
+        std::vector<spx::BlockLanes> lanes;
+        std::vector<spx::BlockCost> costs;
+        for (int e = 1; e <= std::min(widest, ecap_max); ++e) {
+            const size_t cnt = block_lane_count(P, e);
+            const int w = (int)((cnt + 31) / 32);                 // more warps than this only idle
+            if (w > spx::kBlockRows / 32) continue;
+            spx::BlockLanes L;
+            spx::BlockCost c;
+            if (block_lanes(P, w, e, p == 1, h->cplx, h->max_im_diag > 0.0, L, c)) {
+                lanes.push_back(std::move(L));
+                costs.push_back(c);
+            }
+        }
+        if (lanes.empty()) { plan.layouts[0].clear(); return; }
+        std::vector<size_t> keep;
+        for (double per_sm : {1.0, 2.0, 3.0, 5.0, 8.0, 27.0}) {
+            size_t best = 0;
+            for (size_t i = 1; i < lanes.size(); ++i)
+                if (costs[i].time(per_sm) < costs[best].time(per_sm)) best = i;
+            if (std::find(keep.begin(), keep.end(), best) == keep.end()) keep.push_back(best);
+        }
+        for (size_t i : keep) {
+            const spx::BlockLanes &L = lanes[i];
+            at[p].push_back({put(L.row.data(), L.row.size() * 4), put(L.part.data(), L.part.size() * 4),
+                             put(L.shape.data(), L.shape.size() * 4), put(L.src.data(), L.src.size() * 4),
+                             put(L.col.data(), L.col.size() * 2)});
+            BlockPlan::Layout o;
+            o.cost = costs[i];
+            o.warps = L.warps;
+            o.ecap = L.ecap;
+            plan.layouts[p].push_back(o);
+        }
+    }
+    plan.mem.reserve(blob.size());
+    SPX_CUDA(cudaMemcpyAsync(plan.mem.p, blob.data(), blob.size(), cudaMemcpyHostToDevice, h->stream));
+    SPX_CUDA(cudaStreamSynchronize(h->stream));              // blob is pageable
+    const unsigned char *d = plan.mem.p;
+    for (int p = 0; p < 2; ++p)
+        for (size_t i = 0; i < at[p].size(); ++i) {
+            spx::BlockLayout &b = plan.layouts[p][i].dev;
+            b.n = P.n;
+            b.nv = P.nv;
+            b.threads = 32 * plan.layouts[p][i].warps;
+            b.ecap = plan.layouts[p][i].ecap;
+            b.lane_row = reinterpret_cast<const int *>(d + at[p][i].row);
+            b.lane_part = reinterpret_cast<const int *>(d + at[p][i].part);
+            b.warp_shape = reinterpret_cast<const int *>(d + at[p][i].shape);
+            b.src = reinterpret_cast<const int *>(d + at[p][i].src);
+            b.col = reinterpret_cast<const uint16_t *>(d + at[p][i].col);
+            b.row_src = reinterpret_cast<const int *>(d + o_rows);
+            b.vval = reinterpret_cast<const double2 *>(d + o_val);
+            b.vchan = reinterpret_cast<const int *>(d + o_chan);
+            b.vfac = reinterpret_cast<const int *>(d + o_fac);
+        }
+    plan.n = P.n;
+    plan.nv = P.nv;
+    plan.ok = true;
+}
+
+// The plan of the plain acquisition for the handle's coils and initial states.
+void rebuild_plan(spx_handle *h) {
+    std::vector<char> start = h->state_rows;
+    if (h->n_states == 0) {
+        start.resize(h->n);
+        for (int i = 0; i < h->n; ++i) start[i] = h->rho0_host[i].x != 0.0 || h->rho0_host[i].y != 0.0;
+    }
+    build_plan(h, h->component, start, h->plan);
 }
 
 void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32_t *rank,
@@ -465,7 +640,6 @@ void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32
     h->nchan = 1;
     h->n_states = 0;
     h->row_of = inv;
-    SPX_CUDA(cudaStreamSynchronize(h->stream));
     h->n = (int)n;
     h->n_pad = n_pad;
     h->nslices = nslices;
@@ -480,6 +654,17 @@ void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32
     // scales them into (-1, 1) for the packed FP32 layout
     h->lo_scale = g_upper > 0.0 ? std::ldexp(1.0, -std::ilogb(g_upper) - 1) : 1.0;
     h->max_im_diag = max_im_diag;
+    h->ell_col_host = std::move(ell_col);
+    h->rho0_host = std::move(r0);
+    h->coil_row_host = std::move(crow);
+    h->coil_val_host = std::move(cval);
+    h->coil_chan_host.assign(h->coil_row_host.size(), 0);
+    spx::Components comp((int)n);
+    for_each_coupling(h, [&](int r, int c, int) { comp.join(r, c); });
+    h->component.resize(n);
+    for (int i = 0; i < (int)n; ++i) h->component[i] = comp.find(i);
+    rebuild_plan(h);
+    SPX_CUDA(cudaStreamSynchronize(h->stream));
     h->have_system = true;
 }
 
@@ -518,6 +703,10 @@ void upload_coils(spx_handle *h, int32_t nchan, const double *coils) {
         h->d_coil_chan.upload(cchan, h->stream);
     }
     h->nchan = nchan;
+    h->coil_row_host = std::move(crow);
+    h->coil_val_host = std::move(cval);
+    h->coil_chan_host = std::move(cchan);
+    rebuild_plan(h);
     SPX_CUDA(cudaStreamSynchronize(h->stream));
 }
 
@@ -526,26 +715,41 @@ void upload_coils(spx_handle *h, int32_t nchan, const double *coils) {
 // Liouville vectors, orientation after orientation, interleaved complex.
 void set_initial_states(spx_handle *h, int64_t n_states, const double *states) {
     if (!h->have_system) throw SpxError(SPX_ERR_NO_SYSTEM, "no spin system uploaded");
-    if (n_states == 0) { h->n_states = 0; return; }
+    if (n_states == 0) {
+        const bool had = h->n_states != 0;
+        h->n_states = 0;
+        SPX_CUDA(cudaSetDevice(h->device));
+        if (had) rebuild_plan(h);
+        return;
+    }
     if (n_states < 0 || !states) throw SpxError(SPX_ERR_INVALID_ARGUMENT, "bad initial-state array");
     const int n = h->n;
     std::vector<double2> st((size_t)n_states * h->n_pad, make_double2(0, 0));
+    std::vector<char> rows(n, 0);
     for (int64_t o = 0; o < n_states; ++o)
         for (int i = 0; i < n; ++i) {
             const double re = states[2 * ((size_t)o * n + i)], im = states[2 * ((size_t)o * n + i) + 1];
             if (!std::isfinite(re) || !std::isfinite(im)) throw SpxError(SPX_ERR_INVALID_ARGUMENT, "non-finite initial state");
             st[(size_t)o * h->n_pad + h->row_of[i]] = make_double2(re, im);
+            if (re != 0.0 || im != 0.0) rows[h->row_of[i]] = 1;
         }
     SPX_CUDA(cudaSetDevice(h->device));
     h->d_rho0s.upload(st, h->stream);
     SPX_CUDA(cudaStreamSynchronize(h->stream));
     h->n_states = n_states;
+    h->state_rows = std::move(rows);
+    rebuild_plan(h);
 }
 
 // ---------------------------------------------------------------------------
 // Launch configuration
 // ---------------------------------------------------------------------------
 constexpr int kPowderGroup = 64;    // orientations per partial sum of the powder reduction
+
+// spx_options.flags bit of a launch shape that the engine chose itself (the
+// autotuner's): such a run may still take the coupled-state kernels, one whose
+// caller set a shape runs the whole system in that shape.
+constexpr int32_t kOwnShape = 1 << 30;
 
 struct Config {
     int threads, rmax, M, Kmax, grid;
@@ -558,6 +762,13 @@ struct Config {
     int nsl_loc = 0, ell_loc = 0;                 // largest block (slices, ELL entries)
     int traj_m = 1;                               // trajectory outputs: chunk length (1: none)
     bool traj = false;                            // the kernels with trajectory outputs
+    // the coupled-state kernels (block.cuh), if they run: their layout and that
+    // of the spectral bounds (FP32 lanes in both precisions), chunk target, chunk cap, series cap, ladder steps and shared memory
+    const BlockPlan::Layout *blk = nullptr, *blk_bounds = nullptr;
+    double blk_x = 0.0;
+    int blk_M = 0, blk_K = 0, blk_lev = 0;
+    bool blk_cplx = false;
+    size_t blk_smem = 0;
 };
 
 double host_series_terms(double x, double lg, double tol) {
@@ -608,6 +819,10 @@ const void *spx_kernel_f32r_dc_t(int rmax, bool cluster, bool wide);
 const void *spx_kernel_f32c_dc_t(int rmax, bool cluster, bool wide);
 const void *spx_kernel_f64r_dc_t(int rmax, bool cluster, bool wide);
 const void *spx_kernel_f64c_dc_t(int rmax, bool cluster, bool wide);
+// Kernels of block.cuh (kern_block_<value type>.cu): which 0 the spectral
+// bounds, 1 the FP32 and 2 the FP64 propagation.
+const void *spx_block_kernel_r(int ecap, int which);
+const void *spx_block_kernel_c(int ecap, int which);
 namespace {
 
 // Single-CTA kernels for RMAX 1, 2, 4, 6; cluster kernels for RMAX 1, 2, 4;
@@ -661,10 +876,65 @@ bool partition_slices(const spx_handle *h, int cl, Config &c) {
     return true;
 }
 
+const void *block_kernel(bool cplx, int ecap, int which) {
+    const void *k = cplx ? spx_block_kernel_c(ecap, which) : spx_block_kernel_r(ecap, which);
+    if (!k) throw SpxError(SPX_ERR_INTERNAL, "no coupled-state kernel for this layout");
+    return k;
+}
+
+size_t block_smem_for(bool f64, bool cplx, int K, int M, const BlockPlan::Layout &l) {
+    return f64 ? spx::block_smem64(K, M, l.dev.nv, l.dev.threads, l.dev.ecap, l.dev.n, cplx)
+               : spx::block_smem32(K, M, l.dev.nv, l.dev.threads);
+}
+
+// The layout with the least modelled time for a grid.
+const BlockPlan::Layout *best_layout(const std::vector<BlockPlan::Layout> &ls, double per_sm) {
+    const BlockPlan::Layout *best = nullptr;
+    for (const auto &l : ls)
+        if (!best || l.cost.time(per_sm) < best->cost.time(per_sm)) best = &l;
+    return best;
+}
+
+// Whether the run takes the coupled-state kernels, and how: the plan's layout
+// with the least modelled time for this grid.  c holds the whole system's
+// launch shape (so what is refused does not depend on the coupled states).
+void choose_block(spx_handle *h, const BlockPlan *plan, int64_t n_orient, double dt, int64_t nsteps,
+                  const spx_options &opt, int kmax_override, int m_cap, Config &c) {
+    const bool f64 = opt.precision == SPX_FP64;
+    const bool forced = opt.threads > 0 || opt.cluster > 0 || opt.chunk_steps > 0 || opt.chunk_target > 0;
+    if (!plan || !plan->ok || (forced && !(opt.flags & kOwnShape))) return;
+    // FP32 runs of more than 8192 undamped steps keep the whole system: there
+    // FP32 nears the 1e-5 bar and its error decides whether the run is repeated
+    // in FP64, so the decision stays the one it has been (a three-spin system,
+    // 16384 steps: 1.2e-5 on the whole system, 3.5e-6 on its coupled states)
+    if (!f64 && h->max_im_diag == 0.0 && nsteps > 8192) return;
+    const double per_sm = std::ceil((double)n_orient / h->sm_count);
+    const BlockPlan::Layout *best = best_layout(plan->layouts[f64 ? 1 : 0], per_sm);
+    if (!best) return;
+    c.blk_x = opt.chunk_target > 0 ? opt.chunk_target : 300.0;
+    const double lg = (h->g_upper > 0) ? 2.0 * h->max_im_diag / (h->g_upper / 4.0) : 0.0;
+    int K = (int)host_series_terms(std::max(c.blk_x, h->g_upper * dt), std::min(lg, 0.05), c.tol) + 16;
+    c.blk_K = std::min(std::max(K, kmax_override), 8192);
+    // a table's columns: at most 2^18 entries a table (long series come with short chunks)
+    c.blk_M = (int)std::min<int64_t>(std::min(m_cap, std::max(1, (1 << 18) / c.blk_K)), nsteps + 1);
+    c.blk_lev = (int)std::max<int64_t>(4, std::min<int64_t>(spx::kBlockLevels, n_orient / 16));
+    c.blk_smem = block_smem_for(f64, h->cplx, c.blk_K, c.blk_M, *best);
+    const void *kfn = block_kernel(h->cplx, best->ecap, f64 ? 2 : 1);
+    cudaFuncAttributes fa{};
+    SPX_CUDA(cudaFuncGetAttributes(&fa, kfn));
+    if (c.blk_smem + fa.sharedSizeBytes > h->smem_optin) return;
+    SPX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(h->smem_optin - fa.sharedSizeBytes)));
+    c.blk = best;
+    c.blk_cplx = h->cplx;
+    c.blk_bounds = f64 ? best_layout(plan->layouts[0], per_sm) : best;
+}
+
 // traj: the run writes the state at every step (chunks of opt.chunk_steps
-// steps, their intermediate states accumulated in shared memory).
+// steps, their intermediate states accumulated in shared memory).  plan: the
+// run's coupled states, if it may be restricted to them.
 Config choose_config(spx_handle *h, int64_t n_orient, double dt, int64_t nsteps, const spx_options &opt,
-                     int kmax_override, int m_cap = 256, bool traj = false) {
+                     int kmax_override, int m_cap = 256, bool traj = false, const BlockPlan *plan = nullptr) {
     Config c{};
     c.traj = traj;
     const bool f64 = opt.precision == SPX_FP64;
@@ -772,7 +1042,66 @@ Config choose_config(spx_handle *h, int64_t n_orient, double dt, int64_t nsteps,
         if (nclusters < 1) throw SpxError(SPX_ERR_UNSUPPORTED, "no cluster of " + std::to_string(c.cl) + " CTAs fits");
         c.grid = (int)std::min<int64_t>(n_orient, nclusters) * c.cl;
     }
+    choose_block(h, plan, n_orient, dt, nsteps, opt, kmax_override, m_cap, c);
     return c;
+}
+
+// FP32 runs hand the assembled L of every orientation from the bounds to the
+// propagation (both on one layout) while it takes at most 512 MB; larger grids
+// assemble it twice (a radical's 4000 orientations: 96 MB).
+size_t saved_block(const Config &c) {
+    return spx::block_saved(c.blk->dev.ecap, c.blk->dev.threads, c.blk_cplx);
+}
+bool saves_block(int64_t n_orient, bool f64, const Config &c) {
+    return !f64 && (double)n_orient * (double)saved_block(c) <= 64e6;
+}
+
+size_t block_table_entries(const Config &c) { return (size_t)c.blk_lev * c.blk_K * (c.blk_M + 1); }
+
+void reserve_block(BlockBufs &b, int64_t n_orient, bool f64, const Config &c) {
+    b.centre.reserve(n_orient);
+    b.extent.reserve(2);
+    b.lev_half.reserve(c.blk_lev);
+    b.lev.reserve(3 * (size_t)c.blk_lev);
+    b.kcut.reserve((size_t)c.blk_lev * (c.blk_M + 1));
+    b.table.reserve(block_table_entries(c));
+    if (!f64) b.tablef.reserve(block_table_entries(c));
+    if (saves_block(n_orient, f64, c)) b.saved.reserve(n_orient * saved_block(c));
+}
+
+// The buffers' addresses and the configuration in a run descriptor.
+void block_run_buffers(spx::BlockRun &r, const Config &c, double *centre, unsigned long long *extent, double *lev_half,
+                       int *lev, int *kcut, double *table, float *tablef) {
+    r.centre = centre;
+    r.extent = extent;
+    r.lev_half = lev_half;
+    r.nlev = c.blk_lev;
+    r.lev_m = lev;
+    r.lev_k = lev + c.blk_lev;
+    r.lev_raw = lev + 2 * c.blk_lev;
+    r.kcut = kcut;
+    r.table = table;
+    r.tablef = tablef;
+    r.Mcap = c.blk_M;
+    r.Kmax = c.blk_K;
+    r.chunk_x = c.blk_x;
+    r.tol = c.tol;
+}
+
+// Bounds, tables, propagation: three launches on `stream`.
+void launch_block(spx_handle *h, bool f64, const Config &c, spx::DevSystem &sys, spx::BlockRun &r, cudaStream_t stream) {
+    spx::BlockLayout lay = c.blk->dev, blay = c.blk_bounds->dev;
+    SPX_CUDA(cudaMemsetAsync(r.extent, 0, 2 * sizeof(unsigned long long), stream));
+    const dim3 grid((unsigned)r.n_orient);
+    void *bargs[] = {&sys, &blay, &r};
+    SPX_CUDA(cudaLaunchKernel(block_kernel(h->cplx, c.blk_bounds->ecap, 0), grid, dim3((unsigned)blay.threads), bargs, 0,
+                              stream));
+    spx::block_tables_kernel<<<dim3((unsigned)(c.blk_M / 32 + 1), (unsigned)c.blk_lev), 128, 0, stream>>>(r);
+    SPX_CUDA(cudaGetLastError());
+    void *args[] = {&sys, &lay, &r};
+    SPX_CUDA(cudaLaunchKernel(block_kernel(h->cplx, c.blk->ecap, f64 ? 2 : 1), grid,
+                              dim3((unsigned)(lay.threads * (f64 ? 2 : 1))), args, c.blk_smem, stream));
+    h->launches += 3;
 }
 
 // Launch the propagation kernel (plain or cluster launch) on the handle's stream.
@@ -811,7 +1140,8 @@ void reserve_run(spx_handle *h, int64_t n_orient, int64_t nsteps, bool f64, cons
     const size_t npts = ((size_t)nsteps + 1) * h->nchan;       // every channel's points
     const size_t vec_bytes = f64 ? sizeof(double2) : sizeof(float2);
     h->d_fids.reserve(npts * n_orient * vec_bytes);
-    h->d_table.reserve((size_t)c.grid * c.Kmax * (c.M + 1));
+    if (c.blk) reserve_block(h->blk, n_orient, f64, c);
+    else h->d_table.reserve((size_t)c.grid * c.Kmax * (c.M + 1));
     h->d_status.reserve(n_orient);
     h->d_kused.reserve(n_orient);
     h->d_mused.reserve(n_orient);
@@ -850,7 +1180,7 @@ int launch_fp32_check(spx_handle *h, int64_t n_orient, const double *d_al, const
     o64.precision = SPX_FP64;
     o64.lanczos_its = opt.lanczos_its;
     o64 = apply_tuned(h, o64);
-    const Config c = choose_config(h, S, dt, nsteps, o64, 0);
+    const Config c = choose_config(h, S, dt, nsteps, o64, 0, 256, false, &h->plan);
     const size_t npts = ((size_t)nsteps + 1) * h->nchan;
     if (!h->check_stream) {
         SPX_CUDA(cudaStreamCreateWithFlags(&h->check_stream, cudaStreamNonBlocking));
@@ -859,7 +1189,8 @@ int launch_fp32_check(spx_handle *h, int64_t n_orient, const double *d_al, const
     }
     h->d_chk_grid.reserve(3 * (size_t)S);
     h->d_chk_fids.reserve(npts * S * sizeof(double2));
-    h->d_chk_table.reserve((size_t)c.grid * c.Kmax * (c.M + 1));
+    if (c.blk) reserve_block(h->chk_blk, S, true, c);
+    else h->d_chk_table.reserve((size_t)c.grid * c.Kmax * (c.M + 1));
     h->d_chk_status.reserve(S);
     h->d_chk_kused.reserve(S);
     h->d_chk_mused.reserve(S);
@@ -872,6 +1203,24 @@ int launch_fp32_check(spx_handle *h, int64_t n_orient, const double *d_al, const
     for (int j = 0; j < S; ++j) idx[j] = check_index(j, S, n_orient);
     SPX_CUDA(cudaEventRecord(h->ev_fork, h->stream));
     SPX_CUDA(cudaStreamWaitEvent(h->check_stream, h->ev_fork, 0));
+    if (c.blk) {
+        // the checked orientations are picked out of the whole grid on the device
+        spx::DevSystem sys = sys32;
+        spx::BlockRun r{};
+        BlockBufs &b = h->chk_blk;
+        block_run_buffers(r, c, b.centre.p, b.extent.p, b.lev_half.p, b.lev.p, b.kcut.p, b.table.p, nullptr);
+        r.n_orient = S; r.alpha = d_al; r.beta = d_be; r.gamma = d_ga; r.pick = (int)n_orient;
+        r.dt = dt; r.nsteps = (int)nsteps;
+        r.lanczos_its = o64.lanczos_its > 0 ? o64.lanczos_its : 32;
+        r.halfwidth = h->d_chk_halfwidth.p; r.max_im_diag = h->max_im_diag;
+        r.rho0 = sys.rho0; r.rho0s = sys.rho0s; r.rho0_stride = (size_t)h->n_pad;
+        r.fids = h->d_chk_fids.p; r.nchan = h->nchan;
+        r.status = h->d_chk_status.p; r.kused = h->d_chk_kused.p; r.mused = h->d_chk_mused.p;
+        r.matvecs = h->d_chk_matvecs.p;
+        launch_block(h, true, c, sys, r, h->check_stream);
+        SPX_CUDA(cudaEventRecord(h->ev_join, h->check_stream));
+        return 0;
+    }
     double *g = h->d_chk_grid.p;
     for (int j = 0; j < S; ++j) {
         SPX_CUDA(cudaMemcpyAsync(g + j, d_al + idx[j], sizeof(double), cudaMemcpyDeviceToDevice, h->check_stream));
@@ -951,7 +1300,22 @@ void launch_powder(spx_handle *h, int64_t n_orient, const double *d_al, const do
         if (waves && c.grid - take >= std::max(c.cl, c.grid / 2)) c.grid -= take;
     }
     if (timed) SPX_CUDA(cudaEventRecord(h->ev[0], h->stream));
-    launch_chebyshev(h, f64, c, sys, run);
+    if (c.blk) {
+        spx::BlockRun r{};
+        BlockBufs &b = h->blk;
+        block_run_buffers(r, c, b.centre.p, b.extent.p, b.lev_half.p, b.lev.p, b.kcut.p, b.table.p,
+                          f64 ? nullptr : b.tablef.p);
+        if (saves_block(n_orient, f64, c)) r.saved = b.saved.p;
+        r.n_orient = (int)n_orient; r.alpha = d_al; r.beta = d_be; r.gamma = d_ga;
+        r.dt = dt; r.nsteps = (int)nsteps; r.lanczos_its = run.lanczos_its; r.safe_bounds = safe_bounds;
+        r.halfwidth = run.halfwidth; r.max_im_diag = h->max_im_diag;
+        r.rho0 = sys.rho0; r.rho0s = sys.rho0s; r.rho0_stride = (size_t)h->n_pad;
+        r.fids = run.fids; r.nchan = h->nchan;
+        r.status = run.status; r.kused = run.kused; r.mused = run.mused; r.matvecs = run.matvecs;
+        launch_block(h, f64, c, sys, r, h->stream);
+    } else {
+        launch_chebyshev(h, f64, c, sys, run);
+    }
     if (timed) SPX_CUDA(cudaEventRecord(h->ev[1], h->stream));
     // deterministic FP64 powder sum: fixed groups of orientations, fixed order
     const int group = kPowderGroup;
@@ -987,6 +1351,7 @@ void launch_powder(spx_handle *h, int64_t n_orient, const double *d_al, const do
     h->stats.cluster = c.cl;
     h->stats.channels = h->nchan;
     h->stats.smem_bytes = (int32_t)c.smem;
+    h->stats.coupled_dim = c.blk ? c.blk->dev.n : 0;
     h->stats_pending = true;
     h->last_norient = n_orient;
     h->chk_pending = chk;
@@ -1684,12 +2049,13 @@ spx_options apply_tuned(const spx_handle *h, spx_options o) {
         o.threads = h->tuned[p].threads;
         o.cluster = h->tuned[p].cluster;
         o.chunk_target = h->tuned[p].chunk_target;
+        o.flags |= kOwnShape;
     }
     return o;
 }
 
 // shape of a tuning problem: systems with the same key get the same answer
-using TuneKey = std::tuple<int, int, int, int, int, int, int, int>;
+using TuneKey = std::tuple<int, int, int, int, int, int, int, int, int, int>;
 std::mutex g_tune_mutex;
 std::map<TuneKey, spx_options> g_tune_cache;
 
@@ -1697,7 +2063,7 @@ TuneKey tune_key(const spx_handle *h, double dt, int64_t nsteps, int precision) 
     // spectral scale in octaves: the series length per step follows it
     const int scale = (int)std::lround(std::log2(std::max(h->g_upper * dt, 1e-30)));
     return TuneKey{h->n, h->ell_len, h->nslices, h->nstreams, h->cplx ? 1 : 0, precision, scale,
-                   (int)std::min<int64_t>(nsteps, 512)};
+                   (int)std::min<int64_t>(nsteps, 512), h->plan.ok ? h->plan.n : 0, h->nchan};
 }
 
 // Kernel time of one candidate over the sample, or +inf if it cannot run.
@@ -1705,7 +2071,7 @@ double time_candidate(spx_handle *h, int64_t n, const double *d_al, const double
                       const double *d_w, double dt, int64_t nsteps, spx_options o, double2 *d_out) {
     double best = INFINITY;
     try {
-        const Config c = choose_config(h, n, dt, nsteps, o, 0);
+        const Config c = choose_config(h, n, dt, nsteps, o, 0, 256, false, &h->plan);
         for (int rep = 0; rep < 2; ++rep) {           // first launch also loads the kernel
             launch_powder(h, n, d_al, d_be, d_ga, d_w, dt, nsteps, o, d_out, c);
             finish_run(h);
@@ -1737,8 +2103,8 @@ spx_options autotune(spx_handle *h, int64_t n_orient, const double *d_al, const 
     {
         spx_options o1 = base;
         try {
-            const Config c1 = choose_config(h, n, dt, ns, o1, 0);
-            n = std::min<int64_t>(n, c1.grid);
+            const Config c1 = choose_config(h, n, dt, ns, o1, 0, 256, false, &h->plan);
+            if (!c1.blk) n = std::min<int64_t>(n, c1.grid);
         } catch (const SpxError &) {
             n = std::min<int64_t>(n, h->sm_count);
         }
@@ -1753,7 +2119,21 @@ spx_options autotune(spx_handle *h, int64_t n_orient, const double *d_al, const 
     double best_t = INFINITY;
     const int cls[] = {1, 2, 4, 8};
     int cl_min = 0;                 // smallest cluster that fits; it and twice it are tried
+    {
+        // a run over the coupled states has its own layouts: only the series
+        // length per chunk is tuned, beside the whole system's default shape
+        const Config c0 = choose_config(h, n, dt, ns, base, 0, 256, false, &h->plan);
+        if (c0.blk) {
+            best.threads = c0.threads;
+            best.cluster = c0.cl;
+            best.flags = kOwnShape;
+            best.chunk_target = c0.blk_x;
+            best_t = time_candidate(h, n, d_al, d_be, d_ga, w.p, dt, ns, best, out.p);
+            cl_min = -1;
+        }
+    }
     for (int cl : cls) {
+        if (cl_min < 0) break;
         if (cl_min && cl > 2 * cl_min) break;
         // warps: the default for this cluster size, half, and 16
         spx_options o = base;
@@ -1786,6 +2166,7 @@ spx_options autotune(spx_handle *h, int64_t n_orient, const double *d_al, const 
         if (t < best_t) { best_t = t; bc = o; }
     }
     best = bc;
+    best.flags = 0;
     std::lock_guard<std::mutex> lk(g_tune_mutex);
     g_tune_cache[key] = best;
     return best;
@@ -1867,21 +2248,27 @@ void run_powder_noalloc(spx_handle *h, int64_t n_orient, const double *d_al, con
     SPX_CUDA(cudaSetDevice(h->device));
     spx_options opt{};
     opt.precision = precision;
-    const Config c = choose_config(h, n_orient, dt, nsteps, opt, 0, kNoallocChunkCap);
+    const Config c = choose_config(h, n_orient, dt, nsteps, opt, 0, kNoallocChunkCap, false, &h->plan);
     const bool f64 = precision == SPX_FP64;
     const size_t npts = ((size_t)nsteps + 1) * h->nchan;   // all channels' points
     const int group = 64;
     const int ngroups = (int)((n_orient + group - 1) / group);
+    const size_t tables = c.blk ? block_table_entries(c) : (size_t)c.grid * c.Kmax * (c.M + 1);
     // carve the scratch: sizes first, then check, then addresses
-    const size_t sizes[9] = {
-        (size_t)c.grid * c.Kmax * (c.M + 1) * sizeof(double),        // Bessel tables
+    constexpr int kParts = 14;
+    const size_t sizes[kParts] = {
+        tables * sizeof(double),                                      // Bessel tables
         npts * (size_t)n_orient * (f64 ? sizeof(double2) : sizeof(float2)),   // per-orientation FIDs
         (size_t)ngroups * npts * sizeof(double2),                     // FP64 partial sums
         (size_t)n_orient * sizeof(int), (size_t)n_orient * sizeof(int), (size_t)n_orient * sizeof(int),
         (size_t)n_orient * sizeof(long long) + (size_t)n_orient * sizeof(double),
-        sizeof(int), sizeof(int)};
-    size_t offs[9], total = 0;
-    for (int i = 0; i < 9; ++i) {
+        sizeof(int), sizeof(int),
+        // coupled-state kernels: float tables, centres, extents, ladder, columns' terms
+        c.blk && !f64 ? tables * sizeof(float) : 0, c.blk ? (size_t)n_orient * sizeof(double) : 0,
+        c.blk ? 2 * sizeof(unsigned long long) : 0, c.blk ? (size_t)c.blk_lev * (sizeof(double) + 3 * sizeof(int)) : 0,
+        c.blk ? (size_t)c.blk_lev * (c.blk_M + 1) * sizeof(int) : 0};
+    size_t offs[kParts], total = 0;
+    for (int i = 0; i < kParts; ++i) {
         offs[i] = total;
         total += (sizes[i] + 255) & ~(size_t)255;
     }
@@ -1920,7 +2307,24 @@ void run_powder_noalloc(spx_handle *h, int64_t n_orient, const double *d_al, con
     // (run.next_orient) in launch_chebyshev; everything else is written
     // before it is read
     SPX_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), h->stream));
-    launch_chebyshev(h, f64, c, sys, run);
+    if (c.blk) {
+        spx::BlockRun r{};
+        block_run_buffers(r, c, reinterpret_cast<double *>(base + offs[10]),
+                          reinterpret_cast<unsigned long long *>(base + offs[11]),
+                          reinterpret_cast<double *>(base + offs[12]),
+                          reinterpret_cast<int *>(base + offs[12] + c.blk_lev * sizeof(double)),
+                          reinterpret_cast<int *>(base + offs[13]), run.table,
+                          f64 ? nullptr : reinterpret_cast<float *>(base + offs[9]));
+        r.n_orient = run.n_orient; r.alpha = d_al; r.beta = d_be; r.gamma = d_ga;
+        r.dt = dt; r.nsteps = (int)nsteps; r.lanczos_its = run.lanczos_its;
+        r.halfwidth = run.halfwidth; r.max_im_diag = h->max_im_diag;
+        r.rho0 = sys.rho0; r.rho0s = sys.rho0s; r.rho0_stride = (size_t)h->n_pad;
+        r.fids = run.fids; r.nchan = h->nchan;
+        r.status = run.status; r.kused = run.kused; r.mused = run.mused; r.matvecs = run.matvecs;
+        launch_block(h, f64, c, sys, r, h->stream);
+    } else {
+        launch_chebyshev(h, f64, c, sys, run);
+    }
     const dim3 pb(256), pg((unsigned)((npts + 255) / 256), (unsigned)ngroups);
     ++h->launches;  // powder partial sum
     if (f64)
@@ -2033,7 +2437,7 @@ spx_status spx_run_powder(spx_handle *h, int64_t n_orient, const double *alphas,
         SPX_CUDA(cudaMemcpyAsync(g + 2 * n_orient, gammas, b, cudaMemcpyHostToDevice, h->stream));
         SPX_CUDA(cudaMemcpyAsync(g + 3 * n_orient, weights, b, cudaMemcpyHostToDevice, h->stream));
         h->d_fid.reserve(((size_t)nsteps + 1) * h->nchan);
-        Config c = choose_config(h, n_orient, dt, nsteps, o, 0);
+        Config c = choose_config(h, n_orient, dt, nsteps, o, 0, 256, false, &h->plan);
         const bool check = o.precision == SPX_FP32 && !(o.flags & SPX_FLAG_NO_FP32_CHECK);
         launch_powder(h, n_orient, g, g + n_orient, g + 2 * n_orient, g + 3 * n_orient, dt, nsteps, o, h->d_fid.p, c,
                       0, true, RunIO{}, check);
@@ -2054,7 +2458,7 @@ spx_status spx_run_powder(spx_handle *h, int64_t n_orient, const double *alphas,
                 kneed = std::max(kneed, kused[i]);
             }
             if (!retriable) throw;
-            c = choose_config(h, n_orient, dt, nsteps, o, 2 * kneed + 16);
+            c = choose_config(h, n_orient, dt, nsteps, o, 2 * kneed + 16, 256, false, &h->plan);
             retried = true;
             launch_powder(h, n_orient, g, g + n_orient, g + 2 * n_orient, g + 3 * n_orient, dt, nsteps, o,
                           h->d_fid.p, c, 1, true, RunIO{}, check);
@@ -2077,8 +2481,9 @@ spx_status spx_run_powder(spx_handle *h, int64_t n_orient, const double *alphas,
             o64.precision = SPX_FP64;
             o64.threads = o64.cluster = 0;
             o64.chunk_target = 0.0;
+            o64.flags &= ~kOwnShape;
             o64 = apply_tuned(h, o64);
-            const Config c64 = choose_config(h, n_orient, dt, nsteps, o64, 0);
+            const Config c64 = choose_config(h, n_orient, dt, nsteps, o64, 0, 256, false, &h->plan);
             launch_powder(h, n_orient, g, g + n_orient, g + 2 * n_orient, g + 3 * n_orient, dt, nsteps, o64,
                           h->d_fid.p, c64);
             finish_run(h);
@@ -2121,7 +2526,7 @@ spx_status spx_run_powder_device(spx_handle *h, int64_t n_orient, const double *
             throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
         o = apply_tuned(h, o);
         SPX_CUDA(cudaSetDevice(h->device));
-        const Config c = choose_config(h, n_orient, dt, nsteps, o, 0);
+        const Config c = choose_config(h, n_orient, dt, nsteps, o, 0, 256, false, &h->plan);
         const bool check = o.precision == SPX_FP32 && !(o.flags & SPX_FLAG_NO_FP32_CHECK);
         launch_powder(h, n_orient, d_alphas, d_betas, d_gammas, d_weights, dt, nsteps, o,
                       reinterpret_cast<double2 *>(d_fid), c, 0, true, RunIO{}, check);
@@ -2464,7 +2869,7 @@ spx_status spx_batch_create(spx_batch **out, int32_t n, spx_handle *const *handl
             if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
                 throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
             os[i] = apply_tuned(h, o);
-            cfg[i] = choose_config(h, n_orient[i], dt[i], nsteps[i], os[i], 0);
+            cfg[i] = choose_config(h, n_orient[i], dt[i], nsteps[i], os[i], 0, 256, false, &h->plan);
             reserve_run(h, n_orient[i], nsteps[i], os[i].precision == SPX_FP64, cfg[i]);
             SPX_CUDA(cudaStreamSynchronize(h->stream));
         }
@@ -2475,10 +2880,18 @@ spx_status spx_batch_create(spx_batch **out, int32_t n, spx_handle *const *handl
             SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::powder_partial_kernel<float2>)));
             SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::powder_partial_kernel<double2>)));
             SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::powder_combine_kernel)));
-            for (int i = 0; i < n; ++i)
+            SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::block_tables_kernel)));
+            for (int i = 0; i < n; ++i) {
+                if (cfg[i].blk) {
+                    SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(handles[i]->cplx, cfg[i].blk_bounds->ecap, 0)));
+                    SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(handles[i]->cplx, cfg[i].blk->ecap,
+                                                                     os[i].precision == SPX_FP64 ? 2 : 1)));
+                    continue;
+                }
                 SPX_CUDA(cudaFuncGetAttributes(&fa, select_kernel(os[i].precision == SPX_FP64, handles[i]->cplx,
                                                                   cfg[i].rmax, cfg[i].cl > 1, handles[i]->ncoil > 0,
                                                                   false, cfg[i].threads > 512)));
+            }
         }
         b->marks.resize(n + 1, nullptr);
         for (auto &e : b->marks) SPX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

@@ -1612,7 +1612,21 @@ __global__ void powder_partial_kernel(const Vec *__restrict__ fids, const double
     if (t >= npts) return;
     const int o0 = g * group, o1 = min(n_orient, o0 + group);
     double2 s = make_double2(0.0, 0.0);
-    for (int o = o0; o < o1; ++o) {
+    // eight loads in flight: small grids leave too few CTAs to hide their
+    // latency (200 orientations x 1025 points: 25 us one at a time)
+    int o = o0;
+    for (; o + 8 <= o1; o += 8) {
+        Vec v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = fids[(size_t)(o + q) * npts + t];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const double2 d = tod(v[q]);
+            s.x = fma(w[o + q], d.x, s.x);
+            s.y = fma(w[o + q], d.y, s.y);
+        }
+    }
+    for (; o < o1; ++o) {
         const double2 v = tod(fids[(size_t)o * npts + t]);
         s.x = fma(w[o], v.x, s.x);
         s.y = fma(w[o], v.y, s.y);

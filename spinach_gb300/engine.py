@@ -51,7 +51,7 @@ class SpxStats(C.Structure):
                 ('value_streams', C.c_int32), ('real_offdiag', C.c_int32),
                 ('cluster', C.c_int32), ('smem_bytes', C.c_int32), ('channels', C.c_int32),
                 ('retries', C.c_int32), ('fp32_checked', C.c_int32), ('kernel_launches', C.c_int64),
-                ('fp32_rel_error', C.c_double), ('promoted_fp64', C.c_int32), ('reserved', C.c_int32),
+                ('fp32_rel_error', C.c_double), ('promoted_fp64', C.c_int32), ('coupled_dim', C.c_int32),
                 ('fp32_powder_error', C.c_double)]
 
     def as_dict(self) -> dict:
