@@ -29,6 +29,7 @@ namespace spx {
 constexpr int kBlockRows = 512;        // largest number of coupled states
 constexpr int kBlockLevels = 32;       // steps of the half-width ladder (Bessel tables)
 constexpr int kBlockMaxEntries = 24;   // entries of one lane
+constexpr int kBlockTraj = 4;          // steps per chunk of runs that write the state at every step
 
 // One layout of the rows on a CTA's lanes (device pointers).
 struct BlockLayout {
@@ -42,6 +43,7 @@ struct BlockLayout {
     const int *src;             // [ecap][threads] ELL entry of the system, -1 none, -2-i: coil value i
     const uint16_t *col;        // [ecap][threads] state row the entry reads
     const int *row_src;         // [n] row of the system (sliced order)
+    const int *state_pos;       // [n] place of the row in the run's state arrays
     const double2 *vval;        // entry values of the detection rows
     const int *vchan;           // [nv] channel of a detection row
     const int *vfac;            // [nv] 0: times 1, 1: times -1i (imaginary parts of a complex coil)
@@ -69,12 +71,13 @@ struct BlockRun {
     double *table;              // [nlev][Kmax][M+1] (2 - delta_k0) J_k(half j dt)
     float *tablef;              // the same rounded to float, or null
     double max_im_diag;
-    // states
-    const double2 *rho0;        // one initial state (read at row_src, or at the row itself when rho0_own)
-    const double2 *rho0s;       // or one per orientation, rho0_stride apart
-    size_t rho0_stride;
-    int rho0_own;
-    double2 *state_out;         // or null: [n_orient][n] the state after the last step
+    int adjoint;                // propagate under -H + 1i R: the adjoint of exp(-1i L dt)
+    // states (read and written at state_pos)
+    const double2 *rho0;        // one initial state
+    const double2 *rho0s;       // or one per orientation, state_stride apart
+    size_t state_stride;
+    double2 *state_out;         // or null: the state after the last step, state_stride apart
+    void *traj_out;             // or null: [n_orient][nsteps+1][n] the state at every step, in the run's precision
     void *fids;                 // [n_orient][nchan][nsteps+1]; not written when nv == 0
     int nchan;
     double *saved;              // or null: every orientation's assembled L, in lane order (block_saved)
@@ -159,10 +162,11 @@ static __device__ __forceinline__ BlockLane block_lane(const BlockLayout &B, int
 // One lane's entries of an orientation's L: FP64 sums over the value streams
 // (coef: the rotational coefficients), stream by stream, so that the loads of
 // all entries are in flight together; detection rows keep their values.
-// Entries i of the lane with i % NTH == TH (threads that share the lane).
+// sign: -1 for the adjoint generator -H + 1i R.
 template <bool CPLX, int ECAP>
 static __device__ __forceinline__ void block_assemble(const DevSystem &sys, const BlockLayout &B, int ew, int t,
-                                                      const double *coef, double (&re)[ECAP], double (&im)[ECAP]) {
+                                                      const double *coef, double sign, double (&re)[ECAP],
+                                                      double (&im)[ECAP]) {
     int src[ECAP];
 #pragma unroll
     for (int i = 0; i < ECAP; ++i) {
@@ -181,16 +185,19 @@ static __device__ __forceinline__ void block_assemble(const DevSystem &sys, cons
             }
     }
 #pragma unroll
-    for (int i = 0; i < ECAP; ++i)
+    for (int i = 0; i < ECAP; ++i) {
+        re[i] *= sign;
+        im[i] *= sign;
         if (src[i] <= -2) {
             const double2 v = B.vval[-2 - src[i]];
             re[i] = v.x;
             im[i] = v.y;
         }
+    }
 }
 
 // Diagonal entry of system row r.
-static __device__ __forceinline__ double2 block_diagonal(const DevSystem &sys, int r, const double *coef) {
+static __device__ __forceinline__ double2 block_diagonal(const DevSystem &sys, int r, const double *coef, double sign) {
     double2 dg = make_double2(0.0, 0.0);
     for (int s = 0; s < sys.nstreams; ++s) {
         const double c = coef[sys.stream_coef[s]];
@@ -198,6 +205,7 @@ static __device__ __forceinline__ double2 block_diagonal(const DevSystem &sys, i
         dg.x = fma(c, d.x, dg.x);
         dg.y = fma(c, d.y, dg.y);
     }
+    dg.x *= sign;
     return dg;
 }
 
@@ -230,9 +238,8 @@ static __device__ __forceinline__ void block_coefficients(const DevSystem &sys, 
 // Spectral bounds of every orientation: Gershgorin discs, and Lanczos on the
 // Hermitian part, in FP32 for both precisions (the interval is widened by the
 // Ritz residuals and 2% of its width, and the propagation watches the norm).
-// One reduction per Lanczos step: beta^2 = |w|^2 - alpha^2 with the matrix
-// taken about the middle of its discs, where alpha is no larger than the
-// spread.  The assembled L goes to R.saved for the FP32 propagation, which
+// The matrix is taken about the middle of its discs, so that alpha is no larger
+// than the spread.  The assembled L goes to R.saved for the FP32 propagation, which
 // runs on the same layout.
 // ---------------------------------------------------------------------------
 template <bool CPLX, int ECAP>
@@ -249,8 +256,9 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_bounds_kernel(const DevSy
     double2 dg = make_double2(0.0, 0.0);
     {
         double re[ECAP], im[ECAP];
-        block_assemble<CPLX, ECAP>(sys, B, l.ew, tid, s_coef, re, im);
-        if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef);
+        const double sign = R.adjoint ? -1.0 : 1.0;
+        block_assemble<CPLX, ECAP>(sys, B, l.ew, tid, s_coef, sign, re, im);
+        if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef, sign);
         double *save = R.saved ? R.saved + (size_t)o * block_saved(B.ecap, B.threads, CPLX) : nullptr;
 #pragma unroll
         for (int i = 0; i < ECAP; ++i) {
@@ -315,7 +323,9 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_bounds_kernel(const DevSy
     }
     float beta_prev = 0.f;
     int m_eff = 0;
-    const int lits = min(R.lanczos_its, min(kMaxLanczos, B.n));
+    // also beyond n steps: FP32 vectors lose their orthogonality on clustered
+    // spectra, and n steps then miss the ends (more only find them again)
+    const int lits = min(R.lanczos_its, kMaxLanczos);
     const int slot = l.state ? l.row : kBlockRows;
     for (int j = 0; j < lits; ++j) {
         float2 *x = s_x[j & 1];
@@ -333,15 +343,19 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_bounds_kernel(const DevSy
         } else {
             y = make_float2(0.f, 0.f);
         }
-        const float2 sums = reduce(make_float2(q_cur.x * y.x + q_cur.y * y.y, y.x * y.x + y.y * y.y), 0);
-        const float alpha = sums.x, b2 = sums.y - alpha * alpha, beta = b2 > 0.f ? sqrtf(b2) : 0.f;
+        const float alpha = reduce(make_float2(q_cur.x * y.x + q_cur.y * y.y, 0.f), 0).x;
+        y.x -= alpha * q_cur.x;
+        y.y -= alpha * q_cur.y;
+        // beta from the residual itself: |w|^2 - alpha^2 would hide directions
+        // that the start vector holds little of
+        const float beta = sqrtf(reduce(make_float2(y.x * y.x + y.y * y.y, 0.f), 0).x);
         if (tid == 0) { s_al[j] = (double)alpha; s_be[j] = (double)beta; }
         m_eff = j + 1;
-        if (!(b2 > 1e-6f * sums.y)) break;                   // invariant subspace, to the sums' rounding
+        if (!(beta > 1e-12f * (fabsf(alpha) + 1e-30f))) break;      // invariant subspace
         const float inv = 1.f / beta;
         q_prev = q_cur;
-        q_cur.x = (y.x - alpha * q_cur.x) * inv;
-        q_cur.y = (y.y - alpha * q_cur.y) * inv;
+        q_cur.x = y.x * inv;
+        q_cur.y = y.y * inv;
         beta_prev = beta;
     }
     __syncthreads();
@@ -492,12 +506,14 @@ static __global__ void __launch_bounds__(128) block_tables_kernel(const BlockRun
 }
 
 // Dynamic shared memory of the propagation kernels.
-static __host__ __device__ inline size_t block_smem32(int Kmax, int Mcap, int nv, int threads) {
-    return 8 * ((size_t)(Kmax + 2) * (1 + nv) + (size_t)(Mcap + 1) + (size_t)(threads > Mcap ? threads : Mcap));
+static __host__ __device__ inline size_t block_smem32(int Kmax, int Mcap, int nv, int threads, bool traj) {
+    return 8 * ((size_t)(Kmax + 2) * (1 + nv + (traj ? kBlockTraj - 1 : 0)) + (size_t)(Mcap + 1) +
+                (size_t)(threads > Mcap ? threads : Mcap));
 }
-static __host__ __device__ inline size_t block_smem64(int Kmax, int Mcap, int nv, int lanes, int ecap, int n, bool cplx) {
+static __host__ __device__ inline size_t block_smem64(int Kmax, int Mcap, int nv, int lanes, int ecap, int n, bool cplx,
+                                                      bool traj) {
     const size_t rec = (size_t)(2 * lanes > Mcap ? 2 * lanes : Mcap);
-    return 16 * (rec + (size_t)(Mcap + 1) + (size_t)(Kmax + 2) * nv) + 8 * (size_t)(Kmax + 2) +
+    return 16 * (rec + (size_t)(Mcap + 1) + (size_t)(Kmax + 2) * nv) + 8 * (size_t)(Kmax + 2) * (traj ? kBlockTraj : 1) +
            8 * (size_t)ecap * lanes * (cplx ? 2 : 1) + 8 * 4 * (size_t)(n + 1) + 2 * (size_t)ecap * lanes;
 }
 
@@ -550,12 +566,10 @@ static __device__ __forceinline__ BlockSeries block_series(const BlockRun &R, in
 }
 
 // e^{-i c j dt}, j < M: one sine and cosine per thread, turned on by
-// blockDim.x steps at a time (FP64 transcendentals are slow here); the phases
-// of a whole and of the last chunk; and the growth of |t_k|^2 that Im L allows
-// over the last chunk's terms.
+// blockDim.x steps at a time (FP64 transcendentals are slow here), and the
+// phases of a whole and of the last chunk.
 template <class Vec>
-static __device__ __forceinline__ void block_phases(const BlockRun &R, const BlockSeries &S, Vec *phase, double2 *turn,
-                                                    float *allow) {
+static __device__ __forceinline__ void block_phases(const BlockRun &R, const BlockSeries &S, Vec *phase, double2 *turn) {
     const int tid = threadIdx.x, nt = (int)blockDim.x;
     if (tid < S.M) {
         double sn, cs, rs = 0.0, rc = 1.0;
@@ -572,10 +586,6 @@ static __device__ __forceinline__ void block_phases(const BlockRun &R, const Blo
         double sn, cs;
         sincos(-S.cen * (tid == 0 ? S.M : S.j_last) * R.dt, &sn, &cs);
         turn[tid] = make_double2(cs, sn);
-    }
-    if (tid == nt - 1) {
-        const float q = (float)(R.max_im_diag / S.half);
-        *allow = __expf(fminf(80.f, 2.f * S.K * __logf(q + sqrtf(1.f + q * q))));
     }
 }
 
@@ -667,19 +677,22 @@ static __device__ __forceinline__ void block_dispatch(const BlockLane &l, F &&f)
 // ---------------------------------------------------------------------------
 // Propagation, FP32: values in registers, (re, im) in packed f32x2 operations.
 // ---------------------------------------------------------------------------
-template <bool CPLX, int ECAP>
+// TRJ: also the state at every step (R.traj_out), from chunks of at most
+// kBlockTraj steps whose inner states are summed beside the chunk-end state.
+template <bool CPLX, int ECAP, bool TRJ>
 __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const DevSystem sys, const BlockLayout B,
                                                                         const BlockRun R) {
+    constexpr int NT = TRJ ? kBlockTraj - 1 : 0;
     __shared__ double s_coef[kMaxCoef];
     __shared__ float2 s_x[2][kBlockRows + 1];
     __shared__ float s_norm[2][kBlockRows / 32];
     __shared__ double2 s_turn[2];
-    __shared__ float s_allow;
     extern __shared__ __align__(16) unsigned char smem[];
     float2 *s_b = reinterpret_cast<float2 *>(smem);          // chunk-end coefficients (b, b)
     float2 *s_mu = s_b + (R.Kmax + 2);                        // moments, one row per detection row
     float2 *s_phase = s_mu + (size_t)(R.Kmax + 2) * B.nv;
     float2 *s_rec = s_phase + (R.Mcap + 1);
+    [[maybe_unused]] float2 *s_tb = s_rec + (blockDim.x > R.Mcap ? blockDim.x : R.Mcap);   // [step][term] inner states
     const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const BlockLane l = block_lane(B, tid);
     const BlockSeries S = block_series(R, o);
@@ -703,9 +716,10 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
             save += (size_t)(CPLX ? 2 : 1) * B.ecap * B.threads;
             dg = make_double2(save[tid], save[B.threads + tid]);
         } else {
+            const double sign = R.adjoint ? -1.0 : 1.0;
             block_coefficients(sys, R, o, s_coef);
-            block_assemble<CPLX, ECAP>(sys, B, l.ew, tid, s_coef, re, im);
-            if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef);
+            block_assemble<CPLX, ECAP>(sys, B, l.ew, tid, s_coef, sign, re, im);
+            if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef, sign);
         }
         const double sc = l.row < B.n ? scale : 1.0;          // detection rows keep their values
 #pragma unroll
@@ -725,13 +739,20 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
         }
         if (tid < 2) s_b[Kc + tid] = make_float2(0.f, 0.f);
     };
-    block_phases(R, S, s_phase, s_turn, &s_allow);
+    block_phases(R, S, s_phase, s_turn);
     coefficients(M, S.K);
+    if constexpr (TRJ) {
+        for (int q = tid; q < NT * (S.K + 2); q += blockDim.x) {
+            const int k = q / NT, j = 1 + q % NT;
+            const float b = k < S.K && j < M ? (float)(block_sign(k) * S.tab[k * S.ld + j]) : 0.f;
+            s_tb[(size_t)(j - 1) * (R.Kmax + 2) + k] = make_float2(b, b);
+        }
+    }
 
     float2 st = make_float2(0.f, 0.f);
     if (l.state) {
-        const double2 *r0 = R.rho0s ? R.rho0s + (size_t)block_grid_index(R, o) * R.rho0_stride : R.rho0;
-        st = tovec(r0[R.rho0_own ? l.row : B.row_src[l.row]], float2());
+        const double2 *r0 = R.rho0s ? R.rho0s + (size_t)block_grid_index(R, o) * R.state_stride : R.rho0;
+        st = tovec(r0[B.state_pos[l.row]], float2());
     }
     const float2 *mu_row = s_mu + (size_t)(l.row >= B.n ? l.row - B.n : 0) * (R.Kmax + 2);
     float2 *fid_out = reinterpret_cast<float2 *>(R.fids) + (size_t)o * R.nchan * (nsteps + 1);
@@ -757,11 +778,9 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
     const char *x0 = reinterpret_cast<const char *>(&s_x[0][0]), *x1 = reinterpret_cast<const char *>(&s_x[1][0]);
     for (int a = 0; a < S.nchunks; ++a) {
         const bool last = a + 1 == S.nchunks;
-        const bool advance = !last || R.state_out != nullptr;
         const int Kc = last ? min(S.K, S.kcut[S.j_last]) : S.K;
         mv += Kc - 1;
-        if (last && advance) coefficients(S.j_last, Kc);
-        else if (last && tid < 2) s_b[Kc + tid] = make_float2(0.f, 0.f);
+        if (last) coefficients(S.j_last, Kc);
         if (l.state) s_x[0][l.row] = st;
         __syncthreads();
         // Where this lane's result goes: a state row's into the other state
@@ -785,6 +804,14 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
             const f2x b0 = reinterpret_cast<const f2x *>(s_b)[0];
             acc = mul2(b0, tc);
             accl = fma2(b0, tc, sub2(0ull, acc));
+        }
+        [[maybe_unused]] f2x inner[NT + 1];
+        if constexpr (TRJ) {
+            if (l.state)
+                reinterpret_cast<float2 *>(R.traj_out)[((size_t)o * (nsteps + 1) + (size_t)a * M) * B.n + l.row] = st;
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+                inner[j] = mul2(reinterpret_cast<const f2x *>(s_tb + (size_t)j * (R.Kmax + 2))[0], tc);
         }
         auto term = [&](auto ewc, auto rnc, auto oddc, const char *src, int k) {
             constexpr int EW = decltype(ewc)::value, RND = decltype(rnc)::value;
@@ -822,6 +849,11 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
             const f2x Sm = fma2(b, V, acc);
             accl = add2(accl, fma2(b, V, sub2(acc, Sm)));
             acc = Sm;
+            if constexpr (TRJ) {
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+                    inner[j] = fma2(reinterpret_cast<const f2x *>(s_tb + (size_t)j * (R.Kmax + 2))[k], V, inner[j]);
+            }
             ntp = mul2(NEG, tc);
             tc = T;
         };
@@ -832,26 +864,34 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
             }
         };
         block_dispatch<ECAP>(l, terms);
-        const float2 fin = f2up(advance ? add2(acc, accl) : tc);
+        if constexpr (TRJ) {
+            // the states 1 .. M-1 steps into the chunk, up to the last step
+            const int jn = min(M - 1, nsteps - a * M);
+#pragma unroll
+            for (int j = 1; j <= NT; ++j)
+                if (l.state && j <= jn) {
+                    const float2 f = f2up(inner[j - 1]), ph = s_phase[j];
+                    reinterpret_cast<float2 *>(R.traj_out)[((size_t)o * (nsteps + 1) + (size_t)a * M + j) * B.n + l.row] =
+                        make_float2(ph.x * f.x - ph.y * f.y, ph.x * f.y + ph.y * f.x);
+                }
+        }
+        const float2 fin = f2up(add2(acc, accl));
         st = make_float2(0.f, 0.f);
         if (l.state) {
-            st = fin;
-            if (advance) {
-                const double2 ph = s_turn[last ? 1 : 0];
-                st.x = (float)(ph.x * (double)fin.x - ph.y * (double)fin.y);
-                st.y = (float)(ph.y * (double)fin.x + ph.x * (double)fin.y);
-            }
+            const double2 ph = s_turn[last ? 1 : 0];
+            st.x = (float)(ph.x * (double)fin.x - ph.y * (double)fin.y);
+            st.y = (float)(ph.y * (double)fin.x + ph.x * (double)fin.y);
         }
         if (B.nv > 0) block_points<float2, float>(B, R, S, S.tabf, a, Kc, s_mu, s_phase, s_rec, fid_out);
         // a state that grew shows a violated spectral bound (a dissipative L
         // can only shrink it); the norm's barrier also ends this chunk's reads
         const float end_n2 = norm2(st);
         if (!isfinite(end_n2)) status = kDevNonFinite;
-        else if (end_n2 > 16.f * start_n2 * (advance ? 1.f : s_allow) + 1e-30f) status = kDevDiverged;
+        else if (end_n2 > 16.f * start_n2 + 1e-30f) status = kDevDiverged;
         if (status != kDevOk) break;
         start_n2 = end_n2;
     }
-    if (R.state_out && l.state) R.state_out[(size_t)o * B.n + l.row] = tod(st);
+    if (R.state_out && l.state) R.state_out[(size_t)o * R.state_stride + B.state_pos[l.row]] = tod(st);
     if (tid == 0) {
         R.status[o] = status;
         R.kused[o] = S.K;
@@ -869,13 +909,13 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
 // four units; values and columns sit in shared memory, whose loads cost
 // nothing beside them, so that every warp runs just its own entries.
 // ---------------------------------------------------------------------------
-template <bool CPLX>
+template <bool CPLX, bool TRJ>
 __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(const DevSystem sys, const BlockLayout B,
                                                                               const BlockRun R) {
+    constexpr int NT = TRJ ? kBlockTraj - 1 : 0;
     __shared__ double s_coef[kMaxCoef];
     __shared__ double s_norm[2][2 * kBlockRows / 32];
     __shared__ double2 s_turn[2];
-    __shared__ float s_allow;
     extern __shared__ __align__(16) unsigned char smem[];
     const int T = B.threads, n = B.n, xs = n + 1;
     const size_t rec = (size_t)(2 * T > R.Mcap ? 2 * T : R.Mcap);
@@ -885,7 +925,13 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
     double *s_b = reinterpret_cast<double *>(s_mu + (size_t)(R.Kmax + 2) * B.nv);
     double *s_x = s_b + (R.Kmax + 2);                         // [buffer][part][n + 1]
     double *s_val = s_x + 4 * (size_t)xs;                     // [entry][lane], imaginary parts after
-    uint16_t *s_col = reinterpret_cast<uint16_t *>(s_val + (size_t)B.ecap * T * (CPLX ? 2 : 1));
+    [[maybe_unused]] double *s_tb = nullptr;                  // trajectories: [step][term]
+    double *s_end = s_val + (size_t)B.ecap * T * (CPLX ? 2 : 1);
+    if constexpr (TRJ) {
+        s_tb = s_end;
+        s_end += NT * (size_t)(R.Kmax + 2);
+    }
+    uint16_t *s_col = reinterpret_cast<uint16_t *>(s_end);
     const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const int part = tid >= T ? 1 : 0, t = tid - part * T;    // 0: real parts, 1: imaginary parts
     const BlockLane l = block_lane(B, t);
@@ -896,12 +942,12 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
 
     const double scale = 2.0 / S.half;
     block_coefficients(sys, R, o, s_coef);
-    const double sc = l.row < n ? scale : 1.0;
+    const double sc = l.row < n ? scale : 1.0, sign = R.adjoint ? -1.0 : 1.0;
     for (int i = 4 * part; i < l.ew; i += 8) {                // the two threads of a lane take turns
         double re[4], im[4];
         BlockLayout Bi = B;
         Bi.src = B.src + (size_t)i * T;
-        block_assemble<CPLX, 4>(sys, Bi, min(4, l.ew - i), t, s_coef, re, im);
+        block_assemble<CPLX, 4>(sys, Bi, min(4, l.ew - i), t, s_coef, sign, re, im);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             if (i + q < l.ew) {
@@ -912,7 +958,7 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
     }
     double dr = 0.0, dm = 0.0;                                // diagonal; the other part's factor
     if (l.state) {
-        const double2 d = block_diagonal(sys, B.row_src[l.row], s_coef);
+        const double2 d = block_diagonal(sys, B.row_src[l.row], s_coef, sign);
         dr = (d.x - S.cen) * scale;
         dm = (part ? d.y : -d.y) * scale;
     }
@@ -920,14 +966,20 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
         for (int k = tid; k < Kc; k += blockDim.x) s_b[k] = block_sign(k) * S.tab[k * S.ld + j];
         if (tid < 2) s_b[Kc + tid] = 0.0;
     };
-    block_phases(R, S, s_phase, s_turn, &s_allow);
+    block_phases(R, S, s_phase, s_turn);
     coefficients(M, S.K);
+    if constexpr (TRJ) {
+        for (int q = tid; q < NT * (S.K + 2); q += blockDim.x) {
+            const int k = q / NT, j = 1 + q % NT;
+            s_tb[(size_t)(j - 1) * (R.Kmax + 2) + k] = k < S.K && j < M ? block_sign(k) * S.tab[k * S.ld + j] : 0.0;
+        }
+    }
     if (tid < 4) s_x[tid * xs + n] = 0.0;                     // read by lanes without a state row
 
     double st = 0.0;
     if (l.state) {
-        const double2 *r0 = R.rho0s ? R.rho0s + (size_t)block_grid_index(R, o) * R.rho0_stride : R.rho0;
-        const double2 v = r0[R.rho0_own ? l.row : B.row_src[l.row]];
+        const double2 *r0 = R.rho0s ? R.rho0s + (size_t)block_grid_index(R, o) * R.state_stride : R.rho0;
+        const double2 v = r0[B.state_pos[l.row]];
         st = part ? v.y : v.x;
     }
     double *mu_row = reinterpret_cast<double *>(s_mu + (size_t)(l.row >= n ? l.row - n : 0) * (R.Kmax + 2)) + part;
@@ -953,15 +1005,21 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
     const uint16_t *col = s_col + t;
     for (int a = 0; a < S.nchunks; ++a) {
         const bool last = a + 1 == S.nchunks;
-        const bool advance = !last || R.state_out != nullptr;
         const int Kc = last ? min(S.K, S.kcut[S.j_last]) : S.K;
         mv += Kc - 1;
-        if (last && advance) coefficients(S.j_last, Kc);
-        else if (last && tid < 2) s_b[Kc + tid] = 0.0;
+        if (last) coefficients(S.j_last, Kc);
         if (l.state) s_x[part * xs + l.row] = st;
         __syncthreads();
         double tc = st, tp = 0.0, even = s_b[0] * st, odd = 0.0;
-        auto term = [&](int buf, int k, double &acc) {
+        [[maybe_unused]] double ie[NT + 1], io[NT + 1];
+        if constexpr (TRJ) {
+            if (l.state)
+                reinterpret_cast<double *>(
+                    R.traj_out)[2 * (((size_t)o * (nsteps + 1) + (size_t)a * M) * n + l.row) + part] = st;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) { ie[j] = s_tb[(size_t)j * (R.Kmax + 2)] * st; io[j] = 0.0; }
+        }
+        auto term = [&](int buf, int k, double &acc, double *inner) {
             const double *x = s_x + (2 * buf + part) * xs, *xo = s_x + (2 * buf + 1 - part) * xs;
             double y = fma(dr, tc, -tp);
             if (damped) y = fma(dm, xo[own], y);
@@ -995,6 +1053,10 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
                 if (k == 1) y *= 0.5;
                 s_x[(2 * (buf ^ 1) + part) * xs + l.row] = y;
                 acc = fma(s_b[k], y, acc);
+                if constexpr (TRJ) {
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) inner[j] = fma(s_tb[(size_t)j * (R.Kmax + 2) + k], y, inner[j]);
+                }
                 tp = tc;
                 tc = y;
             } else if (l.own) {
@@ -1003,33 +1065,46 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
             __syncthreads();
         };
         for (int k = 1; k <= Kc; k += 2) {
-            term(0, k, odd);
-            if (k + 1 <= Kc) term(1, k + 1, even);
+            term(0, k, odd, io);
+            if (k + 1 <= Kc) term(1, k + 1, even, ie);
         }
         // sum of the terms: even - 1i odd, then the centre's phase; the parts
         // meet in the state buffers
-        st = tc;
-        if (advance) {
+        auto join = [&](double e, double d, double2 ph) {
             if (l.state) {
-                s_x[part * xs + l.row] = even;
-                s_x[(2 + part) * xs + l.row] = odd;
+                s_x[part * xs + l.row] = e;
+                s_x[(2 + part) * xs + l.row] = d;
             }
             __syncthreads();
+            double f = 0.0;
             if (l.state) {
-                const double er = s_x[l.row], ei = s_x[xs + l.row], dr2 = s_x[2 * xs + l.row], di2 = s_x[3 * xs + l.row];
-                const double fr = er + di2, fi = ei - dr2;
-                const double2 ph = s_turn[last ? 1 : 0];
-                st = part ? fma(ph.y, fr, ph.x * fi) : fma(ph.x, fr, -ph.y * fi);
+                const double fr = s_x[l.row] + s_x[3 * xs + l.row], fi = s_x[xs + l.row] - s_x[2 * xs + l.row];
+                f = part ? fma(ph.y, fr, ph.x * fi) : fma(ph.x, fr, -ph.y * fi);
             }
+            __syncthreads();
+            return f;
+        };
+        if constexpr (TRJ) {
+            const int jn = min(M - 1, nsteps - a * M);
+#pragma unroll
+            for (int j = 1; j <= NT; ++j)
+                if (j <= jn) {
+                    const double f = join(ie[j - 1], io[j - 1], s_phase[j]);
+                    if (l.state)
+                        reinterpret_cast<double *>(
+                            R.traj_out)[2 * (((size_t)o * (nsteps + 1) + (size_t)a * M + j) * n + l.row) + part] = f;
+                }
         }
+        st = join(even, odd, s_turn[last ? 1 : 0]);
         if (B.nv > 0) block_points<double2, double>(B, R, S, S.tab, a, Kc, s_mu, s_phase, s_rec, fid_out);
         const double end_n2 = norm2(st);
         if (!isfinite(end_n2)) status = kDevNonFinite;
-        else if (end_n2 > 16.0 * start_n2 * (advance ? 1.0 : (double)s_allow) + 1e-300) status = kDevDiverged;
+        else if (end_n2 > 16.0 * start_n2 + 1e-300) status = kDevDiverged;
         if (status != kDevOk) break;
         start_n2 = end_n2;
     }
-    if (R.state_out && l.state) reinterpret_cast<double *>(R.state_out)[2 * ((size_t)o * n + l.row) + part] = st;
+    if (R.state_out && l.state)
+        reinterpret_cast<double *>(R.state_out)[2 * ((size_t)o * R.state_stride + B.state_pos[l.row]) + part] = st;
     if (tid == 0) {
         R.status[o] = status;
         R.kused[o] = S.K;

@@ -79,7 +79,8 @@ struct Cplx {
 // precision, in one device allocation.
 struct BlockPlan {
     bool ok = false;                 // false: the whole system runs (kernels.cuh)
-    int n = 0, nv = 0, maxchan = 0;
+    int n = 0, nv = 0;
+    std::vector<int> rows;           // system rows (sliced order), ascending
     struct Layout {
         spx::BlockLayout dev{};
         spx::BlockCost cost;
@@ -91,7 +92,7 @@ struct BlockPlan {
 
 // Device buffers of the kernels of block.cuh for one run.
 struct BlockBufs {
-    DevBuf<double> centre, lev_half, table, saved;
+    DevBuf<double> centre, halfwidth, lev_half, table, saved;   // halfwidth: sequences only
     DevBuf<float> tablef;
     DevBuf<unsigned long long> extent;
     DevBuf<int> lev, kcut;           // lev: steps per chunk | table rows | series lengths
@@ -132,6 +133,7 @@ struct spx_handle {
     int nchan = 1;                  // detection channels
     DevBuf<double2> d_rho0s;        // per-orientation initial states (sliced order)
     DevBuf<double2> d_seq[2], d_seq_rho;   // pulse sequences: states between segments
+    DevBuf<int> d_seq_status;              // and the statuses of every launch of one
     std::vector<std::unique_ptr<PulseOp>> pulses;   // pulse superoperators of the last sequence
     DevBuf<double> d_neg_re, d_neg_im;     // echo detection: the adjoint generator's streams
     DevBuf<double2> d_neg_diag;
@@ -231,32 +233,29 @@ void for_each_coupling(const spx_handle *h, F f) {
         }
 }
 
-// The coupled states of a run: rows whose connected component holds both a
-// coil entry and a row with start[row].  component: labels under everything
-// that moves the state (L, and the pulses of a sequence).
-void build_plan(spx_handle *h, const std::vector<int> &component, const std::vector<char> &start, BlockPlan &plan) {
-    const int n = h->n;
+// The plan for the given rows (closed under L's couplings, ascending):
+// state_pos their places in the run's state arrays (null: the system's rows),
+// detect: with detection rows for the handle's coils.
+void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<int> *state_pos, bool detect,
+                BlockPlan &plan) {
     plan.ok = false;
     plan.n = plan.nv = 0;
     plan.layouts[0].clear();
     plan.layouts[1].clear();
-    std::vector<char> seen(n, 0), live(n, 0);
-    for (int r : h->coil_row_host) seen[component[r]] = 1;
-    for (int i = 0; i < n; ++i)
-        if (start[i] && seen[component[i]]) live[component[i]] = 1;
+    plan.rows = rows;
+    if (rows.empty() || rows.size() > (size_t)spx::kBlockRows) return;
+    std::vector<int> own(h->n, -1);
+    for (size_t i = 0; i < rows.size(); ++i) own[rows[i]] = (int)i;
     spx::BlockPattern P;
-    std::vector<int> own(n, -1);
-    for (int i = 0; i < n; ++i)
-        if (live[component[i]]) { own[i] = (int)P.rows.size(); P.rows.push_back(i); }
-    P.n = (int)P.rows.size();
-    if (P.n < 1 || P.n > spx::kBlockRows) return;
+    P.rows = rows;
+    P.n = (int)rows.size();
     P.entries.resize(P.n);
     for_each_coupling(h, [&](int r, int c, int e) {
         if (own[r] >= 0) P.entries[own[r]].push_back({own[c], e});
     });
     // detection rows conj(coil): a complex coil on real values takes a row for
     // its real and one for its imaginary parts (times -1i)
-    for (int ch = 0; ch < h->nchan; ++ch)
+    for (int ch = 0; ch < (detect ? h->nchan : 0); ++ch)
         for (int im = 0; im < (h->cplx ? 1 : 2); ++im) {
             std::vector<spx::BlockPattern::Entry> row;
             for (size_t i = 0; i < h->coil_row_host.size(); ++i) {
@@ -283,6 +282,7 @@ void build_plan(spx_handle *h, const std::vector<int> &component, const std::vec
         return at;
     };
     const size_t o_rows = put(P.rows.data(), P.rows.size() * sizeof(int));
+    const size_t o_pos = state_pos ? put(state_pos->data(), state_pos->size() * sizeof(int)) : o_rows;
     const size_t o_val = put(P.values.data(), P.values.size() * sizeof(double));
     const size_t o_chan = put(P.vchan.data(), P.vchan.size() * sizeof(int));
     const size_t o_fac = put(P.vfac.data(), P.vfac.size() * sizeof(int));
@@ -342,6 +342,7 @@ void build_plan(spx_handle *h, const std::vector<int> &component, const std::vec
             b.src = reinterpret_cast<const int *>(d + at[p][i].src);
             b.col = reinterpret_cast<const uint16_t *>(d + at[p][i].col);
             b.row_src = reinterpret_cast<const int *>(d + o_rows);
+            b.state_pos = reinterpret_cast<const int *>(d + o_pos);
             b.vval = reinterpret_cast<const double2 *>(d + o_val);
             b.vchan = reinterpret_cast<const int *>(d + o_chan);
             b.vfac = reinterpret_cast<const int *>(d + o_fac);
@@ -351,14 +352,29 @@ void build_plan(spx_handle *h, const std::vector<int> &component, const std::vec
     plan.ok = true;
 }
 
+// Rows with a non-zero initial state (of any orientation).
+std::vector<char> start_rows(const spx_handle *h) {
+    if (h->n_states > 0) return h->state_rows;
+    std::vector<char> start(h->n);
+    for (int i = 0; i < h->n; ++i) start[i] = h->rho0_host[i].x != 0.0 || h->rho0_host[i].y != 0.0;
+    return start;
+}
+
+// Rows whose component (label[i]) holds both a coil entry and a start row.
+std::vector<int> live_rows(const spx_handle *h, const std::vector<int> &label, const std::vector<char> &start) {
+    std::vector<char> seen(h->n, 0), live(h->n, 0);
+    for (int r : h->coil_row_host) seen[label[r]] = 1;
+    for (int i = 0; i < h->n; ++i)
+        if (start[i] && seen[label[i]]) live[label[i]] = 1;
+    std::vector<int> rows;
+    for (int i = 0; i < h->n; ++i)
+        if (live[label[i]]) rows.push_back(i);
+    return rows;
+}
+
 // The plan of the plain acquisition for the handle's coils and initial states.
 void rebuild_plan(spx_handle *h) {
-    std::vector<char> start = h->state_rows;
-    if (h->n_states == 0) {
-        start.resize(h->n);
-        for (int i = 0; i < h->n; ++i) start[i] = h->rho0_host[i].x != 0.0 || h->rho0_host[i].y != 0.0;
-    }
-    build_plan(h, h->component, start, h->plan);
+    build_plan(h, live_rows(h, h->component, start_rows(h)), nullptr, true, h->plan);
 }
 
 void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32_t *rank,
@@ -768,6 +784,7 @@ struct Config {
     double blk_x = 0.0;
     int blk_M = 0, blk_K = 0, blk_lev = 0;
     bool blk_cplx = false;
+    int blk_which = 0;                            // the propagation kernel (spx_block_kernel_*)
     size_t blk_smem = 0;
 };
 
@@ -882,9 +899,9 @@ const void *block_kernel(bool cplx, int ecap, int which) {
     return k;
 }
 
-size_t block_smem_for(bool f64, bool cplx, int K, int M, const BlockPlan::Layout &l) {
-    return f64 ? spx::block_smem64(K, M, l.dev.nv, l.dev.threads, l.dev.ecap, l.dev.n, cplx)
-               : spx::block_smem32(K, M, l.dev.nv, l.dev.threads);
+size_t block_smem_for(bool f64, bool cplx, int K, int M, const BlockPlan::Layout &l, bool traj) {
+    return f64 ? spx::block_smem64(K, M, l.dev.nv, l.dev.threads, l.dev.ecap, l.dev.n, cplx, traj)
+               : spx::block_smem32(K, M, l.dev.nv, l.dev.threads, traj);
 }
 
 // The layout with the least modelled time for a grid.
@@ -895,39 +912,51 @@ const BlockPlan::Layout *best_layout(const std::vector<BlockPlan::Layout> &ls, d
     return best;
 }
 
-// Whether the run takes the coupled-state kernels, and how: the plan's layout
-// with the least modelled time for this grid.  c holds the whole system's
-// launch shape (so what is refused does not depend on the coupled states).
-void choose_block(spx_handle *h, const BlockPlan *plan, int64_t n_orient, double dt, int64_t nsteps,
-                  const spx_options &opt, int kmax_override, int m_cap, Config &c) {
-    const bool f64 = opt.precision == SPX_FP64;
-    const bool forced = opt.threads > 0 || opt.cluster > 0 || opt.chunk_steps > 0 || opt.chunk_target > 0;
-    if (!plan || !plan->ok || (forced && !(opt.flags & kOwnShape))) return;
-    // FP32 runs of more than 8192 undamped steps keep the whole system: there
-    // FP32 nears the 1e-5 bar and its error decides whether the run is repeated
-    // in FP64, so the decision stays the one it has been (a three-spin system,
-    // 16384 steps: 1.2e-5 on the whole system, 3.5e-6 on its coupled states)
-    if (!f64 && h->max_im_diag == 0.0 && nsteps > 8192) return;
+// How the coupled-state kernels run a plan: its layout with the least modelled
+// time for this grid, the chunk and the tables; false if they cannot.
+bool configure_block(spx_handle *h, const BlockPlan &plan, int64_t n_orient, double dt, int64_t nsteps, bool f64,
+                     double chunk_target, int kmax_override, int m_cap, bool traj, Config &c) {
+    if (!plan.ok) return false;
     const double per_sm = std::ceil((double)n_orient / h->sm_count);
-    const BlockPlan::Layout *best = best_layout(plan->layouts[f64 ? 1 : 0], per_sm);
-    if (!best) return;
-    c.blk_x = opt.chunk_target > 0 ? opt.chunk_target : 300.0;
+    const BlockPlan::Layout *best = best_layout(plan.layouts[f64 ? 1 : 0], per_sm);
+    if (!best) return false;
+    c.blk_x = chunk_target > 0 ? chunk_target : 300.0;
     const double lg = (h->g_upper > 0) ? 2.0 * h->max_im_diag / (h->g_upper / 4.0) : 0.0;
     int K = (int)host_series_terms(std::max(c.blk_x, h->g_upper * dt), std::min(lg, 0.05), c.tol) + 16;
     c.blk_K = std::min(std::max(K, kmax_override), 8192);
     // a table's columns: at most 2^18 entries a table (long series come with short chunks)
     c.blk_M = (int)std::min<int64_t>(std::min(m_cap, std::max(1, (1 << 18) / c.blk_K)), nsteps + 1);
     c.blk_lev = (int)std::max<int64_t>(4, std::min<int64_t>(spx::kBlockLevels, n_orient / 16));
-    c.blk_smem = block_smem_for(f64, h->cplx, c.blk_K, c.blk_M, *best);
-    const void *kfn = block_kernel(h->cplx, best->ecap, f64 ? 2 : 1);
+    c.blk_smem = block_smem_for(f64, h->cplx, c.blk_K, c.blk_M, *best, traj);
+    c.blk_which = (f64 ? 2 : 1) + (traj ? 2 : 0);
+    const void *kfn = block_kernel(h->cplx, best->ecap, c.blk_which);
     cudaFuncAttributes fa{};
     SPX_CUDA(cudaFuncGetAttributes(&fa, kfn));
-    if (c.blk_smem + fa.sharedSizeBytes > h->smem_optin) return;
+    if (c.blk_smem + fa.sharedSizeBytes > h->smem_optin) return false;
     SPX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(h->smem_optin - fa.sharedSizeBytes)));
     c.blk = best;
     c.blk_cplx = h->cplx;
-    c.blk_bounds = f64 ? best_layout(plan->layouts[0], per_sm) : best;
+    c.blk_bounds = f64 ? best_layout(plan.layouts[0], per_sm) : best;
+    return true;
+}
+
+bool forced_shape(const spx_options &o) {
+    return (o.threads > 0 || o.cluster > 0 || o.chunk_steps > 0 || o.chunk_target > 0) && !(o.flags & kOwnShape);
+}
+
+// Whether a powder run takes the coupled-state kernels.  c holds the whole
+// system's launch shape (so what is refused does not depend on them).
+void choose_block(spx_handle *h, const BlockPlan *plan, int64_t n_orient, double dt, int64_t nsteps,
+                  const spx_options &opt, int kmax_override, int m_cap, Config &c) {
+    const bool f64 = opt.precision == SPX_FP64;
+    if (!plan || !plan->ok || forced_shape(opt)) return;
+    // FP32 runs of more than 8192 undamped steps keep the whole system: there
+    // FP32 nears the 1e-5 bar and its error decides whether the run is repeated
+    // in FP64, so the decision stays the one it has been (a three-spin system,
+    // 16384 steps: 1.2e-5 on the whole system, 3.5e-6 on its coupled states)
+    if (!f64 && h->max_im_diag == 0.0 && nsteps > 8192) return;
+    configure_block(h, *plan, n_orient, dt, nsteps, f64, opt.chunk_target, kmax_override, m_cap, false, c);
 }
 
 // traj: the run writes the state at every step (chunks of opt.chunk_steps
@@ -1088,20 +1117,33 @@ void block_run_buffers(spx::BlockRun &r, const Config &c, double *centre, unsign
     r.tol = c.tol;
 }
 
-// Bounds, tables, propagation: three launches on `stream`.
-void launch_block(spx_handle *h, bool f64, const Config &c, spx::DevSystem &sys, spx::BlockRun &r, cudaStream_t stream) {
-    spx::BlockLayout lay = c.blk->dev, blay = c.blk_bounds->dev;
+// The three launches of a run over the coupled states: spectral bounds (of
+// every orientation), Bessel tables (for one time step) and propagation.
+void launch_bounds(spx_handle *h, const Config &c, spx::DevSystem &sys, spx::BlockRun &r, cudaStream_t stream) {
+    spx::BlockLayout lay = c.blk_bounds->dev;
     SPX_CUDA(cudaMemsetAsync(r.extent, 0, 2 * sizeof(unsigned long long), stream));
-    const dim3 grid((unsigned)r.n_orient);
-    void *bargs[] = {&sys, &blay, &r};
-    SPX_CUDA(cudaLaunchKernel(block_kernel(h->cplx, c.blk_bounds->ecap, 0), grid, dim3((unsigned)blay.threads), bargs, 0,
-                              stream));
+    void *args[] = {&sys, &lay, &r};
+    SPX_CUDA(cudaLaunchKernel(block_kernel(h->cplx, c.blk_bounds->ecap, 0), dim3((unsigned)r.n_orient),
+                              dim3((unsigned)lay.threads), args, 0, stream));
+    ++h->launches;
+}
+void launch_tables(spx_handle *h, const Config &c, spx::BlockRun &r, cudaStream_t stream) {
     spx::block_tables_kernel<<<dim3((unsigned)(c.blk_M / 32 + 1), (unsigned)c.blk_lev), 128, 0, stream>>>(r);
     SPX_CUDA(cudaGetLastError());
+    ++h->launches;
+}
+void launch_propagation(spx_handle *h, const Config &c, spx::DevSystem &sys, spx::BlockRun &r, cudaStream_t stream) {
+    spx::BlockLayout lay = c.blk->dev;
     void *args[] = {&sys, &lay, &r};
-    SPX_CUDA(cudaLaunchKernel(block_kernel(h->cplx, c.blk->ecap, f64 ? 2 : 1), grid,
+    const bool f64 = c.blk_which % 2 == 0;
+    SPX_CUDA(cudaLaunchKernel(block_kernel(h->cplx, c.blk->ecap, c.blk_which), dim3((unsigned)r.n_orient),
                               dim3((unsigned)(lay.threads * (f64 ? 2 : 1))), args, c.blk_smem, stream));
-    h->launches += 3;
+    ++h->launches;
+}
+void launch_block(spx_handle *h, const Config &c, spx::DevSystem &sys, spx::BlockRun &r, cudaStream_t stream) {
+    launch_bounds(h, c, sys, r, stream);
+    launch_tables(h, c, r, stream);
+    launch_propagation(h, c, sys, r, stream);
 }
 
 // Launch the propagation kernel (plain or cluster launch) on the handle's stream.
@@ -1150,6 +1192,60 @@ void reserve_run(spx_handle *h, int64_t n_orient, int64_t nsteps, bool f64, cons
     h->d_counter.reserve(1);
     const int ngroups = (int)((n_orient + kPowderGroup - 1) / kPowderGroup);
     h->d_part.reserve((size_t)ngroups * npts);
+}
+
+// The statistics known at launch (finish_run adds the rest).
+void describe_run(spx_handle *h, int64_t n_orient, int64_t nsteps, int32_t precision, const Config &c) {
+    h->stats = spx_stats{};
+    h->stats.n_orientations = n_orient;
+    h->stats.nsteps = nsteps;
+    h->stats.chunk_steps = c.M;
+    h->stats.threads = c.threads;
+    h->stats.precision = precision;
+    h->stats.dim = h->n;
+    h->stats.nnz = h->nnz;
+    h->stats.ell_entries = h->ell_len;
+    h->stats.value_streams = h->nstreams;
+    h->stats.real_offdiag = h->cplx ? 0 : 1;
+    h->stats.cluster = c.cl;
+    h->stats.channels = h->nchan;
+    h->stats.smem_bytes = (int32_t)c.smem;
+    h->stats.coupled_dim = c.blk ? c.blk->dev.n : 0;
+}
+
+// Weighted sum of the orientations' FIDs: deterministic FP64, fixed groups of
+// orientations in a fixed order.
+void launch_powder_sum(spx_handle *h, bool f64, const void *fids, const double *d_w, int64_t n_orient, size_t npts,
+                       double2 *part, double2 *d_out) {
+    const int group = kPowderGroup;
+    const int ngroups = (int)((n_orient + group - 1) / group);
+    const dim3 pb(256), pg((unsigned)((npts + 255) / 256), (unsigned)ngroups);
+    if (f64)
+        spx::powder_partial_kernel<double2><<<pg, pb, 0, h->stream>>>(
+            reinterpret_cast<const double2 *>(fids), d_w, (int)n_orient, (int)npts, group, part);
+    else
+        spx::powder_partial_kernel<float2><<<pg, pb, 0, h->stream>>>(
+            reinterpret_cast<const float2 *>(fids), d_w, (int)n_orient, (int)npts, group, part);
+    SPX_CUDA(cudaGetLastError());
+    spx::powder_combine_kernel<<<dim3((unsigned)((npts + 255) / 256)), dim3(256), 0, h->stream>>>(part, ngroups,
+                                                                                             (int)npts, d_out);
+    SPX_CUDA(cudaGetLastError());
+    h->launches += 2;
+}
+
+// The uploaded system as the kernels take it.
+spx::DevSystem device_system(const spx_handle *h) {
+    spx::DevSystem sys{};
+    sys.n = h->n; sys.n_pad = h->n_pad; sys.nslices = h->nslices; sys.ell_len = h->ell_len;
+    sys.slice_off = h->d_slice_off.p; sys.ell_col = h->d_ell_col.p;
+    sys.ell_re = h->d_ell_re.p; sys.ell_im = h->cplx ? h->d_ell_im.p : nullptr;
+    sys.diag = h->d_diag.p; sys.stream_coef = h->d_stream_coef.p; sys.nstreams = h->nstreams;
+    sys.ncoef = 1 + 2 * h->nterms; sys.nterms = h->nterms; sys.term_rkm = h->d_term_rkm.p;
+    sys.rho0 = h->d_rho0.p; sys.coil = h->d_coil.p; sys.max_im_diag = h->max_im_diag; sys.lo_scale = h->lo_scale;
+    sys.ncoil = h->ncoil; sys.coil_rows = h->d_coil_rows.p; sys.coil_vals = h->d_coil_vals.p;
+    sys.coil_chan = h->d_coil_chan.p; sys.nchan = h->nchan;
+    sys.rho0s = h->n_states > 0 ? h->d_rho0s.p : nullptr;
+    return sys;
 }
 
 // Initial and final states of one run when they are not the handle's own
@@ -1213,11 +1309,11 @@ int launch_fp32_check(spx_handle *h, int64_t n_orient, const double *d_al, const
         r.dt = dt; r.nsteps = (int)nsteps;
         r.lanczos_its = o64.lanczos_its > 0 ? o64.lanczos_its : 32;
         r.halfwidth = h->d_chk_halfwidth.p; r.max_im_diag = h->max_im_diag;
-        r.rho0 = sys.rho0; r.rho0s = sys.rho0s; r.rho0_stride = (size_t)h->n_pad;
+        r.rho0 = sys.rho0; r.rho0s = sys.rho0s; r.state_stride = (size_t)h->n_pad;
         r.fids = h->d_chk_fids.p; r.nchan = h->nchan;
         r.status = h->d_chk_status.p; r.kused = h->d_chk_kused.p; r.mused = h->d_chk_mused.p;
         r.matvecs = h->d_chk_matvecs.p;
-        launch_block(h, true, c, sys, r, h->check_stream);
+        launch_block(h, c, sys, r, h->check_stream);
         SPX_CUDA(cudaEventRecord(h->ev_join, h->check_stream));
         return 0;
     }
@@ -1256,16 +1352,7 @@ void launch_powder(spx_handle *h, int64_t n_orient, const double *d_al, const do
     const size_t npts = ((size_t)nsteps + 1) * h->nchan;   // the powder sum treats channels as more points
     reserve_run(h, n_orient, nsteps, f64, c);
 
-    spx::DevSystem sys{};
-    sys.n = h->n; sys.n_pad = h->n_pad; sys.nslices = h->nslices; sys.ell_len = h->ell_len;
-    sys.slice_off = h->d_slice_off.p; sys.ell_col = h->d_ell_col.p;
-    sys.ell_re = h->d_ell_re.p; sys.ell_im = h->cplx ? h->d_ell_im.p : nullptr;
-    sys.diag = h->d_diag.p; sys.stream_coef = h->d_stream_coef.p; sys.nstreams = h->nstreams;
-    sys.ncoef = 1 + 2 * h->nterms; sys.nterms = h->nterms; sys.term_rkm = h->d_term_rkm.p;
-    sys.rho0 = h->d_rho0.p; sys.coil = h->d_coil.p; sys.max_im_diag = h->max_im_diag; sys.lo_scale = h->lo_scale;
-    sys.ncoil = h->ncoil; sys.coil_rows = h->d_coil_rows.p; sys.coil_vals = h->d_coil_vals.p;
-    sys.coil_chan = h->d_coil_chan.p; sys.nchan = h->nchan;
-    sys.rho0s = h->n_states > 0 ? h->d_rho0s.p : nullptr;
+    spx::DevSystem sys = device_system(h);
     if (io.rho0) sys.rho0 = io.rho0;
     if (io.rho0s) sys.rho0s = io.rho0s;
     if (io.adjoint) {
@@ -1309,49 +1396,20 @@ void launch_powder(spx_handle *h, int64_t n_orient, const double *d_al, const do
         r.n_orient = (int)n_orient; r.alpha = d_al; r.beta = d_be; r.gamma = d_ga;
         r.dt = dt; r.nsteps = (int)nsteps; r.lanczos_its = run.lanczos_its; r.safe_bounds = safe_bounds;
         r.halfwidth = run.halfwidth; r.max_im_diag = h->max_im_diag;
-        r.rho0 = sys.rho0; r.rho0s = sys.rho0s; r.rho0_stride = (size_t)h->n_pad;
+        r.rho0 = sys.rho0; r.rho0s = sys.rho0s; r.state_stride = (size_t)h->n_pad;
         r.fids = run.fids; r.nchan = h->nchan;
         r.status = run.status; r.kused = run.kused; r.mused = run.mused; r.matvecs = run.matvecs;
-        launch_block(h, f64, c, sys, r, h->stream);
+        launch_block(h, c, sys, r, h->stream);
     } else {
         launch_chebyshev(h, f64, c, sys, run);
     }
     if (timed) SPX_CUDA(cudaEventRecord(h->ev[1], h->stream));
-    // deterministic FP64 powder sum: fixed groups of orientations, fixed order
-    const int group = kPowderGroup;
-    const int ngroups = (int)((n_orient + group - 1) / group);
-    const dim3 pb(256), pg((unsigned)((npts + 255) / 256), (unsigned)ngroups);
-    ++h->launches;  // powder partial sum
-    if (f64)
-        spx::powder_partial_kernel<double2><<<pg, pb, 0, h->stream>>>(
-            reinterpret_cast<const double2 *>(h->d_fids.p), d_w, (int)n_orient, (int)npts, group, h->d_part.p);
-    else
-        spx::powder_partial_kernel<float2><<<pg, pb, 0, h->stream>>>(
-            reinterpret_cast<const float2 *>(h->d_fids.p), d_w, (int)n_orient, (int)npts, group, h->d_part.p);
-    SPX_CUDA(cudaGetLastError());
-    ++h->launches;
-    spx::powder_combine_kernel<<<dim3((unsigned)((npts + 255) / 256)), dim3(256), 0, h->stream>>>(
-        h->d_part.p, ngroups, (int)npts, d_out);
-    SPX_CUDA(cudaGetLastError());
+    launch_powder_sum(h, f64, h->d_fids.p, d_w, n_orient, npts, h->d_part.p, d_out);
     if (chk) SPX_CUDA(cudaStreamWaitEvent(h->stream, h->ev_join, 0));   // the FP64 re-run is part of the run
     if (timed) SPX_CUDA(cudaEventRecord(h->ev[2], h->stream));
     h->stats_timed = timed;
 
-    h->stats = spx_stats{};
-    h->stats.n_orientations = n_orient;
-    h->stats.nsteps = nsteps;
-    h->stats.chunk_steps = c.M;
-    h->stats.threads = c.threads;
-    h->stats.precision = opt.precision;
-    h->stats.dim = h->n;
-    h->stats.nnz = h->nnz;
-    h->stats.ell_entries = h->ell_len;
-    h->stats.value_streams = h->nstreams;
-    h->stats.real_offdiag = h->cplx ? 0 : 1;
-    h->stats.cluster = c.cl;
-    h->stats.channels = h->nchan;
-    h->stats.smem_bytes = (int32_t)c.smem;
-    h->stats.coupled_dim = c.blk ? c.blk->dev.n : 0;
+    describe_run(h, n_orient, nsteps, opt.precision, c);
     h->stats_pending = true;
     h->last_norient = n_orient;
     h->chk_pending = chk;
@@ -1631,6 +1689,410 @@ void upload_grid(spx_handle *h, int64_t n_orient, const double *alphas, const do
     SPX_CUDA(cudaMemcpyAsync(g + 3 * n_orient, weights, b, cudaMemcpyHostToDevice, h->stream));
 }
 
+// ---------------------------------------------------------------------------
+// Pulse sequences on the coupled states: the rows that L and the pulses
+// connect to both the coil and the initial state, in an order of their own
+// (state arrays of n entries), propagated one set of L-connected rows at a
+// time.  A hard pulse is one sparse product with its exponential.
+// ---------------------------------------------------------------------------
+struct HostCsr {
+    std::vector<int> ptr, col;
+    std::vector<double2> val;
+};
+struct SparseOp {
+    DevBuf<int> ptr, col;
+    DevBuf<double2> val;
+    void upload(const HostCsr &m, cudaStream_t s) {
+        ptr.upload(m.ptr, s);
+        col.upload(m.col.empty() ? std::vector<int>{0} : m.col, s);
+        val.upload(m.val.empty() ? std::vector<double2>{make_double2(0, 0)} : m.val, s);
+        SPX_CUDA(cudaStreamSynchronize(s));           // pageable sources
+    }
+};
+
+double2 cmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+
+constexpr int kPulseBlock = 64;        // largest set of states that a pulse operator couples here
+
+// exp(-1i theta P) of a pulse operator given as rows, one connected set of
+// states at a time (a spin's rotation couples a few): scaling and squaring of
+// the Taylor series, 1/2^s scaled to a 1-norm of at most one half.  Entries at
+// or below 1e-15 are rounding residues of the rotation and are dropped.
+// False if a set is larger than kPulseBlock.
+bool pulse_exponential(const std::vector<std::vector<std::pair<int, double2>>> &rows, double theta, HostCsr &out) {
+    const int n = (int)rows.size();
+    spx::Components comp(n);
+    for (int i = 0; i < n; ++i)
+        for (auto &e : rows[i]) comp.join(i, e.first);
+    std::vector<std::vector<int>> sets(n);
+    for (int i = 0; i < n; ++i) sets[comp.find(i)].push_back(i);
+    std::vector<std::vector<std::pair<int, double2>>> res(n);
+    std::vector<int> at(n, -1);
+    for (auto &set : sets) {
+        const int m = (int)set.size();
+        if (m == 0) continue;
+        if (m > kPulseBlock) return false;
+        for (int q = 0; q < m; ++q) at[set[q]] = q;
+        std::vector<double2> A((size_t)m * m, make_double2(0, 0)), X(A), T(A), Y(A);
+        for (int q = 0; q < m; ++q)
+            for (auto &e : rows[set[q]]) {            // -1i theta P
+                double2 &a = A[(size_t)q * m + at[e.first]];
+                a.x += theta * e.second.y;
+                a.y -= theta * e.second.x;
+            }
+        double norm = 0.0;
+        for (int c = 0; c < m; ++c) {
+            double sum = 0.0;
+            for (int r = 0; r < m; ++r) sum += std::hypot(A[(size_t)r * m + c].x, A[(size_t)r * m + c].y);
+            norm = std::max(norm, sum);
+        }
+        int sq = 0;
+        while (norm > 0.5) { norm *= 0.5; ++sq; }
+        const double f = std::ldexp(1.0, -sq);
+        for (auto &a : A) { a.x *= f; a.y *= f; }
+        auto product = [&](const std::vector<double2> &a, const std::vector<double2> &b, std::vector<double2> &c) {
+            for (int r = 0; r < m; ++r)
+                for (int q = 0; q < m; ++q) {
+                    double2 sum = make_double2(0, 0);
+                    for (int k = 0; k < m; ++k) {
+                        const double2 v = cmul(a[(size_t)r * m + k], b[(size_t)k * m + q]);
+                        sum.x += v.x;
+                        sum.y += v.y;
+                    }
+                    c[(size_t)r * m + q] = sum;
+                }
+        };
+        for (int q = 0; q < m; ++q) X[(size_t)q * m + q] = T[(size_t)q * m + q] = make_double2(1, 0);
+        for (int k = 1; k <= 18; ++k) {               // 0.5^19 / 19! < 1e-22
+            product(T, A, Y);
+            for (size_t e = 0; e < Y.size(); ++e) {
+                T[e] = make_double2(Y[e].x / k, Y[e].y / k);
+                X[e].x += T[e].x;
+                X[e].y += T[e].y;
+            }
+        }
+        for (int q = 0; q < sq; ++q) { product(X, X, Y); X.swap(Y); }
+        for (int r = 0; r < m; ++r)
+            for (int c = 0; c < m; ++c) {
+                const double2 v = X[(size_t)r * m + c];
+                if (std::fabs(v.x) > 1e-15 || std::fabs(v.y) > 1e-15) res[set[r]].push_back({set[c], v});
+            }
+    }
+    out = HostCsr{};
+    out.ptr.assign(n + 1, 0);
+    for (int i = 0; i < n; ++i) {
+        for (auto &e : res[i]) { out.col.push_back(e.first); out.val.push_back(e.second); }
+        out.ptr[i + 1] = (int)out.col.size();
+    }
+    return true;
+}
+
+// y = M x for n_states states of n entries each.
+__global__ void sparse_states_kernel(int64_t n_states, int n, const int *__restrict__ ptr, const int *__restrict__ col,
+                                     const double2 *__restrict__ val, const double2 *__restrict__ x, double2 *y) {
+    const int64_t total = n_states * n;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t o = q / n;
+        const int i = (int)(q - o * n);
+        double re = 0.0, im = 0.0;
+        for (int e = ptr[i]; e < ptr[i + 1]; ++e) {
+            const double2 a = val[e], b = x[o * n + col[e]];
+            re = fma(a.x, b.x, fma(-a.y, b.y, re));
+            im = fma(a.x, b.y, fma(a.y, b.x, im));
+        }
+        y[q] = make_double2(re, im);
+    }
+}
+
+// out[o][i] = in[o][rows[i]], states of n_in entries.
+__global__ void gather_states_kernel(int64_t n_states, int n, int n_in, const int *__restrict__ rows,
+                                     const double2 *__restrict__ in, double2 *out) {
+    const int64_t total = n_states * n;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t o = q / n;
+        out[q] = in[o * n_in + rows[q - o * n]];
+    }
+}
+
+unsigned state_blocks(const spx_handle *h, int64_t items) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((items + 255) / 256, (int64_t)h->sm_count * 16));
+}
+
+// The rows a sequence moves, and its pulse operators on them.
+struct CoupledSequence {
+    std::vector<int> rows, at;       // system rows; a row's place among them, or -1
+    std::vector<std::vector<std::vector<std::pair<int, double2>>>> pulses;
+    int n() const { return (int)rows.size(); }
+
+    // Restrict the sequence to the rows that L and the pulses connect.
+    CoupledSequence(spx_handle *h, const std::vector<const spx_csc *> &ops) {
+        spx::Components comp(h->n);
+        for (int i = 0; i < h->n; ++i) comp.join(i, h->component[i]);
+        for (const spx_csc *P : ops) {
+            check_csc(P, h->n, "pulse_op");
+            for_each_entry(P, [&](int64_t r, int64_t c, Cplx v) {
+                if (v.re != 0.0 || v.im != 0.0) comp.join(h->row_of[r], h->row_of[c]);
+            });
+        }
+        std::vector<int> label(h->n);
+        for (int i = 0; i < h->n; ++i) label[i] = comp.find(i);
+        rows = live_rows(h, label, start_rows(h));
+        at.assign(h->n, -1);
+        for (size_t i = 0; i < rows.size(); ++i) at[rows[i]] = (int)i;
+        for (const spx_csc *P : ops) {
+            pulses.emplace_back(rows.size());
+            for_each_entry(P, [&](int64_t r, int64_t c, Cplx v) {
+                const int i = at[h->row_of[r]], j = at[h->row_of[c]];
+                if (i >= 0 && j >= 0 && (v.re != 0.0 || v.im != 0.0)) pulses.back()[i].push_back({j, make_double2(v.re, v.im)});
+            });
+        }
+    }
+    // places of all rows of the L-components that hold one of these places
+    std::vector<char> closure(const spx_handle *h, const std::vector<char> &places) const {
+        std::vector<char> hit(h->n, 0), out(rows.size(), 0);
+        for (size_t i = 0; i < rows.size(); ++i)
+            if (places[i]) hit[h->component[rows[i]]] = 1;
+        for (size_t i = 0; i < rows.size(); ++i) out[i] = hit[h->component[rows[i]]];
+        return out;
+    }
+    std::vector<char> coil_places(const spx_handle *h) const {
+        std::vector<char> p(rows.size(), 0);
+        for (int r : h->coil_row_host)
+            if (at[r] >= 0) p[at[r]] = 1;
+        return closure(h, p);
+    }
+    void plan(spx_handle *h, const std::vector<char> &places, bool detect, BlockPlan &out) const {
+        std::vector<int> r, pos;
+        for (size_t i = 0; i < rows.size(); ++i)
+            if (places[i]) { r.push_back(rows[i]); pos.push_back((int)i); }
+        build_plan(h, r, &pos, detect, out);
+    }
+};
+
+// One set of rows of a sequence with its bounds and tables.
+struct SequenceGroup {
+    BlockPlan plan;
+    BlockBufs bufs;
+    Config c;
+    double table_dt = 0.0;           // time step of the tables held (0: none)
+    bool bounded = false;
+};
+
+// Propagates a group over nsteps steps of dt: bounds on the first call, tables
+// whenever the time step changes (they hold for any step count).
+void run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockRun r, int64_t n_orient,
+               const double *const (&angles)[3], double dt, int64_t nsteps, double tol, bool f64, bool traj, int *status, double *halfwidth) {
+    if (!g.bounded || g.table_dt != dt) {
+        Config c = g.c;
+        c.tol = tol;
+        if (!configure_block(h, g.plan, n_orient, dt, (int64_t)1 << 28, f64, 0.0, 0, traj ? spx::kBlockTraj : 256, traj, c))
+            throw SpxError(SPX_ERR_INTERNAL, "a coupled set of states lost its layout");
+        g.c = c;
+        reserve_block(g.bufs, n_orient, f64, c);
+    }
+    const Config &c = g.c;
+    BlockBufs &b = g.bufs;
+    block_run_buffers(r, c, b.centre.p, b.extent.p, b.lev_half.p, b.lev.p, b.kcut.p, b.table.p, f64 ? nullptr : b.tablef.p);
+    if (saves_block(n_orient, f64, c)) r.saved = b.saved.p;
+    r.n_orient = (int)n_orient; r.alpha = angles[0]; r.beta = angles[1]; r.gamma = angles[2];
+    r.dt = dt; r.lanczos_its = 32;
+    r.max_im_diag = h->max_im_diag; r.halfwidth = halfwidth;
+    r.nchan = 1; r.status = status;
+    r.kused = h->d_kused.p; r.mused = h->d_mused.p; r.matvecs = h->d_matvecs.p;
+    if (!g.bounded) launch_bounds(h, c, sys, r, h->stream);
+    g.bounded = true;
+    if (g.table_dt != dt) {
+        r.nsteps = 1 << 28;                  // chunks as long as the tables allow
+        launch_tables(h, c, r, h->stream);
+        g.table_dt = dt;
+    }
+    r.nsteps = (int)nsteps;
+    launch_propagation(h, c, sys, r, h->stream);
+}
+
+// Statuses of a sequence's launches (after a synchronisation).
+void check_statuses(spx_handle *h, int64_t n_orient, int64_t launches) {
+    std::vector<int> st((size_t)(n_orient * launches));
+    SPX_CUDA(cudaMemcpy(st.data(), h->d_seq_status.p, st.size() * sizeof(int), cudaMemcpyDeviceToHost));
+    for (size_t q = 0; q < st.size(); ++q)
+        if (st[q] != spx::kDevOk)
+            throw SpxError(SPX_ERR_SERIES, "a segment failed its series checks (status " + std::to_string(st[q]) +
+                                               ", orientation #" + std::to_string(q % n_orient) + ")");
+}
+
+// The run on the coupled states, or false if they do not qualify (the caller
+// then runs the whole system).  Arguments are validated and the grid is on the
+// device; total: recorded points.
+bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<const spx_csc *> &pulse_ops,
+                          const std::vector<spx_seq_op> &ops, const spx_options &o, int64_t total, double *fid,
+                          double *fids_per_orient) {
+    if (forced_shape(o)) return false;
+    CoupledSequence seq(h, pulse_ops);
+    const int n = seq.n();
+    if (n == 0) return false;
+    int last_evolve = -1;
+    int64_t evolves = 0, max_steps = 0;
+    for (size_t i = 0; i < ops.size(); ++i)
+        if (ops[i].kind == SPX_SEQ_EVOLVE) {
+            last_evolve = (int)i;
+            ++evolves;
+            max_steps = std::max(max_steps, ops[i].nsteps);
+        }
+    if (last_evolve < 0) return false;
+    // sets of rows: the coil's components together, every other large
+    // component alone, the small ones together
+    std::vector<std::unique_ptr<SequenceGroup>> groups;
+    const std::vector<char> coil = seq.coil_places(h);
+    {
+        std::vector<std::vector<int>> comps(h->n);
+        for (int i = 0; i < n; ++i)
+            if (!coil[i]) comps[h->component[seq.rows[i]]].push_back(i);
+        std::vector<char> small(n, 0);
+        int count = 0;
+        auto flush = [&](std::vector<char> &places) {
+            groups.push_back(std::make_unique<SequenceGroup>());
+            seq.plan(h, places, false, groups.back()->plan);
+            std::fill(places.begin(), places.end(), 0);
+        };
+        for (auto &c : comps) {
+            if (c.empty()) continue;
+            if (c.size() > 24) {
+                std::vector<char> one(n, 0);
+                for (int i : c) one[i] = 1;
+                flush(one);
+                continue;
+            }
+            if (count + (int)c.size() > spx::kBlockRows) { flush(small); count = 0; }
+            for (int i : c) small[i] = 1;
+            count += (int)c.size();
+        }
+        if (count) flush(small);
+        groups.push_back(std::make_unique<SequenceGroup>());      // the coil's last
+        seq.plan(h, coil, true, groups.back()->plan);
+    }
+    for (auto &g : groups)
+        if (!g->plan.ok) return false;
+    // the pulses' exponentials
+    std::map<std::pair<int, double>, std::unique_ptr<SparseOp>> turns;
+    for (auto &q : ops)
+        if (q.kind == SPX_SEQ_PULSE && !turns.count({q.pulse, q.angle})) {
+            HostCsr m;
+            if (!pulse_exponential(seq.pulses[q.pulse], q.angle, m)) return false;
+            auto op = std::make_unique<SparseOp>();
+            op->upload(m, h->stream);
+            turns[{q.pulse, q.angle}] = std::move(op);
+        }
+    const bool f64 = o.precision == SPX_FP64;
+    const size_t vec = f64 ? sizeof(double2) : sizeof(float2);
+    const double *g = h->d_grid.p;
+    const double *const angles[3] = {g, g + n_orient, g + 2 * n_orient};
+    const size_t ns = (size_t)n_orient * n;
+    const bool own_states = h->n_states > 0;
+    h->d_seq[0].reserve(ns);
+    h->d_seq[1].reserve(ns);
+    h->d_seq_rho.reserve(2 * (size_t)n);
+    h->d_fid.reserve((size_t)std::max<int64_t>(total, 1));
+    h->d_fids.reserve((size_t)(max_steps + 1) * n_orient * vec);
+    h->d_part.reserve((size_t)((n_orient + kPowderGroup - 1) / kPowderGroup) * (max_steps + 1));
+    h->d_status.reserve(n_orient);
+    h->d_kused.reserve(n_orient);
+    h->d_mused.reserve(n_orient);
+    h->d_matvecs.reserve(n_orient);
+    h->d_halfwidth.reserve(n_orient);
+    h->d_seq_status.reserve((size_t)(n_orient * evolves * (int64_t)groups.size()));
+    spx::DevSystem sys = device_system(h);
+    DevBuf<int> drows;
+    int cur = 0, rcur = 0;
+    bool per_orient = own_states;
+    if (own_states) {
+        drows.upload(seq.rows, h->stream);
+        ++h->launches;
+        gather_states_kernel<<<state_blocks(h, ns), 256, 0, h->stream>>>(n_orient, n, h->n_pad, drows.p, h->d_rho0s.p,
+                                                                          h->d_seq[0].p);
+        SPX_CUDA(cudaGetLastError());
+    } else {
+        std::vector<double2> r0(n);
+        for (int i = 0; i < n; ++i) r0[i] = h->rho0_host[seq.rows[i]];
+        SPX_CUDA(cudaMemcpyAsync(h->d_seq_rho.p, r0.data(), n * sizeof(double2), cudaMemcpyHostToDevice, h->stream));
+        SPX_CUDA(cudaStreamSynchronize(h->stream));
+    }
+    Config whole{};
+    int64_t at = 0, launched = 0;
+    SPX_CUDA(cudaEventRecord(h->ev[0], h->stream));
+    for (size_t i = 0; i < ops.size(); ++i) {
+        const spx_seq_op &q = ops[i];
+        if (q.kind == SPX_SEQ_PULSE) {
+            const SparseOp &op = *turns[{q.pulse, q.angle}];
+            double2 *x = per_orient ? h->d_seq[cur].p : h->d_seq_rho.p + (size_t)rcur * n;
+            double2 *y = per_orient ? h->d_seq[cur ^ 1].p : h->d_seq_rho.p + (size_t)(rcur ^ 1) * n;
+            const int64_t cnt = per_orient ? n_orient : 1;
+            ++h->launches;
+            sparse_states_kernel<<<state_blocks(h, cnt * n), 256, 0, h->stream>>>(cnt, n, op.ptr.p, op.col.p, op.val.p, x, y);
+            SPX_CUDA(cudaGetLastError());
+            if (per_orient) cur ^= 1; else rcur ^= 1;
+            continue;
+        }
+        // the whole system's configuration: what it refuses stays refused
+        whole = choose_config(h, n_orient, q.dt, q.nsteps, o, 0);
+        const bool last = (int)i == last_evolve;
+        for (size_t k = 0; k < groups.size(); ++k) {
+            const bool detects = k + 1 == groups.size();
+            if (last && !detects) continue;                        // nothing after it reads these states
+            spx::BlockRun r{};
+            if (per_orient) r.rho0s = h->d_seq[cur].p;
+            else r.rho0 = h->d_seq_rho.p + (size_t)rcur * n;
+            r.state_stride = (size_t)n;
+            r.state_out = last ? nullptr : h->d_seq[cur ^ 1].p;
+            r.fids = h->d_fids.p;
+            int *status = last ? h->d_status.p : h->d_seq_status.p + (size_t)(launched++) * n_orient;
+            SequenceGroup &grp = *groups[k];
+            double *half = h->d_halfwidth.p;
+            if (!detects) {
+                grp.bufs.halfwidth.reserve(n_orient);
+                half = grp.bufs.halfwidth.p;
+            }
+            run_group(h, grp, sys, r, n_orient, angles, q.dt, q.nsteps, whole.tol, f64, false, status, half);
+        }
+        if (q.record) {
+            const size_t np = (size_t)q.nsteps + 1;
+            launch_powder_sum(h, f64, h->d_fids.p, g + 3 * n_orient, n_orient, np, h->d_part.p, h->d_fid.p + at);
+            if (fids_per_orient) {
+                // this segment's FIDs of every orientation, into each orientation's row
+                std::vector<unsigned char> tmp(np * (size_t)n_orient * vec);
+                SPX_CUDA(cudaMemcpyAsync(tmp.data(), h->d_fids.p, tmp.size(), cudaMemcpyDeviceToHost, h->stream));
+                SPX_CUDA(cudaStreamSynchronize(h->stream));
+                for (int64_t w = 0; w < n_orient; ++w)
+                    for (size_t j = 0; j < np; ++j) {
+                        const size_t e = (size_t)w * np + j;
+                        double2 v;
+                        if (f64) v = reinterpret_cast<const double2 *>(tmp.data())[e];
+                        else {
+                            const float2 f = reinterpret_cast<const float2 *>(tmp.data())[e];
+                            v = make_double2(f.x, f.y);
+                        }
+                        fids_per_orient[2 * ((size_t)w * total + at + j)] = v.x;
+                        fids_per_orient[2 * ((size_t)w * total + at + j) + 1] = v.y;
+                    }
+            }
+            at += (int64_t)np;
+        }
+        cur ^= 1;
+        per_orient = true;
+    }
+    SPX_CUDA(cudaEventRecord(h->ev[1], h->stream));
+    SPX_CUDA(cudaEventRecord(h->ev[2], h->stream));
+    h->stats_timed = true;
+    whole.blk = groups.back()->c.blk;
+    describe_run(h, n_orient, ops[last_evolve].nsteps, o.precision, whole);
+    h->stats_pending = true;
+    h->last_norient = n_orient;
+    h->chk_pending = 0;
+    finish_run(h);
+    if (launched) check_statuses(h, n_orient, launched);
+    if (total > 0) SPX_CUDA(cudaMemcpy(fid, h->d_fid.p, (size_t)total * sizeof(double2), cudaMemcpyDeviceToHost));
+    return true;
+}
+
 void run_sequence(spx_handle *h, int64_t n_orient, const double *alphas, const double *betas, const double *gammas,
                   const double *weights, int32_t n_pulse, const spx_csc *pulse_ops, int32_t n_ops,
                   const spx_seq_op *ops, const spx_options &o, double *fid, double *fids_per_orient = nullptr) {
@@ -1654,12 +2116,19 @@ void run_sequence(spx_handle *h, int64_t n_orient, const double *alphas, const d
         }
     }
     if (n_orient < 1) throw SpxError(SPX_ERR_INVALID_ARGUMENT, "bad orientation count");
+    {
+        std::vector<const spx_csc *> list;
+        for (int k = 0; k < n_pulse; ++k) list.push_back(&pulse_ops[k]);
+        upload_grid(h, n_orient, alphas, betas, gammas, weights);
+        if (run_coupled_sequence(h, n_orient, list, std::vector<spx_seq_op>(ops, ops + n_ops), o, total, fid,
+                                 fids_per_orient))
+            return;
+    }
     h->pulses.clear();
     for (int k = 0; k < n_pulse; ++k) {
         h->pulses.push_back(std::make_unique<PulseOp>());
         upload_pulse(h, &pulse_ops[k], *h->pulses.back());
     }
-    upload_grid(h, n_orient, alphas, betas, gammas, weights);
     double *g = h->d_grid.p;
     const size_t ns = (size_t)n_orient * h->n_pad;
     h->d_seq[0].reserve(ns);
@@ -1956,6 +2425,235 @@ void echo_outputs(spx_handle *h, int64_t n_orient, int64_t npoints, double scale
     }
 }
 
+// out[o][j] = sum_i conj(v[o][j'][i]) (Pi u[o][j])[i], one warp per (o, j), with
+// j' = j, or the last point minus j when reverse; Pi has v's rows and u's columns.
+template <class Vec>
+__global__ void coupled_echo_kernel(int n_orient, int npoints, int nu, int nv, const int *__restrict__ ptr,
+                                    const int *__restrict__ col, const double2 *__restrict__ val,
+                                    const Vec *__restrict__ u, const Vec *__restrict__ v, int reverse, double2 *out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = (int64_t)n_orient * npoints;
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nw;
+         w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        const int64_t wv = reverse ? w - 2 * (w % npoints) + npoints - 1 : w;
+        const Vec *uu = u + w * nu, *vv = v + wv * nv;
+        double re = 0.0, im = 0.0;
+        for (int i = lane; i < nv; i += 32) {
+            double wr = 0.0, wi = 0.0;
+            for (int e = ptr[i]; e < ptr[i + 1]; ++e) {
+                const double2 a = val[e];
+                const Vec b = uu[col[e]];
+                wr = fma(a.x, (double)b.x, fma(-a.y, (double)b.y, wr));
+                wi = fma(a.x, (double)b.y, fma(a.y, (double)b.x, wi));
+            }
+            const Vec c = vv[i];                 // conj(c) * w
+            re = fma((double)c.x, wr, fma((double)c.y, wi, re));
+            im = fma((double)c.x, wi, fma(-(double)c.y, wr, im));
+        }
+#pragma unroll
+        for (int q = 16; q; q >>= 1) {
+            re += __shfl_xor_sync(0xffffffffu, re, q);
+            im += __shfl_xor_sync(0xffffffffu, im, q);
+        }
+        if (lane == 0) out[w] = make_double2(re, im);
+    }
+}
+
+// M x on the host.
+std::vector<double2> apply_host(const HostCsr &m, const std::vector<double2> &x) {
+    std::vector<double2> y(x.size(), make_double2(0, 0));
+    for (size_t i = 0; i < x.size(); ++i)
+        for (int e = m.ptr[i]; e < m.ptr[i + 1]; ++e) {
+            const double2 v = cmul(m.val[e], x[m.col[e]]);
+            y[i].x += v.x;
+            y[i].y += v.y;
+        }
+    return y;
+}
+
+// The echo core (echo_trajectories) on the coupled states: the adjoint
+// trajectory lives on the coil's rows (or those that `back`, a pulse on the
+// adjoint state after nsteps steps, leads to), the forward one on the rows
+// that the echo pulse connects to them.  out_back: DEER's first adjoint run.
+// False if the states do not qualify.
+bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const spx_csc *> &ops, double first_angle,
+                      const double *back_angle, int echo_op, double tau, int64_t nsteps, const spx_options &o,
+                      bool reverse) {
+    if (forced_shape(o)) return false;
+    CoupledSequence seq(h, ops);
+    const int n = seq.n();
+    if (n == 0) return false;
+    HostCsr first, echo, back;
+    if (!pulse_exponential(seq.pulses[0], first_angle, first) || !pulse_exponential(seq.pulses[echo_op], M_PI, echo)) return false;
+    if (back_angle && !pulse_exponential(seq.pulses[0], *back_angle, back)) return false;
+    std::vector<double2> rho(n), coil(n, make_double2(0, 0));
+    for (int i = 0; i < n; ++i) rho[i] = h->rho0_host[seq.rows[i]];
+    rho = apply_host(first, rho);
+    for (size_t i = 0; i < h->coil_row_host.size(); ++i)
+        if (seq.at[h->coil_row_host[i]] >= 0) coil[seq.at[h->coil_row_host[i]]] = h->coil_val_host[i];
+    // the places a matrix's rows read, and those whose rows read the given places
+    auto reads = [&](const HostCsr &m, const std::vector<char> &rows) {
+        std::vector<char> p(n, 0);
+        for (int i = 0; i < n; ++i)
+            if (rows[i])
+                for (int e = m.ptr[i]; e < m.ptr[i + 1]; ++e) p[m.col[e]] = 1;
+        return p;
+    };
+    const std::vector<char> at_coil = seq.coil_places(h);
+    std::vector<char> vp = at_coil;
+    if (back_angle) {
+        std::vector<char> p(n, 0);
+        for (int i = 0; i < n; ++i)
+            for (int e = back.ptr[i]; e < back.ptr[i + 1]; ++e) p[i] |= at_coil[back.col[e]];
+        vp = seq.closure(h, p);
+    }
+    std::vector<char> excited(n, 0);
+    for (int i = 0; i < n; ++i) excited[i] = rho[i].x != 0.0 || rho[i].y != 0.0;
+    excited = seq.closure(h, excited);
+    std::vector<char> up = seq.closure(h, reads(echo, vp));
+    for (int i = 0; i < n; ++i) up[i] = up[i] && excited[i];
+    SequenceGroup gu, gv, gb;
+    seq.plan(h, up, false, gu.plan);
+    seq.plan(h, vp, false, gv.plan);
+    if (back_angle) seq.plan(h, at_coil, false, gb.plan);
+    if (!gu.plan.ok || !gv.plan.ok || (back_angle && !gb.plan.ok)) return false;
+    const int nu = gu.plan.n, nv = gv.plan.n;
+    HostCsr form;                                   // echo's rows of v and columns of u
+    {
+        std::vector<int> own(n, -1);
+        int q = 0;
+        for (int i = 0; i < n; ++i)
+            if (up[i]) own[i] = q++;
+        form.ptr.push_back(0);
+        for (int i = 0; i < n; ++i) {
+            if (!vp[i]) continue;
+            for (int e = echo.ptr[i]; e < echo.ptr[i + 1]; ++e)
+                if (own[echo.col[e]] >= 0) { form.col.push_back(own[echo.col[e]]); form.val.push_back(echo.val[e]); }
+            form.ptr.push_back((int)form.col.size());
+        }
+    }
+    SparseOp dform, dback;
+    dform.upload(form, h->stream);
+    const bool f64 = o.precision == SPX_FP64;
+    const size_t vec = f64 ? sizeof(double2) : sizeof(float2);
+    const int64_t npoints = nsteps + 1;
+    const double *g = h->d_grid.p;
+    h->d_seq_rho.reserve(2 * (size_t)n);
+    SPX_CUDA(cudaMemcpyAsync(h->d_seq_rho.p, rho.data(), n * sizeof(double2), cudaMemcpyHostToDevice, h->stream));
+    SPX_CUDA(cudaMemcpyAsync(h->d_seq_rho.p + n, coil.data(), n * sizeof(double2), cudaMemcpyHostToDevice, h->stream));
+    SPX_CUDA(cudaStreamSynchronize(h->stream));
+    spx::DevSystem sys = device_system(h);
+    h->d_status.reserve(n_orient);
+    h->d_kused.reserve(n_orient);
+    h->d_mused.reserve(n_orient);
+    h->d_matvecs.reserve(n_orient);
+    h->d_halfwidth.reserve(n_orient);
+    h->d_echo_f.reserve((size_t)n_orient * npoints);
+    h->d_fid.reserve((size_t)npoints);
+    h->d_part.reserve((size_t)((n_orient + kPowderGroup - 1) / kPowderGroup) * npoints);
+    h->d_seq_status.reserve(3 * (size_t)n_orient);
+    SPX_CUDA(cudaEventRecord(h->ev[0], h->stream));
+    const double2 *adj = h->d_seq_rho.p + n;
+    bool adj_each = false;
+    int *status[3];
+    for (int q = 0; q < 3; ++q) status[q] = h->d_seq_status.p + (size_t)q * n_orient;
+    if (back_angle) {
+        const Config whole = choose_config(h, n_orient, tau, nsteps, o, 0);     // refusals of the whole system
+        const size_t ns = (size_t)n_orient * n;
+        h->d_seq[0].reserve(ns);
+        h->d_seq[1].reserve(ns);
+        SPX_CUDA(cudaMemsetAsync(h->d_seq[0].p, 0, ns * sizeof(double2), h->stream));
+        spx::BlockRun r{};
+        r.adjoint = 1;
+        r.rho0 = adj;
+        r.state_stride = (size_t)n;
+        r.state_out = h->d_seq[0].p;
+        const double *const angles[3] = {g, g + n_orient, g + 2 * n_orient};
+        gb.bufs.halfwidth.reserve(n_orient);
+        run_group(h, gb, sys, r, n_orient, angles, tau, nsteps, whole.tol, f64, false, status[2], gb.bufs.halfwidth.p);
+        dback.upload(back, h->stream);
+        ++h->launches;
+        sparse_states_kernel<<<state_blocks(h, ns), 256, 0, h->stream>>>(n_orient, n, dback.ptr.p, dback.col.p, dback.val.p,
+                                                                          h->d_seq[0].p, h->d_seq[1].p);
+        SPX_CUDA(cudaGetLastError());
+        adj = h->d_seq[1].p;
+        adj_each = true;
+    }
+    // orientations in batches whose two trajectories take a quarter of the free
+    // device memory, at most 48 GB
+    size_t free_b = 0, total_b = 0;
+    SPX_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t held = (h->d_traj[0].n + h->d_traj[1].n) * sizeof(double2);
+    const size_t budget = std::min<size_t>((free_b + held) / 4, 48ull << 30);
+    const int64_t batch = std::max<int64_t>(
+        1, std::min<int64_t>(n_orient, (int64_t)(budget / ((size_t)npoints * (nu + nv) * vec))));
+    auto traj = [&](int which, int rows) {
+        h->d_traj[which].reserve(((size_t)batch * npoints * rows * vec + sizeof(double2) - 1) / sizeof(double2));
+        return (void *)h->d_traj[which].p;
+    };
+    void *tu = traj(0, nu), *tv = traj(1, nv);
+    Config whole{};
+    for (int64_t b0 = 0; b0 < n_orient; b0 += batch) {
+        const int64_t nb = std::min(batch, n_orient - b0);
+        bool have = false;
+        for (int m : {kTrajChunk, 2, 1}) {          // the whole system's configuration: its refusals stand
+            spx_options o1 = o;
+            o1.chunk_steps = m;
+            try {
+                whole = choose_config(h, nb, tau, nsteps, o1, 0, 256, true);
+                have = true;
+                break;
+            } catch (const SpxError &e) {
+                if (e.code != SPX_ERR_UNSUPPORTED) throw;
+            }
+        }
+        if (!have) throw SpxError(SPX_ERR_UNSUPPORTED, "the trajectory does not fit a cluster of 8 SMs");
+        const double *const angles[3] = {g + b0, g + n_orient + b0, g + 2 * n_orient + b0};
+        for (int dir = 0; dir < 2; ++dir) {
+            SequenceGroup &grp = dir ? gv : gu;
+            grp.bounded = false;
+            grp.table_dt = 0.0;
+            grp.bufs.halfwidth.reserve(nb);
+            spx::BlockRun r{};
+            r.adjoint = dir;
+            r.state_stride = (size_t)n;
+            if (dir == 0) r.rho0 = h->d_seq_rho.p;
+            else if (adj_each) r.rho0s = adj + (size_t)b0 * n;
+            else r.rho0 = adj;
+            r.traj_out = dir ? tv : tu;
+            const bool final = dir == 1;
+            run_group(h, grp, sys, r, nb, angles, tau, nsteps, whole.tol, f64, true, status[dir] + b0,
+                      final ? h->d_halfwidth.p + b0 : grp.bufs.halfwidth.p);
+        }
+        const int64_t warps = nb * npoints;
+        const int blocks = (int)std::min<int64_t>((warps + 7) / 8, (int64_t)h->sm_count * 16);
+        ++h->launches;
+        if (f64)
+            coupled_echo_kernel<double2><<<blocks, 256, 0, h->stream>>>(
+                (int)nb, (int)npoints, nu, nv, dform.ptr.p, dform.col.p, dform.val.p, (const double2 *)tu,
+                (const double2 *)tv, reverse ? 1 : 0, h->d_echo_f.p + b0 * npoints);
+        else
+            coupled_echo_kernel<float2><<<blocks, 256, 0, h->stream>>>(
+                (int)nb, (int)npoints, nu, nv, dform.ptr.p, dform.col.p, dform.val.p, (const float2 *)tu,
+                (const float2 *)tv, reverse ? 1 : 0, h->d_echo_f.p + b0 * npoints);
+        SPX_CUDA(cudaGetLastError());
+    }
+    launch_powder_sum(h, true, h->d_echo_f.p, g + 3 * n_orient, n_orient, (size_t)npoints, h->d_part.p, h->d_fid.p);
+    SPX_CUDA(cudaEventRecord(h->ev[1], h->stream));
+    SPX_CUDA(cudaEventRecord(h->ev[2], h->stream));
+    SPX_CUDA(cudaMemcpyAsync(h->d_status.p, status[1], n_orient * sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
+    h->stats_timed = true;
+    whole.blk = gv.c.blk;
+    describe_run(h, n_orient, nsteps, o.precision, whole);
+    h->stats_pending = true;
+    h->last_norient = n_orient;
+    h->chk_pending = 0;
+    finish_run(h);
+    if (!back_angle) SPX_CUDA(cudaMemset(status[2], 0, n_orient * sizeof(int)));
+    check_statuses(h, n_orient, 3);
+    return true;
+}
+
 // first_angle: pi/2 for eseem.m, pi/4 for oopeseem.m (the out-of-phase echo).
 void run_eseem(spx_handle *h, int64_t n_orient, const double *alphas, const double *betas, const double *gammas,
                const double *weights, double timestep, int64_t npoints, const spx_csc *pulse_op,
@@ -1967,11 +2665,15 @@ void run_eseem(spx_handle *h, int64_t n_orient, const double *alphas, const doub
     const int64_t nsteps = npoints - 1;
     validate_run(h, n_orient, tau, nsteps);
     if (h->n_pad > 8192) throw SpxError(SPX_ERR_UNSUPPORTED, "echo detection is limited to dimension 8192");
+    upload_grid(h, n_orient, alphas, betas, gammas, weights);
+    if (run_coupled_echo(h, n_orient, {pulse_op}, first_angle, nullptr, 0, tau, nsteps, o, false)) {
+        echo_outputs(h, n_orient, npoints, 1.0, fid, fids_per_orient);
+        return;
+    }
     h->pulses.clear();
     h->pulses.push_back(std::make_unique<PulseOp>());
     upload_pulse(h, pulse_op, *h->pulses.back());
     const PulseOp &P = *h->pulses.back();
-    upload_grid(h, n_orient, alphas, betas, gammas, weights);
     // rho1 = exp(-1i first_angle P) rho0
     h->d_seq_rho.reserve(h->n_pad);
     SPX_CUDA(cudaMemcpyAsync(h->d_seq_rho.p, h->d_rho0.p, h->n_pad * sizeof(double2), cudaMemcpyDeviceToDevice,
@@ -2000,13 +2702,21 @@ void run_deer(spx_handle *h, int64_t n_orient, const double *alphas, const doubl
     validate_run(h, n_orient, stepsize, nsteps);
     const int n_pad = h->n_pad;
     if (n_pad > 8192) throw SpxError(SPX_ERR_UNSUPPORTED, "echo detection is limited to dimension 8192");
+    upload_grid(h, n_orient, alphas, betas, gammas, weights);
+    const double back = -M_PI;
+    if (run_coupled_echo(h, n_orient, {ex_prob, ex_pump}, M_PI / 2, &back, 1, stepsize, nsteps, o, true)) {
+        double nrm = 0.0;
+        for (const double2 &v : h->coil_val_host) nrm += v.x * v.x + v.y * v.y;
+        if (!(nrm > 0.0)) throw SpxError(SPX_ERR_INVALID_ARGUMENT, "the probe coil is zero");
+        echo_outputs(h, n_orient, nsteps + 1, 1.0 / std::sqrt(nrm), fid, fids_per_orient);
+        return;
+    }
     h->pulses.clear();
     for (const spx_csc *q : {ex_prob, ex_pump}) {
         h->pulses.push_back(std::make_unique<PulseOp>());
         upload_pulse(h, q, *h->pulses.back());
     }
     const PulseOp &prob = *h->pulses[0], &pump = *h->pulses[1];
-    upload_grid(h, n_orient, alphas, betas, gammas, weights);
     const double *g = h->d_grid.p;
     h->d_seq_rho.reserve(n_pad);
     SPX_CUDA(cudaMemcpyAsync(h->d_seq_rho.p, h->d_rho0.p, n_pad * sizeof(double2), cudaMemcpyDeviceToDevice,
@@ -2279,16 +2989,7 @@ void run_powder_noalloc(spx_handle *h, int64_t n_orient, const double *d_al, con
                                                 " (use spx_run_powder_device for larger runs)");
     unsigned char *base = static_cast<unsigned char *>(noalloc_scratch(h->device));
     int *flag = reinterpret_cast<int *>(base + offs[7]);
-    spx::DevSystem sys{};
-    sys.n = h->n; sys.n_pad = h->n_pad; sys.nslices = h->nslices; sys.ell_len = h->ell_len;
-    sys.slice_off = h->d_slice_off.p; sys.ell_col = h->d_ell_col.p;
-    sys.ell_re = h->d_ell_re.p; sys.ell_im = h->cplx ? h->d_ell_im.p : nullptr;
-    sys.diag = h->d_diag.p; sys.stream_coef = h->d_stream_coef.p; sys.nstreams = h->nstreams;
-    sys.ncoef = 1 + 2 * h->nterms; sys.nterms = h->nterms; sys.term_rkm = h->d_term_rkm.p;
-    sys.rho0 = h->d_rho0.p; sys.coil = h->d_coil.p; sys.max_im_diag = h->max_im_diag; sys.lo_scale = h->lo_scale;
-    sys.ncoil = h->ncoil; sys.coil_rows = h->d_coil_rows.p; sys.coil_vals = h->d_coil_vals.p;
-    sys.coil_chan = h->d_coil_chan.p; sys.nchan = h->nchan;
-    sys.rho0s = h->n_states > 0 ? h->d_rho0s.p : nullptr;
+    spx::DevSystem sys = device_system(h);
     spx::DevRun run{};
     run.n_orient = (int)n_orient; run.alpha = d_al; run.beta = d_be; run.gamma = d_ga;
     run.dt = dt; run.nsteps = (int)nsteps; run.M = c.M; run.Kmax = c.Kmax; run.tol = c.tol;
@@ -2318,26 +3019,14 @@ void run_powder_noalloc(spx_handle *h, int64_t n_orient, const double *d_al, con
         r.n_orient = run.n_orient; r.alpha = d_al; r.beta = d_be; r.gamma = d_ga;
         r.dt = dt; r.nsteps = (int)nsteps; r.lanczos_its = run.lanczos_its;
         r.halfwidth = run.halfwidth; r.max_im_diag = h->max_im_diag;
-        r.rho0 = sys.rho0; r.rho0s = sys.rho0s; r.rho0_stride = (size_t)h->n_pad;
+        r.rho0 = sys.rho0; r.rho0s = sys.rho0s; r.state_stride = (size_t)h->n_pad;
         r.fids = run.fids; r.nchan = h->nchan;
         r.status = run.status; r.kused = run.kused; r.mused = run.mused; r.matvecs = run.matvecs;
-        launch_block(h, f64, c, sys, r, h->stream);
+        launch_block(h, c, sys, r, h->stream);
     } else {
         launch_chebyshev(h, f64, c, sys, run);
     }
-    const dim3 pb(256), pg((unsigned)((npts + 255) / 256), (unsigned)ngroups);
-    ++h->launches;  // powder partial sum
-    if (f64)
-        spx::powder_partial_kernel<double2><<<pg, pb, 0, h->stream>>>(
-            reinterpret_cast<const double2 *>(run.fids), d_w, (int)n_orient, (int)npts, group, part);
-    else
-        spx::powder_partial_kernel<float2><<<pg, pb, 0, h->stream>>>(
-            reinterpret_cast<const float2 *>(run.fids), d_w, (int)n_orient, (int)npts, group, part);
-    SPX_CUDA(cudaGetLastError());
-    ++h->launches;
-    spx::powder_combine_kernel<<<dim3((unsigned)((npts + 255) / 256)), dim3(256), 0, h->stream>>>(
-        part, ngroups, (int)npts, reinterpret_cast<double2 *>(d_fid));
-    SPX_CUDA(cudaGetLastError());
+    launch_powder_sum(h, f64, run.fids, d_w, n_orient, npts, part, reinterpret_cast<double2 *>(d_fid));
     ++h->launches;
     status_any_kernel<<<dim3(64), dim3(256), 0, h->stream>>>(run.status, (int)n_orient, flag);
     SPX_CUDA(cudaGetLastError());
@@ -2885,7 +3574,7 @@ spx_status spx_batch_create(spx_batch **out, int32_t n, spx_handle *const *handl
                 if (cfg[i].blk) {
                     SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(handles[i]->cplx, cfg[i].blk_bounds->ecap, 0)));
                     SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(handles[i]->cplx, cfg[i].blk->ecap,
-                                                                     os[i].precision == SPX_FP64 ? 2 : 1)));
+                                                                     cfg[i].blk_which)));
                     continue;
                 }
                 SPX_CUDA(cudaFuncGetAttributes(&fa, select_kernel(os[i].precision == SPX_FP64, handles[i]->cplx,
