@@ -11,7 +11,7 @@ SOURCES = [os.path.join(HERE, 'csrc', f) for f in
            [f'kern_{p}_{c}{t}.cu' for p in ('f32r', 'f32c', 'f64r', 'f64c') for c in ('sc', 'dc') for t in ('', '_t')] +
            ['kern_block_r.cu', 'kern_block_c.cu']]
 DEPS = SOURCES + [os.path.join(HERE, 'csrc', 'kernels.cuh'), os.path.join(HERE, 'csrc', 'builder.h'), os.path.join(HERE, 'csrc', 'kern_inst.inc'),
-                  os.path.join(HERE, 'csrc', 'block.cuh'), os.path.join(HERE, 'csrc', 'block_plan.h'),
+                  os.path.join(HERE, 'csrc', 'block.cuh'), os.path.join(HERE, 'csrc', 'block_plan.h'), os.path.join(HERE, 'csrc', 'dense.cuh'),
                   os.path.join(HERE, 'csrc', 'kern_block.inc'),
                   os.path.join(ROOT, 'include', 'spinach_gpu.h')]
 LIB = os.path.join(HERE, 'lib', 'libspinach_gpu.so')

@@ -223,15 +223,81 @@ static __device__ __forceinline__ int block_grid_index(const BlockRun &R, int o)
 // Rotational coefficients of the run's orientation o into coef (all threads call).
 static __device__ __forceinline__ void block_coefficients(const DevSystem &sys, const BlockRun &R, int o, double *coef) {
     o = block_grid_index(R, o);
-    for (int t = threadIdx.x; t < sys.nterms; t += blockDim.x) {
-        double re, im;
-        wigner_element(sys.term_rkm[3 * t], sys.term_rkm[3 * t + 1], sys.term_rkm[3 * t + 2], R.alpha[o], R.beta[o],
-                       R.gamma[o], re, im);
-        coef[1 + 2 * t] = re;
-        coef[2 + 2 * t] = im;
+    wigner_coefficients(sys, R.alpha[o], R.beta[o], R.gamma[o], coef);
+}
+
+// Extreme eigenvalues (low, high) of the tridiagonal matrix (al, be), by one
+// warp: lanes 0-15 bracket the lowest, lanes 16-31 the highest, each round
+// counting the eigenvalues below 16 interior points (Sturm sequences) and
+// shrinking its bracket 17-fold, to 1e-6 of its size.  The counts stay right to
+// the division's rounding; the interval is widened by far more afterwards.
+static __device__ __forceinline__ double2 tridiag_ends(const float *al, const float *be, int m, int lane) {
+    float a = CUDART_INF_F, b = -CUDART_INF_F;
+    for (int i = lane; i < m; i += 32) {
+        const float r = (i > 0 ? fabsf(be[i - 1]) : 0.f) + (i < m - 1 ? fabsf(be[i]) : 0.f);
+        a = fminf(a, al[i] - r);
+        b = fmaxf(b, al[i] + r);
     }
-    if (threadIdx.x == 0) coef[0] = 1.0;
-    __syncthreads();
+#pragma unroll
+    for (int q = 16; q; q >>= 1) {
+        a = fminf(a, __shfl_xor_sync(0xffffffffu, a, q));
+        b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, q));
+    }
+    const bool high = lane >= 16;
+    const int target = high ? m : 1;                             // count >= target: right of the wanted one
+    for (int it = 0; it < 8; ++it) {
+        const float step = (b - a) * (1.f / 17.f), x = a + (float)((lane & 15) + 1) * step;
+        int cnt = 0;
+        float q = al[0] - x;
+        cnt += q < 0.f;
+        for (int i = 1; i < m; ++i) {
+            const float e = be[i - 1];
+            q = al[i] - x - __fdividef(e * e, q == 0.f ? 1e-30f : q);
+            cnt += q < 0.f;
+        }
+        const unsigned mask = (__ballot_sync(0xffffffffu, cnt >= target) >> (high ? 16 : 0)) & 0xffffu;
+        const int j = mask ? __ffs(mask) - 1 : 16;
+        b = mask ? a + (float)(j + 1) * step : b;
+        a = a + (float)j * step;
+        const bool done = !(b - a > 1e-6f * fmaxf(fabsf(a), fabsf(b)) + 1e-30f);
+        if (__all_sync(0xffffffffu, done)) break;
+    }
+    // the outer end of each bracket
+    return make_double2((double)__shfl_sync(0xffffffffu, a, 0), (double)__shfl_sync(0xffffffffu, b, 31));
+}
+
+// |last component| of the tridiagonal matrix's unit eigenvector at theta, by
+// two steps of inverse iteration (one thread; w: work arrays).
+static __device__ float ritz_last(const float *al, const float *be, int m, float theta, float (*w)[kMaxLanczos]) {
+    if (m <= 1) return 1.f;
+    float *y = w[0], *c = w[1], *d = w[2];
+    const float shift = theta + 1e-5f * (fabsf(theta) + 1e-30f);
+    for (int i = 0; i < m; ++i) y[i] = 1.f;
+    for (int it = 0; it < 2; ++it) {
+        float den = al[0] - shift, cp, dp;                       // (T - shift) x = y
+        den = den == 0.f ? 1e-30f : den;
+        cp = c[0] = __fdividef(be[0], den);
+        dp = d[0] = __fdividef(y[0], den);
+        for (int i = 1; i < m; ++i) {
+            const float e = be[i - 1];
+            den = al[i] - shift - e * cp;
+            den = den == 0.f ? 1e-30f : den;
+            const float inv = __fdividef(1.f, den);
+            cp = c[i] = i < m - 1 ? be[i] * inv : 0.f;
+            dp = d[i] = (y[i] - e * dp) * inv;
+        }
+        float x = dp, nrm = x * x;
+        y[m - 1] = x;
+        for (int i = m - 2; i >= 0; --i) {
+            x = d[i] - c[i] * x;
+            y[i] = x;
+            nrm += x * x;
+        }
+        if (!(nrm > 0.f) || !isfinite(nrm)) return 1.f;
+        const float inv = rsqrtf(nrm);
+        for (int i = 0; i < m; ++i) y[i] *= inv;
+    }
+    return fabsf(y[m - 1]);
 }
 
 // ---------------------------------------------------------------------------
@@ -243,32 +309,40 @@ static __device__ __forceinline__ void block_coefficients(const DevSystem &sys, 
 // runs on the same layout.
 // ---------------------------------------------------------------------------
 template <bool CPLX, int ECAP>
-__global__ void __launch_bounds__(kBlockRows, 1) block_bounds_kernel(const DevSystem sys, const BlockLayout B,
+__global__ void __launch_bounds__(kBlockRows, ECAP <= 16 ? 2 : 1) block_bounds_kernel(const DevSystem sys, const BlockLayout B,
                                                                      const BlockRun R) {
     __shared__ double s_coef[kMaxCoef];
     __shared__ float2 s_x[2][kBlockRows + 1];
     __shared__ float2 s_part[2][kBlockRows / 32];
-    __shared__ double s_al[kMaxLanczos], s_be[kMaxLanczos];
+    __shared__ float s_al[kMaxLanczos], s_be[kMaxLanczos];
+    __shared__ float s_work[2][3][kMaxLanczos];
     const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const BlockLane l = block_lane(B, tid);
     block_coefficients(sys, R, o, s_coef);
     BlockEntries<CPLX, ECAP> E;
     double2 dg = make_double2(0.0, 0.0);
     {
-        double re[ECAP], im[ECAP];
         const double sign = R.adjoint ? -1.0 : 1.0;
-        block_assemble<CPLX, ECAP>(sys, B, l.ew, tid, s_coef, sign, re, im);
-        if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef, sign);
         double *save = R.saved ? R.saved + (size_t)o * block_saved(B.ecap, B.threads, CPLX) : nullptr;
+        // four entries at a time: more FP64 sums in registers cost resident CTAs
 #pragma unroll
-        for (int i = 0; i < ECAP; ++i) {
-            E.set(i, re[i], im[i]);
-            E.col[i] = i < l.ew ? B.col[i * B.threads + tid] * (int)sizeof(float2) : 0;
-            if (save && i < l.ew) {
-                save[(size_t)i * B.threads + tid] = re[i];
-                if (CPLX) save[(size_t)(B.ecap + i) * B.threads + tid] = im[i];
+        for (int i0 = 0; i0 < ECAP; i0 += 4) {
+            double re[4], im[4];
+            BlockLayout Bi = B;
+            Bi.src = B.src + (size_t)i0 * B.threads;
+            block_assemble<CPLX, 4>(sys, Bi, l.ew - i0, tid, s_coef, sign, re, im);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int i = i0 + q;
+                E.set(i, re[q], im[q]);
+                E.col[i] = i < l.ew ? B.col[i * B.threads + tid] * (int)sizeof(float2) : 0;
+                if (save && i < l.ew) {
+                    save[(size_t)i * B.threads + tid] = re[q];
+                    if (CPLX) save[(size_t)(B.ecap + i) * B.threads + tid] = im[q];
+                }
             }
         }
+        if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef, sign);
         if (save) {
             double *sd = save + (size_t)(CPLX ? 2 : 1) * B.ecap * B.threads;
             sd[tid] = dg.x;
@@ -349,7 +423,7 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_bounds_kernel(const DevSy
         // beta from the residual itself: |w|^2 - alpha^2 would hide directions
         // that the start vector holds little of
         const float beta = sqrtf(reduce(make_float2(y.x * y.x + y.y * y.y, 0.f), 0).x);
-        if (tid == 0) { s_al[j] = (double)alpha; s_be[j] = (double)beta; }
+        if (tid == 0) { s_al[j] = alpha; s_be[j] = beta; }
         m_eff = j + 1;
         if (!(beta > 1e-12f * (fabsf(alpha) + 1e-30f))) break;      // invariant subspace
         const float inv = 1.f / beta;
@@ -360,11 +434,11 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_bounds_kernel(const DevSy
     }
     __syncthreads();
     if (tid < 32) {
-        double tlo, thi;
-        tridiag_extremes_warp(s_al, s_be, m_eff, tlo, thi, lane);
-        const double bl = fabs(s_be[m_eff - 1]);
-        double rr = 0.0;
-        if (!R.safe_bounds && lane < 2) rr = bl * ritz_last_component(s_al, s_be, m_eff, lane == 0 ? thi : tlo);
+        const double2 ends = tridiag_ends(s_al, s_be, m_eff, lane);
+        const double tlo = ends.x, thi = ends.y;
+        float rr = 0.f;                                          // lane 0 the top, lane 1 the bottom
+        if (!R.safe_bounds && lane < 2)
+            rr = fabsf(s_be[m_eff - 1]) * ritz_last(s_al, s_be, m_eff, lane == 0 ? (float)thi : (float)tlo, s_work[lane]);
         const double rhi = __shfl_sync(0xffffffffu, rr, 0), rlo = __shfl_sync(0xffffffffu, rr, 1);
         if (lane == 0) {
             double hi = gmax, lo = gmin;
@@ -400,69 +474,57 @@ static __device__ __noinline__ double ladder_half(const unsigned long long *exte
     return lev == 0 ? hmax : hmax * exp(-lev * step);
 }
 
-// Column j of a table (bessel_column of kernels.cuh in two passes: the
-// recurrence stores unnormalised values, then eight at a time are scaled, so
-// that their loads overlap), also rounded to float; returns the terms the
-// column needs: the last one above tol (with the growth e^{k lg} that Im L
-// allows), plus two.
-static __device__ int block_column(double *tab, float *tf, int M, int j, int K, double half, double dt, double lg,
-                                   double tol) {
+// Column j of a table by Miller's backward recurrence (bessel_column of
+// kernels.cuh), unnormalised; returns the factor that normalises it and the
+// number of terms that are not zero (kn).
+static __device__ double block_column(double *tab, int M, int j, int K, double half, double dt, int &kn) {
     const size_t ld = (size_t)(M + 1);
     double *col = tab + j;
     const double x = half * j * dt;
-    double inv = 1.0;
-    int kn = min(K, 3);                               // terms that are not zero
+    kn = min(K, 3);
     if (x < 1e-6) {
-        // twice the leading terms, scaled as below
+        // half the leading terms (every term but the first is doubled later)
         col[0] = 1.0 - 0.25 * x * x;
         if (K > 1) col[ld] = 0.5 * x;
         if (K > 2) col[2 * ld] = 0.125 * x * x;
-    } else {
-        kn = min(K, series_terms(x, 0.0, 1e-40, K + 64) + 1);
-        const int base = max(kn, (int)ceil(x));
-        int kst = base + 20 + (int)sqrtf(160.f * base);
-        kst += kst & 1;
-        const double two_over_x = 2.0 / x;
-        const float ftx = (float)two_over_x;
-        float fjp1 = 0.f, fjk = 1e-30f;
-        int k = kst;
-        for (; k > kn; --k) {
-            const float fjm1 = ((float)k * ftx) * fjk - fjp1;
-            fjp1 = fjk;
-            fjk = fjm1;
-            if (fabsf(fjk) > 1e20f) { fjk *= 1e-20f; fjp1 *= 1e-20f; }
-        }
-        double jp1 = fjp1, jk = fjk, even = 0.0;
-        for (; k >= 1; --k) {
-            const double jm1 = (k * two_over_x) * jk - jp1;
-            jp1 = jk;
-            jk = jm1;                                 // J_{k-1}, unnormalised
-            if (k > 1 && (k & 1)) even += jk;
-            col[(size_t)(k - 1) * ld] = jk;
-        }
-        inv = 1.0 / (2.0 * even + jk);                // J_0 + 2 sum J_2k = 1
+        return 1.0;
     }
-    int last = 2;
-    const double two = 2.0 * inv;
-    for (int k0 = 0; k0 < K; k0 += 8) {
-        double v[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = k0 + q < kn ? col[(size_t)(k0 + q) * ld] : 0.0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int k = k0 + q;
-            if (k < K) {
-                v[q] *= k == 0 ? inv : two;
-                col[(size_t)k * ld] = v[q];
-                if (tf) tf[(size_t)k * ld + j] = (float)v[q];
-            }
-        }
+    kn = min(K, series_terms(x, 0.0, 1e-40, K + 64) + 1);
+    const int base = max(kn, (int)ceil(x));
+    int kst = base + 20 + (int)sqrtf(160.f * base);
+    kst += kst & 1;
+    const double two_over_x = 2.0 / x;
+    const float ftx = (float)two_over_x;
+    float fjp1 = 0.f, fjk = 1e-30f;
+    int k = kst;
+    for (; k > kn; --k) {
+        const float fjm1 = ((float)k * ftx) * fjk - fjp1;
+        fjp1 = fjk;
+        fjk = fjm1;
+        if (fabsf(fjk) > 1e20f) { fjk *= 1e-20f; fjp1 *= 1e-20f; }
     }
-    double grow = exp((kn - 1) * lg);
-    const double shrink = exp(-lg);
-    for (int k = kn - 1; k >= 2; --k, grow *= shrink)
-        if (!(fabs(col[(size_t)k * ld]) * grow <= tol)) { last = k + 1; break; }
-    return min(last + 2, K);
+    // an FP64 instruction takes a warp 64 cycles: one conversion and product
+    // for two terms, and only even orders enter the norm
+    double jp1 = fjp1, jk = fjk, even = 0.0;
+    if (k & 1) {                                      // an odd number of terms: one alone first
+        const double jm1 = (k * two_over_x) * jk - jp1;
+        jp1 = jk;
+        jk = jm1;
+        --k;
+        if (k > 0) even += jk;
+        col[(size_t)k * ld] = jk;
+    }
+    for (; k >= 2; k -= 2) {
+        const double f = k * two_over_x;
+        const double a = f * jk - jp1;                // J_{k-1}
+        const double b = (f - two_over_x) * a - jk;   // J_{k-2}
+        col[(size_t)(k - 1) * ld] = a;
+        col[(size_t)(k - 2) * ld] = b;
+        if (k > 2) even += b;
+        jp1 = a;
+        jk = b;
+    }
+    return 1.0 / (2.0 * even + jk);                   // J_0 + 2 sum J_2k = 1
 }
 
 static __global__ void __launch_bounds__(128) block_tables_kernel(const BlockRun R) {
@@ -496,13 +558,53 @@ static __global__ void __launch_bounds__(128) block_tables_kernel(const BlockRun
         }
     }
     __syncthreads();
-    const int j = blockIdx.x * 32 + tid;
-    if (!used || tid >= 32 || j > M) return;
+    if (!used || blockIdx.x * 32 > M) return;
+    __shared__ double s_inv[32];
+    __shared__ int s_kn[32];
+    const int lane = tid & 31, warp = tid >> 5, j = blockIdx.x * 32 + lane;
     const int K = s_k;
+    const size_t ld = (size_t)(M + 1);
     double *tab = R.table + (size_t)lev * R.Kmax * (R.Mcap + 1);
     float *tf = R.tablef ? R.tablef + (size_t)lev * R.Kmax * (R.Mcap + 1) : nullptr;
-    const int kl = block_column(tab, tf, M, j, K, half, R.dt, lg, R.tol);
-    R.kcut[(size_t)lev * (R.Mcap + 1) + j] = kl;
+    // one warp runs the columns' recurrences; all four scale and round them,
+    // eight values of a column in flight
+    if (warp == 0 && j <= M) s_inv[lane] = block_column(tab, M, j, K, half, R.dt, s_kn[lane]);
+    __syncthreads();
+    if (j > M) return;
+    const double inv = s_inv[lane], two = 2.0 * inv;
+    const int kn = s_kn[lane];
+    for (int k0 = 8 * warp; k0 < K; k0 += 32) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = k0 + q < kn ? tab[(size_t)(k0 + q) * ld + j] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int k = k0 + q;
+            if (k < K) {
+                v[q] *= k == 0 ? inv : two;
+                tab[(size_t)k * ld + j] = v[q];
+                if (tf) tf[(size_t)k * ld + j] = (float)v[q];
+            }
+        }
+    }
+    __syncthreads();
+    if (warp != 0) return;
+    // terms the column needs: the last one above the tolerance (with the growth
+    // e^{k lg} that Im L allows), plus two
+    int last = 2;
+    double grow = exp((kn - 1) * lg);
+    const double shrink = exp(-lg);
+    for (int k0 = kn - 1; k0 >= 2 && last == 2; k0 -= 8) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = k0 - q >= 2 ? tab[(size_t)(k0 - q) * ld + j] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if (last == 2 && k0 - q >= 2 && !(fabs(v[q]) * grow <= R.tol)) last = k0 - q + 1;
+            if (lg > 0.0) grow *= shrink;
+        }
+    }
+    R.kcut[(size_t)lev * (R.Mcap + 1) + j] = min(last + 2, K);
 }
 
 // Dynamic shared memory of the propagation kernels.

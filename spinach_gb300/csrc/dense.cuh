@@ -1,0 +1,209 @@
+// FP64 propagation of few coupled states, or of few orientations, by dense
+// matrices instead of series terms.
+//
+// An FP64 series term is a chain of instructions that hold a warp for 64
+// cycles each, and a run of N steps takes thousands of terms one after another
+// on one SM.  Here the N steps take about log2(N) dependent products: the
+// one-step propagator U = exp(-1i L dt) from scaling, a degree-16 Taylor
+// polynomial (six products, Paterson and Stockmeyer, SIAM J. Comput. 2 (1973)
+// 60) and squaring, then its powers U^2, U^4, ... by squaring, the states
+// U^j rho0 (j < m) and the detection rows coil' U^(a m) by doubling their
+// number with each power, and every FID point as one product of a row and a
+// state.  Each product is spread over the whole GPU, all orientations
+// together.  The launcher (engine.cu) takes this path where its FP64 work or
+// its latency is the smaller one.
+//
+// Matrices are stored transposed (S[c * n + r] = U(r, c)), so that a state's
+// rows are neighbours.  The kernels are bound by FP64 instructions; they keep
+// to 40 registers in CTAs of 64 threads, which fit beside the FP32
+// propagation they run along with.
+#pragma once
+
+#include "kernels.cuh"
+
+namespace spx {
+
+constexpr int kDenseThreads = 64;
+
+struct DenseSystem {
+    int n;                      // coupled states
+    int nent;                   // off-diagonal entries
+    const int *ent;             // [nent] column * n + row
+    const int *src;             // [nent] ELL entry of the system
+    const int *row_src;         // [n] row of the system (sliced order)
+};
+
+static __device__ __forceinline__ int dense_grid_index(int pick, int n_orient, int o) {
+    return pick ? (int)(((2 * (long long)o + 1) * pick) / (2 * (long long)n_orient)) : o;
+}
+
+// A = -1i L h (transposed) of every orientation, one CTA each; also the first
+// state and detection rows, and the orientation's status words.
+struct DenseStart {
+    int n_orient, pick;
+    const double *alpha, *beta, *gamma;
+    double h;
+    double2 *A;                 // [o][n][n]
+    const double2 *rho0, *rho0s;
+    size_t state_stride;
+    double2 *V;                 // [o][m][n]
+    int m;
+    double2 *Y;                 // [o][nchan][rows][n]
+    int nchan, rows;
+    int ncoil;                  // coil entries: coupled row, channel, value
+    const int *coil_row, *coil_chan;
+    const double2 *coil_val;
+    int *status, *kused, *mused;
+    long long *matvecs;
+    double *halfwidth;
+    double bound;               // what halfwidth reports: a bound on |L|
+    long long products;
+};
+static __global__ void __launch_bounds__(kDenseThreads) dense_start_kernel(const DevSystem sys, const DenseSystem D,
+                                                                           const DenseStart R) {
+    __shared__ double coef[kMaxCoef];
+    const int o = blockIdx.x, tid = threadIdx.x, n = D.n;
+    const int g = dense_grid_index(R.pick, R.n_orient, o);
+    wigner_coefficients(sys, R.alpha[g], R.beta[g], R.gamma[g], coef);
+    double2 *A = R.A + (size_t)o * n * n;
+    for (int e = tid; e < n * n; e += blockDim.x) A[e] = make_double2(0.0, 0.0);
+    double2 *Y = R.Y + (size_t)o * R.nchan * R.rows * n;
+    for (int e = tid; e < R.nchan * n; e += blockDim.x) Y[(size_t)(e / n) * R.rows * n + e % n] = make_double2(0.0, 0.0);
+    __syncthreads();
+    for (int e = tid; e < D.nent; e += blockDim.x) {
+        double re = 0.0, im = 0.0;
+        for (int s = 0; s < sys.nstreams; ++s) {
+            const double c = coef[sys.stream_coef[s]];
+            re = fma(c, sys.ell_re[(size_t)s * sys.ell_len + D.src[e]], re);
+            if (sys.ell_im) im = fma(c, sys.ell_im[(size_t)s * sys.ell_len + D.src[e]], im);
+        }
+        A[D.ent[e]] = make_double2(im * R.h, -re * R.h);
+    }
+    for (int i = tid; i < n; i += blockDim.x) {
+        double re = 0.0, im = 0.0;
+        for (int s = 0; s < sys.nstreams; ++s) {
+            const double c = coef[sys.stream_coef[s]];
+            const double2 d = sys.diag[(size_t)s * sys.n_pad + D.row_src[i]];
+            re = fma(c, d.x, re);
+            im = fma(c, d.y, im);
+        }
+        A[(size_t)i * n + i] = make_double2(im * R.h, -re * R.h);
+        const double2 *r0 = R.rho0s ? R.rho0s + (size_t)g * R.state_stride : R.rho0;
+        R.V[(size_t)o * R.m * n + i] = r0[D.row_src[i]];
+    }
+    if (tid == 0) {
+        for (int q = 0; q < R.ncoil; ++q) {
+            const double2 v = R.coil_val[q];
+            double2 &y = Y[(size_t)R.coil_chan[q] * R.rows * n + R.coil_row[q]];
+            y = make_double2(y.x + v.x, y.y - v.y);                  // conj(coil)
+        }
+        R.status[o] = kDevOk;
+        R.kused[o] = 16;
+        R.mused[o] = R.m;
+        R.matvecs[o] = R.products * n;
+        R.halfwidth[o] = R.bound;
+    }
+}
+
+static __device__ __forceinline__ void dense_mac(double2 &s, const double2 a, const double2 b) {
+    s.x = fma(a.x, b.x, s.x);
+    s.y = fma(a.x, b.y, s.y);
+    s.x = fma(-a.y, b.y, s.x);
+    s.y = fma(a.y, b.x, s.y);
+}
+
+// C = A B (+ c0 + c1 M1 + c2 M2 + c3 M3 when M1), one element per thread.
+struct DenseSum {
+    const double2 *M1, *M2, *M3;
+    double c0, c1, c2, c3;
+};
+static __device__ __forceinline__ double2 dense_sum(const DenseSum &t, size_t at, bool diagonal, double2 s) {
+    const double2 a = t.M1[at], b = t.M2[at], c = t.M3[at];
+    s.x += (diagonal ? t.c0 : 0.0) + t.c1 * a.x + t.c2 * b.x + t.c3 * c.x;
+    s.y += t.c1 * a.y + t.c2 * b.y + t.c3 * c.y;
+    return s;
+}
+static __global__ void __launch_bounds__(kDenseThreads, 24) dense_product_kernel(int64_t total, int n,
+                                                                                 const double2 *__restrict__ A,
+                                                                                 const double2 *__restrict__ B,
+                                                                                 double2 *__restrict__ C, const DenseSum t) {
+    const int n2 = n * n;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t o = q / n2;
+        const int e = (int)(q - o * n2), r = e / n, c = e - r * n;
+        const double2 *a = A + o * n2 + (size_t)r * n, *b = B + o * n2 + c;
+        double2 s = make_double2(0.0, 0.0);
+        int k = 0;
+        for (; k + 2 <= n; k += 2) {
+            const double2 a0 = a[k], a1 = a[k + 1], b0 = b[(size_t)k * n], b1 = b[(size_t)(k + 1) * n];
+            dense_mac(s, a0, b0);
+            dense_mac(s, a1, b1);
+        }
+        if (k < n) dense_mac(s, a[k], b[(size_t)k * n]);
+        if (t.M1) s = dense_sum(t, (size_t)q, r == c, s);
+        C[q] = s;
+    }
+}
+// C = c0 + c1 M1 + c2 M2 + c3 M3 + c4 M4
+static __global__ void __launch_bounds__(kDenseThreads, 24) dense_sum_kernel(int64_t total, int n, const DenseSum t,
+                                                                             const double2 *M4, double c4, double2 *C) {
+    const int n2 = n * n;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+        const int e = (int)(q % n2);
+        const double2 d = M4[q];
+        C[q] = dense_sum(t, (size_t)q, e / n == e % n, make_double2(c4 * d.x, c4 * d.y));
+    }
+}
+
+// States have .. have + more - 1 from the first `more` ones and a power S (of
+// the propagator, transposed): V[have + j] = U V[j].
+static __global__ void __launch_bounds__(kDenseThreads, 24) dense_states_kernel(int64_t n_orient, int n, int m, int have,
+                                                                                int more, const double2 *__restrict__ S,
+                                                                                double2 *V) {
+    const int per = more * n;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n_orient * per;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t o = q / per;
+        const int e = (int)(q - o * per), j = e / n, r = e - j * n;
+        const double2 *s = S + o * n * n + r, *v = V + (o * m + j) * n;
+        double2 sum = make_double2(0.0, 0.0);
+        for (int k = 0; k < n; ++k) dense_mac(sum, s[(size_t)k * n], v[k]);
+        V[(o * m + have + j) * n + r] = sum;
+    }
+}
+// Detection rows alike: Y[have + j] = Y[j] U, for every channel.
+static __global__ void __launch_bounds__(kDenseThreads, 24) dense_rows_kernel(int64_t n_orient, int n, int nchan, int rows,
+                                                                              int have, int more,
+                                                                              const double2 *__restrict__ S, double2 *Y) {
+    const int per = nchan * more * n;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n_orient * per;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t o = q / per;
+        const int e = (int)(q - o * per), ch = e / (more * n), f = e - ch * more * n, j = f / n, c = f - j * n;
+        double2 *base = Y + ((o * nchan + ch) * rows) * n;
+        const double2 *s = S + (o * n + c) * n, *y = base + (size_t)j * n;
+        double2 sum = make_double2(0.0, 0.0);
+        for (int k = 0; k < n; ++k) dense_mac(sum, s[k], y[k]);
+        base[(size_t)(have + j) * n + c] = sum;
+    }
+}
+// fids[o][ch][a m + j] = Y[a] . V[j]
+static __global__ void __launch_bounds__(kDenseThreads, 24) dense_points_kernel(int64_t n_orient, int n, int nchan, int rows,
+                                                                                int m, int npts,
+                                                                                const double2 *__restrict__ Y,
+                                                                                const double2 *__restrict__ V, double2 *fids,
+                                                                                int *status) {
+    const int64_t per = (int64_t)nchan * npts;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n_orient * per;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t o = q / per;
+        const int e = (int)(q - o * per), ch = e / npts, p = e - ch * npts, a = p / m, j = p - a * m;
+        const double2 *y = Y + ((o * nchan + ch) * rows + a) * n, *v = V + (o * m + j) * n;
+        double2 s = make_double2(0.0, 0.0);
+        for (int k = 0; k < n; ++k) dense_mac(s, y[k], v[k]);
+        fids[q] = s;
+        if (!isfinite(s.x) || !isfinite(s.y)) status[o] = kDevNonFinite;
+    }
+}
+
+}  // namespace spx

@@ -27,6 +27,7 @@
 #include "block.cuh"
 #include "block_plan.h"
 #include "builder.h"
+#include "dense.cuh"
 #include "kernels.cuh"
 
 namespace {
@@ -87,7 +88,17 @@ struct BlockPlan {
         int warps = 0, ecap = 0;
     };
     std::vector<Layout> layouts[2];  // FP32, FP64
+    spx::DenseSystem dense{};        // the same rows for the dense kernels (dense.cuh)
+    int ncoil = 0;                   // coil entries among them
+    const int *coil_row = nullptr, *coil_chan = nullptr;
+    const double2 *coil_val = nullptr;
+    double bound = 0.0;              // on |L| over all orientations, these rows alone
     DevBuf<unsigned char> mem;
+};
+
+// Device buffers of a run of the dense kernels.
+struct DenseBufs {
+    DevBuf<double2> M, V, Y;         // six matrices, states, detection rows
 };
 
 // Device buffers of the kernels of block.cuh for one run.
@@ -153,6 +164,8 @@ struct spx_handle {
     std::vector<char> state_rows;   // rows with a non-zero per-orientation initial state
     BlockPlan plan;
     BlockBufs blk, chk_blk;
+    DenseBufs dense, chk_dense;
+    std::vector<double> row_bound;  // per row: sum of its entries' magnitudes over the value streams
 
     // run buffers
     DevBuf<double> d_grid;       // alpha | beta | gamma | weight
@@ -168,7 +181,8 @@ struct spx_handle {
 
     // FP64 check of FP32 runs: a few orientations re-run in FP64 on a second
     // stream while the FP32 run proceeds (spx_stats.fp32_rel_error)
-    cudaStream_t check_stream = nullptr;
+    cudaStream_t check_stream = nullptr;     // of the highest priority: its launches depend on each other
+    int high_priority = 0;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     DevBuf<double> d_chk_grid;       // alpha | beta | gamma of the checked orientations
     DevBuf<double2> d_chk_rho0s;     // their initial states when per-orientation states are set
@@ -273,6 +287,19 @@ void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<i
             P.vfac.push_back(im);
             ++P.nv;
         }
+    std::vector<int> ent, esrc, crow, cchan;
+    std::vector<double2> cval;
+    for (int i = 0; i < P.n; ++i)
+        for (auto &e : P.entries[i]) { ent.push_back(e.col * P.n + i); esrc.push_back(e.src); }
+    if (detect)
+        for (size_t i = 0; i < h->coil_row_host.size(); ++i)
+            if (own[h->coil_row_host[i]] >= 0) {
+                crow.push_back(own[h->coil_row_host[i]]);
+                cchan.push_back(h->coil_chan_host[i]);
+                cval.push_back(h->coil_val_host[i]);
+            }
+    plan.bound = 0.0;
+    for (int r : rows) plan.bound = std::max(plan.bound, h->row_bound[r]);
     // layouts: the best warp count for a few grid sizes, each precision
     std::vector<unsigned char> blob;
     auto put = [&](const void *p, size_t bytes) {
@@ -286,6 +313,9 @@ void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<i
     const size_t o_val = put(P.values.data(), P.values.size() * sizeof(double));
     const size_t o_chan = put(P.vchan.data(), P.vchan.size() * sizeof(int));
     const size_t o_fac = put(P.vfac.data(), P.vfac.size() * sizeof(int));
+    const size_t o_ent = put(ent.data(), ent.size() * sizeof(int)), o_esrc = put(esrc.data(), esrc.size() * sizeof(int));
+    const size_t o_crow = put(crow.data(), crow.size() * sizeof(int)), o_cchan = put(cchan.data(), cchan.size() * sizeof(int));
+    const size_t o_cval = put(cval.data(), cval.size() * sizeof(double2));
     struct At { size_t row, part, shape, src, col; };
     std::vector<At> at[2];
     for (int p = 0; p < 2; ++p) {
@@ -349,6 +379,12 @@ void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<i
         }
     plan.n = P.n;
     plan.nv = P.nv;
+    plan.dense = {P.n, (int)ent.size(), reinterpret_cast<const int *>(d + o_ent), reinterpret_cast<const int *>(d + o_esrc),
+                  reinterpret_cast<const int *>(d + o_rows)};
+    plan.ncoil = (int)crow.size();
+    plan.coil_row = reinterpret_cast<const int *>(d + o_crow);
+    plan.coil_chan = reinterpret_cast<const int *>(d + o_cchan);
+    plan.coil_val = reinterpret_cast<const double2 *>(d + o_cval);
     plan.ok = true;
 }
 
@@ -581,6 +617,7 @@ void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32
     if (cplx) ell_im.assign((size_t)nst * std::max(ell_len, 1), 0.0);
     std::vector<double2> diag((size_t)nst * n_pad, make_double2(0.0, 0.0));
     double g_upper = 0.0;
+    std::vector<double> row_bound(n_pad, 0.0);
     for (int s = 0; s < nslices; ++s) {
         for (int l = 0; l < 32; ++l) {
             const int row = s * 32 + l;
@@ -613,6 +650,7 @@ void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32
             const int w = (slice_off[s + 1] - slice_off[s]) / 32;
             for (; c < w; ++c) ell_col[(size_t)slice_off[s] + (size_t)c * 32 + l] = (uint16_t)std::min(row, n_pad - 1);
             g_upper = std::max(g_upper, rowsum);
+            row_bound[row] = rowsum;
         }
     }
     for (int i = 0; i < n; ++i) max_im_diag = std::max(max_im_diag, std::fabs(diag[i].y));
@@ -671,6 +709,7 @@ void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32
     h->lo_scale = g_upper > 0.0 ? std::ldexp(1.0, -std::ilogb(g_upper) - 1) : 1.0;
     h->max_im_diag = max_im_diag;
     h->ell_col_host = std::move(ell_col);
+    h->row_bound = std::move(row_bound);
     h->rho0_host = std::move(r0);
     h->coil_row_host = std::move(crow);
     h->coil_val_host = std::move(cval);
@@ -785,6 +824,10 @@ struct Config {
     int blk_M = 0, blk_K = 0, blk_lev = 0;
     bool blk_cplx = false;
     int blk_which = 0;                            // the propagation kernel (spx_block_kernel_*)
+    // FP64 by dense matrices (dense.cuh): states and detection rows kept,
+    // squarings of the scaled exponential
+    const BlockPlan *dense = nullptr;
+    int dense_m = 0, dense_rows = 0, dense_scale = 0;
     size_t blk_smem = 0;
 };
 
@@ -941,6 +984,41 @@ bool configure_block(spx_handle *h, const BlockPlan &plan, int64_t n_orient, dou
     return true;
 }
 
+// Chooses the dense kernels for an FP64 run on the coupled states when their
+// modelled time is below the series': both in cycles, by FP64 instructions (2
+// lanes a cycle on each SM) or by latency (about 6000 cycles from one of the
+// dense launches to the next; the layout's latency for each series term).
+// Measured sides, one orientation of 52 states and 2048 steps: dense 0.25 ms,
+// series 2.3 ms; 1000 of them: series 11 ms, dense 16 ms; 400 of 8 states and
+// 1024 steps: dense 0.2 ms, series 1.4 ms.
+void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, double dt, int64_t nsteps, Config &c) {
+    const double n = plan.n, npts = (double)nsteps + 1.0;
+    // rounding doubles with every squaring; and the matrices take memory
+    if (nsteps > 8192 || 6.0 * n_orient * n * n * sizeof(double2) > 1e9) return;
+    int m = 1, rows = 1, squarings = 0;
+    while ((int64_t)m * rows < nsteps + 1) {
+        if (m <= rows) m *= 2; else rows *= 2;
+        ++squarings;
+    }
+    int scale = 0;
+    while (std::ldexp(plan.bound * dt, -scale) > 0.5) ++scale;
+    const double products = 6.0 + scale + squarings;
+    const double work = 4.0 * n * n * (products * n + m + rows * h->nchan) + 4.0 * n * npts * h->nchan;
+    const double dense = std::max(work * n_orient / (2.0 * h->sm_count), 0.0) + 6000.0 * (products + squarings + 4.0);
+    const double per_sm = std::ceil((double)n_orient / h->sm_count);
+    // the spectral half-width is about an eighth of the row bound (5.6 to 11.5
+    // on the benchmark systems), a chunk's series a quarter longer than its
+    // argument, and a term takes twice the model's cycles alone, 1.5 times in
+    // company
+    const double terms = 1.25 * plan.bound / 8.0 * dt * npts + 30.0;
+    const double series = terms * (per_sm > 2.0 ? 1.5 : 2.0) * c.blk->cost.time(per_sm) + 1e5;
+    if (dense > series) return;
+    c.dense = &plan;
+    c.dense_m = m;
+    c.dense_rows = rows;
+    c.dense_scale = scale;
+}
+
 bool forced_shape(const spx_options &o) {
     return (o.threads > 0 || o.cluster > 0 || o.chunk_steps > 0 || o.chunk_target > 0) && !(o.flags & kOwnShape);
 }
@@ -956,7 +1034,9 @@ void choose_block(spx_handle *h, const BlockPlan *plan, int64_t n_orient, double
     // in FP64, so the decision stays the one it has been (a three-spin system,
     // 16384 steps: 1.2e-5 on the whole system, 3.5e-6 on its coupled states)
     if (!f64 && h->max_im_diag == 0.0 && nsteps > 8192) return;
-    configure_block(h, *plan, n_orient, dt, nsteps, f64, opt.chunk_target, kmax_override, m_cap, false, c);
+    if (configure_block(h, *plan, n_orient, dt, nsteps, f64, opt.chunk_target, kmax_override, m_cap, false, c) && f64 &&
+        kmax_override == 0 && m_cap == 256)
+        choose_dense(h, *plan, n_orient, dt, nsteps, c);
 }
 
 // traj: the run writes the state at every step (chunks of opt.chunk_steps
@@ -1177,12 +1257,92 @@ void launch_chebyshev(spx_handle *h, bool f64, const Config &c, spx::DevSystem &
     SPX_CUDA(cudaLaunchKernelExC(&lc, kfn, args));
 }
 
+void reserve_dense(const spx_handle *h, DenseBufs &b, int64_t n_orient, const Config &c) {
+    const size_t n = (size_t)c.dense->n;
+    b.M.reserve(6 * (size_t)n_orient * n * n);
+    b.V.reserve((size_t)n_orient * c.dense_m * n);
+    b.Y.reserve((size_t)n_orient * h->nchan * c.dense_rows * n);
+}
+
+// An FP64 run by dense matrices: out and the status words as the propagation
+// kernels write them.  pick: see BlockRun.
+void launch_dense(spx_handle *h, const Config &c, spx::DevSystem &sys, DenseBufs &b, int64_t n_orient, int pick,
+                  const double *d_al, const double *d_be, const double *d_ga, double dt, int64_t nsteps, double2 *out,
+                  const spx::DevRun &words, cudaStream_t stream) {
+    const BlockPlan &plan = *c.dense;
+    const int n = plan.n, m = c.dense_m, rows = c.dense_rows;
+    const int64_t total = n_orient * n * n;
+    double2 *M[6];
+    for (int q = 0; q < 6; ++q) M[q] = b.M.p + (size_t)q * total;
+    auto grid = [&](int64_t items) {
+        return dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>((items + spx::kDenseThreads - 1) / spx::kDenseThreads,
+                                                                      (int64_t)h->sm_count * 64)));
+    };
+    spx::DenseStart st{};
+    st.n_orient = (int)n_orient; st.pick = pick;
+    st.alpha = d_al; st.beta = d_be; st.gamma = d_ga;
+    st.h = std::ldexp(dt, -c.dense_scale);
+    st.A = M[0]; st.V = b.V.p; st.m = m; st.Y = b.Y.p; st.nchan = h->nchan; st.rows = rows;
+    st.rho0 = sys.rho0; st.rho0s = sys.rho0s; st.state_stride = (size_t)h->n_pad;
+    st.ncoil = plan.ncoil; st.coil_row = plan.coil_row; st.coil_chan = plan.coil_chan; st.coil_val = plan.coil_val;
+    st.status = words.status; st.kused = words.kused; st.mused = words.mused; st.matvecs = words.matvecs;
+    st.halfwidth = words.halfwidth; st.bound = plan.bound;
+    st.products = 6 + c.dense_scale;
+    spx::dense_start_kernel<<<dim3((unsigned)n_orient), spx::kDenseThreads, 0, stream>>>(sys, plan.dense, st);
+    ++h->launches;
+    auto product = [&](const double2 *A, const double2 *B, double2 *C, const spx::DenseSum &t = spx::DenseSum{}) {
+        spx::dense_product_kernel<<<grid(total), spx::kDenseThreads, 0, stream>>>(total, n, A, B, C, t);
+        ++h->launches;
+    };
+    // exp(A) to degree 16 in powers of A^4: M = A, A^2, A^3, A^4
+    product(M[0], M[0], M[1]);
+    product(M[1], M[0], M[2]);
+    product(M[1], M[1], M[3]);
+    double f[17];
+    f[0] = 1.0;
+    for (int k = 1; k <= 16; ++k) f[k] = f[k - 1] / k;
+    auto quarter = [&](int q) { return spx::DenseSum{M[0], M[1], M[2], f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]}; };
+    spx::dense_sum_kernel<<<grid(total), spx::kDenseThreads, 0, stream>>>(total, n, quarter(3), M[3], f[16], M[4]);
+    ++h->launches;
+    product(M[3], M[4], M[5], quarter(2));
+    product(M[3], M[5], M[4], quarter(1));
+    // without the identity while the step is scaled down: exp(A) - 1 = Z keeps
+    // its digits, and (1 + Z)^2 - 1 = 2 Z + Z^2
+    if (c.dense_scale > 0) f[0] = 0.0;
+    product(M[3], M[4], M[5], quarter(0));
+    double2 *U = M[5], *W = M[4];
+    for (int q = 0; q < c.dense_scale; ++q) {
+        product(U, U, W, spx::DenseSum{U, U, U, q + 1 == c.dense_scale ? 1.0 : 0.0, 2.0, 0.0, 0.0});
+        std::swap(U, W);
+    }
+    auto square = [&] { product(U, U, W); std::swap(U, W); };
+    // states 0 .. m-1 with U, U^2, U^4, ...; then detection rows with U^m, U^2m, ...
+    for (int have = 1; have < m; have *= 2) {
+        spx::dense_states_kernel<<<grid(n_orient * have * n), spx::kDenseThreads, 0, stream>>>(n_orient, n, m, have, have, U,
+                                                                                                b.V.p);
+        ++h->launches;
+        if (2 * have < m || rows > 1) square();
+    }
+    for (int have = 1; have < rows; have *= 2) {
+        spx::dense_rows_kernel<<<grid(n_orient * h->nchan * have * n), spx::kDenseThreads, 0, stream>>>(
+            n_orient, n, h->nchan, rows, have, have, U, b.Y.p);
+        ++h->launches;
+        if (2 * have < rows) square();
+    }
+    const int64_t npts = nsteps + 1;
+    spx::dense_points_kernel<<<grid(n_orient * h->nchan * npts), spx::kDenseThreads, 0, stream>>>(
+        n_orient, n, h->nchan, rows, m, (int)npts, b.Y.p, b.V.p, out, words.status);
+    ++h->launches;
+    SPX_CUDA(cudaGetLastError());
+}
+
 // Device buffers of one run (idempotent; called before graph capture too).
 void reserve_run(spx_handle *h, int64_t n_orient, int64_t nsteps, bool f64, const Config &c) {
     const size_t npts = ((size_t)nsteps + 1) * h->nchan;       // every channel's points
     const size_t vec_bytes = f64 ? sizeof(double2) : sizeof(float2);
     h->d_fids.reserve(npts * n_orient * vec_bytes);
-    if (c.blk) reserve_block(h->blk, n_orient, f64, c);
+    if (c.dense) reserve_dense(h, h->dense, n_orient, c);
+    else if (c.blk) reserve_block(h->blk, n_orient, f64, c);
     else h->d_table.reserve((size_t)c.grid * c.Kmax * (c.M + 1));
     h->d_status.reserve(n_orient);
     h->d_kused.reserve(n_orient);
@@ -1279,13 +1439,14 @@ int launch_fp32_check(spx_handle *h, int64_t n_orient, const double *d_al, const
     const Config c = choose_config(h, S, dt, nsteps, o64, 0, 256, false, &h->plan);
     const size_t npts = ((size_t)nsteps + 1) * h->nchan;
     if (!h->check_stream) {
-        SPX_CUDA(cudaStreamCreateWithFlags(&h->check_stream, cudaStreamNonBlocking));
+        SPX_CUDA(cudaStreamCreateWithPriority(&h->check_stream, cudaStreamNonBlocking, h->high_priority));
         SPX_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
         SPX_CUDA(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
     }
     h->d_chk_grid.reserve(3 * (size_t)S);
     h->d_chk_fids.reserve(npts * S * sizeof(double2));
-    if (c.blk) reserve_block(h->chk_blk, S, true, c);
+    if (c.dense) reserve_dense(h, h->chk_dense, S, c);
+    else if (c.blk) reserve_block(h->chk_blk, S, true, c);
     else h->d_chk_table.reserve((size_t)c.grid * c.Kmax * (c.M + 1));
     h->d_chk_status.reserve(S);
     h->d_chk_kused.reserve(S);
@@ -1299,6 +1460,16 @@ int launch_fp32_check(spx_handle *h, int64_t n_orient, const double *d_al, const
     for (int j = 0; j < S; ++j) idx[j] = check_index(j, S, n_orient);
     SPX_CUDA(cudaEventRecord(h->ev_fork, h->stream));
     SPX_CUDA(cudaStreamWaitEvent(h->check_stream, h->ev_fork, 0));
+    if (c.dense) {
+        spx::DevSystem sys = sys32;
+        spx::DevRun words{};
+        words.status = h->d_chk_status.p; words.kused = h->d_chk_kused.p; words.mused = h->d_chk_mused.p;
+        words.matvecs = h->d_chk_matvecs.p; words.halfwidth = h->d_chk_halfwidth.p;
+        launch_dense(h, c, sys, h->chk_dense, S, (int)n_orient, d_al, d_be, d_ga, dt, nsteps,
+                     reinterpret_cast<double2 *>(h->d_chk_fids.p), words, h->check_stream);
+        SPX_CUDA(cudaEventRecord(h->ev_join, h->check_stream));
+        return 0;
+    }
     if (c.blk) {
         // the checked orientations are picked out of the whole grid on the device
         spx::DevSystem sys = sys32;
@@ -1387,7 +1558,10 @@ void launch_powder(spx_handle *h, int64_t n_orient, const double *d_al, const do
         if (waves && c.grid - take >= std::max(c.cl, c.grid / 2)) c.grid -= take;
     }
     if (timed) SPX_CUDA(cudaEventRecord(h->ev[0], h->stream));
-    if (c.blk) {
+    if (c.dense) {
+        launch_dense(h, c, sys, h->dense, n_orient, 0, d_al, d_be, d_ga, dt, nsteps,
+                     reinterpret_cast<double2 *>(h->d_fids.p), run, h->stream);
+    } else if (c.blk) {
         spx::BlockRun r{};
         BlockBufs &b = h->blk;
         block_run_buffers(r, c, b.centre.p, b.extent.p, b.lev_half.p, b.lev.p, b.kcut.p, b.table.p,
@@ -3069,6 +3243,8 @@ spx_status spx_create(spx_handle **handle, int device) {
         int optin = 0;
         SPX_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
         h->smem_optin = (size_t)optin;
+        int least = 0;
+        SPX_CUDA(cudaDeviceGetStreamPriorityRange(&least, &h->high_priority));
     });
     if (st != SPX_OK) {
         spx_destroy(h);
@@ -3571,6 +3747,16 @@ spx_status spx_batch_create(spx_batch **out, int32_t n, spx_handle *const *handl
             SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::powder_combine_kernel)));
             SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::block_tables_kernel)));
             for (int i = 0; i < n; ++i) {
+                if (cfg[i].dense) {
+                    for (const void *k : {reinterpret_cast<const void *>(&spx::dense_start_kernel),
+                                          reinterpret_cast<const void *>(&spx::dense_product_kernel),
+                                          reinterpret_cast<const void *>(&spx::dense_sum_kernel),
+                                          reinterpret_cast<const void *>(&spx::dense_states_kernel),
+                                          reinterpret_cast<const void *>(&spx::dense_rows_kernel),
+                                          reinterpret_cast<const void *>(&spx::dense_points_kernel)})
+                        SPX_CUDA(cudaFuncGetAttributes(&fa, k));
+                    continue;
+                }
                 if (cfg[i].blk) {
                     SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(handles[i]->cplx, cfg[i].blk_bounds->ecap, 0)));
                     SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(handles[i]->cplx, cfg[i].blk->ecap,

@@ -445,6 +445,62 @@ static __device__ void wigner_element(int rank, int k, int m, double a, double b
     im = d * sin(ph);
 }
 
+// Coefficients 1, Re D_t, Im D_t of all rotational terms into coef, by a CTA
+// (all threads call; the closed forms of wigner_element).  An FP64 instruction
+// takes a warp 64 cycles, so the six sines and cosines (of beta, alpha, gamma
+// and the double angles) are taken once, in lanes side by side, and every
+// d-element is a sum over 1, cos b, cos^2 b, sin b and sin b cos b.
+static __device__ __noinline__ void wigner_coefficients(const DevSystem &sys, double a, double b, double g, double *coef) {
+    __shared__ double2 s_trig[5];                 // cos, sin of b, a, 2a, g, 2g
+    const int tid = threadIdx.x;
+    if (tid < 5) {
+        double sn, cs;
+        sincos(tid == 0 ? b : tid == 1 ? a : tid == 2 ? 2 * a : tid == 3 ? g : 2 * g, &sn, &cs);
+        s_trig[tid] = make_double2(cs, sn);
+    }
+    if (tid == 0) coef[0] = 1.0;
+    __syncthreads();
+    const double cb = s_trig[0].x, sb = s_trig[0].y;
+    for (int t = tid; t < sys.nterms; t += blockDim.x) {
+        const int rank = sys.term_rkm[3 * t], k = sys.term_rkm[3 * t + 1], m = sys.term_rkm[3 * t + 2];
+        double c0 = 0.0, c1 = 0.0, c2 = 0.0, s0 = 0.0, s1 = 0.0;
+        const int p = rank - k, q = rank - m;     // projections
+        if (rank == 1) {
+            const double r2 = 0.70710678118654752;
+            if (p == 0 && q == 0) c1 = 1.0;
+            else if (p == 0) s0 = q > 0 ? r2 : -r2;
+            else if (q == 0) s0 = p > 0 ? -r2 : r2;
+            else { c0 = 0.5; c1 = p == q ? 0.5 : -0.5; }
+        } else {
+            const double r38 = 0.61237243569579452, r32 = 1.2247448713915890;
+            const int ap = abs(p), aq = abs(q);
+            if (ap == 2 && aq == 2) { c0 = c2 = 0.25; c1 = p == q ? 0.5 : -0.5; }
+            else if (ap == 1 && aq == 1) {
+                c1 = 0.5;
+                c0 = p == q ? -0.5 : 0.5;
+                c2 = p == q ? 1.0 : -1.0;
+            } else if (p == 0 && q == 0) { c0 = -0.5; c2 = 1.5; }
+            else if (ap + aq == 2) { c0 = r38; c2 = -r38; }                       // (2, 0), (0, 2)
+            else if (ap + aq == 1) s1 = (p + -q > 0) ? -r32 : r32;                // (1, 0), (0, -1) < 0
+            else {                                                                // (2, 1) and its kin
+                const bool same = (p > 0) == (q > 0);
+                s0 = 0.5;
+                s1 = same ? 0.5 : -0.5;
+                // sign: - for p above q
+                if (p > q) { s0 = -s0; s1 = -s1; }
+            }
+        }
+        const double d = c0 + cb * (c1 + cb * c2) + sb * (s0 + cb * s1);
+        // exp(-1i (p a + q g))
+        double2 ea = p == 0 ? make_double2(1.0, 0.0) : s_trig[abs(p)], eg = q == 0 ? make_double2(1.0, 0.0) : s_trig[2 + abs(q)];
+        if (p > 0) ea.y = -ea.y;
+        if (q > 0) eg.y = -eg.y;
+        coef[1 + 2 * t] = d * (ea.x * eg.x - ea.y * eg.y);
+        coef[2 + 2 * t] = d * (ea.x * eg.y + ea.y * eg.x);
+    }
+    __syncthreads();
+}
+
 // Spectral-bound helpers in FP32: the interval they feed is widened by Ritz
 // residuals and 2% of its width, so FP32 digits suffice, and GB300's FP64
 // division and transcendentals are two orders of magnitude slower.

@@ -84,6 +84,14 @@ def test_coupled_states_match_dense_exponentials(gpu_engine, n, extra, cplx, rel
         assert rel_err(res.fid, WEIGHTS @ ref) <= tol
         assert res.stats['coupled_dim'] in ((n,) if n <= 480 else (0, n))
     assert gpu_engine.run(*ANGLES, WEIGHTS, dt, nsteps, precision=E.FP64).stats['dim'] == n + extra
+    # FP64 of three orientations takes the dense matrices; the entry point
+    # without allocations takes the series
+    import torch
+    g = torch.tensor(np.stack([*ANGLES, WEIGHTS]), device='cuda')
+    out = torch.zeros(2 * (nsteps + 1), dtype=torch.float64, device='cuda')
+    torch.cuda.synchronize()
+    gpu_engine.run_noalloc(*[g[i].data_ptr() for i in range(4)], 3, dt, nsteps, out.data_ptr(), precision=E.FP64)
+    assert rel_err(out.cpu().numpy().view(complex), WEIGHTS @ ref) <= 1e-10
     if relax:           # rates near the spectral width: the whole-system kernel takes its last series for growth
         return
     whole = gpu_engine.run(*ANGLES, WEIGHTS, dt, nsteps, precision=E.FP64, cluster=1)
