@@ -40,11 +40,12 @@ struct BlockLayout {
     const int *lane_row;        // [threads] state row, n + v for detection row v, -1: none
     const int *lane_part;       // [threads] lanes of the row | part index << 8
     const int *warp_shape;      // [threads/32] entries per lane | shuffle rounds << 8
-    const int *src;             // [ecap][threads] ELL entry of the system, -1 none, -2-i: coil value i
-    const uint16_t *col;        // [ecap][threads] state row the entry reads
+    const int *src;             // [ecap][threads] real part of an ELL entry of the system, its imaginary part
+                                // (ell_len later), -1 none, -2-i: value i of the detection rows
+    const uint16_t *col;        // [ecap][threads] state row the entry reads, n + row: 1i times that
     const int *row_src;         // [n] row of the system (sliced order)
     const int *state_pos;       // [n] place of the row in the run's state arrays
-    const double2 *vval;        // entry values of the detection rows
+    const double *vval;         // entry values of the detection rows
     const int *vchan;           // [nv] channel of a detection row
     const int *vfac;            // [nv] 0: times 1, 1: times -1i (imaginary parts of a complex coil)
 };
@@ -68,8 +69,8 @@ struct BlockRun {
     double *lev_half;           // [nlev]
     int *lev_m, *lev_k, *lev_raw;   // [nlev] steps per chunk, table rows, series length before the cap
     int *kcut;                  // [nlev][Mcap+1] terms a column needs
-    double *table;              // [nlev][Kmax][M+1] (2 - delta_k0) J_k(half j dt)
-    float *tablef;              // the same rounded to float, or null
+    double *table;              // [nlev][Kmax][block_row(M)] (2 - delta_k0) J_k(half j dt)
+    float *tablef;              // the same in float, times block_sign(k), or null
     double max_im_diag;
     int adjoint;                // propagate under -H + 1i R: the adjoint of exp(-1i L dt)
     // states (read and written at state_pos)
@@ -86,12 +87,14 @@ struct BlockRun {
 };
 
 // FP32 entries of one lane: values as hi + lo floats, and the byte offset of
-// the state they multiply.
-template <bool CPLX, int ECAP> struct BlockEntries;
-template <int ECAP> struct BlockEntries<false, ECAP> {
+// the state they multiply.  All values are real: a complex system (EXT) keeps
+// 1i x beside x, its entries' real and imaginary parts are entries of their own
+// that read one or the other, and a part that is zero for every orientation is
+// left out (of 1904 entries of a magic-angle-spinning block none has both).
+template <int ECAP> struct BlockEntries {
     float hi[ECAP], lo[ECAP];
     int col[ECAP];
-    __device__ __forceinline__ void set(int i, double re, double) { split(re, hi[i], lo[i]); }
+    __device__ __forceinline__ void set(int i, double v) { split(v, hi[i], lo[i]); }
     // (Y, L, P) += v * x: Y + L + P is the sum.  The product is exact inside the
     // fused multiply-adds, so the low-order part L keeps the product's rounding
     // as well as the sum's; P sums the products of the values' low parts.  Each
@@ -109,30 +112,9 @@ template <int ECAP> struct BlockEntries<false, ECAP> {
     }
     __device__ __forceinline__ float mag(int i) const { return fabsf(hi[i]); }
 };
-template <int ECAP> struct BlockEntries<true, ECAP> {
-    float rh[ECAP], ih[ECAP], rl[ECAP], il[ECAP];
-    int col[ECAP];
-    __device__ __forceinline__ void set(int i, double re, double im) {
-        split(re, rh[i], rl[i]);
-        split(im, ih[i], il[i]);
-    }
-    __device__ __forceinline__ void mac(int i, f2x &Y, f2x &L, f2x &P, f2x X) const {
-        const f2x XS = swap2(X);
-        const f2x H = f2pk(rh[i], rh[i]), G = f2pk(-ih[i], ih[i]);
-        const f2x S = fma2(H, X, Y);
-        L = add2(L, fma2(H, X, sub2(Y, S)));
-        Y = fma2(G, XS, S);
-        L = add2(L, fma2(G, XS, sub2(S, Y)));
-        P = fma2(f2pk(rl[i], rl[i]), X, P);
-        P = fma2(f2pk(-il[i], il[i]), XS, P);
-    }
-    __device__ __forceinline__ void plain(int i, float2 &y, float2 x) const {
-        y.x = fmaf(rh[i], x.x, fmaf(-ih[i], x.y, y.x));
-        y.y = fmaf(rh[i], x.y, fmaf(ih[i], x.x, y.y));
-    }
-    __device__ __forceinline__ float mag(int i) const { return sqrtf(rh[i] * rh[i] + ih[i] * ih[i]); }
-};
-// Barrier of one orientation's CTA; the warps reach it from different loops.
+
+// The CTA's barrier for the terms, whose loops differ between warps (each warp
+// arrives from its own instance of the loop).
 static __device__ __forceinline__ void block_sync() { asm volatile("barrier.sync 0;" ::: "memory"); }
 static __device__ __forceinline__ void st_shared(uint32_t a, f2x v) {
     asm volatile("st.shared.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
@@ -163,36 +145,28 @@ static __device__ __forceinline__ BlockLane block_lane(const BlockLayout &B, int
 // (coef: the rotational coefficients), stream by stream, so that the loads of
 // all entries are in flight together; detection rows keep their values.
 // sign: -1 for the adjoint generator -H + 1i R.
-template <bool CPLX, int ECAP>
+template <int ECAP>
 static __device__ __forceinline__ void block_assemble(const DevSystem &sys, const BlockLayout &B, int ew, int t,
-                                                      const double *coef, double sign, double (&re)[ECAP],
-                                                      double (&im)[ECAP]) {
+                                                      const double *coef, double sign, double (&v)[ECAP]) {
     int src[ECAP];
+    const double *at[ECAP];
 #pragma unroll
     for (int i = 0; i < ECAP; ++i) {
         src[i] = i < ew ? B.src[i * B.threads + t] : -1;
-        re[i] = im[i] = 0.0;
+        at[i] = src[i] < sys.ell_len ? sys.ell_re + src[i] : sys.ell_im + (src[i] - sys.ell_len);
+        v[i] = 0.0;
     }
     for (int s = 0; s < sys.nstreams; ++s) {
         const double c = coef[sys.stream_coef[s]];
-        const double *vr = sys.ell_re + (size_t)s * sys.ell_len;
-        const double *vi = CPLX ? sys.ell_im + (size_t)s * sys.ell_len : nullptr;
+        const size_t off = (size_t)s * sys.ell_len;
 #pragma unroll
         for (int i = 0; i < ECAP; ++i)
-            if (src[i] >= 0) {
-                re[i] = fma(c, vr[src[i]], re[i]);
-                if (CPLX) im[i] = fma(c, vi[src[i]], im[i]);
-            }
+            if (src[i] >= 0) v[i] = fma(c, at[i][off], v[i]);
     }
 #pragma unroll
     for (int i = 0; i < ECAP; ++i) {
-        re[i] *= sign;
-        im[i] *= sign;
-        if (src[i] <= -2) {
-            const double2 v = B.vval[-2 - src[i]];
-            re[i] = v.x;
-            im[i] = v.y;
-        }
+        v[i] *= sign;
+        if (src[i] <= -2) v[i] = B.vval[-2 - src[i]];
     }
 }
 
@@ -211,9 +185,7 @@ static __device__ __forceinline__ double2 block_diagonal(const DevSystem &sys, i
 
 // Doubles of one orientation in BlockRun::saved: the lanes' entries, then
 // their diagonals.
-static __host__ __device__ inline size_t block_saved(int ecap, int threads, bool cplx) {
-    return (size_t)threads * ((cplx ? 2 : 1) * ecap + 2);
-}
+static __host__ __device__ inline size_t block_saved(int ecap, int threads) { return (size_t)threads * (ecap + 2); }
 
 // Index in the grid of the run's orientation o.
 static __device__ __forceinline__ int block_grid_index(const BlockRun &R, int o) {
@@ -308,43 +280,40 @@ static __device__ float ritz_last(const float *al, const float *be, int m, float
 // than the spread.  The assembled L goes to R.saved for the FP32 propagation, which
 // runs on the same layout.
 // ---------------------------------------------------------------------------
-template <bool CPLX, int ECAP>
+template <bool EXT, int ECAP>
 __global__ void __launch_bounds__(kBlockRows, ECAP <= 16 ? 2 : 1) block_bounds_kernel(const DevSystem sys, const BlockLayout B,
                                                                      const BlockRun R) {
     __shared__ double s_coef[kMaxCoef];
-    __shared__ float2 s_x[2][kBlockRows + 1];
+    __shared__ float2 s_x[2][(EXT ? 2 : 1) * kBlockRows + 1];
     __shared__ float2 s_part[2][kBlockRows / 32];
     __shared__ float s_al[kMaxLanczos], s_be[kMaxLanczos];
     __shared__ float s_work[2][3][kMaxLanczos];
     const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const BlockLane l = block_lane(B, tid);
     block_coefficients(sys, R, o, s_coef);
-    BlockEntries<CPLX, ECAP> E;
+    BlockEntries<ECAP> E;
     double2 dg = make_double2(0.0, 0.0);
     {
         const double sign = R.adjoint ? -1.0 : 1.0;
-        double *save = R.saved ? R.saved + (size_t)o * block_saved(B.ecap, B.threads, CPLX) : nullptr;
+        double *save = R.saved ? R.saved + (size_t)o * block_saved(B.ecap, B.threads) : nullptr;
         // four entries at a time: more FP64 sums in registers cost resident CTAs
 #pragma unroll
         for (int i0 = 0; i0 < ECAP; i0 += 4) {
-            double re[4], im[4];
+            double v[4];
             BlockLayout Bi = B;
             Bi.src = B.src + (size_t)i0 * B.threads;
-            block_assemble<CPLX, 4>(sys, Bi, l.ew - i0, tid, s_coef, sign, re, im);
+            block_assemble<4>(sys, Bi, l.ew - i0, tid, s_coef, sign, v);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int i = i0 + q;
-                E.set(i, re[q], im[q]);
+                E.set(i, v[q]);
                 E.col[i] = i < l.ew ? B.col[i * B.threads + tid] * (int)sizeof(float2) : 0;
-                if (save && i < l.ew) {
-                    save[(size_t)i * B.threads + tid] = re[q];
-                    if (CPLX) save[(size_t)(B.ecap + i) * B.threads + tid] = im[q];
-                }
+                if (save && i < l.ew) save[(size_t)i * B.threads + tid] = v[q];
             }
         }
         if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef, sign);
         if (save) {
-            double *sd = save + (size_t)(CPLX ? 2 : 1) * B.ecap * B.threads;
+            double *sd = save + (size_t)B.ecap * B.threads;
             sd[tid] = dg.x;
             sd[B.threads + tid] = dg.y;
         }
@@ -400,10 +369,11 @@ __global__ void __launch_bounds__(kBlockRows, ECAP <= 16 ? 2 : 1) block_bounds_k
     // also beyond n steps: FP32 vectors lose their orthogonality on clustered
     // spectra, and n steps then miss the ends (more only find them again)
     const int lits = min(R.lanczos_its, kMaxLanczos);
-    const int slot = l.state ? l.row : kBlockRows;
+    const int slot = l.state ? l.row : (EXT ? 2 : 1) * kBlockRows, slot2 = l.state ? B.n + l.row : slot;
     for (int j = 0; j < lits; ++j) {
         float2 *x = s_x[j & 1];
         x[slot] = q_cur;
+        if (EXT) x[slot2] = make_float2(-q_cur.y, q_cur.x);
         __syncthreads();
         float2 y = make_float2(0.f, 0.f);
         const char *xb = reinterpret_cast<const char *>(x);
@@ -474,11 +444,18 @@ static __device__ __noinline__ double ladder_half(const unsigned long long *exte
     return lev == 0 ? hmax : hmax * exp(-lev * step);
 }
 
+// (-1i)^k is this sign times 1 (even k) or -1i (odd k).
+static __device__ __forceinline__ double block_sign(int k) { return (k & 2) ? -1.0 : 1.0; }
+
+// Table rows are a multiple of 16 bytes long, so that a thread takes the
+// values of neighbouring columns in one load.
+static __host__ __device__ inline int block_row(int M) { return (M + 4) & ~3; }
+
 // Column j of a table by Miller's backward recurrence (bessel_column of
 // kernels.cuh), unnormalised; returns the factor that normalises it and the
 // number of terms that are not zero (kn).
 static __device__ double block_column(double *tab, int M, int j, int K, double half, double dt, int &kn) {
-    const size_t ld = (size_t)(M + 1);
+    const size_t ld = (size_t)block_row(M);
     double *col = tab + j;
     const double x = half * j * dt;
     kn = min(K, 3);
@@ -563,9 +540,9 @@ static __global__ void __launch_bounds__(128) block_tables_kernel(const BlockRun
     __shared__ int s_kn[32];
     const int lane = tid & 31, warp = tid >> 5, j = blockIdx.x * 32 + lane;
     const int K = s_k;
-    const size_t ld = (size_t)(M + 1);
-    double *tab = R.table + (size_t)lev * R.Kmax * (R.Mcap + 1);
-    float *tf = R.tablef ? R.tablef + (size_t)lev * R.Kmax * (R.Mcap + 1) : nullptr;
+    const size_t ld = (size_t)block_row(M), at = (size_t)lev * R.Kmax * block_row(R.Mcap);
+    double *tab = R.table + at;
+    float *tf = R.tablef ? R.tablef + at : nullptr;
     // one warp runs the columns' recurrences; all four scale and round them,
     // eight values of a column in flight
     if (warp == 0 && j <= M) s_inv[lane] = block_column(tab, M, j, K, half, R.dt, s_kn[lane]);
@@ -583,7 +560,7 @@ static __global__ void __launch_bounds__(128) block_tables_kernel(const BlockRun
             if (k < K) {
                 v[q] *= k == 0 ? inv : two;
                 tab[(size_t)k * ld + j] = v[q];
-                if (tf) tf[(size_t)k * ld + j] = (float)v[q];
+                if (tf) tf[(size_t)k * ld + j] = (float)((k == 0 ? 2.0 : block_sign(k)) * v[q]);   // FP32 moments 0 are halved
             }
         }
     }
@@ -607,25 +584,34 @@ static __global__ void __launch_bounds__(128) block_tables_kernel(const BlockRun
     R.kcut[(size_t)lev * (R.Mcap + 1) + j] = min(last + 2, K);
 }
 
-// Dynamic shared memory of the propagation kernels.
+constexpr int kBlockPoints32 = 4, kBlockPoints64 = 1;      // points a thread sums together (block_points)
+
+// Shared memory for the points' partial sums, and all dynamic shared memory of
+// the propagation kernels.
+static __host__ __device__ inline size_t block_rec(int Mcap, int threads, int points) {
+    return (size_t)points * (size_t)(threads > Mcap / points + 1 ? threads : Mcap / points + 1);
+}
 static __host__ __device__ inline size_t block_smem32(int Kmax, int Mcap, int nv, int threads, bool traj) {
     return 8 * ((size_t)(Kmax + 2) * (1 + nv + (traj ? kBlockTraj - 1 : 0)) + (size_t)(Mcap + 1) +
-                (size_t)(threads > Mcap ? threads : Mcap));
+                block_rec(Mcap, threads, kBlockPoints32));
 }
-static __host__ __device__ inline size_t block_smem64(int Kmax, int Mcap, int nv, int lanes, int ecap, int n, bool cplx,
+static __host__ __device__ inline size_t block_smem64(int Kmax, int Mcap, int nv, int lanes, int ecap, int n, bool ext,
                                                       bool traj) {
-    const size_t rec = (size_t)(2 * lanes > Mcap ? 2 * lanes : Mcap);
-    return 16 * (rec + (size_t)(Mcap + 1) + (size_t)(Kmax + 2) * nv) + 8 * (size_t)(Kmax + 2) * (traj ? kBlockTraj : 1) +
-           8 * (size_t)ecap * lanes * (cplx ? 2 : 1) + 8 * 4 * (size_t)(n + 1) + 2 * (size_t)ecap * lanes;
+    return 16 * (block_rec(Mcap, 2 * lanes, kBlockPoints64) + (size_t)(Mcap + 1) + (size_t)(Kmax + 2) * nv) +
+           8 * (size_t)(Kmax + 2) * (traj ? kBlockTraj : 1) +
+           8 * (size_t)ecap * lanes + 8 * 4 * ((ext ? 2 : 1) * (size_t)n + 1) + 2 * (size_t)ecap * lanes;
 }
-
-// (-1i)^k is this sign times 1 (even k) or -1i (odd k).
-static __device__ __forceinline__ double block_sign(int k) { return (k & 2) ? -1.0 : 1.0; }
 
 // (-1i) * t as a packed pair
 static __device__ __forceinline__ f2x turn2(f2x t) {
     const float2 f = f2up(t);
     return f2pk(f.y, -f.x);
+}
+
+// 1i * t
+static __device__ __forceinline__ f2x rot2(f2x t) {
+    const float2 f = f2up(t);
+    return f2pk(-f.y, f.x);
 }
 
 // What a CTA knows of its orientation's series.
@@ -649,12 +635,12 @@ static __device__ __forceinline__ BlockSeries block_series(const BlockRun &R, in
     S.half = R.lev_half[lev];
     S.M = R.lev_m[lev];
     const int Kb = R.lev_k[lev];
-    const size_t at = (size_t)lev * R.Kmax * (R.Mcap + 1);
+    const size_t at = (size_t)lev * R.Kmax * block_row(R.Mcap);
     S.kcut = R.kcut + (size_t)lev * (R.Mcap + 1);
     S.K = Kb > 0 ? S.kcut[S.M] : 0;
     S.tab = R.table + at;
     S.tabf = R.tablef ? R.tablef + at : nullptr;
-    S.ld = (size_t)(S.M + 1);
+    S.ld = (size_t)block_row(S.M);
     S.nchunks = (R.nsteps + S.M) / S.M;
     S.j_last = R.nsteps - (S.nchunks - 1) * S.M;
     S.ok = !(Kb == 0 || (R.lev_raw[lev] + 2 > R.Kmax && S.K >= Kb - 2));
@@ -692,60 +678,76 @@ static __device__ __forceinline__ void block_phases(const BlockRun &R, const Blo
 }
 
 // FID points of chunk a: f_j = e^{-i c j dt} sum_k J_k(s j dt) (-1i)^k mu_k.
-// tr: the table in the run's precision.  Every thread calls, after a barrier;
-// the caller's next barrier ends it.
+// tr: the table in the run's precision.  After a barrier; the caller's next
+// barrier ends it.  An FP32 thread sums four neighbouring points over a part of
+// the terms: one 16-byte table load (from L2) and one moment serve all of them
+// (three spins, 200 orientations: 0.78 ms with one point a thread, 0.66 with
+// two, 0.65 with four; seven spins 1.68, 1.60, 1.54).  FP64 is bound by its
+// instructions and takes one point.
 template <class Vec, class Real>
 static __device__ __forceinline__ void block_points(const BlockLayout &B, const BlockRun &R, const BlockSeries &S,
                                                     const Real *tr, int a, int Kc, const Vec *s_mu, const Vec *s_phase,
                                                     Vec *s_rec, Vec *fid_out) {
-    const int tid = threadIdx.x, nt = (int)blockDim.x, M = S.M;
+    constexpr int N = sizeof(Real) == 4 ? kBlockPoints32 : kBlockPoints64, UN = 8;
+    using Wide = std::conditional_t<sizeof(Real) == 4, float4, double>;
+    const int M = S.M, tid = threadIdx.x, nt = blockDim.x;
     const int np = min(M, R.nsteps + 1 - a * M);                // points of this chunk
-    const int parts = max(1, nt / M);
+    const int cols = (np + N - 1) / N;                           // threads for all of them
+    const int parts = max(1, nt / cols);
     const int kper = ((Kc + parts - 1) / parts + 3) & ~3;
     const size_t ld = S.ld;
     for (int v = 0; v < B.nv; ++v) {
         const Vec *mu = s_mu + (size_t)v * (R.Kmax + 2);
         if (v > 0) __syncthreads();                              // s_rec reused
-        for (int jj = tid; jj < M * parts; jj += nt) {
-            const int j = jj % M, k0 = (jj / M) * kper, k1 = min(min(Kc, k0 + kper), S.kcut[j]);
-            Vec e = vzero<Vec>(), d = vzero<Vec>();              // even and odd terms
-            int k = k0;
-            // the table sits in L2: 16 loads in flight, then 4, then one
-            auto add = [&](auto nc) {
-                constexpr int N = decltype(nc)::value;
-                for (; k + N <= k1; k += N) {
-                    Real J[N];
+        for (int jj = tid; jj < cols * parts; jj += nt) {
+            const int j = (jj % cols) * N, part = jj / cols;
+            const int k0 = part * kper, k1 = min(min(Kc, k0 + kper), S.kcut[min(j + N - 1, M - 1)]);
+            Vec e[N], d[N];                                      // even and odd terms
 #pragma unroll
-                    for (int q = 0; q < N; ++q) J[q] = tr[(size_t)(k + q) * ld + j];
+            for (int q = 0; q < N; ++q) e[q] = d[q] = vzero<Vec>();
+            const Real *col = tr + j;
+            // the float table holds the signs of (-1i)^k, the double one does not
+            auto term = [&](int k, int odd, bool minus, const Wide &w) {
+                const Vec m = mu[k];
+                const Real *J = reinterpret_cast<const Real *>(&w);
 #pragma unroll
-                    for (int q = 0; q < N; ++q) {
-                        const Vec m = mu[k + q];
-                        const Real b = (q & 2) ? -J[q] : J[q];
-                        Vec &t = (q & 1) ? d : e;
-                        t.x += b * m.x;
-                        t.y += b * m.y;
-                    }
+                for (int q = 0; q < N; ++q) {
+                    const Real b = sizeof(Real) == 8 && minus ? -J[q] : J[q];
+                    Vec &t = odd ? d[q] : e[q];
+                    t.x += b * m.x;
+                    t.y += b * m.y;
                 }
             };
-            add(std::integral_constant<int, 16>{});
-            add(std::integral_constant<int, 4>{});
-            for (; k < k1; ++k) {
-                const Real b = (Real)block_sign(k) * tr[(size_t)k * ld + j];
-                Vec &t = (k & 1) ? d : e;
-                t.x += b * mu[k].x;
-                t.y += b * mu[k].y;
+            int k = k0;
+            for (; k + UN <= k1; k += UN) {
+                Wide w[UN];
+#pragma unroll
+                for (int u = 0; u < UN; ++u) w[u] = *reinterpret_cast<const Wide *>(col + (size_t)(k + u) * ld);
+#pragma unroll
+                for (int u = 0; u < UN; ++u) term(k + u, u & 1, u & 2, w[u]);
             }
-            Vec f;                                               // e - 1i d
-            f.x = e.x + d.y;
-            f.y = e.y - d.x;
-            s_rec[jj] = f;
+            for (; k < k1; ++k) {
+                const Wide w = *reinterpret_cast<const Wide *>(col + (size_t)k * ld);
+                if (k & 1) term(k, 1, k & 2, w);
+                else term(k, 0, k & 2, w);
+            }
+#pragma unroll
+            for (int q = 0; q < N; ++q) {
+                Vec f;                                           // e - 1i d
+                f.x = e[q].x + d[q].y;
+                f.y = e[q].y - d[q].x;
+                s_rec[part * cols * N + j + q] = f;
+            }
         }
         __syncthreads();
         Vec *out = fid_out + (size_t)B.vchan[v] * (R.nsteps + 1) + (size_t)a * M;
         const bool first = v == 0 || B.vchan[v] != B.vchan[v - 1];
         for (int j = tid; j < np; j += nt) {
             Vec f = s_rec[j];
-            for (int q = 1; q < parts; ++q) { f.x += s_rec[q * M + j].x; f.y += s_rec[q * M + j].y; }
+            for (int q = 1; q < parts; ++q) {
+                f.x += s_rec[q * cols * N + j].x;
+                f.y += s_rec[q * cols * N + j].y;
+            }
             const Vec ph = s_phase[j];
             Vec g;
             g.x = ph.x * f.x - ph.y * f.y;
@@ -781,20 +783,23 @@ static __device__ __forceinline__ void block_dispatch(const BlockLane &l, F &&f)
 // ---------------------------------------------------------------------------
 // TRJ: also the state at every step (R.traj_out), from chunks of at most
 // kBlockTraj steps whose inner states are summed beside the chunk-end state.
-template <bool CPLX, int ECAP, bool TRJ>
-__global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const DevSystem sys, const BlockLayout B,
-                                                                        const BlockRun R) {
+// The launch bounds set the registers: 96 up to 16 entries (80 for 8 gives
+// seven spins, 1000 orientations, 1.62 ms for 1.54), 128 for 24.
+template <bool EXT, int ECAP, bool TRJ>
+__global__ void __launch_bounds__(ECAP == 24 ? 512 : 640, 1)
+    block_chebyshev_kernel(const DevSystem sys, const BlockLayout B, const BlockRun R) {
     constexpr int NT = TRJ ? kBlockTraj - 1 : 0;
     __shared__ double s_coef[kMaxCoef];
-    __shared__ float2 s_x[2][kBlockRows + 1];
-    __shared__ float s_norm[2][kBlockRows / 32];
+    constexpr int XN = (EXT ? 2 : 1) * kBlockRows;            // the last slot takes what no one reads
+    __shared__ float2 s_x[2][XN + 1];
+    __shared__ float s_norm[2][kBlockRows / 32 + 2];
     __shared__ double2 s_turn[2];
     extern __shared__ __align__(16) unsigned char smem[];
     float2 *s_b = reinterpret_cast<float2 *>(smem);          // chunk-end coefficients (b, b)
     float2 *s_mu = s_b + (R.Kmax + 2);                        // moments, one row per detection row
     float2 *s_phase = s_mu + (size_t)(R.Kmax + 2) * B.nv;
     float2 *s_rec = s_phase + (R.Mcap + 1);
-    [[maybe_unused]] float2 *s_tb = s_rec + (blockDim.x > R.Mcap ? blockDim.x : R.Mcap);   // [step][term] inner states
+    [[maybe_unused]] float2 *s_tb = s_rec + block_rec(R.Mcap, blockDim.x, kBlockPoints32);  // [step][term] inner states
     const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const BlockLane l = block_lane(B, tid);
     const BlockSeries S = block_series(R, o);
@@ -802,31 +807,28 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
     const int nsteps = R.nsteps, M = S.M;
 
     // 2 L~ = 2 (L - c) / s: the recurrence is t_{k+1} = 2 L~ t_k - t_{k-1}
-    BlockEntries<CPLX, ECAP> E;
+    BlockEntries<ECAP> E;
     float dh = 0.f, dl = 0.f, di = 0.f;
     {
         const double scale = 2.0 / S.half;
-        double re[ECAP], im[ECAP];
+        double v[ECAP];
         double2 dg = make_double2(0.0, 0.0);
         if (R.saved) {
-            const double *save = R.saved + (size_t)o * block_saved(B.ecap, B.threads, CPLX);
+            const double *save = R.saved + (size_t)o * block_saved(B.ecap, B.threads);
 #pragma unroll
-            for (int i = 0; i < ECAP; ++i) {
-                re[i] = i < l.ew ? save[(size_t)i * B.threads + tid] : 0.0;
-                im[i] = CPLX && i < l.ew ? save[(size_t)(B.ecap + i) * B.threads + tid] : 0.0;
-            }
-            save += (size_t)(CPLX ? 2 : 1) * B.ecap * B.threads;
+            for (int i = 0; i < ECAP; ++i) v[i] = i < l.ew ? save[(size_t)i * B.threads + tid] : 0.0;
+            save += (size_t)B.ecap * B.threads;
             dg = make_double2(save[tid], save[B.threads + tid]);
         } else {
             const double sign = R.adjoint ? -1.0 : 1.0;
             block_coefficients(sys, R, o, s_coef);
-            block_assemble<CPLX, ECAP>(sys, B, l.ew, tid, s_coef, sign, re, im);
+            block_assemble<ECAP>(sys, B, l.ew, tid, s_coef, sign, v);
             if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef, sign);
         }
         const double sc = l.row < B.n ? scale : 1.0;          // detection rows keep their values
 #pragma unroll
         for (int i = 0; i < ECAP; ++i) {
-            E.set(i, re[i] * sc, im[i] * sc);
+            E.set(i, v[i] * sc);
             E.col[i] = i < l.ew ? B.col[i * B.threads + tid] * (int)sizeof(float2) : 0;
         }
         if (l.state) {
@@ -876,14 +878,17 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
     float start_n2 = norm2(st);
 
     const f2x DH = f2pk(dh, dh), DL = f2pk(dl, dl), DI = f2pk(-di, di);
-    const f2x NEG = l.state ? f2pk(-1.f, -1.f) : 0ull, HALF = l.state ? f2pk(0.5f, 0.5f) : f2pk(1.f, 1.f);
+    const f2x NEG = l.state ? f2pk(-1.f, -1.f) : 0ull;
     const char *x0 = reinterpret_cast<const char *>(&s_x[0][0]), *x1 = reinterpret_cast<const char *>(&s_x[1][0]);
     for (int a = 0; a < S.nchunks; ++a) {
         const bool last = a + 1 == S.nchunks;
         const int Kc = last ? min(S.K, S.kcut[S.j_last]) : S.K;
         mv += Kc - 1;
         if (last) coefficients(S.j_last, Kc);
-        if (l.state) s_x[0][l.row] = st;
+        if (l.state) {
+            s_x[0][l.row] = make_float2(0.5f * st.x, 0.5f * st.y);
+            if (EXT) s_x[0][B.n + l.row] = make_float2(-0.5f * st.y, 0.5f * st.x);
+        }
         __syncthreads();
         // Where this lane's result goes: a state row's into the other state
         // buffer, a detection row's into its moments (one further each term),
@@ -897,15 +902,18 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
             ad[0] = ad[1] + 8;
             inc = 16;
         } else {
-            ad[0] = ad[1] = smem_u32(&s_x[0][kBlockRows]);
+            ad[0] = ad[1] = smem_u32(&s_x[0][XN]);
         }
+        const uint32_t ext = l.state ? 8u * (uint32_t)B.n : 0u;
         // ntp = -t_{k-2}, so that a row's sum starts from it without another operation
         f2x tc = f2pk(st.x, st.y), ntp = 0ull;
-        f2x acc, accl;
+        // chunk-end sums over even and odd terms, each with its low-order part
+        f2x acc[2], accl[2] = {0ull, 0ull};
         {
             const f2x b0 = reinterpret_cast<const f2x *>(s_b)[0];
-            acc = mul2(b0, tc);
-            accl = fma2(b0, tc, sub2(0ull, acc));
+            acc[0] = mul2(b0, tc);
+            accl[0] = fma2(b0, tc, sub2(0ull, acc[0]));
+            acc[1] = 0ull;
         }
         [[maybe_unused]] f2x inner[NT + 1];
         if constexpr (TRJ) {
@@ -915,6 +923,9 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
             for (int j = 0; j < NT; ++j)
                 inner[j] = mul2(reinterpret_cast<const f2x *>(s_tb + (size_t)j * (R.Kmax + 2))[0], tc);
         }
+        // t_1 = L~ t_0: the first term works on t_0 / 2
+        f2x neg = add2(NEG, NEG);
+        tc = mul2(f2pk(0.5f, 0.5f), tc);
         auto term = [&](auto ewc, auto rnc, auto oddc, const char *src, int k) {
             constexpr int EW = decltype(ewc)::value, RND = decltype(rnc)::value;
             constexpr bool ODD = decltype(oddc)::value;
@@ -943,26 +954,26 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
                 Y = Sm;
             }
             f2x T = add2(Y, Lw);
-            if (k == 1) T = mul2(T, HALF);
             st_shared(ad[ODD], T);
+            if (EXT && l.state) st_shared(ad[ODD] + ext, rot2(T));
             ad[ODD] += inc;
             block_sync();
-            const f2x V = ODD ? turn2(T) : T;
-            const f2x Sm = fma2(b, V, acc);
-            accl = add2(accl, fma2(b, V, sub2(acc, Sm)));
-            acc = Sm;
+            const f2x Sm = fma2(b, T, acc[ODD]);
+            accl[ODD] = add2(accl[ODD], fma2(b, T, sub2(acc[ODD], Sm)));
+            acc[ODD] = Sm;
             if constexpr (TRJ) {
 #pragma unroll
                 for (int j = 0; j < NT; ++j)
-                    inner[j] = fma2(reinterpret_cast<const f2x *>(s_tb + (size_t)j * (R.Kmax + 2))[k], V, inner[j]);
+                    inner[j] = fma2(reinterpret_cast<const f2x *>(s_tb + (size_t)j * (R.Kmax + 2))[k], ODD ? turn2(T) : T, inner[j]);
             }
-            ntp = mul2(NEG, tc);
+            ntp = mul2(neg, tc);
             tc = T;
         };
         auto terms = [&](auto ewc, auto rnc) {
             for (int k = 1; k <= Kc; k += 2) {
                 term(ewc, rnc, std::true_type{}, x0, k);
-                if (k + 1 <= Kc) term(ewc, rnc, std::false_type{}, x1, k + 1);
+                neg = NEG;
+                if (k < Kc) term(ewc, rnc, std::false_type{}, x1, k + 1);
             }
         };
         block_dispatch<ECAP>(l, terms);
@@ -977,7 +988,12 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
                         make_float2(ph.x * f.x - ph.y * f.y, ph.x * f.y + ph.y * f.x);
                 }
         }
-        const float2 fin = f2up(add2(acc, accl));
+        float2 fin;
+        {
+            // even - 1i odd, rounded once
+            const f2x O = turn2(acc[1]), Sm = add2(acc[0], O);
+            fin = f2up(add2(Sm, add2(add2(O, sub2(acc[0], Sm)), add2(accl[0], turn2(accl[1])))));
+        }
         st = make_float2(0.f, 0.f);
         if (l.state) {
             const double2 ph = s_turn[last ? 1 : 0];
@@ -1011,7 +1027,7 @@ __global__ void __launch_bounds__(kBlockRows, 1) block_chebyshev_kernel(const De
 // four units; values and columns sit in shared memory, whose loads cost
 // nothing beside them, so that every warp runs just its own entries.
 // ---------------------------------------------------------------------------
-template <bool CPLX, bool TRJ>
+template <bool EXT, bool TRJ>
 __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(const DevSystem sys, const BlockLayout B,
                                                                               const BlockRun R) {
     constexpr int NT = TRJ ? kBlockTraj - 1 : 0;
@@ -1019,16 +1035,18 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
     __shared__ double s_norm[2][2 * kBlockRows / 32];
     __shared__ double2 s_turn[2];
     extern __shared__ __align__(16) unsigned char smem[];
-    const int T = B.threads, n = B.n, xs = n + 1;
-    const size_t rec = (size_t)(2 * T > R.Mcap ? 2 * T : R.Mcap);
+    const int T = B.threads, n = B.n, xs = (EXT ? 2 : 1) * n + 1;
+    const size_t rec = block_rec(R.Mcap, 2 * T, kBlockPoints64);
     double2 *s_rec = reinterpret_cast<double2 *>(smem);
     double2 *s_phase = s_rec + rec;
     double2 *s_mu = s_phase + (R.Mcap + 1);
     double *s_b = reinterpret_cast<double *>(s_mu + (size_t)(R.Kmax + 2) * B.nv);
-    double *s_x = s_b + (R.Kmax + 2);                         // [buffer][part][n + 1]
-    double *s_val = s_x + 4 * (size_t)xs;                     // [entry][lane], imaginary parts after
+    // [buffer][part]: a part of the states, with EXT also that part of 1i times
+    // them, and a slot that lanes without a state row read
+    double *s_x = s_b + (R.Kmax + 2);
+    double *s_val = s_x + 4 * (size_t)xs;                     // [entry][lane]
     [[maybe_unused]] double *s_tb = nullptr;                  // trajectories: [step][term]
-    double *s_end = s_val + (size_t)B.ecap * T * (CPLX ? 2 : 1);
+    double *s_end = s_val + (size_t)B.ecap * T;
     if constexpr (TRJ) {
         s_tb = s_end;
         s_end += NT * (size_t)(R.Kmax + 2);
@@ -1046,15 +1064,14 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
     block_coefficients(sys, R, o, s_coef);
     const double sc = l.row < n ? scale : 1.0, sign = R.adjoint ? -1.0 : 1.0;
     for (int i = 4 * part; i < l.ew; i += 8) {                // the two threads of a lane take turns
-        double re[4], im[4];
+        double v[4];
         BlockLayout Bi = B;
         Bi.src = B.src + (size_t)i * T;
-        block_assemble<CPLX, 4>(sys, Bi, min(4, l.ew - i), t, s_coef, sign, re, im);
+        block_assemble<4>(sys, Bi, min(4, l.ew - i), t, s_coef, sign, v);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             if (i + q < l.ew) {
-                s_val[(size_t)(i + q) * T + t] = re[q] * sc;
-                if (CPLX) s_val[(size_t)(B.ecap + i + q) * T + t] = im[q] * sc;
+                s_val[(size_t)(i + q) * T + t] = v[q] * sc;
                 s_col[(size_t)(i + q) * T + t] = B.col[(size_t)(i + q) * T + t];
             }
     }
@@ -1076,7 +1093,7 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
             s_tb[(size_t)(j - 1) * (R.Kmax + 2) + k] = k < S.K && j < M ? block_sign(k) * S.tab[k * S.ld + j] : 0.0;
         }
     }
-    if (tid < 4) s_x[tid * xs + n] = 0.0;                     // read by lanes without a state row
+    if (tid < 4) s_x[tid * xs + xs - 1] = 0.0;
 
     double st = 0.0;
     if (l.state) {
@@ -1102,15 +1119,20 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
     };
     double start_n2 = norm2(st);
 
-    const int own = l.state ? l.row : n;                      // where the diagonal's other part is read
-    const double *val = s_val + t, *vim = s_val + (size_t)B.ecap * T + t;
+    const int own = l.state ? l.row : xs - 1;                 // where the diagonal's other part is read
+    const double *val = s_val + t;
+    // a state's part, and that part of 1i times it in the other part's array
+    auto store = [&](int buf, double y) {
+        s_x[(2 * buf + part) * xs + l.row] = y;
+        if (EXT) s_x[(2 * buf + 1 - part) * xs + n + l.row] = part ? -y : y;
+    };
     const uint16_t *col = s_col + t;
     for (int a = 0; a < S.nchunks; ++a) {
         const bool last = a + 1 == S.nchunks;
         const int Kc = last ? min(S.K, S.kcut[S.j_last]) : S.K;
         mv += Kc - 1;
         if (last) coefficients(S.j_last, Kc);
-        if (l.state) s_x[part * xs + l.row] = st;
+        if (l.state) store(0, st);
         __syncthreads();
         double tc = st, tp = 0.0, even = s_b[0] * st, odd = 0.0;
         [[maybe_unused]] double ie[NT + 1], io[NT + 1];
@@ -1127,25 +1149,16 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
             if (damped) y = fma(dm, xo[own], y);
             int i = 0;
             for (; i + 4 <= l.ew; i += 4) {
-                double v[4], w[4], X[4], Xo[4];
+                double v[4], X[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const int c = col[(i + q) * T];
                     v[q] = val[(i + q) * T];
-                    X[q] = x[c];
-                    if (CPLX) { w[q] = vim[(i + q) * T]; Xo[q] = xo[c]; }
+                    X[q] = x[col[(i + q) * T]];
                 }
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    y = fma(v[q], X[q], y);
-                    if (CPLX) y = fma(part ? w[q] : -w[q], Xo[q], y);
-                }
+                for (int q = 0; q < 4; ++q) y = fma(v[q], X[q], y);
             }
-            for (; i < l.ew; ++i) {
-                const int c = col[i * T];
-                y = fma(val[i * T], x[c], y);
-                if (CPLX) y = fma(part ? vim[i * T] : -vim[i * T], xo[c], y);
-            }
+            for (; i < l.ew; ++i) y = fma(val[i * T], x[col[i * T]], y);
             for (int r = 0; r < l.rounds; ++r) {
                 const double u = __shfl_xor_sync(0xffffffffu, y, 1 << r);
                 if ((l.parts >> r) > 1) y += u;
@@ -1153,7 +1166,7 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
             tp = 0.0;
             if (l.state) {
                 if (k == 1) y *= 0.5;
-                s_x[(2 * (buf ^ 1) + part) * xs + l.row] = y;
+                store(buf ^ 1, y);
                 acc = fma(s_b[k], y, acc);
                 if constexpr (TRJ) {
 #pragma unroll

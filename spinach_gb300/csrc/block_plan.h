@@ -28,11 +28,11 @@ struct Components {
 // The coupled rows and everything a layout needs, in numbers of their own
 // (0 .. n-1, in the order of the system's rows).
 struct BlockPattern {
-    struct Entry { int col, src; };           // src: ELL entry, or -2-i for value i of a detection row
+    struct Entry { int col, src; };           // as BlockLayout::col and src
     int n = 0, nv = 0;
     std::vector<int> rows;                    // system row of every coupled row
     std::vector<std::vector<Entry>> entries;  // n state rows, then nv detection rows
-    std::vector<double> values;               // detection rows' values (re, im)
+    std::vector<double> values;               // detection rows' values
     std::vector<int> vchan, vfac;
 };
 
@@ -47,22 +47,25 @@ struct BlockLanes {
     std::vector<uint16_t> col;
 };
 
-// Cost model of a term (cycles): what its warps issue and how long it takes end
-// to end.  FP32 (measured on GB300): an entry is five packed multiply-adds of
-// two FMA cycles and a load, a split row's reduction step about 55 cycles, the
-// rest of a term about 130.  FP64: one instruction holds a warp and its FP64
+// Cost model of a term (cycles): what its warps issue, and how long it takes end
+// to end (the busiest of the SM's four units, warp w on unit w mod 4).  FP32
+// (measured on GB300): an entry is five packed multiply-adds of two FMA cycles
+// and a load, a split row's reduction step about 55 cycles, the rest of a term
+// 45 to issue and about 120 of latency.  FP64: one instruction holds a warp and its FP64
 // unit for 64 cycles and the SM has four units; a row is two lanes (real and
-// imaginary part), each with one instruction per entry (two for complex
-// values) and reduction step and three or four of its own.
+// imaginary part), each with one instruction per entry and reduction step and
+// three or four of its own.
 struct BlockCost {
     double issue = 0.0;        // all warps of one orientation, cycles of the SM's unit
     double latency = 0.0;
     int warps = 0;             // of one orientation's CTA
     int warps_per_sm = 16;     // resident, by registers
-    // relative time of n orientations per SM
+    // relative time of n orientations per SM: rounds of as many as fit, the last
+    // with what is left
     double time(double per_sm) const {
-        const double res = std::max(1.0, std::min(per_sm, std::floor((double)warps_per_sm / warps)));
-        return std::ceil(per_sm / res) * std::max(latency, res * issue);
+        const double res = std::max(1.0, std::floor((double)warps_per_sm / warps)), full = std::floor(per_sm / res);
+        const double rest = std::ceil(per_sm - full * res);
+        return full * std::max(latency, res * issue) + (rest > 0.0 ? std::max(latency, rest * issue) : 0.0);
     }
 };
 
@@ -85,7 +88,7 @@ inline size_t block_lane_count(const BlockPattern &P, int e) {
 
 // The layout on `warps` warps with at most e entries per lane; false if the
 // rows do not fit.
-inline bool block_lanes(const BlockPattern &P, int warps, int e, bool f64, bool cplx, bool damped, BlockLanes &L,
+inline bool block_lanes(const BlockPattern &P, int warps, int e, bool f64, bool damped, BlockLanes &L,
                         BlockCost &cost) {
     if (block_lane_count(P, e) > 32u * (size_t)warps) return false;
     const int T = 32 * warps, nr = P.n + P.nv;
@@ -129,9 +132,8 @@ inline bool block_lanes(const BlockPattern &P, int warps, int e, bool f64, bool 
     double unit[4] = {0.0, 0.0, 0.0, 0.0};
     for (int w = 0; w < warps; ++w) {
         L.shape[w] = ew[w] | (rounds[w] << 8);
-        const double c = cplx ? 2.0 : 1.0;
         if (f64) {
-            const double n = 64.0 * (c * ew[w] + rounds[w] + (damped ? 4.0 : 3.0));
+            const double n = 64.0 * (ew[w] + rounds[w] + (damped ? 4.0 : 3.0));
             cost.issue += 2.0 * n / 4.0;
             unit[w % 4] += n;
             unit[(w + warps) % 4] += n;
@@ -142,14 +144,14 @@ inline bool block_lanes(const BlockPattern &P, int warps, int e, bool f64, bool 
             const int step = cap <= 8 ? 1 : cap / 8;
             const double n = rounds[w] ? cap : std::max(step, (ew[w] + step - 1) / step * step);
             const double r = rounds[w] > 2 ? 5 : rounds[w];
-            cost.issue += (11.0 * c * n + 20.0 * r + 45.0) / 4.0;
-            cost.latency = std::max(cost.latency, 130.0 + 11.0 * c * n + 55.0 * r);
+            const double own = 11.0 * n + 20.0 * r + 45.0;
+            cost.issue += own / 4.0;
+            unit[w % 4] += own;
+            cost.latency = std::max(cost.latency, own + 35.0 * r);
         }
     }
-    if (f64) {
-        for (double u : unit) cost.latency = std::max(cost.latency, u);
-        cost.latency += 200.0;
-    }
+    for (double u : unit) cost.latency = std::max(cost.latency, u);
+    cost.latency += f64 ? 200.0 : 120.0;
     if (cost.warps > 1) cost.latency += 30.0;
     return true;
 }

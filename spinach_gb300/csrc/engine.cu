@@ -157,6 +157,7 @@ struct spx_handle {
     // coupled states of the plain acquisition (rebuilt with the coils and the
     // initial states) and what finding them takes
     std::vector<uint16_t> ell_col_host;
+    std::vector<unsigned char> ell_parts;       // per ELL entry: 1 a real part, 2 an imaginary part in some stream
     std::vector<int> component;     // connected component of every row under L
     std::vector<double2> rho0_host;             // sliced order
     std::vector<int> coil_row_host, coil_chan_host;
@@ -264,8 +265,13 @@ void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<i
     P.rows = rows;
     P.n = (int)rows.size();
     P.entries.resize(P.n);
+    std::vector<int> ent, esrc;                   // the whole entries, for the dense kernels
     for_each_coupling(h, [&](int r, int c, int e) {
-        if (own[r] >= 0) P.entries[own[r]].push_back({own[c], e});
+        if (own[r] < 0) return;
+        ent.push_back(own[c] * P.n + own[r]);
+        esrc.push_back(e);
+        if (h->ell_parts[e] & 1) P.entries[own[r]].push_back({own[c], e});
+        if (h->ell_parts[e] & 2) P.entries[own[r]].push_back({P.n + own[c], h->ell_len + e});
     });
     // detection rows conj(coil): a complex coil on real values takes a row for
     // its real and one for its imaginary parts (times -1i)
@@ -276,10 +282,13 @@ void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<i
                 const int r = own[h->coil_row_host[i]];
                 const double2 v = h->coil_val_host[i];
                 if (h->coil_chan_host[i] != ch || r < 0) continue;
-                if (!h->cplx && (im ? v.y : v.x) == 0.0) continue;
-                row.push_back({r, -2 - (int)(P.values.size() / 2)});
-                P.values.push_back(h->cplx || !im ? v.x : v.y);
-                P.values.push_back(h->cplx ? -v.y : 0.0);
+                auto add = [&](int col, double x) {
+                    if (x == 0.0) return;
+                    row.push_back({col, -2 - (int)P.values.size()});
+                    P.values.push_back(x);
+                };
+                if (h->cplx) { add(r, v.x); add(P.n + r, -v.y); }
+                else add(r, im ? v.y : v.x);
             }
             if (im && row.empty()) continue;
             P.entries.push_back(row);
@@ -287,10 +296,8 @@ void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<i
             P.vfac.push_back(im);
             ++P.nv;
         }
-    std::vector<int> ent, esrc, crow, cchan;
+    std::vector<int> crow, cchan;
     std::vector<double2> cval;
-    for (int i = 0; i < P.n; ++i)
-        for (auto &e : P.entries[i]) { ent.push_back(e.col * P.n + i); esrc.push_back(e.src); }
     if (detect)
         for (size_t i = 0; i < h->coil_row_host.size(); ++i)
             if (own[h->coil_row_host[i]] >= 0) {
@@ -319,7 +326,7 @@ void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<i
     struct At { size_t row, part, shape, src, col; };
     std::vector<At> at[2];
     for (int p = 0; p < 2; ++p) {
-        const int ecap_max = p == 1 ? 32 : h->cplx ? 16 : spx::kBlockMaxEntries;
+        const int ecap_max = p == 1 ? 32 : spx::kBlockMaxEntries;
         int widest = 1;
         for (auto &r : P.entries) widest = std::max(widest, (int)r.size());
         std::vector<spx::BlockLanes> lanes;
@@ -330,14 +337,14 @@ void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<i
             if (w > spx::kBlockRows / 32) continue;
             spx::BlockLanes L;
             spx::BlockCost c;
-            if (block_lanes(P, w, e, p == 1, h->cplx, h->max_im_diag > 0.0, L, c)) {
+            if (block_lanes(P, w, e, p == 1, h->max_im_diag > 0.0, L, c)) {
                 lanes.push_back(std::move(L));
                 costs.push_back(c);
             }
         }
         if (lanes.empty()) { plan.layouts[0].clear(); return; }
         std::vector<size_t> keep;
-        for (double per_sm : {1.0, 2.0, 3.0, 5.0, 8.0, 27.0}) {
+        for (double per_sm : {0.5, 1.5, 2.5, 4.5, 7.0, 13.0, 27.0}) {
             size_t best = 0;
             for (size_t i = 1; i < lanes.size(); ++i)
                 if (costs[i].time(per_sm) < costs[best].time(per_sm)) best = i;
@@ -373,7 +380,7 @@ void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<i
             b.col = reinterpret_cast<const uint16_t *>(d + at[p][i].col);
             b.row_src = reinterpret_cast<const int *>(d + o_rows);
             b.state_pos = reinterpret_cast<const int *>(d + o_pos);
-            b.vval = reinterpret_cast<const double2 *>(d + o_val);
+            b.vval = reinterpret_cast<const double *>(d + o_val);
             b.vchan = reinterpret_cast<const int *>(d + o_chan);
             b.vfac = reinterpret_cast<const int *>(d + o_fac);
         }
@@ -708,6 +715,12 @@ void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32
     // scales them into (-1, 1) for the packed FP32 layout
     h->lo_scale = g_upper > 0.0 ? std::ldexp(1.0, -std::ilogb(g_upper) - 1) : 1.0;
     h->max_im_diag = max_im_diag;
+    h->ell_parts.assign(std::max(ell_len, 1), 0);
+    for (int q = 0; q < nst; ++q)
+        for (int e = 0; e < ell_len; ++e) {
+            if (std::fabs(ell_re[(size_t)q * ell_len + e]) > im_tol) h->ell_parts[e] |= 1;
+            if (cplx && std::fabs(ell_im[(size_t)q * ell_len + e]) > im_tol) h->ell_parts[e] |= 2;
+        }
     h->ell_col_host = std::move(ell_col);
     h->row_bound = std::move(row_bound);
     h->rho0_host = std::move(r0);
@@ -822,7 +835,6 @@ struct Config {
     const BlockPlan::Layout *blk = nullptr, *blk_bounds = nullptr;
     double blk_x = 0.0;
     int blk_M = 0, blk_K = 0, blk_lev = 0;
-    bool blk_cplx = false;
     int blk_which = 0;                            // the propagation kernel (spx_block_kernel_*)
     // FP64 by dense matrices (dense.cuh): states and detection rows kept,
     // squarings of the scaled exponential
@@ -960,7 +972,7 @@ const BlockPlan::Layout *best_layout(const std::vector<BlockPlan::Layout> &ls, d
 bool configure_block(spx_handle *h, const BlockPlan &plan, int64_t n_orient, double dt, int64_t nsteps, bool f64,
                      double chunk_target, int kmax_override, int m_cap, bool traj, Config &c) {
     if (!plan.ok) return false;
-    const double per_sm = std::ceil((double)n_orient / h->sm_count);
+    const double per_sm = (double)n_orient / h->sm_count;
     const BlockPlan::Layout *best = best_layout(plan.layouts[f64 ? 1 : 0], per_sm);
     if (!best) return false;
     c.blk_x = chunk_target > 0 ? chunk_target : 300.0;
@@ -979,7 +991,6 @@ bool configure_block(spx_handle *h, const BlockPlan &plan, int64_t n_orient, dou
     SPX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(h->smem_optin - fa.sharedSizeBytes)));
     c.blk = best;
-    c.blk_cplx = h->cplx;
     c.blk_bounds = f64 ? best_layout(plan.layouts[0], per_sm) : best;
     return true;
 }
@@ -1005,7 +1016,7 @@ void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, 
     const double products = 6.0 + scale + squarings;
     const double work = 4.0 * n * n * (products * n + m + rows * h->nchan) + 4.0 * n * npts * h->nchan;
     const double dense = std::max(work * n_orient / (2.0 * h->sm_count), 0.0) + 6000.0 * (products + squarings + 4.0);
-    const double per_sm = std::ceil((double)n_orient / h->sm_count);
+    const double per_sm = (double)n_orient / h->sm_count;
     // the spectral half-width is about an eighth of the row bound (5.6 to 11.5
     // on the benchmark systems), a chunk's series a quarter longer than its
     // argument, and a term takes twice the model's cycles alone, 1.5 times in
@@ -1159,13 +1170,13 @@ Config choose_config(spx_handle *h, int64_t n_orient, double dt, int64_t nsteps,
 // propagation (both on one layout) while it takes at most 512 MB; larger grids
 // assemble it twice (a radical's 4000 orientations: 96 MB).
 size_t saved_block(const Config &c) {
-    return spx::block_saved(c.blk->dev.ecap, c.blk->dev.threads, c.blk_cplx);
+    return spx::block_saved(c.blk->dev.ecap, c.blk->dev.threads);
 }
 bool saves_block(int64_t n_orient, bool f64, const Config &c) {
     return !f64 && (double)n_orient * (double)saved_block(c) <= 64e6;
 }
 
-size_t block_table_entries(const Config &c) { return (size_t)c.blk_lev * c.blk_K * (c.blk_M + 1); }
+size_t block_table_entries(const Config &c) { return (size_t)c.blk_lev * c.blk_K * spx::block_row(c.blk_M); }
 
 void reserve_block(BlockBufs &b, int64_t n_orient, bool f64, const Config &c) {
     b.centre.reserve(n_orient);

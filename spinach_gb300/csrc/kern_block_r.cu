@@ -1,4 +1,4 @@
-// Instantiations of the coupled-state kernels for one value type.
-#define SPX_INST_CPLX 0
+// Instantiations of the coupled-state kernels for real values.
+#define SPX_INST_EXT 0
 #define SPX_INST_FN spx_block_kernel_r
 #include "kern_block.inc"
