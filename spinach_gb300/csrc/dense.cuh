@@ -1,5 +1,6 @@
-// FP64 propagation of few coupled states, or of few orientations, by dense
-// matrices instead of series terms.
+// Propagation of few coupled states, or of few orientations, by dense matrices
+// in FP64 instead of series terms, for FP64 runs and, rounded at the end, for
+// FP32 runs that are over sooner this way.
 //
 // An FP64 series term is a chain of instructions that hold a warp for 64
 // cycles each, and a run of N steps takes thousands of terms one after another
@@ -187,12 +188,20 @@ static __global__ void __launch_bounds__(kDenseThreads, 24) dense_rows_kernel(in
         base[(size_t)(have + j) * n + c] = sum;
     }
 }
+// Orientations whose points an FP32 run also keeps unrounded (its check against
+// FP64): number j is orientation ((2 j + 1) of n) / (2 count).
+struct DenseCheck {
+    double2 *fids;              // [count][nchan][npts]
+    int *status;                // [count]
+    int count;
+};
 // fids[o][ch][a m + j] = Y[a] . V[j]
+template <class Vec>
 static __global__ void __launch_bounds__(kDenseThreads, 24) dense_points_kernel(int64_t n_orient, int n, int nchan, int rows,
                                                                                 int m, int npts,
                                                                                 const double2 *__restrict__ Y,
-                                                                                const double2 *__restrict__ V, double2 *fids,
-                                                                                int *status) {
+                                                                                const double2 *__restrict__ V, Vec *fids,
+                                                                                int *status, const DenseCheck check) {
     const int64_t per = (int64_t)nchan * npts;
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n_orient * per;
          q += (int64_t)gridDim.x * blockDim.x) {
@@ -201,8 +210,14 @@ static __global__ void __launch_bounds__(kDenseThreads, 24) dense_points_kernel(
         const double2 *y = Y + ((o * nchan + ch) * rows + a) * n, *v = V + (o * m + j) * n;
         double2 s = make_double2(0.0, 0.0);
         for (int k = 0; k < n; ++k) dense_mac(s, y[k], v[k]);
-        fids[q] = s;
-        if (!isfinite(s.x) || !isfinite(s.y)) status[o] = kDevNonFinite;
+        fids[q] = tovec(s, Vec());
+        const bool finite = isfinite(s.x) && isfinite(s.y);
+        if (!finite) status[o] = kDevNonFinite;
+        for (int c = 0; c < check.count; ++c)
+            if (((2 * (long long)c + 1) * n_orient) / (2 * (long long)check.count) == o) {
+                check.fids[c * per + e] = s;
+                if (!finite) check.status[c] = kDevNonFinite;
+            }
     }
 }
 

@@ -836,7 +836,7 @@ struct Config {
     double blk_x = 0.0;
     int blk_M = 0, blk_K = 0, blk_lev = 0;
     int blk_which = 0;                            // the propagation kernel (spx_block_kernel_*)
-    // FP64 by dense matrices (dense.cuh): states and detection rows kept,
+    // by dense matrices (dense.cuh): states and detection rows kept,
     // squarings of the scaled exponential
     const BlockPlan *dense = nullptr;
     int dense_m = 0, dense_rows = 0, dense_scale = 0;
@@ -995,14 +995,16 @@ bool configure_block(spx_handle *h, const BlockPlan &plan, int64_t n_orient, dou
     return true;
 }
 
-// Chooses the dense kernels for an FP64 run on the coupled states when their
-// modelled time is below the series': both in cycles, by FP64 instructions (2
-// lanes a cycle on each SM) or by latency (about 6000 cycles from one of the
+// Chooses the dense kernels for a run on the coupled states when their modelled
+// time is below the series': both in cycles, by FP64 instructions (2 lanes a
+// cycle on each SM) or by latency (6000 cycles and 470 a state from one of the
 // dense launches to the next; the layout's latency for each series term).
-// Measured sides, one orientation of 52 states and 2048 steps: dense 0.25 ms,
-// series 2.3 ms; 1000 of them: series 11 ms, dense 16 ms; 400 of 8 states and
-// 1024 steps: dense 0.2 ms, series 1.4 ms.
-void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, double dt, int64_t nsteps, Config &c) {
+// Measured sides (coupled states, orientations, steps): FP64 52, 1, 2048: dense
+// 0.5 ms, series 2.3 ms; 52, 1000, 2048: 16 and 11 ms; 8, 400, 1024: 0.2 and
+// 1.4 ms.  FP32 6, 200, 1024: 0.17 and 0.65 ms; 20, 200, 1024: 0.56 and 1.02;
+// 20, 1000, 1024: 1.86 and 1.28; 52, 1, 1024: 0.50 and 0.36; 70, 1, 1024: 0.67
+// and 1.09.
+void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, double dt, int64_t nsteps, bool f64, Config &c) {
     const double n = plan.n, npts = (double)nsteps + 1.0;
     // rounding doubles with every squaring; and the matrices take memory
     if (nsteps > 8192 || 6.0 * n_orient * n * n * sizeof(double2) > 1e9) return;
@@ -1015,14 +1017,15 @@ void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, 
     while (std::ldexp(plan.bound * dt, -scale) > 0.5) ++scale;
     const double products = 6.0 + scale + squarings;
     const double work = 4.0 * n * n * (products * n + m + rows * h->nchan) + 4.0 * n * npts * h->nchan;
-    const double dense = std::max(work * n_orient / (2.0 * h->sm_count), 0.0) + 6000.0 * (products + squarings + 4.0);
+    const double dense = std::max(work * n_orient / (2.0 * h->sm_count), 0.0) + (6000.0 + 470.0 * n) * (products + squarings + 4.0);
     const double per_sm = (double)n_orient / h->sm_count;
     // the spectral half-width is about an eighth of the row bound (5.6 to 11.5
     // on the benchmark systems), a chunk's series a quarter longer than its
-    // argument, and a term takes twice the model's cycles alone, 1.5 times in
-    // company
+    // argument, and an FP64 term takes twice the model's cycles alone, 1.5 times
+    // in company; FP32 terms 0.85 to 1.5 times, after 130 us of bounds and tables
     const double terms = 1.25 * plan.bound / 8.0 * dt * npts + 30.0;
-    const double series = terms * (per_sm > 2.0 ? 1.5 : 2.0) * c.blk->cost.time(per_sm) + 1e5;
+    const double factor = f64 ? (per_sm > 2.0 ? 1.5 : 2.0) : per_sm > 2.0 ? 1.5 : per_sm > 1.0 ? 1.2 : 0.85;
+    const double series = terms * factor * c.blk->cost.time(per_sm) + (f64 ? 1e5 : 2.5e5);
     if (dense > series) return;
     c.dense = &plan;
     c.dense_m = m;
@@ -1045,9 +1048,9 @@ void choose_block(spx_handle *h, const BlockPlan *plan, int64_t n_orient, double
     // in FP64, so the decision stays the one it has been (a three-spin system,
     // 16384 steps: 1.2e-5 on the whole system, 3.5e-6 on its coupled states)
     if (!f64 && h->max_im_diag == 0.0 && nsteps > 8192) return;
-    if (configure_block(h, *plan, n_orient, dt, nsteps, f64, opt.chunk_target, kmax_override, m_cap, false, c) && f64 &&
+    if (configure_block(h, *plan, n_orient, dt, nsteps, f64, opt.chunk_target, kmax_override, m_cap, false, c) &&
         kmax_override == 0 && m_cap == 256)
-        choose_dense(h, *plan, n_orient, dt, nsteps, c);
+        choose_dense(h, *plan, n_orient, dt, nsteps, f64, c);
 }
 
 // traj: the run writes the state at every step (chunks of opt.chunk_steps
@@ -1275,11 +1278,12 @@ void reserve_dense(const spx_handle *h, DenseBufs &b, int64_t n_orient, const Co
     b.Y.reserve((size_t)n_orient * h->nchan * c.dense_rows * n);
 }
 
-// An FP64 run by dense matrices: out and the status words as the propagation
-// kernels write them.  pick: see BlockRun.
+// A run by dense matrices: out (of type Vec) and the status words as the
+// propagation kernels write them.  pick: see BlockRun.
+template <class Vec>
 void launch_dense(spx_handle *h, const Config &c, spx::DevSystem &sys, DenseBufs &b, int64_t n_orient, int pick,
-                  const double *d_al, const double *d_be, const double *d_ga, double dt, int64_t nsteps, double2 *out,
-                  const spx::DevRun &words, cudaStream_t stream) {
+                  const double *d_al, const double *d_be, const double *d_ga, double dt, int64_t nsteps, Vec *out,
+                  const spx::DevRun &words, cudaStream_t stream, const spx::DenseCheck &check = spx::DenseCheck{}) {
     const BlockPlan &plan = *c.dense;
     const int n = plan.n, m = c.dense_m, rows = c.dense_rows;
     const int64_t total = n_orient * n * n;
@@ -1341,8 +1345,8 @@ void launch_dense(spx_handle *h, const Config &c, spx::DevSystem &sys, DenseBufs
         if (2 * have < rows) square();
     }
     const int64_t npts = nsteps + 1;
-    spx::dense_points_kernel<<<grid(n_orient * h->nchan * npts), spx::kDenseThreads, 0, stream>>>(
-        n_orient, n, h->nchan, rows, m, (int)npts, b.Y.p, b.V.p, out, words.status);
+    spx::dense_points_kernel<Vec><<<grid(n_orient * h->nchan * npts), spx::kDenseThreads, 0, stream>>>(
+        n_orient, n, h->nchan, rows, m, (int)npts, b.Y.p, b.V.p, out, words.status, check);
     ++h->launches;
     SPX_CUDA(cudaGetLastError());
 }
@@ -1558,7 +1562,19 @@ void launch_powder(spx_handle *h, int64_t n_orient, const double *d_al, const do
     run.next_orient = h->d_counter.p;
 
     int chk = 0;
-    if (fp32_check && !f64) {
+    spx::DenseCheck kept{};
+    if (fp32_check && !f64 && c.dense) {
+        // an FP32 run by dense matrices is an FP64 run that is rounded at the
+        // end: the check takes its unrounded points
+        chk = (int)std::min<int64_t>(kCheckOrients, n_orient);
+        h->d_chk_fids.reserve(npts * chk * sizeof(double2));
+        h->d_chk_status.reserve(chk);
+        h->chk_index.resize(chk);
+        for (int j = 0; j < chk; ++j) h->chk_index[j] = check_index(j, chk, n_orient);
+        static_assert(spx::kDevOk == 0, "status words start at zero");
+        SPX_CUDA(cudaMemsetAsync(h->d_chk_status.p, 0, chk * sizeof(int), h->stream));
+        kept = {reinterpret_cast<double2 *>(h->d_chk_fids.p), h->d_chk_status.p, chk};
+    } else if (fp32_check && !f64) {
         // the FP64 re-run takes its CTAs' SMs; an FP32 run of several waves
         // keeps the rest (a single-wave grid keeps every CTA: fewer would add
         // a wave)
@@ -1570,8 +1586,12 @@ void launch_powder(spx_handle *h, int64_t n_orient, const double *d_al, const do
     }
     if (timed) SPX_CUDA(cudaEventRecord(h->ev[0], h->stream));
     if (c.dense) {
-        launch_dense(h, c, sys, h->dense, n_orient, 0, d_al, d_be, d_ga, dt, nsteps,
-                     reinterpret_cast<double2 *>(h->d_fids.p), run, h->stream);
+        if (f64)
+            launch_dense(h, c, sys, h->dense, n_orient, 0, d_al, d_be, d_ga, dt, nsteps,
+                         reinterpret_cast<double2 *>(h->d_fids.p), run, h->stream);
+        else
+            launch_dense(h, c, sys, h->dense, n_orient, 0, d_al, d_be, d_ga, dt, nsteps,
+                         reinterpret_cast<float2 *>(h->d_fids.p), run, h->stream, kept);
     } else if (c.blk) {
         spx::BlockRun r{};
         BlockBufs &b = h->blk;
@@ -1590,7 +1610,7 @@ void launch_powder(spx_handle *h, int64_t n_orient, const double *d_al, const do
     }
     if (timed) SPX_CUDA(cudaEventRecord(h->ev[1], h->stream));
     launch_powder_sum(h, f64, h->d_fids.p, d_w, n_orient, npts, h->d_part.p, d_out);
-    if (chk) SPX_CUDA(cudaStreamWaitEvent(h->stream, h->ev_join, 0));   // the FP64 re-run is part of the run
+    if (chk && !kept.count) SPX_CUDA(cudaStreamWaitEvent(h->stream, h->ev_join, 0));   // the FP64 re-run is part of the run
     if (timed) SPX_CUDA(cudaEventRecord(h->ev[2], h->stream));
     h->stats_timed = timed;
 
@@ -3764,7 +3784,8 @@ spx_status spx_batch_create(spx_batch **out, int32_t n, spx_handle *const *handl
                                           reinterpret_cast<const void *>(&spx::dense_sum_kernel),
                                           reinterpret_cast<const void *>(&spx::dense_states_kernel),
                                           reinterpret_cast<const void *>(&spx::dense_rows_kernel),
-                                          reinterpret_cast<const void *>(&spx::dense_points_kernel)})
+                                          reinterpret_cast<const void *>(&spx::dense_points_kernel<float2>),
+                                          reinterpret_cast<const void *>(&spx::dense_points_kernel<double2>)})
                         SPX_CUDA(cudaFuncGetAttributes(&fa, k));
                     continue;
                 }
