@@ -59,11 +59,14 @@ struct DenseStart {
     double *halfwidth;
     double bound;               // what halfwidth reports: a bound on |L|
     long long products;
+    int *sym;                   // [o] whether A equals its transpose (null: not wanted)
 };
-static __global__ void __launch_bounds__(kDenseThreads) dense_start_kernel(const DevSystem sys, const DenseSystem D,
+static __global__ void __launch_bounds__(256) dense_start_kernel(const DevSystem sys, const DenseSystem D,
                                                                            const DenseStart R) {
     __shared__ double coef[kMaxCoef];
+    __shared__ int differs;
     const int o = blockIdx.x, tid = threadIdx.x, n = D.n;
+    if (tid == 0) differs = 0;
     const int g = dense_grid_index(R.pick, R.n_orient, o);
     wigner_coefficients(sys, R.alpha[g], R.beta[g], R.gamma[g], coef);
     double2 *A = R.A + (size_t)o * n * n;
@@ -92,7 +95,14 @@ static __global__ void __launch_bounds__(kDenseThreads) dense_start_kernel(const
         const double2 *r0 = R.rho0s ? R.rho0s + (size_t)g * R.state_stride : R.rho0;
         R.V[(size_t)o * R.m * n + i] = r0[D.row_src[i]];
     }
+    if (R.sym) __syncthreads();
+    for (int e = tid; R.sym && e < D.nent; e += blockDim.x) {
+        const double2 a = A[D.ent[e]], b = A[(size_t)(D.ent[e] % n) * n + D.ent[e] / n];
+        if (a.x != b.x || a.y != b.y) differs = 1;
+    }
+    if (R.sym) __syncthreads();
     if (tid == 0) {
+        if (R.sym) R.sym[o] = differs ? 0 : 1;
         for (int q = 0; q < R.ncoil; ++q) {
             const double2 v = R.coil_val[q];
             double2 &y = Y[(size_t)R.coil_chan[q] * R.rows * n + R.coil_row[q]];
@@ -124,14 +134,38 @@ static __device__ __forceinline__ double2 dense_sum(const DenseSum &t, size_t at
     s.y += t.c1 * a.y + t.c2 * b.y + t.c3 * c.y;
     return s;
 }
+// Element u of the upper triangle with diagonal of an m x m matrix, rows r and
+// m-1-r side by side (m+1 elements).
+static __device__ __forceinline__ int2 dense_upper(int u, int m) {
+    const int r = u / (m + 1), c = u - r * (m + 1);
+    return c < m - r ? make_int2(r, r + c) : make_int2(m - 1 - r, c - 1);
+}
+// TRI: the first n (n+1) / 2 elements are the upper triangle.  An orientation
+// whose A equals its transpose (real couplings; relaxation may be complex) has
+// only products that do, so its lower triangles are copies: half of the FP64
+// instructions that bind this kernel (two orientations of 252 states, 2048
+// steps: products 5.9 -> 3.1 ms).  From kDenseTri states on: below, latency
+// binds it and the longer index chain costs more (6 states: 1.5 us a product).
+constexpr int kDenseTri = 32;
+template <bool TRI>
 static __global__ void __launch_bounds__(kDenseThreads, 24) dense_product_kernel(int64_t total, int n,
+                                                                                 const int *__restrict__ sym,
                                                                                  const double2 *__restrict__ A,
                                                                                  const double2 *__restrict__ B,
                                                                                  double2 *__restrict__ C, const DenseSum t) {
-    const int n2 = n * n;
+    const int n2 = n * n, upper = (n2 + n) / 2;
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
         const int64_t o = q / n2;
-        const int e = (int)(q - o * n2), r = e / n, c = e - r * n;
+        const int e = (int)(q - o * n2);
+        int r = e / n, c = e - r * n;
+        bool same = false;
+        if (TRI) {
+            same = sym[o] != 0;
+            if (e >= upper && same) continue;
+            const int2 at = dense_upper(e < upper ? e : e - upper, e < upper ? n : n - 1);
+            r = e < upper ? at.x : at.y + 1;
+            c = e < upper ? at.y : at.x;
+        }
         const double2 *a = A + o * n2 + (size_t)r * n, *b = B + o * n2 + c;
         double2 s = make_double2(0.0, 0.0);
         int k = 0;
@@ -141,8 +175,10 @@ static __global__ void __launch_bounds__(kDenseThreads, 24) dense_product_kernel
             dense_mac(s, a1, b1);
         }
         if (k < n) dense_mac(s, a[k], b[(size_t)k * n]);
-        if (t.M1) s = dense_sum(t, (size_t)q, r == c, s);
-        C[q] = s;
+        const int64_t to = o * n2 + (int64_t)r * n + c;
+        if (t.M1) s = dense_sum(t, (size_t)to, r == c, s);
+        C[to] = s;
+        if (TRI && same && r != c) C[o * n2 + (int64_t)c * n + r] = s;
     }
 }
 // C = c0 + c1 M1 + c2 M2 + c3 M3 + c4 M4

@@ -99,6 +99,7 @@ struct BlockPlan {
 // Device buffers of a run of the dense kernels.
 struct DenseBufs {
     DevBuf<double2> M, V, Y;         // six matrices, states, detection rows
+    DevBuf<int> sym;                 // whether an orientation's matrix is symmetric
 };
 
 // Device buffers of the kernels of block.cuh for one run.
@@ -1016,7 +1017,8 @@ void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, 
     int scale = 0;
     while (std::ldexp(plan.bound * dt, -scale) > 0.5) ++scale;
     const double products = 6.0 + scale + squarings;
-    const double work = 4.0 * n * n * (products * n + m + rows * h->nchan) + 4.0 * n * npts * h->nchan;
+    const double half = h->cplx || n < spx::kDenseTri ? 1.0 : 0.5;    // real couplings: symmetric products
+    const double work = 4.0 * n * n * (half * products * n + m + rows * h->nchan) + 4.0 * n * npts * h->nchan;
     const double dense = std::max(work * n_orient / (2.0 * h->sm_count), 0.0) + (6000.0 + 470.0 * n) * (products + squarings + 4.0);
     const double per_sm = (double)n_orient / h->sm_count;
     // the spectral half-width is about an eighth of the row bound (5.6 to 11.5
@@ -1274,6 +1276,7 @@ void launch_chebyshev(spx_handle *h, bool f64, const Config &c, spx::DevSystem &
 void reserve_dense(const spx_handle *h, DenseBufs &b, int64_t n_orient, const Config &c) {
     const size_t n = (size_t)c.dense->n;
     b.M.reserve(6 * (size_t)n_orient * n * n);
+    b.sym.reserve(n_orient);
     b.V.reserve((size_t)n_orient * c.dense_m * n);
     b.Y.reserve((size_t)n_orient * h->nchan * c.dense_rows * n);
 }
@@ -1303,10 +1306,13 @@ void launch_dense(spx_handle *h, const Config &c, spx::DevSystem &sys, DenseBufs
     st.status = words.status; st.kused = words.kused; st.mused = words.mused; st.matvecs = words.matvecs;
     st.halfwidth = words.halfwidth; st.bound = plan.bound;
     st.products = 6 + c.dense_scale;
-    spx::dense_start_kernel<<<dim3((unsigned)n_orient), spx::kDenseThreads, 0, stream>>>(sys, plan.dense, st);
+    const bool tri = n >= spx::kDenseTri && !h->cplx;
+    st.sym = tri ? b.sym.p : nullptr;
+    spx::dense_start_kernel<<<dim3((unsigned)n_orient), n < spx::kDenseTri ? spx::kDenseThreads : 256, 0, stream>>>(sys, plan.dense, st);
     ++h->launches;
     auto product = [&](const double2 *A, const double2 *B, double2 *C, const spx::DenseSum &t = spx::DenseSum{}) {
-        spx::dense_product_kernel<<<grid(total), spx::kDenseThreads, 0, stream>>>(total, n, A, B, C, t);
+        if (tri) spx::dense_product_kernel<true><<<grid(total), spx::kDenseThreads, 0, stream>>>(total, n, b.sym.p, A, B, C, t);
+        else spx::dense_product_kernel<false><<<grid(total), spx::kDenseThreads, 0, stream>>>(total, n, nullptr, A, B, C, t);
         ++h->launches;
     };
     // exp(A) to degree 16 in powers of A^4: M = A, A^2, A^3, A^4
@@ -3780,7 +3786,8 @@ spx_status spx_batch_create(spx_batch **out, int32_t n, spx_handle *const *handl
             for (int i = 0; i < n; ++i) {
                 if (cfg[i].dense) {
                     for (const void *k : {reinterpret_cast<const void *>(&spx::dense_start_kernel),
-                                          reinterpret_cast<const void *>(&spx::dense_product_kernel),
+                                          reinterpret_cast<const void *>(&spx::dense_product_kernel<false>),
+                                          reinterpret_cast<const void *>(&spx::dense_product_kernel<true>),
                                           reinterpret_cast<const void *>(&spx::dense_sum_kernel),
                                           reinterpret_cast<const void *>(&spx::dense_states_kernel),
                                           reinterpret_cast<const void *>(&spx::dense_rows_kernel),
