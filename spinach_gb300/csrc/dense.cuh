@@ -61,18 +61,15 @@ struct DenseStart {
     long long products;
     int *sym;                   // [o] whether A equals its transpose (null: not wanted)
 };
-static __global__ void __launch_bounds__(256) dense_start_kernel(const DevSystem sys, const DenseSystem D,
-                                                                           const DenseStart R) {
-    __shared__ double coef[kMaxCoef];
-    __shared__ int differs;
-    const int o = blockIdx.x, tid = threadIdx.x, n = D.n;
-    if (tid == 0) differs = 0;
+// The CTA assembles A and sets the first state v, the first detection row of
+// every channel y (apart by ystride) and the status words; ends with a barrier.
+static __device__ __forceinline__ void dense_start(const DevSystem &sys, const DenseSystem &D, const DenseStart &R, int o,
+                                                   double *coef, double2 *A, double2 *v, double2 *y, size_t ystride) {
+    const int tid = threadIdx.x, n = D.n;
     const int g = dense_grid_index(R.pick, R.n_orient, o);
     wigner_coefficients(sys, R.alpha[g], R.beta[g], R.gamma[g], coef);
-    double2 *A = R.A + (size_t)o * n * n;
     for (int e = tid; e < n * n; e += blockDim.x) A[e] = make_double2(0.0, 0.0);
-    double2 *Y = R.Y + (size_t)o * R.nchan * R.rows * n;
-    for (int e = tid; e < R.nchan * n; e += blockDim.x) Y[(size_t)(e / n) * R.rows * n + e % n] = make_double2(0.0, 0.0);
+    for (int e = tid; e < R.nchan * n; e += blockDim.x) y[(size_t)(e / n) * ystride + e % n] = make_double2(0.0, 0.0);
     __syncthreads();
     for (int e = tid; e < D.nent; e += blockDim.x) {
         double re = 0.0, im = 0.0;
@@ -93,20 +90,13 @@ static __global__ void __launch_bounds__(256) dense_start_kernel(const DevSystem
         }
         A[(size_t)i * n + i] = make_double2(im * R.h, -re * R.h);
         const double2 *r0 = R.rho0s ? R.rho0s + (size_t)g * R.state_stride : R.rho0;
-        R.V[(size_t)o * R.m * n + i] = r0[D.row_src[i]];
+        v[i] = r0[D.row_src[i]];
     }
-    if (R.sym) __syncthreads();
-    for (int e = tid; R.sym && e < D.nent; e += blockDim.x) {
-        const double2 a = A[D.ent[e]], b = A[(size_t)(D.ent[e] % n) * n + D.ent[e] / n];
-        if (a.x != b.x || a.y != b.y) differs = 1;
-    }
-    if (R.sym) __syncthreads();
     if (tid == 0) {
-        if (R.sym) R.sym[o] = differs ? 0 : 1;
         for (int q = 0; q < R.ncoil; ++q) {
-            const double2 v = R.coil_val[q];
-            double2 &y = Y[(size_t)R.coil_chan[q] * R.rows * n + R.coil_row[q]];
-            y = make_double2(y.x + v.x, y.y - v.y);                  // conj(coil)
+            const double2 w = R.coil_val[q];
+            double2 &t = y[(size_t)R.coil_chan[q] * ystride + R.coil_row[q]];
+            t = make_double2(t.x + w.x, t.y - w.y);                  // conj(coil)
         }
         R.status[o] = kDevOk;
         R.kused[o] = 16;
@@ -114,6 +104,24 @@ static __global__ void __launch_bounds__(256) dense_start_kernel(const DevSystem
         R.matvecs[o] = R.products * n;
         R.halfwidth[o] = R.bound;
     }
+    __syncthreads();
+}
+static __global__ void __launch_bounds__(256) dense_start_kernel(const DevSystem sys, const DenseSystem D,
+                                                                 const DenseStart R) {
+    __shared__ double coef[kMaxCoef];
+    __shared__ int differs;
+    const int o = blockIdx.x, n = D.n;
+    if (threadIdx.x == 0) differs = 0;
+    double2 *A = R.A + (size_t)o * n * n;
+    dense_start(sys, D, R, o, coef, A, R.V + (size_t)o * R.m * n, R.Y + (size_t)o * R.nchan * R.rows * n,
+                (size_t)R.rows * n);
+    if (!R.sym) return;
+    for (int e = threadIdx.x; e < D.nent; e += blockDim.x) {
+        const double2 a = A[D.ent[e]], b = A[(size_t)(D.ent[e] % n) * n + D.ent[e] / n];
+        if (a.x != b.x || a.y != b.y) differs = 1;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) R.sym[o] = differs ? 0 : 1;
 }
 
 static __device__ __forceinline__ void dense_mac(double2 &s, const double2 a, const double2 b) {
@@ -128,6 +136,18 @@ struct DenseSum {
     const double2 *M1, *M2, *M3;
     double c0, c1, c2, c3;
 };
+// sum over k of a[k] b[k n]
+static __device__ __forceinline__ double2 dense_dot(const double2 *a, const double2 *b, int n) {
+    double2 s = make_double2(0.0, 0.0);
+    int k = 0;
+    for (; k + 2 <= n; k += 2) {
+        const double2 a0 = a[k], a1 = a[k + 1], b0 = b[(size_t)k * n], b1 = b[(size_t)(k + 1) * n];
+        dense_mac(s, a0, b0);
+        dense_mac(s, a1, b1);
+    }
+    if (k < n) dense_mac(s, a[k], b[(size_t)k * n]);
+    return s;
+}
 static __device__ __forceinline__ double2 dense_sum(const DenseSum &t, size_t at, bool diagonal, double2 s) {
     const double2 a = t.M1[at], b = t.M2[at], c = t.M3[at];
     s.x += (diagonal ? t.c0 : 0.0) + t.c1 * a.x + t.c2 * b.x + t.c3 * c.x;
@@ -167,14 +187,7 @@ static __global__ void __launch_bounds__(kDenseThreads, 24) dense_product_kernel
             c = e < upper ? at.y : at.x;
         }
         const double2 *a = A + o * n2 + (size_t)r * n, *b = B + o * n2 + c;
-        double2 s = make_double2(0.0, 0.0);
-        int k = 0;
-        for (; k + 2 <= n; k += 2) {
-            const double2 a0 = a[k], a1 = a[k + 1], b0 = b[(size_t)k * n], b1 = b[(size_t)(k + 1) * n];
-            dense_mac(s, a0, b0);
-            dense_mac(s, a1, b1);
-        }
-        if (k < n) dense_mac(s, a[k], b[(size_t)k * n]);
+        double2 s = dense_dot(a, b, n);
         const int64_t to = o * n2 + (int64_t)r * n + c;
         if (t.M1) s = dense_sum(t, (size_t)to, r == c, s);
         C[to] = s;
@@ -254,6 +267,106 @@ static __global__ void __launch_bounds__(kDenseThreads, 24) dense_points_kernel(
                 check.fids[c * per + e] = s;
                 if (!finite) check.status[c] = kDevNonFinite;
             }
+    }
+}
+
+// The whole run of an orientation in one CTA, its matrices in shared memory, the
+// same sums in the same order: for few states, where a product is a few
+// instructions and the chain of launches took the time.  Bound by FP64 latency.
+// 6 states, 1024 steps, 200 orientations: 0.17 ms in launches, 0.067 so; 8
+// states 0.21 and 0.081; at 18 to 20 states no faster, with 256 threads either.
+constexpr int kDenseOne = 16;            // most states
+constexpr int kDenseOneThreads = 128;
+struct DenseOne {
+    int scale, npts;
+    double f[17];                        // Taylor coefficients
+};
+static __host__ __device__ inline size_t dense_one_smem(int n, int m, int rows, int nchan) {
+    return sizeof(double2) * (size_t)n * (6 * (size_t)n + m + (size_t)nchan * rows);
+}
+template <class Vec>
+static __global__ void __launch_bounds__(kDenseOneThreads) dense_one_kernel(const DevSystem sys, const DenseSystem D,
+                                                                            const DenseStart R, const DenseOne P, Vec *fids,
+                                                                            const DenseCheck check) {
+    __shared__ double coef[kMaxCoef];
+    extern __shared__ __align__(16) unsigned char dense_smem[];
+    const int o = blockIdx.x, tid = threadIdx.x, n = D.n, n2 = n * n;
+    double2 *M[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) M[q] = reinterpret_cast<double2 *>(dense_smem) + q * n2;
+    double2 *V = M[5] + n2, *Y = V + R.m * n;
+    dense_start(sys, D, R, o, coef, M[0], V, Y, (size_t)R.rows * n);
+    auto product = [&](const double2 *A, const double2 *B, double2 *C, const DenseSum &t) {
+        for (int e = tid; e < n2; e += kDenseOneThreads) {
+            const int r = e / n, c = e - r * n;
+            double2 s = dense_dot(A + r * n, B + c, n);
+            if (t.M1) s = dense_sum(t, e, r == c, s);
+            C[e] = s;
+        }
+        __syncthreads();
+    };
+    const DenseSum none = {};
+    const double *f = P.f;
+    auto quarter = [&](int q, double f0) { return DenseSum{M[0], M[1], M[2], f0, f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]}; };
+    product(M[0], M[0], M[1], none);
+    product(M[1], M[0], M[2], none);
+    product(M[1], M[1], M[3], none);
+    for (int e = tid; e < n2; e += kDenseOneThreads)
+        M[4][e] = dense_sum(quarter(3, f[12]), e, e / n == e % n, make_double2(f[16] * M[3][e].x, f[16] * M[3][e].y));
+    __syncthreads();
+    product(M[3], M[4], M[5], quarter(2, f[8]));
+    product(M[3], M[5], M[4], quarter(1, f[4]));
+    product(M[3], M[4], M[5], quarter(0, P.scale > 0 ? 0.0 : f[0]));
+    double2 *U = M[5], *W = M[4];
+    auto turn = [&] { double2 *t = U; U = W; W = t; };
+    for (int q = 0; q < P.scale; ++q) {
+        product(U, U, W, DenseSum{U, U, U, q + 1 == P.scale ? 1.0 : 0.0, 2.0, 0.0, 0.0});
+        turn();
+    }
+    for (int have = 1; have < R.m; have *= 2) {
+        for (int e = tid; e < have * n; e += kDenseOneThreads) {
+            const int j = e / n, r = e - j * n;
+            double2 s = make_double2(0.0, 0.0);
+            for (int k = 0; k < n; ++k) dense_mac(s, U[k * n + r], V[j * n + k]);
+            V[(have + j) * n + r] = s;
+        }
+        __syncthreads();
+        if (2 * have < R.m || R.rows > 1) {
+            product(U, U, W, none);
+            turn();
+        }
+    }
+    for (int have = 1; have < R.rows; have *= 2) {
+        for (int e = tid; e < R.nchan * have * n; e += kDenseOneThreads) {
+            const int ch = e / (have * n), x = e - ch * have * n, j = x / n, c = x - j * n;
+            double2 *y = Y + (size_t)ch * R.rows * n;
+            double2 s = make_double2(0.0, 0.0);
+            for (int k = 0; k < n; ++k) dense_mac(s, U[c * n + k], y[j * n + k]);
+            y[(have + j) * n + c] = s;
+        }
+        __syncthreads();
+        if (2 * have < R.rows) {
+            product(U, U, W, none);
+            turn();
+        }
+    }
+    const int per = R.nchan * P.npts;
+    int at = -1;                                              // of the checked orientations
+    for (int c = 0; c < check.count; ++c)
+        if (((2 * (long long)c + 1) * R.n_orient) / (2 * (long long)check.count) == o) at = c;
+    bool finite = true;
+    for (int e = tid; e < per; e += kDenseOneThreads) {
+        const int ch = e / P.npts, p = e - ch * P.npts, a = p / R.m, j = p - a * R.m;
+        const double2 *y = Y + ((size_t)ch * R.rows + a) * n, *v = V + (size_t)j * n;
+        double2 s = make_double2(0.0, 0.0);
+        for (int k = 0; k < n; ++k) dense_mac(s, y[k], v[k]);
+        fids[(size_t)o * per + e] = tovec(s, Vec());
+        if (at >= 0) check.fids[(size_t)at * per + e] = s;
+        finite = finite && isfinite(s.x) && isfinite(s.y);
+    }
+    if (!finite) {
+        R.status[o] = kDevNonFinite;
+        if (at >= 0) check.status[at] = kDevNonFinite;
     }
 }
 

@@ -841,6 +841,7 @@ struct Config {
     // squarings of the scaled exponential
     const BlockPlan *dense = nullptr;
     int dense_m = 0, dense_rows = 0, dense_scale = 0;
+    bool dense_one = false;                       // one CTA per orientation
     size_t blk_smem = 0;
 };
 
@@ -1002,7 +1003,7 @@ bool configure_block(spx_handle *h, const BlockPlan &plan, int64_t n_orient, dou
 // dense launches to the next; the layout's latency for each series term).
 // Measured sides (coupled states, orientations, steps): FP64 52, 1, 2048: dense
 // 0.5 ms, series 2.3 ms; 52, 1000, 2048: 16 and 11 ms; 8, 400, 1024: 0.2 and
-// 1.4 ms.  FP32 6, 200, 1024: 0.17 and 0.65 ms; 20, 200, 1024: 0.56 and 1.02;
+// 1.4 ms.  FP32 6, 200, 1024: 0.07 and 0.65 ms (one CTA an orientation); 20, 200, 1024: 0.56 and 1.02;
 // 20, 1000, 1024: 1.86 and 1.28; 52, 1, 1024: 0.50 and 0.36; 70, 1, 1024: 0.67
 // and 1.09.
 void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, double dt, int64_t nsteps, bool f64, Config &c) {
@@ -1016,10 +1017,13 @@ void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, 
     }
     int scale = 0;
     while (std::ldexp(plan.bound * dt, -scale) > 0.5) ++scale;
+    const bool one = plan.n <= spx::kDenseOne && spx::dense_one_smem(plan.n, m, rows, h->nchan) <= 96 * 1024;
     const double products = 6.0 + scale + squarings;
     const double half = h->cplx || n < spx::kDenseTri ? 1.0 : 0.5;    // real couplings: symmetric products
     const double work = 4.0 * n * n * (half * products * n + m + rows * h->nchan) + 4.0 * n * npts * h->nchan;
-    const double dense = std::max(work * n_orient / (2.0 * h->sm_count), 0.0) + (6000.0 + 470.0 * n) * (products + squarings + 4.0);
+    const double chain = products + squarings + 4.0;
+    const double dense = one ? work * std::ceil((double)n_orient / h->sm_count) / 2.0 + 800.0 * chain + 2e4
+                             : work * n_orient / (2.0 * h->sm_count) + (6000.0 + 470.0 * n) * chain;
     const double per_sm = (double)n_orient / h->sm_count;
     // the spectral half-width is about an eighth of the row bound (5.6 to 11.5
     // on the benchmark systems), a chunk's series a quarter longer than its
@@ -1033,6 +1037,7 @@ void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, 
     c.dense_m = m;
     c.dense_rows = rows;
     c.dense_scale = scale;
+    c.dense_one = one;
 }
 
 bool forced_shape(const spx_options &o) {
@@ -1274,6 +1279,7 @@ void launch_chebyshev(spx_handle *h, bool f64, const Config &c, spx::DevSystem &
 }
 
 void reserve_dense(const spx_handle *h, DenseBufs &b, int64_t n_orient, const Config &c) {
+    if (c.dense_one) return;
     const size_t n = (size_t)c.dense->n;
     b.M.reserve(6 * (size_t)n_orient * n * n);
     b.sym.reserve(n_orient);
@@ -1289,6 +1295,33 @@ void launch_dense(spx_handle *h, const Config &c, spx::DevSystem &sys, DenseBufs
                   const spx::DevRun &words, cudaStream_t stream, const spx::DenseCheck &check = spx::DenseCheck{}) {
     const BlockPlan &plan = *c.dense;
     const int n = plan.n, m = c.dense_m, rows = c.dense_rows;
+    spx::DenseStart st{};
+    st.n_orient = (int)n_orient; st.pick = pick;
+    st.alpha = d_al; st.beta = d_be; st.gamma = d_ga;
+    st.h = std::ldexp(dt, -c.dense_scale);
+    st.m = m; st.nchan = h->nchan; st.rows = rows;
+    st.rho0 = sys.rho0; st.rho0s = sys.rho0s; st.state_stride = (size_t)h->n_pad;
+    st.ncoil = plan.ncoil; st.coil_row = plan.coil_row; st.coil_chan = plan.coil_chan; st.coil_val = plan.coil_val;
+    st.status = words.status; st.kused = words.kused; st.mused = words.mused; st.matvecs = words.matvecs;
+    st.halfwidth = words.halfwidth; st.bound = plan.bound;
+    st.products = 6 + c.dense_scale;
+    const int64_t npts = nsteps + 1;
+    double f[17];
+    f[0] = 1.0;
+    for (int k = 1; k <= 16; ++k) f[k] = f[k - 1] / k;
+    if (c.dense_one) {
+        spx::DenseOne one{c.dense_scale, (int)npts, {}};
+        std::copy(f, f + 17, one.f);
+        const size_t smem = spx::dense_one_smem(n, m, rows, h->nchan);
+        if (smem > 40 * 1024)
+            SPX_CUDA(cudaFuncSetAttribute(spx::dense_one_kernel<Vec>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)(96 * 1024)));
+        spx::dense_one_kernel<Vec><<<dim3((unsigned)n_orient), spx::kDenseOneThreads, smem, stream>>>(sys, plan.dense, st, one,
+                                                                                                    out, check);
+        SPX_CUDA(cudaGetLastError());
+        ++h->launches;
+        return;
+    }
     const int64_t total = n_orient * n * n;
     double2 *M[6];
     for (int q = 0; q < 6; ++q) M[q] = b.M.p + (size_t)q * total;
@@ -1296,16 +1329,7 @@ void launch_dense(spx_handle *h, const Config &c, spx::DevSystem &sys, DenseBufs
         return dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>((items + spx::kDenseThreads - 1) / spx::kDenseThreads,
                                                                       (int64_t)h->sm_count * 64)));
     };
-    spx::DenseStart st{};
-    st.n_orient = (int)n_orient; st.pick = pick;
-    st.alpha = d_al; st.beta = d_be; st.gamma = d_ga;
-    st.h = std::ldexp(dt, -c.dense_scale);
-    st.A = M[0]; st.V = b.V.p; st.m = m; st.Y = b.Y.p; st.nchan = h->nchan; st.rows = rows;
-    st.rho0 = sys.rho0; st.rho0s = sys.rho0s; st.state_stride = (size_t)h->n_pad;
-    st.ncoil = plan.ncoil; st.coil_row = plan.coil_row; st.coil_chan = plan.coil_chan; st.coil_val = plan.coil_val;
-    st.status = words.status; st.kused = words.kused; st.mused = words.mused; st.matvecs = words.matvecs;
-    st.halfwidth = words.halfwidth; st.bound = plan.bound;
-    st.products = 6 + c.dense_scale;
+    st.A = M[0]; st.V = b.V.p; st.Y = b.Y.p;
     const bool tri = n >= spx::kDenseTri && !h->cplx;
     st.sym = tri ? b.sym.p : nullptr;
     spx::dense_start_kernel<<<dim3((unsigned)n_orient), n < spx::kDenseTri ? spx::kDenseThreads : 256, 0, stream>>>(sys, plan.dense, st);
@@ -1319,9 +1343,6 @@ void launch_dense(spx_handle *h, const Config &c, spx::DevSystem &sys, DenseBufs
     product(M[0], M[0], M[1]);
     product(M[1], M[0], M[2]);
     product(M[1], M[1], M[3]);
-    double f[17];
-    f[0] = 1.0;
-    for (int k = 1; k <= 16; ++k) f[k] = f[k - 1] / k;
     auto quarter = [&](int q) { return spx::DenseSum{M[0], M[1], M[2], f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]}; };
     spx::dense_sum_kernel<<<grid(total), spx::kDenseThreads, 0, stream>>>(total, n, quarter(3), M[3], f[16], M[4]);
     ++h->launches;
@@ -1350,7 +1371,6 @@ void launch_dense(spx_handle *h, const Config &c, spx::DevSystem &sys, DenseBufs
         ++h->launches;
         if (2 * have < rows) square();
     }
-    const int64_t npts = nsteps + 1;
     spx::dense_points_kernel<Vec><<<grid(n_orient * h->nchan * npts), spx::kDenseThreads, 0, stream>>>(
         n_orient, n, h->nchan, rows, m, (int)npts, b.Y.p, b.V.p, out, words.status, check);
     ++h->launches;
@@ -3786,6 +3806,8 @@ spx_status spx_batch_create(spx_batch **out, int32_t n, spx_handle *const *handl
             for (int i = 0; i < n; ++i) {
                 if (cfg[i].dense) {
                     for (const void *k : {reinterpret_cast<const void *>(&spx::dense_start_kernel),
+                                          reinterpret_cast<const void *>(&spx::dense_one_kernel<float2>),
+                                          reinterpret_cast<const void *>(&spx::dense_one_kernel<double2>),
                                           reinterpret_cast<const void *>(&spx::dense_product_kernel<false>),
                                           reinterpret_cast<const void *>(&spx::dense_product_kernel<true>),
                                           reinterpret_cast<const void *>(&spx::dense_sum_kernel),
