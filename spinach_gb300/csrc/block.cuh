@@ -141,6 +141,24 @@ static __device__ __forceinline__ BlockLane block_lane(const BlockLayout &B, int
     return l;
 }
 
+// The thread whose part of the layout a thread plays.  An SM's warp slots belong
+// to its four units by turns, so CTAs of two warps would all put their first
+// warp, the one with the wide rows, on the same two units: every other pair of
+// CTAs plays the parts the other way round (seven spins, 1000 orientations: 1.54
+// -> 1.38 ms; CTAs of three warps and more are spread well enough, and turning
+// those too costs 3 to 15 %).  Ends with a barrier where it takes one.
+static __device__ __forceinline__ int block_role(int nwarps) {
+    if (nwarps != 2) return threadIdx.x;
+    __shared__ int s_turned;
+    if (threadIdx.x == 0) {
+        unsigned slot;
+        asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
+        s_turned = (slot >> 2) & 1;
+    }
+    __syncthreads();
+    return threadIdx.x ^ (32 * s_turned);
+}
+
 // One lane's entries of an orientation's L: FP64 sums over the value streams
 // (coef: the rotational coefficients), stream by stream, so that the loads of
 // all entries are in flight together; detection rows keep their values.
@@ -801,7 +819,8 @@ __global__ void __launch_bounds__(ECAP == 24 ? 512 : 640, 1)
     float2 *s_rec = s_phase + (R.Mcap + 1);
     [[maybe_unused]] float2 *s_tb = s_rec + block_rec(R.Mcap, blockDim.x, kBlockPoints32);  // [step][term] inner states
     const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const BlockLane l = block_lane(B, tid);
+    const int role = block_role(nwarps);
+    const BlockLane l = block_lane(B, role);
     const BlockSeries S = block_series(R, o);
     if (!S.ok) return;
     const int nsteps = R.nsteps, M = S.M;
@@ -816,20 +835,20 @@ __global__ void __launch_bounds__(ECAP == 24 ? 512 : 640, 1)
         if (R.saved) {
             const double *save = R.saved + (size_t)o * block_saved(B.ecap, B.threads);
 #pragma unroll
-            for (int i = 0; i < ECAP; ++i) v[i] = i < l.ew ? save[(size_t)i * B.threads + tid] : 0.0;
+            for (int i = 0; i < ECAP; ++i) v[i] = i < l.ew ? save[(size_t)i * B.threads + role] : 0.0;
             save += (size_t)B.ecap * B.threads;
-            dg = make_double2(save[tid], save[B.threads + tid]);
+            dg = make_double2(save[role], save[B.threads + role]);
         } else {
             const double sign = R.adjoint ? -1.0 : 1.0;
             block_coefficients(sys, R, o, s_coef);
-            block_assemble<ECAP>(sys, B, l.ew, tid, s_coef, sign, v);
+            block_assemble<ECAP>(sys, B, l.ew, role, s_coef, sign, v);
             if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef, sign);
         }
         const double sc = l.row < B.n ? scale : 1.0;          // detection rows keep their values
 #pragma unroll
         for (int i = 0; i < ECAP; ++i) {
             E.set(i, v[i] * sc);
-            E.col[i] = i < l.ew ? B.col[i * B.threads + tid] * (int)sizeof(float2) : 0;
+            E.col[i] = i < l.ew ? B.col[i * B.threads + role] * (int)sizeof(float2) : 0;
         }
         if (l.state) {
             split((dg.x - S.cen) * scale, dh, dl);

@@ -150,7 +150,7 @@ struct spx_handle {
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::string err;
     int sm_count = 0;
-    size_t smem_optin = 0;
+    size_t smem_optin = 0, smem_sm = 0;     // shared memory of a CTA at most, and of an SM
 
     // uploaded system
     bool have_system = false;
@@ -868,7 +868,7 @@ struct Config {
     const BlockPlan *dense = nullptr;
     int dense_m = 0, dense_rows = 0, dense_scale = 0;
     bool dense_one = false;                       // one CTA per orientation
-    size_t blk_smem = 0;
+    size_t blk_smem = 0, blk_even = 0;            // blk_even: no SM takes more CTAs than its share
 };
 
 double host_series_terms(double x, double lg, double tol) {
@@ -1018,6 +1018,9 @@ bool configure_block(spx_handle *h, const BlockPlan &plan, int64_t n_orient, dou
     if (c.blk_smem + fa.sharedSizeBytes > h->smem_optin) return false;
     SPX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(h->smem_optin - fa.sharedSizeBytes)));
+    const size_t even = (size_t)(n_orient + h->sm_count - 1) / h->sm_count, own = fa.sharedSizeBytes + 1024;
+    const size_t part = (h->smem_sm / (even + 1) + 256) & ~(size_t)15;
+    c.blk_even = part > own ? std::max(c.blk_smem, part - own) : c.blk_smem;
     c.blk = best;
     c.blk_bounds = f64 ? best_layout(plan.layouts[0], per_sm) : best;
     return true;
@@ -1656,6 +1659,11 @@ void launch_powder(spx_handle *h, int64_t n_orient, const double *d_al, const do
         r.rho0 = sys.rho0; r.rho0s = sys.rho0s; r.state_stride = (size_t)h->n_pad;
         r.fids = run.fids; r.nchan = h->nchan;
         r.status = run.status; r.kused = run.kused; r.mused = run.mused; r.matvecs = run.matvecs;
+        // launched beside the check's kernels, a grid of less than a wave piles up
+        // on the SMs that are free first (200 orientations of a rotor-frame
+        // system, 128 threads each: 3.3 to 5.8 ms, 3.3 with even shares); beside
+        // other systems of a batch even shares would cost 8 %
+        if (chk) c.blk_smem = c.blk_even;
         launch_block(h, c, sys, r, h->stream);
     } else {
         launch_chebyshev(h, f64, c, sys, run);
@@ -3358,6 +3366,8 @@ spx_status spx_create(spx_handle **handle, int device) {
         int optin = 0;
         SPX_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
         h->smem_optin = (size_t)optin;
+        SPX_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
+        h->smem_sm = (size_t)optin;
         int least = 0;
         SPX_CUDA(cudaDeviceGetStreamPriorityRange(&least, &h->high_priority));
     });
