@@ -77,7 +77,23 @@ def measured_peaks():
     return 6800.0, 'fallback'
 
 
-def profile_traffic(name='powder_chebyshev_c1.md'):
+def coupled_nnz(L):
+    """Non-zeros of L in the rows that connect the initial state with the coil."""
+    import scipy.sparse as sp
+    from scipy.sparse.csgraph import connected_components
+    P = abs(L.R) + abs(L.I)
+    for Q in L.terms.values():
+        P = P + abs(Q)
+    P = sp.csr_matrix(P)
+    P.data[P.data < 1e-12 * P.data.max()] = 0.0
+    P.eliminate_zeros()
+    of = connected_components(P, directed=False)[1]
+    dense = lambda v: np.asarray(v.todense() if sp.issparse(v) else v).ravel()
+    rows = np.isin(of, np.intersect1d(of[dense(L.rho0) != 0], of[dense(L.coil) != 0]))
+    return int(P[rows].nnz)
+
+
+def profile_traffic(name='block_chebyshev_c1.md'):
     """Per-launch DRAM bytes of the propagation kernel from the committed ncu summary."""
     p = os.path.join(ROOT, 'profiles', name)
     if not os.path.exists(p):
@@ -395,13 +411,17 @@ def run_gpu(args):
                   'how': 'two orientations re-run in FP64 on a second stream inside every FP32 run '
                          '(spx_stats.fp32_*); the timed steps include it'}
 
-    # roofline of the dominant kernel (powder_chebyshev_kernel).  L and the
-    # state live in shared memory, so the bound is on chip: the FP32 pipe,
+    # roofline of the dominant kernel, over the states it propagates (those that
+    # couple to the coils where the run is restricted to them).  L lives in
+    # registers and the state in shared memory (whole systems: both in shared
+    # memory), so the bound is on chip: the FP32 pipe,
     # with the algorithmic flops of the sparse branch (8 flops per stored
     # non-zero per matvec) against 128 lanes x 2 flops per SM at the sampled
     # clock; shared-memory bandwidth beside it; the HBM figure is the
     # effective bandwidth a streaming SpMV would need for the same matvecs
     nnz, n = stats['nnz'], stats['dim']
+    if stats['coupled_dim']:
+        nnz, n = coupled_nnz(L), stats['coupled_dim']
     matvecs = stats['matvecs']
     k_ms = statistics.mean(kernel_ms)
     clk = clk.summary()
@@ -465,11 +485,13 @@ def run_gpu(args):
             'roofline': {'bound': 'fp32', 'achieved': achieved, 'peak': fp32_peak, 'unit': 'TFLOP/s',
                          'frac': achieved / fp32_peak, 'traffic': traffic,
                          'traffic_source': 'ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of this '
-                                           'workload, profiles/powder_chebyshev_c1.md (not measured in this run)'
+                                           'workload, profiles/block_chebyshev_c1.md (not measured in this run)'
                          if traffic is not None else None,
                          'peak_source': f'nominal FP32 pipe: {sms} SMs x 128 lanes x 2 flops at the sampled '
                                         f'{mhz:.0f} MHz (MEASURED_PEAKS.json has no FP32 figure)',
-                         'kernel': 'powder_chebyshev_kernel', 'kernel_ms': k_ms, 'matvecs': matvecs,
+                         'kernel': 'block_bounds, block_tables and block_chebyshev kernels' if stats['coupled_dim']
+                         else 'powder_chebyshev_kernel', 'kernel_ms': k_ms, 'matvecs': matvecs,
+                         'states': n, 'non_zeros': nnz,
                          'algorithmic_flops': alg_flops,
                          'useful_flops': useful_flops, 'useful_frac': useful_flops / (k_ms / 1e3) / 1e12 / fp32_peak,
                          'smem': {'achieved_gbs': eff_gbs, 'peak_gbs': smem_peak, 'frac': eff_gbs / smem_peak,
@@ -481,7 +503,7 @@ def run_gpu(args):
                          'note': 'achieved = 8 flops per stored non-zero per matvec (the sparse-branch count) '
                                  'x matvecs executed / kernel time (CUDA events on the engine stream); '
                                  'useful_flops counts 4 flops per real off-diagonal value; the compensated '
-                                 'FP32 arithmetic (hi+lo values, Kahan row sums) executes about 4x these flops'},
+                                 'FP32 arithmetic (hi+lo values, error-free row sums) executes about 4x these flops'},
             'cpu_baseline': cpu,
             'surrogate': sur,
             'surrogate_c4': sur4,

@@ -3255,35 +3255,50 @@ void run_powder_noalloc(spx_handle *h, int64_t n_orient, const double *d_al, con
     SPX_CUDA(cudaSetDevice(h->device));
     spx_options opt{};
     opt.precision = precision;
-    const Config c = choose_config(h, n_orient, dt, nsteps, opt, 0, kNoallocChunkCap, false, &h->plan);
+    Config c = choose_config(h, n_orient, dt, nsteps, opt, 0, kNoallocChunkCap, false, &h->plan);
     const bool f64 = precision == SPX_FP64;
     const size_t npts = ((size_t)nsteps + 1) * h->nchan;   // all channels' points
     const int group = 64;
     const int ngroups = (int)((n_orient + group - 1) / group);
-    const size_t tables = c.blk ? block_table_entries(c) : (size_t)c.grid * c.Kmax * (c.M + 1);
     // carve the scratch: sizes first, then check, then addresses
     constexpr int kParts = 14;
-    const size_t sizes[kParts] = {
-        tables * sizeof(double),                                      // Bessel tables
-        npts * (size_t)n_orient * (f64 ? sizeof(double2) : sizeof(float2)),   // per-orientation FIDs
-        (size_t)ngroups * npts * sizeof(double2),                     // FP64 partial sums
-        (size_t)n_orient * sizeof(int), (size_t)n_orient * sizeof(int), (size_t)n_orient * sizeof(int),
-        (size_t)n_orient * sizeof(long long) + (size_t)n_orient * sizeof(double),
-        sizeof(int), sizeof(int),
-        // coupled-state kernels: float tables, centres, extents, ladder, columns' terms
-        c.blk && !f64 ? tables * sizeof(float) : 0, c.blk ? (size_t)n_orient * sizeof(double) : 0,
-        c.blk ? 2 * sizeof(unsigned long long) : 0, c.blk ? (size_t)c.blk_lev * (sizeof(double) + 3 * sizeof(int)) : 0,
-        c.blk ? (size_t)c.blk_lev * (c.blk_M + 1) * sizeof(int) : 0};
     size_t offs[kParts], total = 0;
-    for (int i = 0; i < kParts; ++i) {
-        offs[i] = total;
-        total += (sizes[i] + 255) & ~(size_t)255;
-    }
+    auto carve = [&] {
+        const size_t tables = c.blk ? block_table_entries(c) : (size_t)c.grid * c.Kmax * (c.M + 1);
+        const size_t sizes[kParts] = {
+            tables * sizeof(double),                                      // Bessel tables
+            npts * (size_t)n_orient * (f64 ? sizeof(double2) : sizeof(float2)),   // per-orientation FIDs
+            (size_t)ngroups * npts * sizeof(double2),                     // FP64 partial sums
+            (size_t)n_orient * sizeof(int), (size_t)n_orient * sizeof(int), (size_t)n_orient * sizeof(int),
+            (size_t)n_orient * sizeof(long long) + (size_t)n_orient * sizeof(double),
+            sizeof(int), sizeof(int),
+            // coupled-state kernels: float tables, centres, extents, ladder, columns' terms
+            c.blk && !f64 ? tables * sizeof(float) : 0, c.blk ? (size_t)n_orient * sizeof(double) : 0,
+            c.blk ? 2 * sizeof(unsigned long long) : 0,
+            c.blk ? (size_t)c.blk_lev * (sizeof(double) + 3 * sizeof(int)) : 0,
+            c.blk ? (size_t)c.blk_lev * (c.blk_M + 1) * sizeof(int) : 0};
+        total = 0;
+        for (int i = 0; i < kParts; ++i) {
+            offs[i] = total;
+            total += (sizes[i] + 255) & ~(size_t)255;
+        }
+    };
+    // what the whole system needs decides what is refused; the coupled states
+    // run where they fit too
+    const BlockPlan::Layout *coupled = c.blk;
+    c.blk = nullptr;
+    carve();
     if (total > SPX_NOALLOC_SCRATCH_BYTES)
         throw SpxError(SPX_ERR_UNSUPPORTED, "this run needs " + std::to_string(total) +
                                                 " bytes of scratch; spx_run_powder_noalloc holds " +
                                                 std::to_string((size_t)SPX_NOALLOC_SCRATCH_BYTES) +
                                                 " (use spx_run_powder_device for larger runs)");
+    c.blk = coupled;
+    carve();
+    if (total > SPX_NOALLOC_SCRATCH_BYTES) {
+        c.blk = nullptr;
+        carve();
+    }
     unsigned char *base = static_cast<unsigned char *>(noalloc_scratch(h->device));
     int *flag = reinterpret_cast<int *>(base + offs[7]);
     spx::DevSystem sys = device_system(h);
