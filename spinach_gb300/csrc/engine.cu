@@ -3124,7 +3124,7 @@ spx_options autotune(spx_handle *h, int64_t n_orient, const double *d_al, const 
     std::vector<double> hw((size_t)n, 1.0 / (double)n);
     SPX_CUDA(cudaMemcpyAsync(w.p, hw.data(), n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     DevBuf<double2> out;
-    out.reserve((size_t)ns + 1);
+    out.reserve(((size_t)ns + 1) * h->nchan);
     spx_options best = base;
     double best_t = INFINITY;
     const int cls[] = {1, 2, 4, 8};
