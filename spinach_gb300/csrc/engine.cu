@@ -2178,14 +2178,25 @@ struct SequenceGroup {
     bool bounded = false;
 };
 
+// Tables of a sequence hold for any step count: their chunks are as long as
+// the tables allow.
+constexpr int64_t kAnySteps = (int64_t)1 << 28;
+
+// The group's configuration for a time step and a tolerance; false if its
+// series is too long for the coupled-state kernels' shared memory.
+bool configure_group(spx_handle *h, SequenceGroup &g, int64_t n_orient, double dt, double tol, bool f64, bool traj,
+                     Config &c) {
+    c.tol = tol;
+    return configure_block(h, g.plan, n_orient, dt, kAnySteps, f64, 0.0, 0, traj ? spx::kBlockTraj : 256, traj, c);
+}
+
 // Propagates a group over nsteps steps of dt: bounds on the first call, tables
-// whenever the time step changes (they hold for any step count).
+// whenever the time step changes.
 void run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockRun r, int64_t n_orient,
                const double *const (&angles)[3], double dt, int64_t nsteps, double tol, bool f64, bool traj, int *status, double *halfwidth) {
     if (!g.bounded || g.table_dt != dt) {
         Config c = g.c;
-        c.tol = tol;
-        if (!configure_block(h, g.plan, n_orient, dt, (int64_t)1 << 28, f64, 0.0, 0, traj ? spx::kBlockTraj : 256, traj, c))
+        if (!configure_group(h, g, n_orient, dt, tol, f64, traj, c))
             throw SpxError(SPX_ERR_INTERNAL, "a coupled set of states lost its layout");
         g.c = c;
         reserve_block(g.bufs, n_orient, f64, c);
@@ -2202,7 +2213,7 @@ void run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockR
     if (!g.bounded) launch_bounds(h, c, sys, r, h->stream);
     g.bounded = true;
     if (g.table_dt != dt) {
-        r.nsteps = 1 << 28;                  // chunks as long as the tables allow
+        r.nsteps = (int)kAnySteps;
         launch_tables(h, c, r, h->stream);
         g.table_dt = dt;
     }
@@ -2287,6 +2298,21 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
     const double *g = h->d_grid.p;
     const double *const angles[3] = {g, g + n_orient, g + 2 * n_orient};
     const size_t ns = (size_t)n_orient * n;
+    // every segment has to fit before the first one starts (long series: steps
+    // of several thousand in |L| dt).  The whole system's configurations come
+    // first: what they refuse stays refused.
+    std::vector<Config> wholes(ops.size());
+    for (size_t i = 0; i < ops.size(); ++i)
+        if (ops[i].kind == SPX_SEQ_EVOLVE) wholes[i] = choose_config(h, n_orient, ops[i].dt, ops[i].nsteps, o, 0);
+    std::vector<double> fits;                    // time steps known to
+    for (size_t i = 0; i < ops.size(); ++i) {
+        if (ops[i].kind != SPX_SEQ_EVOLVE || std::find(fits.begin(), fits.end(), ops[i].dt) != fits.end()) continue;
+        for (auto &grp : groups) {
+            Config c{};
+            if (!configure_group(h, *grp, n_orient, ops[i].dt, wholes[i].tol, f64, false, c)) return false;
+        }
+        fits.push_back(ops[i].dt);
+    }
     const bool own_states = h->n_states > 0;
     h->d_seq[0].reserve(ns);
     h->d_seq[1].reserve(ns);
@@ -2332,8 +2358,7 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
             if (per_orient) cur ^= 1; else rcur ^= 1;
             continue;
         }
-        // the whole system's configuration: what it refuses stays refused
-        whole = choose_config(h, n_orient, q.dt, q.nsteps, o, 0);
+        whole = wholes[i];
         const bool last = (int)i == last_evolve;
         for (size_t k = 0; k < groups.size(); ++k) {
             const bool detects = k + 1 == groups.size();
@@ -2859,6 +2884,8 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
     for (int q = 0; q < 3; ++q) status[q] = h->d_seq_status.p + (size_t)q * n_orient;
     if (back_angle) {
         const Config whole = choose_config(h, n_orient, tau, nsteps, o, 0);     // refusals of the whole system
+        Config c{};
+        if (!configure_group(h, gb, n_orient, tau, whole.tol, f64, false, c)) return false;
         const size_t ns = (size_t)n_orient * n;
         h->d_seq[0].reserve(ns);
         h->d_seq[1].reserve(ns);
@@ -2908,6 +2935,10 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
             }
         }
         if (!have) throw SpxError(SPX_ERR_UNSUPPORTED, "the trajectory does not fit a cluster of 8 SMs");
+        for (SequenceGroup *grp : {&gu, &gv}) {
+            Config c{};
+            if (!configure_group(h, *grp, nb, tau, whole.tol, f64, true, c)) return false;
+        }
         const double *const angles[3] = {g + b0, g + n_orient + b0, g + 2 * n_orient + b0};
         for (int dir = 0; dir < 2; ++dir) {
             SequenceGroup &grp = dir ? gv : gu;

@@ -61,3 +61,32 @@ def test_autotune_of_several_channels(engine_lib, nchan, prec, tol):
             assert rel_err(res.fid[ch], _fid(H, R, rho0, coils[ch], 0.2, 600)) <= tol
     finally:
         eng.close()
+
+
+def _shift_operator(n):
+    return sp.csc_matrix(np.diag(np.ones(n - 1), 1) + np.diag(np.ones(n - 1), -1))
+
+
+def test_steps_too_long_for_the_coupled_kernels_take_the_whole_system(gpu_engine):
+    """Series of several thousand terms outgrow the coupled kernels' shared memory
+    before they outgrow the whole system's: FP64 detection rows of a complex coil,
+    FP32 trajectories.  The phases reach 1e4, which leaves FP64 about 1e-12 of
+    them and FP32 1e-3."""
+    n = 4
+    H, R, rho0, coil = _chain(n, 5)
+    P = _shift_operator(n)
+    H *= 4800.0 / np.abs(H).sum(1).max()
+    _upload(gpu_engine, H, R, rho0, coil)
+    res = gpu_engine.run_sequence(*ANGLES, WEIGHTS, [P], [('evolve', 2, 1.0), ('pulse', 0, 0.3), ('evolve', 1, 1.0)],
+                                  precision=E.FP64)
+    first = _fid(H, R, rho0, coil, 1.0, 2)
+    after = sl.expm(-0.3j * P.toarray()) @ sl.expm(-2j * H) @ rho0
+    ref = np.concatenate([first, _fid(H, R, after, coil, 1.0, 1)])
+    assert rel_err(res.fid, ref) <= 1e-10 and res.stats['coupled_dim'] == 0
+    H *= 5300.0 / 4800.0
+    _upload(gpu_engine, H, R, rho0, coil)
+    res = gpu_engine.run_eseem(*ANGLES, WEIGHTS, 2.0, 3, P, precision=E.FP32)
+    U, Pi = sl.expm(-1j * H), sl.expm(-1j * np.pi * P.toarray())
+    v = sl.expm(-0.5j * np.pi * P.toarray()) @ rho0
+    ref = [np.vdot(coil, np.linalg.matrix_power(U, j) @ Pi @ np.linalg.matrix_power(U, j) @ v) for j in range(3)]
+    assert rel_err(res.fid, ref) <= 1e-3 and res.stats['coupled_dim'] == 0
