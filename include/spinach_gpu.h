@@ -403,7 +403,9 @@ spx_status spx_autotune(spx_handle *handle, int64_t n_orient, const double *d_al
  * arguments of spx_run_powder_device, one entry per handle) -- into one CUDA
  * graph whose per-system launches sit on parallel branches.  The handles'
  * buffers are sized at creation; the handles must not run anything else
- * while the batch exists.
+ * while the batch exists.  What is uploaded to a handle meanwhile (a system,
+ * coils, initial states) is what the next launch runs: it captures the graph
+ * again first.
  */
 typedef struct spx_batch spx_batch;
 spx_status spx_batch_create(spx_batch **batch, int32_t n, spx_handle *const *handles, const int64_t *n_orient,

@@ -179,6 +179,7 @@ struct spx_handle {
     DevBuf<double2> d_echo_val;
     int64_t n_states = 0;           // their count (0: one initial state for all)
     std::vector<int> row_of;        // sliced-ELL row of every basis state
+    int64_t revision = 0;           // counts uploads: systems, coils, initial states
 
     // coupled states of the plain acquisition (rebuilt with the coils and the
     // initial states) and what finding them takes
@@ -443,7 +444,10 @@ std::vector<int> live_rows(const spx_handle *h, const std::vector<int> &label, c
 }
 
 // The plan of the plain acquisition for the handle's coils and initial states.
+// It lies where the plan before it lay if it fits there, so a graph that was
+// captured with that one (spx_batch) may not run any more: hence the revision.
 void rebuild_plan(spx_handle *h) {
+    ++h->revision;
     build_plan(h, live_rows(h, h->component, start_rows(h)), nullptr, true, h->plan);
 }
 
@@ -704,6 +708,7 @@ void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32
 
     SPX_CUDA(cudaSetDevice(h->device));
     h->have_system = false;
+    ++h->revision;
     h->d_slice_off.upload(slice_off, h->stream);
     h->slice_off_host = slice_off;
     h->d_ell_col.upload(ell_col, h->stream);
@@ -3823,13 +3828,23 @@ spx_status spx_autotune(spx_handle *h, int64_t n_orient, const double *d_alphas,
 // Batched powders: one CUDA graph, one branch per system
 // ---------------------------------------------------------------------------
 struct spx_batch {
+    // one system's run, as given to spx_batch_create
+    struct Run {
+        spx_handle *h;
+        int64_t n_orient;
+        const double *alphas, *betas, *gammas, *weights;
+        double dt;
+        int64_t nsteps;
+        spx_options opt;
+        double2 *fid;
+        int64_t revision;                // of the handle when the graph was captured
+    };
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     std::vector<cudaEvent_t> marks;      // fork / join events used while capturing
-    std::vector<spx_handle *> hs;
-    std::vector<int64_t> n_orient;
+    std::vector<Run> runs;
     std::string err;
     bool launched = false;
 };
@@ -3853,6 +3868,83 @@ spx_status batch_guarded(spx_batch *b, F f) {
     } catch (const std::exception &e) {
         if (b) b->err = e.what();
         return SPX_ERR_INTERNAL;
+    }
+}
+
+// Captures the batch's graph for what its handles hold now.
+void capture_batch(spx_batch *b) {
+    const size_t n = b->runs.size();
+    // launch shapes and buffers first: nothing may allocate while capturing
+    std::vector<Config> cfg(n);
+    std::vector<spx_options> os(n);
+    for (size_t i = 0; i < n; ++i) {
+        const spx_batch::Run &r = b->runs[i];
+        os[i] = apply_tuned(r.h, r.opt);
+        cfg[i] = choose_config(r.h, r.n_orient, r.dt, r.nsteps, os[i], 0, 256, false, &r.h->plan);
+        reserve_run(r.h, r.n_orient, r.nsteps, os[i].precision == SPX_FP64, cfg[i]);
+        SPX_CUDA(cudaStreamSynchronize(r.h->stream));
+    }
+    // load every kernel the graph will hold before capturing (lazy module loading
+    // would otherwise happen inside the capture)
+    {
+        cudaFuncAttributes fa{};
+        SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::powder_partial_kernel<float2>)));
+        SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::powder_partial_kernel<double2>)));
+        SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::powder_combine_kernel)));
+        SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::block_tables_kernel)));
+        for (size_t i = 0; i < n; ++i) {
+            const spx_handle *h = b->runs[i].h;
+            if (cfg[i].dense) {
+                for (const void *k : {reinterpret_cast<const void *>(&spx::dense_start_kernel),
+                                      reinterpret_cast<const void *>(&spx::dense_one_kernel<float2>),
+                                      reinterpret_cast<const void *>(&spx::dense_one_kernel<double2>),
+                                      reinterpret_cast<const void *>(&spx::dense_product_kernel<false>),
+                                      reinterpret_cast<const void *>(&spx::dense_product_kernel<true>),
+                                      reinterpret_cast<const void *>(&spx::dense_sum_kernel),
+                                      reinterpret_cast<const void *>(&spx::dense_states_kernel),
+                                      reinterpret_cast<const void *>(&spx::dense_rows_kernel),
+                                      reinterpret_cast<const void *>(&spx::dense_points_kernel<float2>),
+                                      reinterpret_cast<const void *>(&spx::dense_points_kernel<double2>)})
+                    SPX_CUDA(cudaFuncGetAttributes(&fa, k));
+                continue;
+            }
+            if (cfg[i].blk) {
+                SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(h->cplx, cfg[i].blk_bounds->ecap, 0)));
+                SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(h->cplx, cfg[i].blk->ecap, cfg[i].blk_which)));
+                continue;
+            }
+            SPX_CUDA(cudaFuncGetAttributes(&fa, select_kernel(os[i].precision == SPX_FP64, h->cplx, cfg[i].rmax,
+                                                              cfg[i].cl > 1, h->ncoil > 0, false,
+                                                              cfg[i].threads > 512)));
+        }
+    }
+    cudaGraph_t graph = nullptr;
+    SPX_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+    try {
+        SPX_CUDA(cudaEventRecord(b->marks[n], b->stream));             // fork
+        for (size_t i = 0; i < n; ++i) {
+            const spx_batch::Run &r = b->runs[i];
+            SPX_CUDA(cudaStreamWaitEvent(r.h->stream, b->marks[n], 0));
+            launch_powder(r.h, r.n_orient, r.alphas, r.betas, r.gammas, r.weights, r.dt, r.nsteps, os[i], r.fid, cfg[i],
+                          0, false);
+            SPX_CUDA(cudaEventRecord(b->marks[i], r.h->stream));        // join
+            SPX_CUDA(cudaStreamWaitEvent(b->stream, b->marks[i], 0));
+        }
+    } catch (...) {
+        cudaStreamEndCapture(b->stream, &graph);
+        if (graph) cudaGraphDestroy(graph);
+        throw;
+    }
+    SPX_CUDA(cudaStreamEndCapture(b->stream, &graph));
+    cudaGraphExec_t exec = nullptr;
+    const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
+    cudaGraphDestroy(graph);
+    SPX_CUDA(ie);
+    if (b->exec) cudaGraphExecDestroy(b->exec);
+    b->exec = exec;
+    for (spx_batch::Run &r : b->runs) {
+        r.h->stats_pending = false;
+        r.revision = r.h->revision;
     }
 }
 
@@ -3898,83 +3990,18 @@ spx_status spx_batch_create(spx_batch **out, int32_t n, spx_handle *const *handl
         SPX_CUDA(cudaSetDevice(b->device));
         SPX_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
         for (auto &e : b->ev) SPX_CUDA(cudaEventCreate(&e));
-        // launch shapes and buffers first: nothing may allocate while capturing
-        std::vector<Config> cfg(n);
-        std::vector<spx_options> os(n);
         for (int i = 0; i < n; ++i) {
-            spx_handle *h = handles[i];
-            finish_run(h);
+            finish_run(handles[i]);
             spx_options o{};
             if (opts) o = opts[i];
             if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
                 throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
-            os[i] = apply_tuned(h, o);
-            cfg[i] = choose_config(h, n_orient[i], dt[i], nsteps[i], os[i], 0, 256, false, &h->plan);
-            reserve_run(h, n_orient[i], nsteps[i], os[i].precision == SPX_FP64, cfg[i]);
-            SPX_CUDA(cudaStreamSynchronize(h->stream));
-        }
-        // load every kernel the graph will hold before capturing (lazy module loading
-        // would otherwise happen inside the capture)
-        {
-            cudaFuncAttributes fa{};
-            SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::powder_partial_kernel<float2>)));
-            SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::powder_partial_kernel<double2>)));
-            SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::powder_combine_kernel)));
-            SPX_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(&spx::block_tables_kernel)));
-            for (int i = 0; i < n; ++i) {
-                if (cfg[i].dense) {
-                    for (const void *k : {reinterpret_cast<const void *>(&spx::dense_start_kernel),
-                                          reinterpret_cast<const void *>(&spx::dense_one_kernel<float2>),
-                                          reinterpret_cast<const void *>(&spx::dense_one_kernel<double2>),
-                                          reinterpret_cast<const void *>(&spx::dense_product_kernel<false>),
-                                          reinterpret_cast<const void *>(&spx::dense_product_kernel<true>),
-                                          reinterpret_cast<const void *>(&spx::dense_sum_kernel),
-                                          reinterpret_cast<const void *>(&spx::dense_states_kernel),
-                                          reinterpret_cast<const void *>(&spx::dense_rows_kernel),
-                                          reinterpret_cast<const void *>(&spx::dense_points_kernel<float2>),
-                                          reinterpret_cast<const void *>(&spx::dense_points_kernel<double2>)})
-                        SPX_CUDA(cudaFuncGetAttributes(&fa, k));
-                    continue;
-                }
-                if (cfg[i].blk) {
-                    SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(handles[i]->cplx, cfg[i].blk_bounds->ecap, 0)));
-                    SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(handles[i]->cplx, cfg[i].blk->ecap,
-                                                                     cfg[i].blk_which)));
-                    continue;
-                }
-                SPX_CUDA(cudaFuncGetAttributes(&fa, select_kernel(os[i].precision == SPX_FP64, handles[i]->cplx,
-                                                                  cfg[i].rmax, cfg[i].cl > 1, handles[i]->ncoil > 0,
-                                                                  false, cfg[i].threads > 512)));
-            }
+            b->runs.push_back({handles[i], n_orient[i], d_alphas[i], d_betas[i], d_gammas[i], d_weights[i], dt[i],
+                               nsteps[i], o, reinterpret_cast<double2 *>(d_fids[i]), 0});
         }
         b->marks.resize(n + 1, nullptr);
         for (auto &e : b->marks) SPX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        cudaGraph_t graph = nullptr;
-        SPX_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        try {
-            SPX_CUDA(cudaEventRecord(b->marks[n], b->stream));             // fork
-            for (int i = 0; i < n; ++i) {
-                spx_handle *h = handles[i];
-                SPX_CUDA(cudaStreamWaitEvent(h->stream, b->marks[n], 0));
-                launch_powder(h, n_orient[i], d_alphas[i], d_betas[i], d_gammas[i], d_weights[i], dt[i], nsteps[i],
-                              os[i], reinterpret_cast<double2 *>(d_fids[i]), cfg[i], 0, false);
-                SPX_CUDA(cudaEventRecord(b->marks[i], h->stream));          // join
-                SPX_CUDA(cudaStreamWaitEvent(b->stream, b->marks[i], 0));
-            }
-        } catch (...) {
-            cudaStreamEndCapture(b->stream, &graph);
-            if (graph) cudaGraphDestroy(graph);
-            throw;
-        }
-        SPX_CUDA(cudaStreamEndCapture(b->stream, &graph));
-        const cudaError_t ie = cudaGraphInstantiate(&b->exec, graph, 0);
-        cudaGraphDestroy(graph);
-        SPX_CUDA(ie);
-        for (int i = 0; i < n; ++i) {
-            handles[i]->stats_pending = false;
-            b->hs.push_back(handles[i]);
-            b->n_orient.push_back(n_orient[i]);
-        }
+        capture_batch(b);
     });
     if (st != SPX_OK) {
         g_batch_create_error = b->err;
@@ -3993,13 +4020,22 @@ spx_status spx_batch_launch(spx_batch *b, void *stream) {
     return batch_guarded(b, [&] {
         SPX_CUDA(cudaSetDevice(b->device));
         cudaStream_t s = stream ? (cudaStream_t)stream : b->stream;
+        // a system, coils or initial states uploaded since: the graph's launches
+        // hold the sizes and places of what was there before
+        bool stale = false;
+        for (const spx_batch::Run &r : b->runs) stale = stale || r.revision != r.h->revision;
+        if (stale) {
+            if (b->launched) SPX_CUDA(cudaEventSynchronize(b->ev[1]));
+            for (const spx_batch::Run &r : b->runs) validate_run(r.h, r.n_orient, r.dt, r.nsteps);
+            capture_batch(b);
+        }
         SPX_CUDA(cudaEventRecord(b->ev[0], s));
         SPX_CUDA(cudaGraphLaunch(b->exec, s));
         SPX_CUDA(cudaEventRecord(b->ev[1], s));
-        for (size_t i = 0; i < b->hs.size(); ++i) {
-            b->hs[i]->stats_pending = true;
-            b->hs[i]->stats_timed = false;
-            b->hs[i]->last_norient = b->n_orient[i];
+        for (const spx_batch::Run &r : b->runs) {
+            r.h->stats_pending = true;
+            r.h->stats_timed = false;
+            r.h->last_norient = r.n_orient;
         }
         b->launched = true;
     });
@@ -4014,9 +4050,9 @@ spx_status spx_batch_synchronize(spx_batch *b, double *ms) {
         float t = 0.f;
         SPX_CUDA(cudaEventElapsedTime(&t, b->ev[0], b->ev[1]));
         if (ms) *ms = t;
-        for (size_t i = 0; i < b->hs.size(); ++i) {
+        for (size_t i = 0; i < b->runs.size(); ++i) {
             try {
-                finish_run(b->hs[i]);
+                finish_run(b->runs[i].h);
             } catch (const SpxError &e) {
                 throw SpxError(e.code, "system #" + std::to_string(i) + ": " + e.what());
             }

@@ -90,3 +90,56 @@ def test_steps_too_long_for_the_coupled_kernels_take_the_whole_system(gpu_engine
     v = sl.expm(-0.5j * np.pi * P.toarray()) @ rho0
     ref = [np.vdot(coil, np.linalg.matrix_power(U, j) @ Pi @ np.linalg.matrix_power(U, j) @ v) for j in range(3)]
     assert rel_err(res.fid, ref) <= 1e-3 and res.stats['coupled_dim'] == 0
+
+
+@pytest.mark.parametrize('prec,tol', [(E.FP64, 1e-10), (E.FP32, 1e-5)])
+def test_batch_follows_later_uploads(engine_lib, prec, tol):
+    """A captured batch runs what its handles hold at the launch: initial states in
+    another block (of other size), other coils, another system."""
+    import torch
+    H, Q, R, rho0, coil, block = _system(20, 70, False, True, 1, 2, 11)
+    rest = np.setdiff1d(np.arange(90), block)
+    H2, Q2, R2, rho2, coil2, block2 = _system(45, 60, True, True, 2, 1, 12)
+    dt, nsteps = 0.3, 80
+    eng, other = E.Engine(0), E.Engine(0)
+    batch = None
+    up = lambda e, *s: e.upload(sp.csc_matrix(s[0]), {(2, 2, 1): sp.csc_matrix(s[1])}, sp.csc_matrix(s[2]), s[3], s[4])
+    try:
+        up(eng, H, Q, R, rho0, coil)
+        up(other, H2, Q2, R2, rho2, coil2)
+        _, ptr = _device_grid()
+        outs = [torch.zeros(2 * (nsteps + 1), dtype=torch.float64, device='cuda') for _ in range(2)]
+        torch.cuda.synchronize()
+        batch = E.Batch([(e, 3, *ptr, dt, nsteps, o.data_ptr(), prec) for e, o in zip((eng, other), outs)])
+        full = np.arange(90)
+
+        def check(ref):
+            for _ in range(2):
+                batch.launch()
+                batch.synchronize()
+                assert rel_err(outs[0].cpu().numpy().view(complex), WEIGHTS @ ref) <= tol
+                ref2 = _reference(H2, Q2, R2, rho2, coil2, block2, dt, nsteps)
+                assert rel_err(outs[1].cpu().numpy().view(complex), WEIGHTS @ ref2) <= tol
+
+        check(_reference(H, Q, R, rho0, coil, block, dt, nsteps))
+        far = np.zeros(90, complex)
+        far[rest[3]], far[rest[40]] = 2.0, -1.0
+        states = np.zeros((3, 90), complex)
+        states[:, rest[0]] = [1.0, -2.0, 0.5]
+        eng.upload_coils([far])
+        eng.set_initial_states(states)
+        check(np.array([_reference(H, Q, R, states[o], far, full, dt, nsteps)[o] for o in range(3)]))
+        states[:, block[2]] = [0.3, 0.2, 0.1]
+        eng.upload_coils([far + coil])
+        eng.set_initial_states(states)
+        check(np.array([_reference(H, Q, R, states[o], far + coil, full, dt, nsteps)[o] for o in range(3)]))
+        up(eng, H2, Q2, R2, rho2, coil2)
+        check(_reference(H2, Q2, R2, rho2, coil2, block2, dt, nsteps))
+        eng.set_initial_states(np.zeros((2, 105), complex))
+        with pytest.raises(E.SpxError, match='per-orientation initial states'):
+            batch.launch()
+    finally:
+        if batch is not None:
+            batch.close()
+        eng.close()
+        other.close()
