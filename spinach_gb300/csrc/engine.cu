@@ -159,6 +159,7 @@ struct spx_handle {
     int64_t nnz = 0;
     double g_upper = 0.0;      // upper bound of the spectral radius of H over all orientations
     double max_im_diag = 0.0;
+    double max_growth = 0.0;   // largest rate at which a state grows (relaxation of the wrong sign)
     double lo_scale = 1.0;     // power of two scaling every assembled off-diagonal entry into (-1, 1)
     DevBuf<int> d_slice_off, d_stream_coef, d_term_rkm;
     std::vector<int> slice_off_host;
@@ -691,7 +692,11 @@ void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32
             row_bound[row] = rowsum;
         }
     }
-    for (int i = 0; i < n; ++i) max_im_diag = std::max(max_im_diag, std::fabs(diag[i].y));
+    double max_growth = 0.0;
+    for (int i = 0; i < n; ++i) {
+        max_im_diag = std::max(max_im_diag, std::fabs(diag[i].y));
+        max_growth = std::max(max_growth, diag[i].y);
+    }
     std::vector<int> stream_coef(nst);
     for (int q = 0; q < nst; ++q) stream_coef[q] = keep[q];     // slot in the coefficient vector
     std::vector<int> term_rkm(3 * std::max(n_terms, 1), 0);
@@ -747,6 +752,7 @@ void upload_system(spx_handle *h, const spx_csc *I, int32_t n_terms, const int32
     // scales them into (-1, 1) for the packed FP32 layout
     h->lo_scale = g_upper > 0.0 ? std::ldexp(1.0, -std::ilogb(g_upper) - 1) : 1.0;
     h->max_im_diag = max_im_diag;
+    h->max_growth = max_growth;
     h->ell_parts.assign(std::max(ell_len, 1), 0);
     for (int q = 0; q < nst; ++q)
         for (int e = 0; e < ell_len; ++e) {
@@ -1078,12 +1084,20 @@ bool forced_shape(const spx_options &o) {
     return (o.threads > 0 || o.cluster > 0 || o.chunk_steps > 0 || o.chunk_target > 0) && !(o.flags & kOwnShape);
 }
 
+// Whether the state could grow to more than four times its norm, which the
+// whole-system kernel refuses as diverged (its chunks' norm check).  The dense
+// matrices watch no norm, and the coupled-state kernels neither the other states
+// nor chunks as long, so a run that this may happen to is the whole system's.
+bool may_diverge(const spx_handle *h, double dt, int64_t nsteps) {
+    return h->max_growth * dt * (double)nsteps > 1.3862943611198906;       // ln 4
+}
+
 // Whether a powder run takes the coupled-state kernels.  c holds the whole
 // system's launch shape (so what is refused does not depend on them).
 void choose_block(spx_handle *h, const BlockPlan *plan, int64_t n_orient, double dt, int64_t nsteps,
                   const spx_options &opt, int kmax_override, int m_cap, Config &c) {
     const bool f64 = opt.precision == SPX_FP64;
-    if (!plan || !plan->ok || forced_shape(opt)) return;
+    if (!plan || !plan->ok || forced_shape(opt) || may_diverge(h, dt, nsteps)) return;
     // FP32 runs of more than 8192 undamped steps keep the whole system: there
     // FP32 nears the 1e-5 bar and its error decides whether the run is repeated
     // in FP64, so the decision stays the one it has been (a three-spin system,
@@ -2243,6 +2257,8 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
                           const std::vector<spx_seq_op> &ops, const spx_options &o, int64_t total, double *fid,
                           double *fids_per_orient) {
     if (forced_shape(o)) return false;
+    for (auto &q : ops)
+        if (q.kind == SPX_SEQ_EVOLVE && may_diverge(h, q.dt, q.nsteps)) return false;
     CoupledSequence seq(h, pulse_ops);
     const int n = seq.n();
     if (n == 0) return false;
@@ -2809,7 +2825,7 @@ std::vector<double2> apply_host(const HostCsr &m, const std::vector<double2> &x)
 bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const spx_csc *> &ops, double first_angle,
                       const double *back_angle, int echo_op, double tau, int64_t nsteps, const spx_options &o,
                       bool reverse) {
-    if (forced_shape(o)) return false;
+    if (forced_shape(o) || may_diverge(h, tau, nsteps)) return false;
     CoupledSequence seq(h, ops);
     const int n = seq.n();
     if (n == 0) return false;

@@ -143,3 +143,30 @@ def test_batch_follows_later_uploads(engine_lib, prec, tol):
             batch.close()
         eng.close()
         other.close()
+
+
+@pytest.mark.parametrize('n', [1, 6, 20, 70])
+@pytest.mark.parametrize('prec,tol', [(E.FP64, 1e-10), (E.FP32, 1e-5)])
+def test_growing_states_are_refused_at_every_size(gpu_engine, n, prec, tol):
+    """A relaxation matrix of the wrong sign: refused when the state may grow
+    fourfold, whichever kernels the size would take; run when it cannot."""
+    P = _shift_operator(n) if n > 1 else sp.csc_matrix((1, 1), dtype=complex)
+    for rate in (0.05, 0.3, 3.0):                       # over 45 steps of 0.7: factors of 5 and more
+        _upload(gpu_engine, *_chain(n, n, -rate))
+        with pytest.raises(E.SpxError, match='series did not converge'):
+            gpu_engine.run(*ANGLES, WEIGHTS, 0.7, 45, precision=prec)
+        with pytest.raises(E.SpxError, match='series did not converge'):
+            gpu_engine.run_sequence(*ANGLES, WEIGHTS, [P], [('evolve', 45, 0.7)], precision=prec)
+        with pytest.raises(E.SpxError, match='series did not converge'):
+            gpu_engine.run_eseem(*ANGLES, WEIGHTS, 45 * 1.4, 46, P, precision=prec)
+    mild = _chain(n, n, -0.03)                          # 45 steps: 2.6
+    _upload(gpu_engine, *mild)
+    res = gpu_engine.run(*ANGLES, WEIGHTS, 0.7, 45, precision=prec)
+    assert rel_err(res.fid, _fid(*mild, 0.7, 45)) <= tol
+    # growth where nothing is detected is refused too
+    H, R, rho0, coil = _chain(n, n, 0.01)
+    H2, R2, rho2, _ = _chain(9, 2, -0.3)
+    H, R = sl.block_diag(H, H2), sl.block_diag(R, R2)
+    _upload(gpu_engine, H, R, np.concatenate([rho0, rho2]), np.concatenate([coil, np.zeros(9)]))
+    with pytest.raises(E.SpxError, match='series did not converge'):
+        gpu_engine.run(*ANGLES, WEIGHTS, 0.7, 45, precision=prec)
