@@ -671,18 +671,19 @@ static __device__ __forceinline__ BlockSeries block_series(const BlockRun &R, in
     return S;
 }
 
-// e^{-i c j dt}, j < M: one sine and cosine per thread, turned on by
+// size e^{-i c j dt}, j < M: one sine and cosine per thread, turned on by
 // blockDim.x steps at a time (FP64 transcendentals are slow here), and the
 // phases of a whole and of the last chunk.
 template <class Vec>
-static __device__ __forceinline__ void block_phases(const BlockRun &R, const BlockSeries &S, Vec *phase, double2 *turn) {
+static __device__ __forceinline__ void block_phases(const BlockRun &R, const BlockSeries &S, double size, Vec *phase,
+                                                    double2 *turn) {
     const int tid = threadIdx.x, nt = (int)blockDim.x;
     if (tid < S.M) {
         double sn, cs, rs = 0.0, rc = 1.0;
         sincos(-S.cen * tid * R.dt, &sn, &cs);
         if (S.M > nt) sincos(-S.cen * nt * R.dt, &rs, &rc);
         for (int j = tid; j < S.M; j += nt) {
-            phase[j] = tovec(make_double2(cs, sn), Vec());
+            phase[j] = tovec(make_double2(size * cs, size * sn), Vec());
             const double c2 = cs * rc - sn * rs;
             sn = sn * rc + cs * rs;
             cs = c2;
@@ -810,7 +811,7 @@ __global__ void __launch_bounds__(ECAP == 24 ? 512 : 640, 1)
     __shared__ double s_coef[kMaxCoef];
     constexpr int XN = (EXT ? 2 : 1) * kBlockRows;            // the last slot takes what no one reads
     __shared__ float2 s_x[2][XN + 1];
-    __shared__ float s_norm[2][kBlockRows / 32 + 2];
+    __shared__ float s_norm[2][kBlockRows / 32 + 2], s_size;
     __shared__ double2 s_turn[2];
     extern __shared__ __align__(16) unsigned char smem[];
     float2 *s_b = reinterpret_cast<float2 *>(smem);          // chunk-end coefficients (b, b)
@@ -862,7 +863,6 @@ __global__ void __launch_bounds__(ECAP == 24 ? 512 : 640, 1)
         }
         if (tid < 2) s_b[Kc + tid] = make_float2(0.f, 0.f);
     };
-    block_phases(R, S, s_phase, s_turn);
     coefficients(M, S.K);
     if constexpr (TRJ) {
         for (int q = tid; q < NT * (S.K + 2); q += blockDim.x) {
@@ -876,6 +876,25 @@ __global__ void __launch_bounds__(ECAP == 24 ? 512 : 640, 1)
     if (l.state) {
         const double2 *r0 = R.rho0s ? R.rho0s + (size_t)block_grid_index(R, o) * R.state_stride : R.rho0;
         st = tovec(r0[B.state_pos[l.row]], float2());
+    }
+    // The state is carried in units of a power of two that puts the first one's
+    // largest part near one, so that the squares of the norm check fit a float
+    // whatever its size (in its own, states above 1.8e19 have an infinite norm
+    // and a bound violated below 1e-15 goes unnoticed).  The outputs' phases turn
+    // it back, so a chunk has no more work (scaling in the norm instead took 200
+    // orientations of a rotor-frame system, with their short chunks, 1 % longer).
+    {
+        float m = fmaxf(fabsf(st.x), fabsf(st.y));
+#pragma unroll
+        for (int q = 16; q; q >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, q));
+        if (lane == 0) s_norm[1][warp] = m;
+        __syncthreads();
+        for (int w = 0; w < nwarps; ++w) m = fmaxf(m, s_norm[1][w]);
+        const int e = m > 0.f ? max(-100, min(100, ilogbf(m))) : 0;
+        if (tid == 0) s_size = ldexpf(1.f, e);
+        st.x = ldexpf(st.x, -e);
+        st.y = ldexpf(st.y, -e);
+        block_phases(R, S, ldexp(1.0, e), s_phase, s_turn);
     }
     const float2 *mu_row = s_mu + (size_t)(l.row >= B.n ? l.row - B.n : 0) * (R.Kmax + 2);
     float2 *fid_out = reinterpret_cast<float2 *>(R.fids) + (size_t)o * R.nchan * (nsteps + 1);
@@ -937,7 +956,8 @@ __global__ void __launch_bounds__(ECAP == 24 ? 512 : 640, 1)
         [[maybe_unused]] f2x inner[NT + 1];
         if constexpr (TRJ) {
             if (l.state)
-                reinterpret_cast<float2 *>(R.traj_out)[((size_t)o * (nsteps + 1) + (size_t)a * M) * B.n + l.row] = st;
+                reinterpret_cast<float2 *>(R.traj_out)[((size_t)o * (nsteps + 1) + (size_t)a * M) * B.n + l.row] =
+                    make_float2(s_size * st.x, s_size * st.y);
 #pragma unroll
             for (int j = 0; j < NT; ++j)
                 inner[j] = mul2(reinterpret_cast<const f2x *>(s_tb + (size_t)j * (R.Kmax + 2))[0], tc);
@@ -1028,7 +1048,8 @@ __global__ void __launch_bounds__(ECAP == 24 ? 512 : 640, 1)
         if (status != kDevOk) break;
         start_n2 = end_n2;
     }
-    if (R.state_out && l.state) R.state_out[(size_t)o * R.state_stride + B.state_pos[l.row]] = tod(st);
+    if (R.state_out && l.state)
+        R.state_out[(size_t)o * R.state_stride + B.state_pos[l.row]] = tod(make_float2(s_size * st.x, s_size * st.y));
     if (tid == 0) {
         R.status[o] = status;
         R.kused[o] = S.K;
@@ -1104,7 +1125,7 @@ __global__ void __launch_bounds__(2 * kBlockRows, 1) block_chebyshev64_kernel(co
         for (int k = tid; k < Kc; k += blockDim.x) s_b[k] = block_sign(k) * S.tab[k * S.ld + j];
         if (tid < 2) s_b[Kc + tid] = 0.0;
     };
-    block_phases(R, S, s_phase, s_turn);
+    block_phases(R, S, 1.0, s_phase, s_turn);
     coefficients(M, S.K);
     if constexpr (TRJ) {
         for (int q = tid; q < NT * (S.K + 2); q += blockDim.x) {

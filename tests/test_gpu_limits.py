@@ -170,3 +170,33 @@ def test_growing_states_are_refused_at_every_size(gpu_engine, n, prec, tol):
     _upload(gpu_engine, H, R, np.concatenate([rho0, rho2]), np.concatenate([coil, np.zeros(9)]))
     with pytest.raises(E.SpxError, match='series did not converge'):
         gpu_engine.run(*ANGLES, WEIGHTS, 0.7, 45, precision=prec)
+
+
+def _outlier(half=30, out=11.0, coupling=1e-3):
+    """Two clusters of states at +-10 and one at `out`: two Lanczos steps find the
+    clusters and miss it, so lanczos_its=2 gives an interval about 10.7 (with its
+    margins) instead of 11.  Scaled by it the outlier lies at cosh(0.19), and a
+    series of argument x amplifies its rounding by exp(x sinh 0.19)."""
+    H = np.diag(np.concatenate([np.full(half, 10.0), np.full(half, -10.0), [out]]))
+    for i in range(1, len(H)):
+        H[i, i - 1] = H[i - 1, i] = coupling
+    n = len(H)
+    rho0, coil = np.ones(n, complex), np.zeros(n, complex)
+    coil[0] = coil[n - 1] = 1.0
+    return H, np.zeros((n, n)), rho0, coil
+
+
+@pytest.mark.parametrize('size', [1.0, 1e25, 1e37, 1e-20, 1e-36])
+def test_fp32_states_of_extreme_size(gpu_engine, size):
+    """The FP32 kernels' norm check holds for initial states of any size: large and
+    small ones run, and a violated spectral bound is noticed and mended."""
+    H, R, rho0, coil = _chain(20, 3)
+    _upload(gpu_engine, H, R, rho0 * size, coil)
+    res = gpu_engine.run(*ANGLES, WEIGHTS, 0.7, 45, precision=E.FP32, fp32_check=False)
+    assert rel_err(res.fid / size, _fid(H, R, rho0, coil, 0.7, 45)) <= 1e-5
+    H, R, rho0, coil = _outlier()
+    _upload(gpu_engine, H, R, rho0 * size, coil)
+    # one chunk of argument 175: exp(34) of 2^-24, far above the fourfold growth
+    res = gpu_engine.run(*ANGLES, WEIGHTS, 0.28, 59, precision=E.FP32, lanczos_its=2, fp32_check=False)
+    assert res.stats['retries'] == 1 and res.stats['coupled_dim'] == len(H)
+    assert rel_err(res.fid / size, _fid(H, R, rho0, coil, 0.28, 59)) <= 1e-5
