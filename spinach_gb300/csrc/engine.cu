@@ -2212,7 +2212,8 @@ bool configure_group(spx_handle *h, SequenceGroup &g, int64_t n_orient, double d
 // Propagates a group over nsteps steps of dt: bounds on the first call, tables
 // whenever the time step changes.
 void run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockRun r, int64_t n_orient,
-               const double *const (&angles)[3], double dt, int64_t nsteps, double tol, bool f64, bool traj, int *status, double *halfwidth) {
+               const double *const (&angles)[3], double dt, int64_t nsteps, double tol, int lanczos_its, bool f64, bool traj,
+               int *status, double *halfwidth) {
     if (!g.bounded || g.table_dt != dt) {
         Config c = g.c;
         if (!configure_group(h, g, n_orient, dt, tol, f64, traj, c))
@@ -2225,7 +2226,7 @@ void run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockR
     block_run_buffers(r, c, b.centre.p, b.extent.p, b.lev_half.p, b.lev.p, b.kcut.p, b.table.p, f64 ? nullptr : b.tablef.p);
     if (saves_block(n_orient, f64, c)) r.saved = b.saved.p;
     r.n_orient = (int)n_orient; r.alpha = angles[0]; r.beta = angles[1]; r.gamma = angles[2];
-    r.dt = dt; r.lanczos_its = 32;
+    r.dt = dt; r.lanczos_its = lanczos_its > 0 ? lanczos_its : 32;
     r.max_im_diag = h->max_im_diag; r.halfwidth = halfwidth;
     r.nchan = 1; r.status = status;
     r.kused = h->d_kused.p; r.mused = h->d_mused.p; r.matvecs = h->d_matvecs.p;
@@ -2397,7 +2398,7 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
                 grp.bufs.halfwidth.reserve(n_orient);
                 half = grp.bufs.halfwidth.p;
             }
-            run_group(h, grp, sys, r, n_orient, angles, q.dt, q.nsteps, whole.tol, f64, false, status, half);
+            run_group(h, grp, sys, r, n_orient, angles, q.dt, q.nsteps, whole.tol, o.lanczos_its, f64, false, status, half);
         }
         if (q.record) {
             const size_t np = (size_t)q.nsteps + 1;
@@ -2918,7 +2919,8 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
         r.state_out = h->d_seq[0].p;
         const double *const angles[3] = {g, g + n_orient, g + 2 * n_orient};
         gb.bufs.halfwidth.reserve(n_orient);
-        run_group(h, gb, sys, r, n_orient, angles, tau, nsteps, whole.tol, f64, false, status[2], gb.bufs.halfwidth.p);
+        run_group(h, gb, sys, r, n_orient, angles, tau, nsteps, whole.tol, o.lanczos_its, f64, false, status[2],
+                  gb.bufs.halfwidth.p);
         dback.upload(back, h->stream);
         ++h->launches;
         sparse_states_kernel<<<state_blocks(h, ns), 256, 0, h->stream>>>(n_orient, n, dback.ptr.p, dback.col.p, dback.val.p,
@@ -2974,7 +2976,7 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
             else r.rho0 = adj;
             r.traj_out = dir ? tv : tu;
             const bool final = dir == 1;
-            run_group(h, grp, sys, r, nb, angles, tau, nsteps, whole.tol, f64, true, status[dir] + b0,
+            run_group(h, grp, sys, r, nb, angles, tau, nsteps, whole.tol, o.lanczos_its, f64, true, status[dir] + b0,
                       final ? h->d_halfwidth.p + b0 : grp.bufs.halfwidth.p);
         }
         const int64_t warps = nb * npoints;

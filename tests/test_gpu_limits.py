@@ -200,3 +200,53 @@ def test_fp32_states_of_extreme_size(gpu_engine, size):
     res = gpu_engine.run(*ANGLES, WEIGHTS, 0.28, 59, precision=E.FP32, lanczos_its=2, fp32_check=False)
     assert res.stats['retries'] == 1 and res.stats['coupled_dim'] == len(H)
     assert rel_err(res.fid / size, _fid(H, R, rho0, coil, 0.28, 59)) <= 1e-5
+
+
+def _call(eng, name, program, opt, npts, fill=None):
+    """A pulse program or an echo on the three orientations through the C entry
+    points: status, powder points and every orientation's."""
+    import ctypes as C
+    n = eng.dim
+    P = E._CscHolder(_shift_operator(n), n)
+    fid, fids = np.full(2 * npts, fill if fill else 0.0), np.full(2 * npts * 3, fill if fill else 0.0)
+    grid = [E._dptr(np.ascontiguousarray(a)) for a in (*ANGLES, WEIGHTS)]
+    if name == 'sequence':
+        ops = (E.SpxSeqOp * len(program))(*[E.SpxSeqOp(E.SEQ_EVOLVE, 0, 0.0, ns, dt, 1, 0) for ns, dt in program])
+        st = eng.lib.spx_run_sequence(eng.h, 3, *grid, 1, (E.SpxCsc * 1)(P.struct), len(program), ops, C.byref(opt),
+                                      E._dptr(fid), E._dptr(fids))
+    elif name == 'eseem':
+        ns, dt = program
+        st = eng.lib.spx_run_eseem(eng.h, 3, *grid, 2 * dt, ns + 1, C.byref(P.struct), C.byref(opt), E._dptr(fid),
+                                   E._dptr(fids))
+    else:
+        ns, dt = program
+        st = eng.lib.spx_run_deer(eng.h, 3, *grid, dt, ns, C.byref(P.struct), C.byref(P.struct), C.byref(opt),
+                                  E._dptr(fid), E._dptr(fids))
+    return st, fid, fids
+
+
+@pytest.mark.parametrize('prec', [E.FP64, E.FP32])
+@pytest.mark.parametrize('name', ['sequence', 'eseem', 'deer'])
+def test_lanczos_steps_reach_sequences_and_echoes(engine_lib, name, prec):
+    """Two Lanczos steps give the outlier's system an interval that misses it (and
+    a refusal: these entry points do not retry); 32 and 48 hold it."""
+    import ctypes as C
+    eng = E.Engine(0)
+    try:
+        _upload(eng, *_outlier(half=12))                    # pulses connect all 25 states
+        program, npts = ([(79, 0.33)], 80) if name == 'sequence' else ((79, 0.33), 80)
+        half = {}
+        for its in (0, 2, 32, 48):
+            st, fid, _ = _call(eng, name, program, E.SpxOptions(prec, 0, 0, 0, 0.0, 0.0, its, 0), npts)
+            s = E.SpxStats()
+            eng.lib.spx_get_stats(eng.h, C.byref(s))
+            half[its] = (st, s.max_half_width, fid)
+            assert s.coupled_dim == 25
+        assert half[2][1] < 0.99 * half[32][1]              # 10.46 and 10.61 by the formula of the bounds
+        if name == 'sequence':                              # chunks long enough to grow
+            assert half[2][0] == 5
+        for its in (0, 48):
+            assert half[its][0] == 0 and abs(half[its][1] / half[32][1] - 1) <= 1e-3
+        assert np.array_equal(half[0][2], half[32][2])
+    finally:
+        eng.close()
