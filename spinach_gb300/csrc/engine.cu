@@ -1761,15 +1761,18 @@ FP32Error fp32_error(const std::vector<const float2 *> &f32, const double2 *f64,
     return out;
 }
 
-// Synchronise, read per-orientation status and fill the statistics; fid, if
-// given: also the powder FID of h->d_fid.  All results are copied behind the run
-// into one pinned buffer of the handle (runs of more than kStage bytes of them:
-// pageable memory) and waited for once: a copy of its own for each of the eleven
-// took a 200-orientation run of three spins 271 us; it takes 181.
-void finish_run(spx_handle *h, double *fid = nullptr) {
+// Synchronise, read per-orientation status and fill the statistics.  All results
+// are copied behind the run into one pinned buffer of the handle (runs of more
+// than kStage bytes of them: pageable memory) and waited for once: a copy of its
+// own for each of the eleven took a 200-orientation run of three spins 271 us;
+// it takes 181.  want_fid: also the powder FID of h->d_fid, which is returned in
+// that buffer, where it lies until the handle's next run (null if it does not
+// fit: then it is still in h->d_fid).  The caller's arrays are left to the
+// caller, who writes them once nothing can fail any more.
+const double *finish_run(spx_handle *h, bool want_fid = false) {
     if (!h->stats_pending) {
         SPX_CUDA(cudaStreamSynchronize(h->stream));
-        return;
+        return nullptr;
     }
     h->stats_pending = false;
     const int64_t no = h->last_norient;
@@ -1787,7 +1790,6 @@ void finish_run(spx_handle *h, double *fid = nullptr) {
     const size_t p_status = piece(h->d_status.p, no * sizeof(int)), p_kused = piece(h->d_kused.p, no * sizeof(int)),
                  p_mused = piece(h->d_mused.p, no * sizeof(int)), p_mv = piece(h->d_matvecs.p, no * sizeof(long long)),
                  p_hw = piece(h->d_halfwidth.p, no * sizeof(double));
-    const size_t p_fid = fid ? piece(h->d_fid.p, npts * sizeof(double2)) : 0;
     size_t p_cst = 0, p_f64 = 0, p_f32 = 0, p_pw = 0, p_w = 0;
     if (S > 0) {
         p_cst = piece(h->d_chk_status.p, S * sizeof(int));
@@ -1800,6 +1802,8 @@ void finish_run(spx_handle *h, double *fid = nullptr) {
         p_pw = piece(h->chk_out, npts * sizeof(double2));
         p_w = piece(h->chk_w, no * sizeof(double));
     }
+    want_fid = want_fid && total + npts * sizeof(double2) <= kStage;
+    const size_t p_fid = want_fid ? piece(h->d_fid.p, npts * sizeof(double2)) : 0;
     std::vector<unsigned char> pageable;
     unsigned char *base;
     if (total <= kStage) {
@@ -1862,7 +1866,6 @@ void finish_run(spx_handle *h, double *fid = nullptr) {
             h->stats.fp32_powder_error = e.powder;
         }
     }
-    if (fid) std::memcpy(fid, words(p_fid), npts * sizeof(double2));
     if (failed) {
         static const char *why[] = {"ok", "series longer than the coefficient table", "state norm grew (spectral bound violated)",
                                     "non-finite state", "launch configuration has too few threads"};
@@ -1870,6 +1873,7 @@ void finish_run(spx_handle *h, double *fid = nullptr) {
         throw SpxError(SPX_ERR_SERIES, std::to_string(failed) + " orientation(s) failed, first #" +
                                            std::to_string(first_bad) + ": " + w);
     }
+    return want_fid ? reinterpret_cast<const double *>(words(p_fid)) : nullptr;
 }
 
 void validate_run(spx_handle *h, int64_t n_orient, double dt, int64_t nsteps) {
@@ -2366,6 +2370,7 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
     }
     Config whole{};
     int64_t at = 0, launched = 0;
+    std::vector<std::vector<unsigned char>> each;      // recorded segments, until all of them are known to be good
     SPX_CUDA(cudaEventRecord(h->ev[0], h->stream));
     for (size_t i = 0; i < ops.size(); ++i) {
         const spx_seq_op &q = ops[i];
@@ -2404,22 +2409,11 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
             const size_t np = (size_t)q.nsteps + 1;
             launch_powder_sum(h, f64, h->d_fids.p, g + 3 * n_orient, n_orient, np, h->d_part.p, h->d_fid.p + at);
             if (fids_per_orient) {
-                // this segment's FIDs of every orientation, into each orientation's row
-                std::vector<unsigned char> tmp(np * (size_t)n_orient * vec);
-                SPX_CUDA(cudaMemcpyAsync(tmp.data(), h->d_fids.p, tmp.size(), cudaMemcpyDeviceToHost, h->stream));
+                // this segment's FIDs of every orientation
+                each.emplace_back(np * (size_t)n_orient * vec);
+                SPX_CUDA(cudaMemcpyAsync(each.back().data(), h->d_fids.p, each.back().size(), cudaMemcpyDeviceToHost,
+                                         h->stream));
                 SPX_CUDA(cudaStreamSynchronize(h->stream));
-                for (int64_t w = 0; w < n_orient; ++w)
-                    for (size_t j = 0; j < np; ++j) {
-                        const size_t e = (size_t)w * np + j;
-                        double2 v;
-                        if (f64) v = reinterpret_cast<const double2 *>(tmp.data())[e];
-                        else {
-                            const float2 f = reinterpret_cast<const float2 *>(tmp.data())[e];
-                            v = make_double2(f.x, f.y);
-                        }
-                        fids_per_orient[2 * ((size_t)w * total + at + j)] = v.x;
-                        fids_per_orient[2 * ((size_t)w * total + at + j) + 1] = v.y;
-                    }
             }
             at += (int64_t)np;
         }
@@ -2437,6 +2431,24 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
     finish_run(h);
     if (launched) check_statuses(h, n_orient, launched);
     if (total > 0) SPX_CUDA(cudaMemcpy(fid, h->d_fid.p, (size_t)total * sizeof(double2), cudaMemcpyDeviceToHost));
+    at = 0;
+    for (const std::vector<unsigned char> &seg : each) {
+        // into each orientation's row
+        const size_t np = seg.size() / ((size_t)n_orient * vec);
+        for (int64_t w = 0; w < n_orient; ++w)
+            for (size_t j = 0; j < np; ++j) {
+                const size_t e = (size_t)w * np + j;
+                double2 v;
+                if (f64) v = reinterpret_cast<const double2 *>(seg.data())[e];
+                else {
+                    const float2 f = reinterpret_cast<const float2 *>(seg.data())[e];
+                    v = make_double2(f.x, f.y);
+                }
+                fids_per_orient[2 * ((size_t)w * total + at + j)] = v.x;
+                fids_per_orient[2 * ((size_t)w * total + at + j) + 1] = v.y;
+            }
+        at += (int64_t)np;
+    }
     return true;
 }
 
@@ -3509,8 +3521,9 @@ spx_status spx_run_powder(spx_handle *h, int64_t n_orient, const double *alphas,
         launch_powder(h, n_orient, g, g + n_orient, g + 2 * n_orient, g + 3 * n_orient, dt, nsteps, o, h->d_fid.p, c,
                       0, true, RunIO{}, check);
         bool retried = false;
+        const double *staged = nullptr;
         try {
-            finish_run(h, fid);
+            staged = finish_run(h, true);
         } catch (const SpxError &e) {
             // one retry: a wider coefficient table if that was the only problem,
             // otherwise the conservative spectral bound
@@ -3528,7 +3541,7 @@ spx_status spx_run_powder(spx_handle *h, int64_t n_orient, const double *alphas,
             retried = true;
             launch_powder(h, n_orient, g, g + n_orient, g + 2 * n_orient, g + 3 * n_orient, dt, nsteps, o,
                           h->d_fid.p, c, 1, true, RunIO{}, check);
-            finish_run(h, fid);
+            staged = finish_run(h, true);
         }
         h->stats.retries = retried ? 1 : 0;
         // the bar applies to what the caller receives: the powder FID, and
@@ -3551,7 +3564,7 @@ spx_status spx_run_powder(spx_handle *h, int64_t n_orient, const double *alphas,
             const Config c64 = choose_config(h, n_orient, dt, nsteps, o64, 0, 256, false, &h->plan);
             launch_powder(h, n_orient, g, g + n_orient, g + 2 * n_orient, g + 3 * n_orient, dt, nsteps, o64,
                           h->d_fid.p, c64);
-            finish_run(h, fid);
+            staged = finish_run(h, true);
             h->stats.fp32_checked = s32.fp32_checked;
             h->stats.fp32_rel_error = s32.fp32_rel_error;
             h->stats.fp32_powder_error = s32.fp32_powder_error;
@@ -3559,6 +3572,9 @@ spx_status spx_run_powder(spx_handle *h, int64_t n_orient, const double *alphas,
             h->stats.retries = s32.retries;
             o.precision = SPX_FP64;
         }
+        const size_t fid_bytes = ((size_t)nsteps + 1) * h->nchan * sizeof(double2);
+        if (staged) std::memcpy(fid, staged, fid_bytes);
+        else SPX_CUDA(cudaMemcpy(fid, h->d_fid.p, fid_bytes, cudaMemcpyDeviceToHost));
         if (fids_per_orient) {
             const size_t cnt = ((size_t)nsteps + 1) * h->nchan * n_orient;
             if (o.precision == SPX_FP64) {

@@ -250,3 +250,42 @@ def test_lanczos_steps_reach_sequences_and_echoes(engine_lib, name, prec):
         assert np.array_equal(half[0][2], half[32][2])
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize('prec', [E.FP64, E.FP32])
+def test_a_failed_run_leaves_the_output_untouched(engine_lib, prec):
+    import ctypes as C
+    eng = E.Engine(0)
+    try:
+        # whole system (growing) and coupled states (a violated bound, not retried)
+        _upload(eng, *_chain(20, 3, -3.0))
+        fid, fids = np.full(2 * 46, 7.0), np.full(2 * 46 * 3, 7.0)
+        grid = [E._dptr(np.ascontiguousarray(a)) for a in (*ANGLES, WEIGHTS)]
+        opt = E.SpxOptions(prec, 0, 0, 0, 0.0, 0.0, 0, 0)
+        assert eng.lib.spx_run_powder(eng.h, 3, *grid, 0.7, 45, C.byref(opt), E._dptr(fid), E._dptr(fids)) == 5
+        assert np.all(fid == 7.0) and np.all(fids == 7.0)
+        _upload(eng, *_outlier(half=12))
+        opt.lanczos_its = 2
+        st, fid, fids = _call(eng, 'sequence', [(2, 0.01), (79, 0.33)], opt, 83, fill=7.0)
+        assert st == 5 and np.all(fid == 7.0) and np.all(fids == 7.0)
+        # the same program with the default bounds: every point is written
+        opt.lanczos_its = 0
+        st, fid, fids = _call(eng, 'sequence', [(2, 0.01), (79, 0.33)], opt, 83, fill=7.0)
+        each = fids.view(complex).reshape(3, 83)
+        assert st == 0 and rel_err(WEIGHTS @ each, fid.view(complex)) <= 1e-6 and not np.any(fids == 7.0)
+    finally:
+        eng.close()
+
+
+def test_outputs_larger_than_the_pinned_stage(gpu_engine):
+    """FIDs of more than 8 MB come straight from the device."""
+    H, R, rho0, coil = _chain(6, 4)
+    _upload(gpu_engine, H, R, rho0, coil)
+    nsteps = 600000                                         # 9.6 MB
+    res = gpu_engine.run(*[a[:1] for a in ANGLES], WEIGHTS[:1], 0.01, nsteps, precision=E.FP64)
+    e, V = np.linalg.eigh(H)
+    a = (coil.conj() @ V) * (V.T @ rho0)
+    at = np.array([0, 1, 7777, 299999, nsteps])
+    ref = WEIGHTS[0] * np.array([np.sum(a * np.exp(-1j * e * 0.01 * k)) for k in at])
+    # rounding of 2400 chunks, of which each adds a few 2^-53
+    assert np.abs(res.fid[at] - ref).max() <= 1e-10 * np.abs(ref).max()
