@@ -93,7 +93,13 @@ typedef struct {
  * on the others.  A run whose options set threads, cluster, chunk_steps or
  * chunk_target takes the whole system in that shape.
  */
-/* Statistics of the last spx_run_powder* call on a handle. */
+/*
+ * Statistics of the last run on a handle.  After a pulse program or an echo on
+ * the coupled states the times span the whole program; matvecs, max_terms,
+ * chunk_steps, the half-widths and coupled_dim are those of its last series over
+ * all orientations: the coil's states in the last segment, or the adjoint
+ * trajectory of an echo.  (On the whole system everything is the last launch's.)
+ */
 typedef struct {
     int64_t n_orientations;
     int64_t nsteps;

@@ -2214,10 +2214,11 @@ bool configure_group(spx_handle *h, SequenceGroup &g, int64_t n_orient, double d
 }
 
 // Propagates a group over nsteps steps of dt: bounds on the first call, tables
-// whenever the time step changes.
+// whenever the time step changes.  first: place of the orientations among the
+// call's (status and halfwidth are given where they start).
 void run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockRun r, int64_t n_orient,
                const double *const (&angles)[3], double dt, int64_t nsteps, double tol, int lanczos_its, bool f64, bool traj,
-               int *status, double *halfwidth) {
+               int *status, double *halfwidth, int64_t first = 0) {
     if (!g.bounded || g.table_dt != dt) {
         Config c = g.c;
         if (!configure_group(h, g, n_orient, dt, tol, f64, traj, c))
@@ -2233,7 +2234,7 @@ void run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockR
     r.dt = dt; r.lanczos_its = lanczos_its > 0 ? lanczos_its : 32;
     r.max_im_diag = h->max_im_diag; r.halfwidth = halfwidth;
     r.nchan = 1; r.status = status;
-    r.kused = h->d_kused.p; r.mused = h->d_mused.p; r.matvecs = h->d_matvecs.p;
+    r.kused = h->d_kused.p + first; r.mused = h->d_mused.p + first; r.matvecs = h->d_matvecs.p + first;
     if (!g.bounded) launch_bounds(h, c, sys, r, h->stream);
     g.bounded = true;
     if (g.table_dt != dt) {
@@ -2989,7 +2990,7 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
             r.traj_out = dir ? tv : tu;
             const bool final = dir == 1;
             run_group(h, grp, sys, r, nb, angles, tau, nsteps, whole.tol, o.lanczos_its, f64, true, status[dir] + b0,
-                      final ? h->d_halfwidth.p + b0 : grp.bufs.halfwidth.p);
+                      final ? h->d_halfwidth.p + b0 : grp.bufs.halfwidth.p, b0);
         }
         const int64_t warps = nb * npoints;
         const int blocks = (int)std::min<int64_t>((warps + 7) / 8, (int64_t)h->sm_count * 16);

@@ -289,3 +289,38 @@ def test_outputs_larger_than_the_pinned_stage(gpu_engine):
     ref = WEIGHTS[0] * np.array([np.sum(a * np.exp(-1j * e * 0.01 * k)) for k in at])
     # rounding of 2400 chunks, of which each adds a few 2^-53
     assert np.abs(res.fid[at] - ref).max() <= 1e-10 * np.abs(ref).max()
+
+
+def test_echo_in_several_batches(engine_lib):
+    """With little free memory the trajectories of an echo come in batches; points
+    and statistics are those of one batch (whose ladder of half-widths may lie a
+    step of 1/16 octave off)."""
+    import torch
+    n, no, npoints, dt = 100, 200, 2048, 0.01
+    H, R, rho0, coil = _chain(n, 6, 0.01)
+    P = sp.csc_matrix(sl.block_diag(*[[[0.0, 1.0], [1.0, 0.0]]] * (n // 2)))
+    rng = np.random.default_rng(2)
+    grid = (*rng.uniform(0, 3, (3, no)), rng.uniform(0.1, 1, no))
+    Q = sp.csc_matrix(np.diag(rng.normal(size=n)).astype(complex))
+    res = []
+    for limited in (True, False):
+        eng, hold = E.Engine(0), None
+        try:
+            eng.upload(sp.csc_matrix(H.astype(complex)), {(2, 2, 1): Q}, sp.csc_matrix(R.astype(complex)), rho0, coil)
+            if limited:
+                # 3 GB left, of which a quarter takes 120 orientations' trajectories
+                torch.cuda.empty_cache()
+                hold = torch.empty(torch.cuda.mem_get_info()[0] - (3 << 30), dtype=torch.uint8, device='cuda')
+            res.append(eng.run_eseem(*grid, 2 * dt, npoints, P, precision=E.FP64, per_orientation=True))
+        finally:
+            eng.close()
+            del hold
+            torch.cuda.empty_cache()
+    a, b = res
+    for o in range(no):
+        assert rel_err(a.fids[o], b.fids[o]) <= 1e-10, o
+    assert rel_err(a.fid, b.fid) <= 1e-10
+    assert a.stats['coupled_dim'] == n and a.stats['n_orientations'] == no
+    assert a.stats['chunk_steps'] == b.stats['chunk_steps']
+    for key in ('min_half_width', 'max_half_width', 'matvecs', 'max_terms'):
+        assert abs(a.stats[key] / b.stats[key] - 1) <= 0.1, key
