@@ -854,7 +854,8 @@ constexpr int kPowderGroup = 64;    // orientations per partial sum of the powde
 
 // spx_options.flags bit of a launch shape that the engine chose itself (the
 // autotuner's): such a run may still take the coupled-state kernels, one whose
-// caller set a shape runs the whole system in that shape.
+// caller set a shape (or a chunk length beside the tuner's) runs the whole
+// system in that shape.  Never a caller's (given_options).
 constexpr int32_t kOwnShape = 1 << 30;
 
 struct Config {
@@ -1081,7 +1082,17 @@ void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, 
 }
 
 bool forced_shape(const spx_options &o) {
-    return (o.threads > 0 || o.cluster > 0 || o.chunk_steps > 0 || o.chunk_target > 0) && !(o.flags & kOwnShape);
+    return o.chunk_steps > 0 || ((o.threads > 0 || o.cluster > 0 || o.chunk_target > 0) && !(o.flags & kOwnShape));
+}
+
+// The caller's options (null: the defaults).
+spx_options given_options(const spx_options *opt) {
+    spx_options o{};
+    if (opt) o = *opt;
+    if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
+        throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
+    o.flags &= ~kOwnShape;
+    return o;
 }
 
 // Whether the state could grow to more than four times its norm, which the
@@ -3498,10 +3509,7 @@ spx_status spx_run_powder(spx_handle *h, int64_t n_orient, const double *alphas,
             if (!std::isfinite(alphas[o]) || !std::isfinite(betas[o]) || !std::isfinite(gammas[o]) ||
                 !std::isfinite(weights[o]))
                 throw SpxError(SPX_ERR_INVALID_ARGUMENT, "non-finite grid entry");
-        spx_options o{};
-        if (opt) o = *opt;
-        if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
-            throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
+        spx_options o = given_options(opt);
         o = apply_tuned(h, o);
         SPX_CUDA(cudaSetDevice(h->device));
         h->d_grid.reserve(4 * (size_t)n_orient);
@@ -3600,10 +3608,7 @@ spx_status spx_run_powder_device(spx_handle *h, int64_t n_orient, const double *
         validate_run(h, n_orient, dt, nsteps);
         if (!d_alphas || !d_betas || !d_gammas || !d_weights || !d_fid)
             throw SpxError(SPX_ERR_INVALID_ARGUMENT, "NULL device pointer");
-        spx_options o{};
-        if (opt) o = *opt;
-        if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
-            throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
+        spx_options o = given_options(opt);
         o = apply_tuned(h, o);
         SPX_CUDA(cudaSetDevice(h->device));
         const Config c = choose_config(h, n_orient, dt, nsteps, o, 0, 256, false, &h->plan);
@@ -3664,10 +3669,7 @@ spx_status spx_run_cpmg(spx_handle *h, int64_t n_orient, const double *alphas, c
             if (!std::isfinite(alphas[o]) || !std::isfinite(betas[o]) || !std::isfinite(gammas[o]) ||
                 !std::isfinite(weights[o]))
                 throw SpxError(SPX_ERR_INVALID_ARGUMENT, "non-finite grid entry");
-        spx_options o{};
-        if (opt) o = *opt;
-        if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
-            throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
+        spx_options o = given_options(opt);
         o = apply_tuned(h, o);
         SPX_CUDA(cudaSetDevice(h->device));
         run_cpmg(h, n_orient, alphas, betas, gammas, weights, dt, npoints, nloops, pulse_op, o, fid, fids_per_orient);
@@ -3685,10 +3687,7 @@ spx_status spx_run_sequence(spx_handle *h, int64_t n_orient, const double *alpha
             if (!std::isfinite(alphas[o]) || !std::isfinite(betas[o]) || !std::isfinite(gammas[o]) ||
                 !std::isfinite(weights[o]))
                 throw SpxError(SPX_ERR_INVALID_ARGUMENT, "non-finite grid entry");
-        spx_options o{};
-        if (opt) o = *opt;
-        if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
-            throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
+        spx_options o = given_options(opt);
         o = apply_tuned(h, o);
         SPX_CUDA(cudaSetDevice(h->device));
         run_sequence(h, n_orient, alphas, betas, gammas, weights, n_pulse, pulse_ops, n_ops, ops, o, fid,
@@ -3709,10 +3708,7 @@ spx_status run_echo_entry(spx_handle *h, int64_t n_orient, const double *alphas,
             if (!std::isfinite(alphas[o]) || !std::isfinite(betas[o]) || !std::isfinite(gammas[o]) ||
                 !std::isfinite(weights[o]))
                 throw SpxError(SPX_ERR_INVALID_ARGUMENT, "non-finite grid entry");
-        spx_options o{};
-        if (opt) o = *opt;
-        if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
-            throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
+        spx_options o = given_options(opt);
         SPX_CUDA(cudaSetDevice(h->device));
         run_eseem(h, n_orient, alphas, betas, gammas, weights, timestep, npoints, pulse_op, first_angle, o, fid,
                   fids_per_orient);
@@ -3746,10 +3742,7 @@ spx_status spx_run_deer(spx_handle *h, int64_t n_orient, const double *alphas, c
             if (!std::isfinite(alphas[o]) || !std::isfinite(betas[o]) || !std::isfinite(gammas[o]) ||
                 !std::isfinite(weights[o]))
                 throw SpxError(SPX_ERR_INVALID_ARGUMENT, "non-finite grid entry");
-        spx_options o{};
-        if (opt) o = *opt;
-        if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
-            throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
+        spx_options o = given_options(opt);
         SPX_CUDA(cudaSetDevice(h->device));
         run_deer(h, n_orient, alphas, betas, gammas, weights, stepsize, nsteps, ex_prob, ex_pump, o, fid,
                  fids_per_orient);
@@ -4027,10 +4020,7 @@ spx_status spx_batch_create(spx_batch **out, int32_t n, spx_handle *const *handl
         for (auto &e : b->ev) SPX_CUDA(cudaEventCreate(&e));
         for (int i = 0; i < n; ++i) {
             finish_run(handles[i]);
-            spx_options o{};
-            if (opts) o = opts[i];
-            if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
-                throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
+            const spx_options o = given_options(opts ? &opts[i] : nullptr);
             b->runs.push_back({handles[i], n_orient[i], d_alphas[i], d_betas[i], d_gammas[i], d_weights[i], dt[i],
                                nsteps[i], o, reinterpret_cast<double2 *>(d_fids[i]), 0});
         }

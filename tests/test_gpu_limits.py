@@ -324,3 +324,31 @@ def test_echo_in_several_batches(engine_lib):
     assert a.stats['chunk_steps'] == b.stats['chunk_steps']
     for key in ('min_half_width', 'max_half_width', 'matvecs', 'max_terms'):
         assert abs(a.stats[key] / b.stats[key] - 1) <= 0.1, key
+
+
+@pytest.mark.parametrize('prec', [E.FP64, E.FP32])
+def test_chunk_length_and_flags_of_the_caller_on_a_tuned_handle(engine_lib, prec):
+    """A chunk length takes the whole system, tuned or not; a bit of the flags that
+    means nothing does not turn a forced shape into the engine's own."""
+    import ctypes as C
+    eng = E.Engine(0)
+    try:
+        H, R, rho0, coil = _chain(40, 5)
+        _upload(eng, H, R, rho0, coil)
+        ref = WEIGHTS.sum() * _fid(H, R, rho0, coil, 0.3, 100)
+        _, ptr = _device_grid()
+        for tuned in (False, True):
+            if tuned:
+                eng.autotune(*ptr[:3], 3, 0.3, 100, prec)
+            res = eng.run(*ANGLES, WEIGHTS, 0.3, 100, precision=prec, chunk_steps=10)
+            assert res.stats['coupled_dim'] == 0 and res.stats['chunk_steps'] == 10
+            assert rel_err(res.fid, ref) <= (1e-10 if prec else 1e-5)
+            res = eng.run(*ANGLES, WEIGHTS, 0.3, 100, precision=prec)
+            assert res.stats['coupled_dim'] == 40
+            fid = np.zeros(2 * 101)
+            grid = [E._dptr(np.ascontiguousarray(a)) for a in (*ANGLES, WEIGHTS)]
+            opt = E.SpxOptions(prec, 0, 96, 1, 0.0, 0.0, 0, 1 << 30)
+            assert eng.lib.spx_run_powder(eng.h, 3, *grid, 0.3, 100, C.byref(opt), E._dptr(fid), None) == 0
+            assert eng.stats()['coupled_dim'] == 0 and eng.stats()['threads'] == 96
+    finally:
+        eng.close()
