@@ -91,7 +91,8 @@ typedef struct {
  * coils: the connected components of the Liouvillian's pattern that hold both
  * coil and initial-state entries, at most 512 states.  The FIDs do not depend
  * on the others.  A run whose options set threads, cluster, chunk_steps or
- * chunk_target takes the whole system in that shape.
+ * chunk_target takes the whole system in that shape, unless threads, cluster and
+ * chunk_target are what spx_autotune returned for such a system.
  */
 /*
  * Statistics of the last run on a handle.  After a pulse program or an echo on
@@ -393,10 +394,13 @@ spx_status spx_upload_coils(spx_handle *handle, int32_t nchan, const double *coi
  * per orientation (1, 2, 4, 8), warps per CTA, series length per chunk -- on
  * one wave of the given device-resident orientations over at most 512 steps,
  * and keeps the fastest in the handle: later runs whose options leave
- * threads, cluster and chunk_target at 0 use it.  Results are cached per
- * system shape (dimension, ELL size, value streams, precision, spectral
- * scale) for the life of the process.  best (may be NULL) receives the chosen
- * options; spx_stats reports what a run used.
+ * threads, cluster and chunk_target at 0, or hand back what was returned, use
+ * it.  Where runs restrict themselves to the coupled states only the series
+ * length per chunk of their kernels is tuned, and the whole system's default
+ * shape is returned.  Results are cached per system shape (dimension, ELL size,
+ * value streams, coupled states, precision, spectral scale) for the life of
+ * the process.  best (may be NULL) receives the chosen options; spx_stats
+ * reports what a run used.
  */
 spx_status spx_autotune(spx_handle *handle, int64_t n_orient, const double *d_alphas, const double *d_betas,
                         const double *d_gammas, double dt, int64_t nsteps, int32_t precision,

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -135,6 +136,13 @@ struct BlockBufs {
     DevBuf<int> lev, kcut;           // lev: steps per chunk | table rows | series lengths
 };
 
+// What the autotuner chose for a system: `shape` is what spx_autotune returns.
+struct TunedShape {
+    spx_options shape{};             // whole-system launch shape (threads, cluster, chunk_target)
+    bool coupled = false;            // the coupled states run: shape is the whole system's default
+    double blk_target = 0.0;         // and this their series argument of a chunk (0: the default)
+};
+
 // A pulse superoperator as CSR rows in the sliced order, with its 1-norm.
 struct PulseOp {
     DevBuf<int> ptr, col;
@@ -232,9 +240,9 @@ struct spx_handle {
     bool stats_timed = true;        // kernel events recorded (not inside a captured graph)
     int64_t last_norient = 0;
 
-    // autotuned launch shape per precision (threads, cluster, chunk_target)
+    // the autotuner's choice per precision
     bool has_tuned[2] = {false, false};
-    spx_options tuned[2] = {};
+    TunedShape tuned[2];
 };
 
 namespace {
@@ -852,11 +860,16 @@ void set_initial_states(spx_handle *h, int64_t n_states, const double *states) {
 // ---------------------------------------------------------------------------
 constexpr int kPowderGroup = 64;    // orientations per partial sum of the powder reduction
 
-// spx_options.flags bit of a launch shape that the engine chose itself (the
-// autotuner's): such a run may still take the coupled-state kernels, one whose
-// caller set a shape (or a chunk length beside the tuner's) runs the whole
-// system in that shape.  Never a caller's (given_options).
-constexpr int32_t kOwnShape = 1 << 30;
+// The options of a run: the caller's, and what the autotuner adds.  A run whose
+// caller set a shape, or a chunk length beside the tuner's, takes the whole
+// system in that shape; one in a shape of the engine's own may still take the
+// coupled-state kernels.
+struct RunOptions : spx_options {
+    bool own = false;                // threads, cluster and chunk_target are the tuner's
+    double blk_target = 0.0;         // TunedShape::blk_target
+    RunOptions() : spx_options{} {}
+    RunOptions(const spx_options &o) : spx_options(o) {}
+};
 
 struct Config {
     int threads, rmax, M, Kmax, grid;
@@ -1081,8 +1094,8 @@ void choose_dense(const spx_handle *h, const BlockPlan &plan, int64_t n_orient, 
     c.dense_one = one;
 }
 
-bool forced_shape(const spx_options &o) {
-    return o.chunk_steps > 0 || ((o.threads > 0 || o.cluster > 0 || o.chunk_target > 0) && !(o.flags & kOwnShape));
+bool forced_shape(const RunOptions &o) {
+    return o.chunk_steps > 0 || ((o.threads > 0 || o.cluster > 0 || o.chunk_target > 0) && !o.own);
 }
 
 // The caller's options (null: the defaults).
@@ -1091,7 +1104,6 @@ spx_options given_options(const spx_options *opt) {
     if (opt) o = *opt;
     if (o.precision != SPX_FP32 && o.precision != SPX_FP64)
         throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
-    o.flags &= ~kOwnShape;
     return o;
 }
 
@@ -1106,7 +1118,7 @@ bool may_diverge(const spx_handle *h, double dt, int64_t nsteps) {
 // Whether a powder run takes the coupled-state kernels.  c holds the whole
 // system's launch shape (so what is refused does not depend on them).
 void choose_block(spx_handle *h, const BlockPlan *plan, int64_t n_orient, double dt, int64_t nsteps,
-                  const spx_options &opt, int kmax_override, int m_cap, Config &c) {
+                  const RunOptions &opt, int kmax_override, int m_cap, Config &c) {
     const bool f64 = opt.precision == SPX_FP64;
     if (!plan || !plan->ok || forced_shape(opt) || may_diverge(h, dt, nsteps)) return;
     // FP32 runs of more than 8192 undamped steps keep the whole system: there
@@ -1114,7 +1126,7 @@ void choose_block(spx_handle *h, const BlockPlan *plan, int64_t n_orient, double
     // in FP64, so the decision stays the one it has been (a three-spin system,
     // 16384 steps: 1.2e-5 on the whole system, 3.5e-6 on its coupled states)
     if (!f64 && h->max_im_diag == 0.0 && nsteps > 8192) return;
-    if (configure_block(h, *plan, n_orient, dt, nsteps, f64, opt.chunk_target, kmax_override, m_cap, false, c) &&
+    if (configure_block(h, *plan, n_orient, dt, nsteps, f64, opt.blk_target, kmax_override, m_cap, false, c) &&
         kmax_override == 0 && m_cap == 256)
         choose_dense(h, *plan, n_orient, dt, nsteps, f64, c);
 }
@@ -1122,7 +1134,7 @@ void choose_block(spx_handle *h, const BlockPlan *plan, int64_t n_orient, double
 // traj: the run writes the state at every step (chunks of opt.chunk_steps
 // steps, their intermediate states accumulated in shared memory).  plan: the
 // run's coupled states, if it may be restricted to them.
-Config choose_config(spx_handle *h, int64_t n_orient, double dt, int64_t nsteps, const spx_options &opt,
+Config choose_config(spx_handle *h, int64_t n_orient, double dt, int64_t nsteps, const RunOptions &opt,
                      int kmax_override, int m_cap = 256, bool traj = false, const BlockPlan *plan = nullptr) {
     Config c{};
     c.traj = traj;
@@ -1522,7 +1534,7 @@ struct RunIO {
     bool adjoint = false;              // propagate under -H + 1i R (the adjoint of L, negated)
 };
 
-spx_options apply_tuned(const spx_handle *h, spx_options o);
+RunOptions apply_tuned(const spx_handle *h, const spx_options &given);
 
 constexpr int kCheckOrients = SPX_FP32_CHECKED_ORIENTATIONS;   // orientations of an FP32 run re-run in FP64
 
@@ -1533,12 +1545,12 @@ int check_index(int j, int S, int64_t n_orient) { return (int)(((2 * (int64_t)j 
 // (forked from the handle's stream) and return its CTA count, so that the
 // FP32 launch can leave those SMs to it.
 int launch_fp32_check(spx_handle *h, int64_t n_orient, const double *d_al, const double *d_be, const double *d_ga,
-                      double dt, int64_t nsteps, const spx_options &opt, const spx::DevSystem &sys32) {
+                      double dt, int64_t nsteps, const RunOptions &opt, const spx::DevSystem &sys32) {
     const int S = (int)std::min<int64_t>(kCheckOrients, n_orient);
-    spx_options o64{};
-    o64.precision = SPX_FP64;
-    o64.lanczos_its = opt.lanczos_its;
-    o64 = apply_tuned(h, o64);
+    spx_options given{};
+    given.precision = SPX_FP64;
+    given.lanczos_its = opt.lanczos_its;
+    const RunOptions o64 = apply_tuned(h, given);
     const Config c = choose_config(h, S, dt, nsteps, o64, 0, 256, false, &h->plan);
     const size_t npts = ((size_t)nsteps + 1) * h->nchan;
     if (!h->check_stream) {
@@ -1619,7 +1631,7 @@ int launch_fp32_check(spx_handle *h, int64_t n_orient, const double *d_al, const
 
 void launch_powder(spx_handle *h, int64_t n_orient, const double *d_al, const double *d_be,
                    const double *d_ga, const double *d_w, double dt, int64_t nsteps,
-                   const spx_options &opt, double2 *d_out, const Config &c_in, int safe_bounds = 0, bool timed = true,
+                   const RunOptions &opt, double2 *d_out, const Config &c_in, int safe_bounds = 0, bool timed = true,
                    const RunIO &io = RunIO{}, bool fp32_check = false) {
     const bool f64 = opt.precision == SPX_FP64;
     Config c = c_in;
@@ -2271,7 +2283,7 @@ void check_statuses(spx_handle *h, int64_t n_orient, int64_t launches) {
 // then runs the whole system).  Arguments are validated and the grid is on the
 // device; total: recorded points.
 bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<const spx_csc *> &pulse_ops,
-                          const std::vector<spx_seq_op> &ops, const spx_options &o, int64_t total, double *fid,
+                          const std::vector<spx_seq_op> &ops, const RunOptions &o, int64_t total, double *fid,
                           double *fids_per_orient) {
     if (forced_shape(o)) return false;
     for (auto &q : ops)
@@ -2466,7 +2478,7 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
 
 void run_sequence(spx_handle *h, int64_t n_orient, const double *alphas, const double *betas, const double *gammas,
                   const double *weights, int32_t n_pulse, const spx_csc *pulse_ops, int32_t n_ops,
-                  const spx_seq_op *ops, const spx_options &o, double *fid, double *fids_per_orient = nullptr) {
+                  const spx_seq_op *ops, const RunOptions &o, double *fid, double *fids_per_orient = nullptr) {
     if (h->nchan != 1) throw SpxError(SPX_ERR_UNSUPPORTED, "pulse sequences take one coil");
     if (h->n_states > 0 && h->n_states != n_orient)
         throw SpxError(SPX_ERR_INVALID_ARGUMENT, "the grid size differs from the number of per-orientation initial states");
@@ -2563,7 +2575,7 @@ void run_sequence(spx_handle *h, int64_t n_orient, const double *alphas, const d
 // (npoints + 2*npoints*nloops points).
 void run_cpmg(spx_handle *h, int64_t n_orient, const double *alphas, const double *betas, const double *gammas,
               const double *weights, double dt, int64_t npoints, int32_t nloops, const spx_csc *pulse_op,
-              const spx_options &o, double *fid, double *fids_per_orient) {
+              const RunOptions &o, double *fid, double *fids_per_orient) {
     // experiments/cpmg.m:77-90: both positive integers
     if (npoints < 1 || nloops < 1) throw SpxError(SPX_ERR_INVALID_ARGUMENT, "npoints and nloops must be positive");
     std::vector<spx_seq_op> prog;
@@ -2720,7 +2732,7 @@ void negate_generator(spx_handle *h) {
 // conj(v[o][k]) * Pi * u[o][j] with k = j, or k = nsteps - j when reverse;
 // d_fid = their weighted sum in orientation order.
 void echo_trajectories(spx_handle *h, int64_t n_orient, const double *g, double tau, int64_t nsteps,
-                       const spx_options &o, const double2 *adj0, bool reverse) {
+                       const RunOptions &o, const double2 *adj0, bool reverse) {
     const int n_pad = h->n_pad;
     const int64_t npoints = nsteps + 1;
     // the states at every step come from chunks of a few steps (their
@@ -2728,7 +2740,7 @@ void echo_trajectories(spx_handle *h, int64_t n_orient, const double *g, double 
     // most of their series on the truncation tail); orientations in batches
     // whose two trajectories take a quarter of the free device memory (at
     // most 48 GB): few batches, so few partly filled waves
-    spx_options o1 = o;
+    RunOptions o1 = o;
     size_t free_b = 0, total_b = 0;
     SPX_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t budget = std::min<size_t>(free_b / 4, 48ull << 30);
@@ -2848,7 +2860,7 @@ std::vector<double2> apply_host(const HostCsr &m, const std::vector<double2> &x)
 // that the echo pulse connects to them.  out_back: DEER's first adjoint run.
 // False if the states do not qualify.
 bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const spx_csc *> &ops, double first_angle,
-                      const double *back_angle, int echo_op, double tau, int64_t nsteps, const spx_options &o,
+                      const double *back_angle, int echo_op, double tau, int64_t nsteps, const RunOptions &o,
                       bool reverse) {
     if (forced_shape(o) || may_diverge(h, tau, nsteps)) return false;
     CoupledSequence seq(h, ops);
@@ -2971,7 +2983,7 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
         const int64_t nb = std::min(batch, n_orient - b0);
         bool have = false;
         for (int m : {kTrajChunk, 2, 1}) {          // the whole system's configuration: its refusals stand
-            spx_options o1 = o;
+            RunOptions o1 = o;
             o1.chunk_steps = m;
             try {
                 whole = choose_config(h, nb, tau, nsteps, o1, 0, 256, true);
@@ -3035,7 +3047,7 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
 // first_angle: pi/2 for eseem.m, pi/4 for oopeseem.m (the out-of-phase echo).
 void run_eseem(spx_handle *h, int64_t n_orient, const double *alphas, const double *betas, const double *gammas,
                const double *weights, double timestep, int64_t npoints, const spx_csc *pulse_op,
-               double first_angle, const spx_options &o, double *fid, double *fids_per_orient) {
+               double first_angle, const RunOptions &o, double *fid, double *fids_per_orient) {
     if (h->nchan != 1 || h->n_states != 0)
         throw SpxError(SPX_ERR_UNSUPPORTED, "pulse sequences take one coil and one initial state");
     if (npoints < 1) throw SpxError(SPX_ERR_INVALID_ARGUMENT, "npoints must be positive");
@@ -3073,7 +3085,7 @@ void run_eseem(spx_handle *h, int64_t n_orient, const double *alphas, const doub
 // w read backwards against the forward trajectory from rho1.
 void run_deer(spx_handle *h, int64_t n_orient, const double *alphas, const double *betas, const double *gammas,
               const double *weights, double stepsize, int64_t nsteps, const spx_csc *ex_prob,
-              const spx_csc *ex_pump, const spx_options &o, double *fid, double *fids_per_orient) {
+              const spx_csc *ex_pump, const RunOptions &o, double *fid, double *fids_per_orient) {
     if (h->nchan != 1 || h->n_states != 0)
         throw SpxError(SPX_ERR_UNSUPPORTED, "pulse sequences take one coil and one initial state");
     if (nsteps < 1) throw SpxError(SPX_ERR_INVALID_ARGUMENT, "nsteps must be a positive integer");
@@ -3130,33 +3142,65 @@ void run_deer(spx_handle *h, int64_t n_orient, const double *alphas, const doubl
 // ---------------------------------------------------------------------------
 // Autotuner
 // ---------------------------------------------------------------------------
-// Options left at zero take the handle's tuned launch shape for that precision.
-spx_options apply_tuned(const spx_handle *h, spx_options o) {
-    const int p = o.precision == SPX_FP64 ? 1 : 0;
-    if (h->has_tuned[p] && o.threads == 0 && o.cluster == 0 && o.chunk_target == 0.0) {
-        o.threads = h->tuned[p].threads;
-        o.cluster = h->tuned[p].cluster;
-        o.chunk_target = h->tuned[p].chunk_target;
-        o.flags |= kOwnShape;
-    }
-    return o;
-}
-
-// shape of a tuning problem: systems with the same key get the same answer
-using TuneKey = std::tuple<int, int, int, int, int, int, int, int, int, int>;
+// shape of a tuning problem: systems with the same key get the same answer.
+// First what describes the system and its coupled states, then the run.
+using SystemKey = std::tuple<int, int, int, int, int, int, int, int>;
+using TuneKey = std::pair<SystemKey, std::tuple<int, int, int>>;
 std::mutex g_tune_mutex;
-std::map<TuneKey, spx_options> g_tune_cache;
+std::map<TuneKey, TunedShape> g_tune_cache;
 
-TuneKey tune_key(const spx_handle *h, double dt, int64_t nsteps, int precision) {
+SystemKey system_key(const spx_handle *h, int precision) {
+    return SystemKey{h->n, h->ell_len, h->nslices, h->nstreams, h->cplx ? 1 : 0, precision,
+                     h->plan.ok ? h->plan.n : 0, h->nchan};
+}
+// kernels: 0 the whole system's, 1 the coupled states', 2 the dense matrices.
+TuneKey tune_key(const spx_handle *h, double dt, int64_t nsteps, int precision, int kernels) {
     // spectral scale in octaves: the series length per step follows it
     const int scale = (int)std::lround(std::log2(std::max(h->g_upper * dt, 1e-30)));
-    return TuneKey{h->n, h->ell_len, h->nslices, h->nstreams, h->cplx ? 1 : 0, precision, scale,
-                   (int)std::min<int64_t>(nsteps, 512), h->plan.ok ? h->plan.n : 0, h->nchan};
+    return TuneKey{system_key(h, precision), {scale, (int)std::min<int64_t>(nsteps, 512), kernels}};
+}
+
+bool same_shape(const spx_options &a, const spx_options &b) {
+    return a.threads == b.threads && a.cluster == b.cluster && a.chunk_target == b.chunk_target;
+}
+
+// The tuner's choice that options ask for: the handle's where they leave the
+// shape at zero, else one that spx_autotune returned, for this handle or another
+// one with such a system; null for neither.
+const TunedShape *tuned_shape(const spx_handle *h, const spx_options &o) {
+    const int p = o.precision == SPX_FP64 ? 1 : 0;
+    const bool left = o.threads == 0 && o.cluster == 0 && o.chunk_target == 0.0;
+    if (h->has_tuned[p] && (left || same_shape(o, h->tuned[p].shape))) return &h->tuned[p];
+    if (left || o.threads == 0 || o.cluster == 0) return nullptr;
+    const SystemKey key = system_key(h, o.precision);
+    std::lock_guard<std::mutex> lk(g_tune_mutex);              // entries are never erased
+    for (auto it = g_tune_cache.lower_bound(TuneKey{key, {INT_MIN, INT_MIN, INT_MIN}});
+         it != g_tune_cache.end() && it->first.first == key; ++it)
+        if (same_shape(o, it->second.shape)) return &it->second;
+    return nullptr;
+}
+
+// The run's options with the tuner's choice in them.
+RunOptions apply_tuned(const spx_handle *h, const spx_options &given) {
+    RunOptions o(given);
+    const TunedShape *t = tuned_shape(h, given);
+    if (!t || (t->coupled && o.chunk_steps > 0)) return o;
+    if (t->coupled) {
+        o.threads = o.cluster = 0;             // the whole system's default, should it run after all
+        o.chunk_target = 0.0;
+        o.blk_target = t->blk_target;
+    } else {
+        o.threads = t->shape.threads;
+        o.cluster = t->shape.cluster;
+        o.chunk_target = t->shape.chunk_target;
+    }
+    o.own = true;
+    return o;
 }
 
 // Kernel time of one candidate over the sample, or +inf if it cannot run.
 double time_candidate(spx_handle *h, int64_t n, const double *d_al, const double *d_be, const double *d_ga,
-                      const double *d_w, double dt, int64_t nsteps, spx_options o, double2 *d_out) {
+                      const double *d_w, double dt, int64_t nsteps, const RunOptions &o, double2 *d_out) {
     double best = INFINITY;
     try {
         const Config c = choose_config(h, n, dt, nsteps, o, 0, 256, false, &h->plan);
@@ -3173,29 +3217,28 @@ double time_candidate(spx_handle *h, int64_t n, const double *d_al, const double
     return best;
 }
 
-spx_options autotune(spx_handle *h, int64_t n_orient, const double *d_al, const double *d_be, const double *d_ga,
-                     double dt, int64_t nsteps, int precision) {
-    const TuneKey key = tune_key(h, dt, nsteps, precision);
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mutex);
-        auto it = g_tune_cache.find(key);
-        if (it != g_tune_cache.end()) return it->second;
-    }
-    spx_options base{};
+TunedShape autotune(spx_handle *h, int64_t n_orient, const double *d_al, const double *d_be, const double *d_ga,
+                    double dt, int64_t nsteps, int precision) {
+    RunOptions base;
     base.precision = precision;
     // sample: one wave of single-CTA orientations (at most 1024), at most 512
     // steps (several chunks, so long chunks are not penalised; a 256-step
     // sample picked shorter chunks and made the c2 graph 2 % slower)
     const int64_t ns = std::min<int64_t>(nsteps, 512);
     int64_t n = std::min<int64_t>(n_orient, 1024);
+    Config c0{};                     // the default; a refused one leaves the shapes below to try
+    try {
+        c0 = choose_config(h, n, dt, ns, base, 0, 256, false, &h->plan);
+        if (!c0.blk) n = std::min<int64_t>(n, c0.grid);
+    } catch (const SpxError &) {
+        c0 = Config{};
+        n = std::min<int64_t>(n, h->sm_count);
+    }
+    const TuneKey key = tune_key(h, dt, nsteps, precision, c0.dense ? 2 : c0.blk ? 1 : 0);
     {
-        spx_options o1 = base;
-        try {
-            const Config c1 = choose_config(h, n, dt, ns, o1, 0, 256, false, &h->plan);
-            if (!c1.blk) n = std::min<int64_t>(n, c1.grid);
-        } catch (const SpxError &) {
-            n = std::min<int64_t>(n, h->sm_count);
-        }
+        std::lock_guard<std::mutex> lk(g_tune_mutex);
+        auto it = g_tune_cache.find(key);
+        if (it != g_tune_cache.end()) return it->second;
     }
     DevBuf<double> w;
     w.reserve((size_t)n);
@@ -3203,60 +3246,65 @@ spx_options autotune(spx_handle *h, int64_t n_orient, const double *d_al, const 
     SPX_CUDA(cudaMemcpyAsync(w.p, hw.data(), n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     DevBuf<double2> out;
     out.reserve(((size_t)ns + 1) * h->nchan);
-    spx_options best = base;
-    double best_t = INFINITY;
-    const int cls[] = {1, 2, 4, 8};
-    int cl_min = 0;                 // smallest cluster that fits; it and twice it are tried
-    {
-        // a run over the coupled states has its own layouts: only the series
-        // length per chunk is tuned, beside the whole system's default shape
-        const Config c0 = choose_config(h, n, dt, ns, base, 0, 256, false, &h->plan);
-        if (c0.blk) {
-            best.threads = c0.threads;
-            best.cluster = c0.cl;
-            best.flags = kOwnShape;
-            best.chunk_target = c0.blk_x;
-            best_t = time_candidate(h, n, d_al, d_be, d_ga, w.p, dt, ns, best, out.p);
-            cl_min = -1;
-        }
-    }
-    for (int cl : cls) {
-        if (cl_min < 0) break;
-        if (cl_min && cl > 2 * cl_min) break;
-        // warps: the default for this cluster size, half, and 16
-        spx_options o = base;
-        o.cluster = cl;
-        Config c0{};
-        try {
-            c0 = choose_config(h, n, dt, ns, o, 0);
-        } catch (const SpxError &) {
-            continue;
-        }
-        if (!cl_min) cl_min = cl;
-        const int nw0 = c0.threads / 32;
-        std::vector<int> nws = {nw0, std::max(1, nw0 / 2), 16};
-        std::sort(nws.begin(), nws.end());
-        nws.erase(std::unique(nws.begin(), nws.end()), nws.end());
-        for (int nw : nws) {
-            o.threads = nw * 32;
-            const double t = time_candidate(h, n, d_al, d_be, d_ga, w.p, dt, ns, o, out.p);
-            if (t < best_t) { best_t = t; best = o; }
-        }
-    }
-    if (!std::isfinite(best_t)) throw SpxError(SPX_ERR_UNSUPPORTED, "no launch shape could run this system");
-    // series length per chunk for the best shape
+    auto time = [&](const RunOptions &o) { return time_candidate(h, n, d_al, d_be, d_ga, w.p, dt, ns, o, out.p); };
+    // series length per chunk
     const double targets[] = {450.0, 300.0, 150.0, 60.0};
-    spx_options bc = best;
-    for (double tx : targets) {
-        spx_options o = best;
-        o.chunk_target = tx;
-        const double t = time_candidate(h, n, d_al, d_be, d_ga, w.p, dt, ns, o, out.p);
-        if (t < best_t) { best_t = t; bc = o; }
+    TunedShape best;
+    best.shape = base;
+    double best_t = INFINITY;
+    if (c0.blk) {
+        // a run over the coupled states has its own layouts: only the series length
+        // per chunk is tuned (the dense matrices have none); the whole system keeps
+        // its default shape, which is the one returned
+        best.coupled = true;
+        best.shape.threads = c0.threads;
+        best.shape.cluster = c0.cl;
+        best.shape.chunk_target = c0.chunk_x;
+        if (!c0.dense) {
+            for (double tx : targets) {
+                RunOptions o = base;
+                o.blk_target = tx;
+                const double t = time(o);
+                if (t < best_t) { best_t = t; best.blk_target = tx; }
+            }
+            if (!std::isfinite(best_t)) throw SpxError(SPX_ERR_UNSUPPORTED, "no launch shape could run this system");
+        }
+    } else {
+        const int cls[] = {1, 2, 4, 8};
+        int cl_min = 0;              // smallest cluster that fits; it and twice it are tried
+        for (int cl : cls) {
+            if (cl_min && cl > 2 * cl_min) break;
+            // warps: the default for this cluster size, half, and 16
+            RunOptions o = base;
+            o.cluster = cl;
+            Config c{};
+            try {
+                c = choose_config(h, n, dt, ns, o, 0);
+            } catch (const SpxError &) {
+                continue;
+            }
+            if (!cl_min) cl_min = cl;
+            const int nw0 = c.threads / 32;
+            std::vector<int> nws = {nw0, std::max(1, nw0 / 2), 16};
+            std::sort(nws.begin(), nws.end());
+            nws.erase(std::unique(nws.begin(), nws.end()), nws.end());
+            for (int nw : nws) {
+                o.threads = nw * 32;
+                const double t = time(o);
+                if (t < best_t) { best_t = t; best.shape = o; }
+            }
+        }
+        if (!std::isfinite(best_t)) throw SpxError(SPX_ERR_UNSUPPORTED, "no launch shape could run this system");
+        const RunOptions shape = best.shape;
+        for (double tx : targets) {
+            RunOptions o = shape;
+            o.chunk_target = tx;
+            const double t = time(o);
+            if (t < best_t) { best_t = t; best.shape = o; }
+        }
     }
-    best = bc;
-    best.flags = 0;
     std::lock_guard<std::mutex> lk(g_tune_mutex);
-    g_tune_cache[key] = best;
+    g_tune_cache.emplace(key, best);
     return best;
 }
 
@@ -3509,8 +3557,7 @@ spx_status spx_run_powder(spx_handle *h, int64_t n_orient, const double *alphas,
             if (!std::isfinite(alphas[o]) || !std::isfinite(betas[o]) || !std::isfinite(gammas[o]) ||
                 !std::isfinite(weights[o]))
                 throw SpxError(SPX_ERR_INVALID_ARGUMENT, "non-finite grid entry");
-        spx_options o = given_options(opt);
-        o = apply_tuned(h, o);
+        RunOptions o = apply_tuned(h, given_options(opt));
         SPX_CUDA(cudaSetDevice(h->device));
         h->d_grid.reserve(4 * (size_t)n_orient);
         double *g = h->d_grid.p;
@@ -3564,12 +3611,11 @@ spx_status spx_run_powder(spx_handle *h, int64_t n_orient, const double *alphas,
             // the FP32 result misses the bar on the checked orientations: run
             // the whole grid again in FP64 and return that
             const spx_stats s32 = h->stats;
-            spx_options o64 = o;
-            o64.precision = SPX_FP64;
-            o64.threads = o64.cluster = 0;
-            o64.chunk_target = 0.0;
-            o64.flags &= ~kOwnShape;
-            o64 = apply_tuned(h, o64);
+            spx_options given64 = o;
+            given64.precision = SPX_FP64;
+            given64.threads = given64.cluster = 0;
+            given64.chunk_target = 0.0;
+            const RunOptions o64 = apply_tuned(h, given64);
             const Config c64 = choose_config(h, n_orient, dt, nsteps, o64, 0, 256, false, &h->plan);
             launch_powder(h, n_orient, g, g + n_orient, g + 2 * n_orient, g + 3 * n_orient, dt, nsteps, o64,
                           h->d_fid.p, c64);
@@ -3608,8 +3654,7 @@ spx_status spx_run_powder_device(spx_handle *h, int64_t n_orient, const double *
         validate_run(h, n_orient, dt, nsteps);
         if (!d_alphas || !d_betas || !d_gammas || !d_weights || !d_fid)
             throw SpxError(SPX_ERR_INVALID_ARGUMENT, "NULL device pointer");
-        spx_options o = given_options(opt);
-        o = apply_tuned(h, o);
+        RunOptions o = apply_tuned(h, given_options(opt));
         SPX_CUDA(cudaSetDevice(h->device));
         const Config c = choose_config(h, n_orient, dt, nsteps, o, 0, 256, false, &h->plan);
         const bool check = o.precision == SPX_FP32 && !(o.flags & SPX_FLAG_NO_FP32_CHECK);
@@ -3669,8 +3714,7 @@ spx_status spx_run_cpmg(spx_handle *h, int64_t n_orient, const double *alphas, c
             if (!std::isfinite(alphas[o]) || !std::isfinite(betas[o]) || !std::isfinite(gammas[o]) ||
                 !std::isfinite(weights[o]))
                 throw SpxError(SPX_ERR_INVALID_ARGUMENT, "non-finite grid entry");
-        spx_options o = given_options(opt);
-        o = apply_tuned(h, o);
+        RunOptions o = apply_tuned(h, given_options(opt));
         SPX_CUDA(cudaSetDevice(h->device));
         run_cpmg(h, n_orient, alphas, betas, gammas, weights, dt, npoints, nloops, pulse_op, o, fid, fids_per_orient);
     });
@@ -3687,8 +3731,7 @@ spx_status spx_run_sequence(spx_handle *h, int64_t n_orient, const double *alpha
             if (!std::isfinite(alphas[o]) || !std::isfinite(betas[o]) || !std::isfinite(gammas[o]) ||
                 !std::isfinite(weights[o]))
                 throw SpxError(SPX_ERR_INVALID_ARGUMENT, "non-finite grid entry");
-        spx_options o = given_options(opt);
-        o = apply_tuned(h, o);
+        RunOptions o = apply_tuned(h, given_options(opt));
         SPX_CUDA(cudaSetDevice(h->device));
         run_sequence(h, n_orient, alphas, betas, gammas, weights, n_pulse, pulse_ops, n_ops, ops, o, fid,
                      fids_per_orient);
@@ -3842,11 +3885,11 @@ spx_status spx_autotune(spx_handle *h, int64_t n_orient, const double *d_alphas,
         if (precision != SPX_FP32 && precision != SPX_FP64) throw SpxError(SPX_ERR_INVALID_ARGUMENT, "unknown precision");
         SPX_CUDA(cudaSetDevice(h->device));
         finish_run(h);
-        const spx_options o = autotune(h, n_orient, d_alphas, d_betas, d_gammas, dt, nsteps, precision);
+        const TunedShape t = autotune(h, n_orient, d_alphas, d_betas, d_gammas, dt, nsteps, precision);
         const int p = precision == SPX_FP64 ? 1 : 0;
-        h->tuned[p] = o;
+        h->tuned[p] = t;
         h->has_tuned[p] = true;
-        if (best) *best = o;
+        if (best) *best = t.shape;
     });
 }
 
@@ -3904,7 +3947,7 @@ void capture_batch(spx_batch *b) {
     const size_t n = b->runs.size();
     // launch shapes and buffers first: nothing may allocate while capturing
     std::vector<Config> cfg(n);
-    std::vector<spx_options> os(n);
+    std::vector<RunOptions> os(n);
     for (size_t i = 0; i < n; ++i) {
         const spx_batch::Run &r = b->runs[i];
         os[i] = apply_tuned(r.h, r.opt);

@@ -352,3 +352,54 @@ def test_chunk_length_and_flags_of_the_caller_on_a_tuned_handle(engine_lib, prec
             assert eng.stats()['coupled_dim'] == 0 and eng.stats()['threads'] == 96
     finally:
         eng.close()
+
+
+def test_autotuned_options_handed_back_keep_the_coupled_states(engine_lib):
+    """What spx_autotune returns may be passed to runs of the handle, or of another
+    one with such a system; a shape changed by the caller is forced."""
+    import torch
+    H, R, rho0, coil = _chain(41, 5, 0.02)
+    ref = WEIGHTS.sum() * _fid(H, R, rho0, coil, 0.3, 700)
+    _, ptr = _device_grid()
+    eng, other = E.Engine(0), E.Engine(0)
+    try:
+        for e in (eng, other):
+            _upload(e, H, R, rho0, coil)
+        for prec, tol in ((E.FP64, 1e-10), (E.FP32, 1e-5)):
+            untuned = eng.run(*ANGLES, WEIGHTS, 0.3, 700, precision=prec).stats
+            best = eng.autotune(*ptr[:3], 3, 0.3, 700, prec)
+            for e in (eng, other):
+                res = e.run(*ANGLES, WEIGHTS, 0.3, 700, precision=prec, **best)
+                assert res.stats['coupled_dim'] == 41 and rel_err(res.fid, ref) <= tol
+                assert res.stats['threads'] == untuned['threads'] and res.stats['cluster'] == untuned['cluster']
+                forced = dict(best, threads=best['threads'] + 32)
+                res = e.run(*ANGLES, WEIGHTS, 0.3, 700, precision=prec, **forced)
+                assert res.stats['coupled_dim'] == 0 and rel_err(res.fid, ref) <= tol
+    finally:
+        eng.close()
+        other.close()
+
+
+def test_autotune_where_the_whole_system_takes_short_chunks(engine_lib):
+    """2370 states beside 30 coupled ones: the whole system's default has a shorter
+    series per chunk than the coupled states', and both have to be tunable."""
+    n, m, dt, nsteps = 2400, 2370, 0.05, 600
+    rng = np.random.default_rng(n)
+    A = sp.diags([rng.normal(size=m)] + [rng.normal(size=m - k) for k in (1, 2, 3, 5, 8, 13, 21, 34)],
+                 [0, 1, 2, 3, 5, 8, 13, 21, 34])
+    A = A + sp.triu(A, 1).T
+    B, R, rho0, coil = _chain(n - m, 7)
+    H = sp.block_diag([A, B], format='csc').astype(complex)
+    z = np.zeros(m)
+    eng = E.Engine(0)
+    try:
+        eng.upload(H, {}, sp.csc_matrix((n, n), dtype=complex), np.concatenate([z, rho0]), np.concatenate([z, coil]))
+        _, ptr = _device_grid()
+        for prec, tol in ((E.FP64, 1e-10), (E.FP32, 1e-5)):
+            best = eng.autotune(*ptr[:3], 3, dt, nsteps, prec)
+            for options in ({}, best):
+                res = eng.run(*ANGLES, WEIGHTS, dt, nsteps, precision=prec, **options)
+                assert res.stats['coupled_dim'] == n - m
+                assert rel_err(res.fid, WEIGHTS.sum() * _fid(B, R, rho0, coil, dt, nsteps)) <= tol
+    finally:
+        eng.close()
