@@ -2005,6 +2005,7 @@ void upload_pulse(spx_handle *h, const spx_csc *P, PulseOp &op) {
 // exp(-1i * theta * P) on n_states states of n_pad entries (sliced order).
 void apply_pulse(spx_handle *h, const PulseOp &op, double theta, int64_t n_states, double2 *states) {
     const double x = op.norm1 * std::fabs(theta);
+    if (!(x < 2147483647.0)) throw SpxError(SPX_ERR_INVALID_ARGUMENT, "pulse operator times angle overflows");
     const int nsub = std::max(1, (int)std::ceil(x));
     const int nterms = 25;                     // 1 / 25! < 1e-25 per substep
     const size_t smem = 3 * (size_t)h->n_pad * sizeof(double2);
@@ -2062,8 +2063,9 @@ constexpr int kPulseBlock = 64;        // largest set of states that a pulse ope
 
 // exp(-1i theta P) of a pulse operator given as rows, one connected set of
 // states at a time (a spin's rotation couples a few): scaling and squaring of
-// the Taylor series, 1/2^s scaled to a 1-norm of at most one half.  Entries at
-// or below 1e-15 are rounding residues of the rotation and are dropped.
+// the Taylor series, 1/2^s scaled to a 1-norm of at most one half.  Of a rotation
+// that was scaled down, entries at or below 1e-15 are rounding residues and are
+// dropped; a smaller rotation's small entries are what it does.
 // False if a set is larger than kPulseBlock.
 bool pulse_exponential(const std::vector<std::vector<std::pair<int, double2>>> &rows, double theta, HostCsr &out) {
     const int n = (int)rows.size();
@@ -2090,8 +2092,9 @@ bool pulse_exponential(const std::vector<std::vector<std::pair<int, double2>>> &
         for (int c = 0; c < m; ++c) {
             double sum = 0.0;
             for (int r = 0; r < m; ++r) sum += std::hypot(A[(size_t)r * m + c].x, A[(size_t)r * m + c].y);
-            norm = std::max(norm, sum);
+            if (!(sum <= norm)) norm = sum;           // NaN too
         }
+        if (!std::isfinite(norm)) throw SpxError(SPX_ERR_INVALID_ARGUMENT, "pulse operator times angle overflows");
         int sq = 0;
         while (norm > 0.5) { norm *= 0.5; ++sq; }
         const double f = std::ldexp(1.0, -sq);
@@ -2118,10 +2121,11 @@ bool pulse_exponential(const std::vector<std::vector<std::pair<int, double2>>> &
             }
         }
         for (int q = 0; q < sq; ++q) { product(X, X, Y); X.swap(Y); }
+        const double residue = sq > 0 ? 1e-15 : 0.0;
         for (int r = 0; r < m; ++r)
             for (int c = 0; c < m; ++c) {
                 const double2 v = X[(size_t)r * m + c];
-                if (std::fabs(v.x) > 1e-15 || std::fabs(v.y) > 1e-15) res[set[r]].push_back({set[c], v});
+                if (std::fabs(v.x) > residue || std::fabs(v.y) > residue) res[set[r]].push_back({set[c], v});
             }
     }
     out = HostCsr{};

@@ -403,3 +403,22 @@ def test_autotune_where_the_whole_system_takes_short_chunks(engine_lib):
                 assert rel_err(res.fid, WEIGHTS.sum() * _fid(B, R, rho0, coil, dt, nsteps)) <= tol
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize('n', [4, 70])                     # 70: the pulse connects more states than the coupled path takes
+def test_pulses_of_extreme_angles(gpu_engine, n):
+    """A tiny rotation moves its tiny part of the state (relative to it, FP64's
+    digits), and an angle that overflows the operator is an error."""
+    H, R, _, _ = _chain(n, 8)
+    P = _shift_operator(n)
+    rho0, coil = np.zeros(n, complex), np.zeros(n, complex)
+    rho0[0], coil[1] = 1.0, 1.0
+    H[0, 1] = H[1, 0] = 0.0                                 # detected states are reached by the pulse alone
+    _upload(gpu_engine, H, R, rho0, coil)
+    for angle in (1e-3, 1e-16, 1e-200):
+        res = gpu_engine.run_sequence(*ANGLES, WEIGHTS, [P], [('pulse', 0, angle), ('evolve', 20, 0.1)], precision=E.FP64)
+        v = -1j * np.eye(n)[1] * angle if angle < 1e-10 else sl.expm(-1j * angle * P.toarray()) @ rho0
+        assert rel_err(res.fid / angle, _fid(H, R, v / angle, coil, 0.1, 20)) <= 1e-10
+    for op, angle in ((1e10 * P, 1e300), (1e308 * P, 1.0)):
+        with pytest.raises(E.SpxError, match='overflows'):
+            gpu_engine.run_sequence(*ANGLES, WEIGHTS, [op], [('pulse', 0, angle), ('evolve', 2, 0.1)], precision=E.FP64)
