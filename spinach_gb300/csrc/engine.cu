@@ -883,11 +883,11 @@ struct Config {
     int traj_m = 1;                               // trajectory outputs: chunk length (1: none)
     bool traj = false;                            // the kernels with trajectory outputs
     // the coupled-state kernels (block.cuh), if they run: their layout and that
-    // of the spectral bounds (FP32 lanes in both precisions), chunk target, chunk cap, series cap, ladder steps and shared memory
+    // of the spectral bounds (an FP32 layout in both precisions), chunk target, chunk cap, series cap, ladder steps and shared memory
     const BlockPlan::Layout *blk = nullptr, *blk_bounds = nullptr;
     double blk_x = 0.0;
     int blk_M = 0, blk_K = 0, blk_lev = 0;
-    int blk_which = 0;                            // the propagation kernel (spx_block_kernel_*)
+    int blk_which = 0, blk_bounds_which = 0;      // the propagation and bounds kernels (spx_block_kernel_*)
     // by dense matrices (dense.cuh): states and detection rows kept,
     // squarings of the scaled exponential
     const BlockPlan *dense = nullptr;
@@ -944,8 +944,8 @@ const void *spx_kernel_f32r_dc_t(int rmax, bool cluster, bool wide);
 const void *spx_kernel_f32c_dc_t(int rmax, bool cluster, bool wide);
 const void *spx_kernel_f64r_dc_t(int rmax, bool cluster, bool wide);
 const void *spx_kernel_f64c_dc_t(int rmax, bool cluster, bool wide);
-// Kernels of block.cuh (kern_block_<value type>.cu): which 0 the spectral
-// bounds, 1 the FP32 and 2 the FP64 propagation.
+// Kernels of block.cuh (kern_block_<value type>.cu): which 0 the FP32 and 5 the
+// FP64 spectral bounds, 1 the FP32 and 2 the FP64 propagation.
 const void *spx_block_kernel_r(int ecap, int which);
 const void *spx_block_kernel_c(int ecap, int which);
 namespace {
@@ -1048,6 +1048,7 @@ bool configure_block(spx_handle *h, const BlockPlan &plan, int64_t n_orient, dou
     c.blk_even = part > own ? std::max(c.blk_smem, part - own) : c.blk_smem;
     c.blk = best;
     c.blk_bounds = f64 ? best_layout(plan.layouts[0], per_sm) : best;
+    c.blk_bounds_which = f64 ? 5 : 0;
     return true;
 }
 
@@ -1295,7 +1296,7 @@ void launch_bounds(spx_handle *h, const Config &c, spx::DevSystem &sys, spx::Blo
     spx::BlockLayout lay = c.blk_bounds->dev;
     SPX_CUDA(cudaMemsetAsync(r.extent, 0, 2 * sizeof(unsigned long long), stream));
     void *args[] = {&sys, &lay, &r};
-    SPX_CUDA(cudaLaunchKernel(block_kernel(h->cplx, c.blk_bounds->ecap, 0), dim3((unsigned)r.n_orient),
+    SPX_CUDA(cudaLaunchKernel(block_kernel(h->cplx, c.blk_bounds->ecap, c.blk_bounds_which), dim3((unsigned)r.n_orient),
                               dim3((unsigned)lay.threads), args, 0, stream));
     ++h->launches;
 }
@@ -3984,7 +3985,7 @@ void capture_batch(spx_batch *b) {
                 continue;
             }
             if (cfg[i].blk) {
-                SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(h->cplx, cfg[i].blk_bounds->ecap, 0)));
+                SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(h->cplx, cfg[i].blk_bounds->ecap, cfg[i].blk_bounds_which)));
                 SPX_CUDA(cudaFuncGetAttributes(&fa, block_kernel(h->cplx, cfg[i].blk->ecap, cfg[i].blk_which)));
                 continue;
             }

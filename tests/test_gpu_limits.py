@@ -422,3 +422,29 @@ def test_pulses_of_extreme_angles(gpu_engine, n):
     for op, angle in ((1e10 * P, 1e300), (1e308 * P, 1.0)):
         with pytest.raises(E.SpxError, match='overflows'):
             gpu_engine.run_sequence(*ANGLES, WEIGHTS, [op], [('pulse', 0, angle), ('evolve', 2, 0.1)], precision=E.FP64)
+
+
+def test_fp64_runs_take_their_bounds_in_fp64(gpu_engine):
+    """The Gershgorin interval of the retry after a violated bound, and the Lanczos
+    interval, of a spectrum whose centre is 500 times its width: FP32 sums would
+    widen the discs by a part in 1e6 of the centre."""
+    shift, dt, nsteps = 1.05e4, 0.38, 8300                  # more steps than the dense matrices take
+    H, R, rho0, coil = _outlier()
+    H = H + shift * np.eye(len(H))
+    _upload(gpu_engine, H, R, rho0, coil)
+    d = np.diag(H)
+    rad = np.abs(H).sum(1) - np.abs(d)
+    safe = 0.505 * ((d + rad).max() - (d - rad).min()) + 1e-9 * d.max()
+    e, V = np.linalg.eigh(H - shift * np.eye(len(H)))
+    a = (coil.conj() @ V) * (V.T @ rho0)
+    at = np.array([0, 1, 255, 256, nsteps])
+    ref = np.array([np.sum(a * np.exp(-1j * e * dt * k)) * np.exp(-1j * shift * dt * k) for k in at])
+    for its, retries in ((2, 1), (0, 0)):
+        res = gpu_engine.run(*ANGLES, WEIGHTS, dt, nsteps, precision=E.FP64, lanczos_its=its)
+        assert res.stats['coupled_dim'] == len(H) and res.stats['retries'] == retries
+        # phases of 3e7: 4e-9 of them are lost to their rounding
+        assert np.abs(res.fid[at] - ref).max() <= 1e-6 * np.abs(ref).max()
+        if retries:
+            assert abs(res.stats['max_half_width'] / safe - 1) <= 1e-9
+        else:
+            assert res.stats['max_half_width'] <= safe * (1 + 1e-9)
