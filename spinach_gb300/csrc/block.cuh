@@ -1096,8 +1096,8 @@ __global__ void __launch_bounds__(ECAP == 24 ? 512 : 640, 1)
 }
 
 // ---------------------------------------------------------------------------
-// Propagation, FP64.  An FP64 instruction takes a warp 64 cycles here (2 lanes
-// of each of the SM's four FP64 units a cycle), so the terms are bound by the
+// Propagation, FP64.  An FP64 instruction takes a warp 64 cycles here (half a
+// lane a cycle on each of the SM's four units), so the terms are bound by the
 // FP64 instructions of a warp and nothing else: the real and imaginary parts
 // of a row sit in two lanes of different warps (thread t and t + lanes), which
 // halves a warp's instructions per term and spreads one orientation over the
