@@ -2220,26 +2220,39 @@ struct CoupledSequence {
     }
 };
 
-// One set of rows of a sequence with its bounds and tables.
-struct SequenceGroup {
-    BlockPlan plan;
-    BlockBufs bufs;
-    Config c;
-    double table_dt = 0.0;           // time step of the tables held (0: none)
-    bool bounded = false;
-};
-
 // Tables of a sequence hold for any step count: their chunks are as long as
 // the tables allow.
 constexpr int64_t kAnySteps = (int64_t)1 << 28;
 
-// The group's configuration for a time step and a tolerance; false if its
-// series is too long for the coupled-state kernels' shared memory.
-bool configure_group(spx_handle *h, SequenceGroup &g, int64_t n_orient, double dt, double tol, bool f64, bool traj,
-                     Config &c) {
-    c.tol = tol;
-    return configure_block(h, g.plan, n_orient, dt, kAnySteps, f64, 0.0, 0, traj ? spx::kBlockTraj : 256, traj, c);
-}
+// One set of rows of a sequence with its bounds and tables.
+struct SequenceGroup {
+    BlockPlan plan;
+    BlockBufs bufs;
+    struct Setting {
+        int64_t n_orient;
+        double dt;
+        bool fits;
+        Config c;
+    };
+    std::vector<std::unique_ptr<Setting>> settings;
+    Config c;                        // the one its buffers are set up for
+    double table_dt = 0.0;           // time step of the tables held (0: none)
+    bool bounded = false;
+
+    // The configuration for a grid and a time step, worked out once; null if the
+    // series is too long for the coupled-state kernels' shared memory.
+    const Config *configure(spx_handle *h, int64_t n_orient, double dt, double tol, bool f64, bool traj) {
+        for (auto &s : settings)
+            if (s->n_orient == n_orient && s->dt == dt) return s->fits ? &s->c : nullptr;
+        settings.push_back(std::make_unique<Setting>());
+        Setting &s = *settings.back();
+        s.n_orient = n_orient;
+        s.dt = dt;
+        s.c.tol = tol;
+        s.fits = configure_block(h, plan, n_orient, dt, kAnySteps, f64, 0.0, 0, traj ? spx::kBlockTraj : 256, traj, s.c);
+        return s.fits ? &s.c : nullptr;
+    }
+};
 
 // Propagates a group over nsteps steps of dt: bounds on the first call, tables
 // whenever the time step changes.  first: place of the orientations among the
@@ -2248,11 +2261,10 @@ void run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockR
                const double *const (&angles)[3], double dt, int64_t nsteps, double tol, int lanczos_its, bool f64, bool traj,
                int *status, double *halfwidth, int64_t first = 0) {
     if (!g.bounded || g.table_dt != dt) {
-        Config c = g.c;
-        if (!configure_group(h, g, n_orient, dt, tol, f64, traj, c))
-            throw SpxError(SPX_ERR_INTERNAL, "a coupled set of states lost its layout");
-        g.c = c;
-        reserve_block(g.bufs, n_orient, f64, c);
+        const Config *set = g.configure(h, n_orient, dt, tol, f64, traj);
+        if (!set) throw SpxError(SPX_ERR_INTERNAL, "a coupled set of states lost its layout");
+        g.c = *set;
+        reserve_block(g.bufs, n_orient, f64, g.c);
     }
     const Config &c = g.c;
     BlockBufs &b = g.bufs;
@@ -2359,15 +2371,10 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
     std::vector<Config> wholes(ops.size());
     for (size_t i = 0; i < ops.size(); ++i)
         if (ops[i].kind == SPX_SEQ_EVOLVE) wholes[i] = choose_config(h, n_orient, ops[i].dt, ops[i].nsteps, o, 0);
-    std::vector<double> fits;                    // time steps known to
-    for (size_t i = 0; i < ops.size(); ++i) {
-        if (ops[i].kind != SPX_SEQ_EVOLVE || std::find(fits.begin(), fits.end(), ops[i].dt) != fits.end()) continue;
-        for (auto &grp : groups) {
-            Config c{};
-            if (!configure_group(h, *grp, n_orient, ops[i].dt, wholes[i].tol, f64, false, c)) return false;
-        }
-        fits.push_back(ops[i].dt);
-    }
+    for (size_t i = 0; i < ops.size(); ++i)
+        for (auto &grp : groups)
+            if (ops[i].kind == SPX_SEQ_EVOLVE && !grp->configure(h, n_orient, ops[i].dt, wholes[i].tol, f64, false))
+                return false;
     const bool own_states = h->n_states > 0;
     h->d_seq[0].reserve(ns);
     h->d_seq[1].reserve(ns);
@@ -2947,8 +2954,7 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
     for (int q = 0; q < 3; ++q) status[q] = h->d_seq_status.p + (size_t)q * n_orient;
     if (back_angle) {
         const Config whole = choose_config(h, n_orient, tau, nsteps, o, 0);     // refusals of the whole system
-        Config c{};
-        if (!configure_group(h, gb, n_orient, tau, whole.tol, f64, false, c)) return false;
+        if (!gb.configure(h, n_orient, tau, whole.tol, f64, false)) return false;
         const size_t ns = (size_t)n_orient * n;
         h->d_seq[0].reserve(ns);
         h->d_seq[1].reserve(ns);
@@ -2999,10 +3005,8 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
             }
         }
         if (!have) throw SpxError(SPX_ERR_UNSUPPORTED, "the trajectory does not fit a cluster of 8 SMs");
-        for (SequenceGroup *grp : {&gu, &gv}) {
-            Config c{};
-            if (!configure_group(h, *grp, nb, tau, whole.tol, f64, true, c)) return false;
-        }
+        for (SequenceGroup *grp : {&gu, &gv})
+            if (!grp->configure(h, nb, tau, whole.tol, f64, true)) return false;
         const double *const angles[3] = {g + b0, g + n_orient + b0, g + 2 * n_orient + b0};
         for (int dir = 0; dir < 2; ++dir) {
             SequenceGroup &grp = dir ? gv : gu;

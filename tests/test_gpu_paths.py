@@ -61,3 +61,18 @@ def test_programs_beyond_the_coupled_limits_take_the_whole_system(gpu_engine, n,
             v = U @ v
         ref += WEIGHTS[o] * np.array(f)
     assert rel_err(res.fid, ref) <= tol
+
+
+@pytest.mark.parametrize('prec,tol', [(E.FP64, 1e-10), (E.FP32, 1e-5)])
+@pytest.mark.parametrize('n,cplx', [(31, False), (64, True), (256, False)])
+def test_damped_systems_whole_and_on_the_coupled_states(gpu_engine, n, cplx, prec, tol):
+    """Rates far below the spectral width: the whole-system kernel (whose norm check
+    of the last series refuses rates near it) and the coupled states agree."""
+    H, Q, R, rho0, coil, block = _system(n, 20, cplx, True, 1, 2, n)
+    R = 0.02 * R
+    dt, nsteps = 0.1, 600
+    ref = WEIGHTS @ _reference(H, Q, R, rho0, coil, block, dt, nsteps)
+    gpu_engine.upload(sp.csc_matrix(H), {(2, 2, 1): sp.csc_matrix(Q)}, sp.csc_matrix(R), rho0, coil)
+    for options, states in (({}, n), ({'cluster': 1}, 0)):
+        res = gpu_engine.run(*ANGLES, WEIGHTS, dt, nsteps, precision=prec, **options)
+        assert res.stats['coupled_dim'] == states and rel_err(res.fid, ref) <= tol
