@@ -2228,43 +2228,27 @@ constexpr int64_t kAnySteps = (int64_t)1 << 28;
 struct SequenceGroup {
     BlockPlan plan;
     BlockBufs bufs;
-    struct Setting {
-        int64_t n_orient;
-        double dt;
-        bool fits;
-        Config c;
-    };
-    std::vector<std::unique_ptr<Setting>> settings;
-    Config c;                        // the one its buffers are set up for
+    Config c;
     double table_dt = 0.0;           // time step of the tables held (0: none)
     bool bounded = false;
-
-    // The configuration for a grid and a time step, worked out once; null if the
-    // series is too long for the coupled-state kernels' shared memory.
-    const Config *configure(spx_handle *h, int64_t n_orient, double dt, double tol, bool f64, bool traj) {
-        for (auto &s : settings)
-            if (s->n_orient == n_orient && s->dt == dt) return s->fits ? &s->c : nullptr;
-        settings.push_back(std::make_unique<Setting>());
-        Setting &s = *settings.back();
-        s.n_orient = n_orient;
-        s.dt = dt;
-        s.c.tol = tol;
-        s.fits = configure_block(h, plan, n_orient, dt, kAnySteps, f64, 0.0, 0, traj ? spx::kBlockTraj : 256, traj, s.c);
-        return s.fits ? &s.c : nullptr;
-    }
 };
 
 // Propagates a group over nsteps steps of dt: bounds on the first call, tables
 // whenever the time step changes.  first: place of the orientations among the
-// call's (status and halfwidth are given where they start).
-void run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockRun r, int64_t n_orient,
+// call's (status and halfwidth are given where they start).  False, and nothing
+// launched, if the series is too long for the coupled-state kernels' shared
+// memory (|L| dt of several thousand): the whole call then starts again on the
+// whole system.
+bool run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockRun r, int64_t n_orient,
                const double *const (&angles)[3], double dt, int64_t nsteps, double tol, int lanczos_its, bool f64, bool traj,
                int *status, double *halfwidth, int64_t first = 0) {
     if (!g.bounded || g.table_dt != dt) {
-        const Config *set = g.configure(h, n_orient, dt, tol, f64, traj);
-        if (!set) throw SpxError(SPX_ERR_INTERNAL, "a coupled set of states lost its layout");
-        g.c = *set;
-        reserve_block(g.bufs, n_orient, f64, g.c);
+        Config c{};
+        c.tol = tol;
+        if (!configure_block(h, g.plan, n_orient, dt, kAnySteps, f64, 0.0, 0, traj ? spx::kBlockTraj : 256, traj, c))
+            return false;
+        g.c = c;
+        reserve_block(g.bufs, n_orient, f64, c);
     }
     const Config &c = g.c;
     BlockBufs &b = g.bufs;
@@ -2284,6 +2268,7 @@ void run_group(spx_handle *h, SequenceGroup &g, spx::DevSystem &sys, spx::BlockR
     }
     r.nsteps = (int)nsteps;
     launch_propagation(h, c, sys, r, h->stream);
+    return true;
 }
 
 // Statuses of a sequence's launches (after a synchronisation).
@@ -2365,16 +2350,6 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
     const double *g = h->d_grid.p;
     const double *const angles[3] = {g, g + n_orient, g + 2 * n_orient};
     const size_t ns = (size_t)n_orient * n;
-    // every segment has to fit before the first one starts (long series: steps
-    // of several thousand in |L| dt).  The whole system's configurations come
-    // first: what they refuse stays refused.
-    std::vector<Config> wholes(ops.size());
-    for (size_t i = 0; i < ops.size(); ++i)
-        if (ops[i].kind == SPX_SEQ_EVOLVE) wholes[i] = choose_config(h, n_orient, ops[i].dt, ops[i].nsteps, o, 0);
-    for (size_t i = 0; i < ops.size(); ++i)
-        for (auto &grp : groups)
-            if (ops[i].kind == SPX_SEQ_EVOLVE && !grp->configure(h, n_orient, ops[i].dt, wholes[i].tol, f64, false))
-                return false;
     const bool own_states = h->n_states > 0;
     h->d_seq[0].reserve(ns);
     h->d_seq[1].reserve(ns);
@@ -2421,7 +2396,8 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
             if (per_orient) cur ^= 1; else rcur ^= 1;
             continue;
         }
-        whole = wholes[i];
+        // the whole system's configuration: what it refuses stays refused
+        whole = choose_config(h, n_orient, q.dt, q.nsteps, o, 0);
         const bool last = (int)i == last_evolve;
         for (size_t k = 0; k < groups.size(); ++k) {
             const bool detects = k + 1 == groups.size();
@@ -2439,7 +2415,9 @@ bool run_coupled_sequence(spx_handle *h, int64_t n_orient, const std::vector<con
                 grp.bufs.halfwidth.reserve(n_orient);
                 half = grp.bufs.halfwidth.p;
             }
-            run_group(h, grp, sys, r, n_orient, angles, q.dt, q.nsteps, whole.tol, o.lanczos_its, f64, false, status, half);
+            if (!run_group(h, grp, sys, r, n_orient, angles, q.dt, q.nsteps, whole.tol, o.lanczos_its, f64, false, status,
+                           half))
+                return false;
         }
         if (q.record) {
             const size_t np = (size_t)q.nsteps + 1;
@@ -2954,7 +2932,6 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
     for (int q = 0; q < 3; ++q) status[q] = h->d_seq_status.p + (size_t)q * n_orient;
     if (back_angle) {
         const Config whole = choose_config(h, n_orient, tau, nsteps, o, 0);     // refusals of the whole system
-        if (!gb.configure(h, n_orient, tau, whole.tol, f64, false)) return false;
         const size_t ns = (size_t)n_orient * n;
         h->d_seq[0].reserve(ns);
         h->d_seq[1].reserve(ns);
@@ -2966,8 +2943,9 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
         r.state_out = h->d_seq[0].p;
         const double *const angles[3] = {g, g + n_orient, g + 2 * n_orient};
         gb.bufs.halfwidth.reserve(n_orient);
-        run_group(h, gb, sys, r, n_orient, angles, tau, nsteps, whole.tol, o.lanczos_its, f64, false, status[2],
-                  gb.bufs.halfwidth.p);
+        if (!run_group(h, gb, sys, r, n_orient, angles, tau, nsteps, whole.tol, o.lanczos_its, f64, false, status[2],
+                       gb.bufs.halfwidth.p))
+            return false;
         dback.upload(back, h->stream);
         ++h->launches;
         sparse_states_kernel<<<state_blocks(h, ns), 256, 0, h->stream>>>(n_orient, n, dback.ptr.p, dback.col.p, dback.val.p,
@@ -3005,8 +2983,6 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
             }
         }
         if (!have) throw SpxError(SPX_ERR_UNSUPPORTED, "the trajectory does not fit a cluster of 8 SMs");
-        for (SequenceGroup *grp : {&gu, &gv})
-            if (!grp->configure(h, nb, tau, whole.tol, f64, true)) return false;
         const double *const angles[3] = {g + b0, g + n_orient + b0, g + 2 * n_orient + b0};
         for (int dir = 0; dir < 2; ++dir) {
             SequenceGroup &grp = dir ? gv : gu;
@@ -3021,8 +2997,9 @@ bool run_coupled_echo(spx_handle *h, int64_t n_orient, const std::vector<const s
             else r.rho0 = adj;
             r.traj_out = dir ? tv : tu;
             const bool final = dir == 1;
-            run_group(h, grp, sys, r, nb, angles, tau, nsteps, whole.tol, o.lanczos_its, f64, true, status[dir] + b0,
-                      final ? h->d_halfwidth.p + b0 : grp.bufs.halfwidth.p, b0);
+            if (!run_group(h, grp, sys, r, nb, angles, tau, nsteps, whole.tol, o.lanczos_its, f64, true, status[dir] + b0,
+                           final ? h->d_halfwidth.p + b0 : grp.bufs.halfwidth.p, b0))
+                return false;
         }
         const int64_t warps = nb * npoints;
         const int blocks = (int)std::min<int64_t>((warps + 7) / 8, (int64_t)h->sm_count * 16);
