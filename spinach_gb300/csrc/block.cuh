@@ -106,6 +106,11 @@ template <int ECAP> struct BlockEntries {
         Y = S;
         P = fma2(f2pk(lo[i], lo[i]), X, P);
     }
+    __device__ __forceinline__ void plain(int i, float2 &y, float2 x) const {
+        y.x = fmaf(hi[i], x.x, y.x);
+        y.y = fmaf(hi[i], x.y, y.y);
+    }
+    __device__ __forceinline__ float mag(int i) const { return fabsf(hi[i]); }
 };
 
 // The CTA's barrier for the terms, whose loops differ between warps (each warp
@@ -286,39 +291,25 @@ static __device__ float ritz_last(const float *al, const float *be, int m, float
 }
 
 // ---------------------------------------------------------------------------
-// Spectral bounds of every orientation: Gershgorin discs, and Lanczos on the
-// Hermitian part, in the run's precision (the interval is widened by the Ritz
-// residuals and 2% of its width, and the propagation watches the norm).  The
-// matrix is taken about the middle of its discs, so that alpha is no larger than
-// the spread.  Real couplings keep real vectors.  The assembled L goes to R.saved
-// for the FP32 propagation, which runs on the same layout.
-//
-// Bound by latency: a step is one product and two sums over the CTA, 32 times.
-// FP64 instructions take a warp 64 cycles, so the FP64 kernel runs just its
-// warp's entries (seven spins, 1000 orientations, 2048 steps in FP64: 13.94 ms,
-// with FP32 bounds 13.84).
+// Spectral bounds of every orientation of FP32 runs: Gershgorin discs, and Lanczos
+// on the Hermitian part, in FP32 (the interval is widened by the Ritz residuals
+// and 2% of its width, and the propagation watches the norm).
+// The matrix is taken about the middle of its discs, so that alpha is no larger
+// than the spread.  The assembled L goes to R.saved for the FP32 propagation, which
+// runs on the same layout.
 // ---------------------------------------------------------------------------
-template <class Real> struct RealPair;
-template <> struct RealPair<float> { using type = float2; };
-template <> struct RealPair<double> { using type = double2; };
-
-template <bool EXT, int ECAP, class Real>
-__global__ void __launch_bounds__(kBlockRows, sizeof(Real) == 4 && ECAP <= 16 ? 2 : 1)
-    block_bounds_kernel(const DevSystem sys, const BlockLayout B, const BlockRun R) {
-    constexpr bool F64 = sizeof(Real) == 8;
-    using Pair = typename RealPair<Real>::type;
-    using Vec = std::conditional_t<EXT, Pair, Real>;          // a state's part of a Lanczos vector
-    constexpr int XN = (EXT ? 2 : 1) * kBlockRows;            // the last slot takes what no one reads
+template <bool EXT, int ECAP>
+__global__ void __launch_bounds__(kBlockRows, ECAP <= 16 ? 2 : 1) block_bounds_kernel(const DevSystem sys, const BlockLayout B,
+                                                                     const BlockRun R) {
     __shared__ double s_coef[kMaxCoef];
-    __shared__ Vec s_x[2][XN + 1];
-    __shared__ Pair s_part[2][kBlockRows / 32];
+    __shared__ float2 s_x[2][(EXT ? 2 : 1) * kBlockRows + 1];
+    __shared__ float2 s_part[2][kBlockRows / 32];
     __shared__ float s_al[kMaxLanczos], s_be[kMaxLanczos];
     __shared__ float s_work[2][3][kMaxLanczos];
     const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const BlockLane l = block_lane(B, tid);
     block_coefficients(sys, R, o, s_coef);
-    Real val[ECAP];
-    int col[ECAP];                                            // byte offsets
+    BlockEntries<ECAP> E;
     double2 dg = make_double2(0.0, 0.0);
     {
         const double sign = R.adjoint ? -1.0 : 1.0;
@@ -333,8 +324,8 @@ __global__ void __launch_bounds__(kBlockRows, sizeof(Real) == 4 && ECAP <= 16 ? 
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int i = i0 + q;
-                val[i] = (Real)v[q];
-                col[i] = i < l.ew ? B.col[i * B.threads + tid] * (int)sizeof(Vec) : 0;
+                E.set(i, v[q]);
+                E.col[i] = i < l.ew ? B.col[i * B.threads + tid] * (int)sizeof(float2) : 0;
                 if (save && i < l.ew) save[(size_t)i * B.threads + tid] = v[q];
             }
         }
@@ -346,23 +337,175 @@ __global__ void __launch_bounds__(kBlockRows, sizeof(Real) == 4 && ECAP <= 16 ? 
         }
     }
     int par = 0;
+    // sums (op 0) or maxima (op 1) of both components over the CTA; the slots
+    // alternate, so one barrier each
+    auto reduce = [&](float2 v, int op) {
+#pragma unroll
+        for (int q = 16; q; q >>= 1) {
+            const float ux = __shfl_xor_sync(0xffffffffu, v.x, q), uy = __shfl_xor_sync(0xffffffffu, v.y, q);
+            v.x = op ? fmaxf(v.x, ux) : v.x + ux;
+            v.y = op ? fmaxf(v.y, uy) : v.y + uy;
+        }
+        if (nwarps == 1) return v;
+        if (lane == 0) s_part[par][warp] = v;
+        __syncthreads();
+        v = s_part[par][0];
+        for (int w = 1; w < nwarps; ++w) {
+            const float2 u = s_part[par][w];
+            v.x = op ? fmaxf(v.x, u.x) : v.x + u.x;
+            v.y = op ? fmaxf(v.y, u.y) : v.y + u.y;
+        }
+        par ^= 1;
+        return v;
+    };
+    auto join = [&](float v) {                                // sum over the parts of a row
+        for (int r = 0; r < l.rounds; ++r) {
+            const float u = __shfl_xor_sync(0xffffffffu, v, 1 << r);
+            if ((l.parts >> r) > 1) v += u;
+        }
+        return v;
+    };
+    float rad = 0.f;
+#pragma unroll
+    for (int i = 0; i < ECAP; ++i) rad += E.mag(i);
+    rad = join(rad);
+    // float sums: 4e-6 of the row covers their rounding
+    const float dgf = (float)dg.x, slack = 4e-6f * (fabsf(dgf) + rad);
+    const float2 g = reduce(l.state ? make_float2(dgf + rad + slack, -(dgf - rad - slack))
+                                    : make_float2(-CUDART_INF_F, -CUDART_INF_F), 1);
+    const double gmax = g.x, gmin = -g.y, mid = 0.5 * (gmax + gmin);
+    const float dre = (float)(dg.x - mid);
+
+    float2 q_cur = make_float2(0.f, 0.f), q_prev = q_cur;
+    if (l.state) q_cur.x = 1.0f + 0.37f * __sinf(1.7f * (float)l.row + 0.3f);
+    {
+        const float inv = rsqrtf(reduce(make_float2(q_cur.x * q_cur.x, 0.f), 0).x);
+        q_cur.x *= inv;
+    }
+    float beta_prev = 0.f;
+    int m_eff = 0;
+    // also beyond n steps: FP32 vectors lose their orthogonality on clustered
+    // spectra, and n steps then miss the ends (more only find them again)
+    const int lits = min(R.lanczos_its, kMaxLanczos);
+    const int slot = l.state ? l.row : (EXT ? 2 : 1) * kBlockRows, slot2 = l.state ? B.n + l.row : slot;
+    for (int j = 0; j < lits; ++j) {
+        float2 *x = s_x[j & 1];
+        x[slot] = q_cur;
+        if (EXT) x[slot2] = make_float2(-q_cur.y, q_cur.x);
+        __syncthreads();
+        float2 y = make_float2(0.f, 0.f);
+        const char *xb = reinterpret_cast<const char *>(x);
+#pragma unroll
+        for (int i = 0; i < ECAP; ++i) E.plain(i, y, *reinterpret_cast<const float2 *>(xb + E.col[i]));
+        y.x = join(y.x);
+        y.y = join(y.y);
+        if (l.state) {
+            y.x += dre * q_cur.x - beta_prev * q_prev.x;
+            y.y += dre * q_cur.y - beta_prev * q_prev.y;
+        } else {
+            y = make_float2(0.f, 0.f);
+        }
+        const float alpha = reduce(make_float2(q_cur.x * y.x + q_cur.y * y.y, 0.f), 0).x;
+        y.x -= alpha * q_cur.x;
+        y.y -= alpha * q_cur.y;
+        // beta from the residual itself: |w|^2 - alpha^2 would hide directions
+        // that the start vector holds little of
+        const float beta = sqrtf(reduce(make_float2(y.x * y.x + y.y * y.y, 0.f), 0).x);
+        if (tid == 0) { s_al[j] = alpha; s_be[j] = beta; }
+        m_eff = j + 1;
+        if (!(beta > 1e-12f * (fabsf(alpha) + 1e-30f))) break;      // invariant subspace
+        const float inv = 1.f / beta;
+        q_prev = q_cur;
+        q_cur.x = y.x * inv;
+        q_cur.y = y.y * inv;
+        beta_prev = beta;
+    }
+    __syncthreads();
+    if (tid < 32) {
+        const double2 ends = tridiag_ends(s_al, s_be, m_eff, lane);
+        const double tlo = ends.x, thi = ends.y;
+        float rr = 0.f;                                          // lane 0 the top, lane 1 the bottom
+        if (!R.safe_bounds && lane < 2)
+            rr = fabsf(s_be[m_eff - 1]) * ritz_last(s_al, s_be, m_eff, lane == 0 ? (float)thi : (float)tlo, s_work[lane]);
+        const double rhi = __shfl_sync(0xffffffffu, rr, 0), rlo = __shfl_sync(0xffffffffu, rr, 1);
+        if (lane == 0) {
+            double hi = gmax, lo = gmin;
+            if (!R.safe_bounds) {
+                const double wid = thi - tlo;
+                hi = fmin(mid + thi + rhi + 0.02 * wid, gmax);
+                lo = fmax(mid + tlo - rlo - 0.02 * wid, gmin);
+                if (!(hi >= lo)) { hi = gmax; lo = gmin; }
+            }
+            const double scale = fmax(fabs(hi), fabs(lo));
+            const double half = fmax(0.5 * (hi - lo) * 1.01 + 1e-9 * scale, R.max_im_diag) + 1e-30;
+            R.centre[o] = 0.5 * (hi + lo);
+            R.halfwidth[o] = half;
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(half);   // half > 0
+            atomicMax(R.extent, bits);
+            atomicMax(R.extent + 1, ~bits);
+        }
+    }
+}
+
+// The same in FP64 for FP64 runs.  Real couplings keep real vectors.  Bound by
+// latency: a step is one product and two sums over the CTA, 32 times, and an FP64
+// instruction takes a warp 64 cycles, so it runs just its warp's entries, on the
+// layout that the host finds cheapest for it (with FP32 bounds and with these:
+// seven spins, 1000 orientations, 2048 steps in FP64 13.67 and 13.58 ms; one
+// orientation of a radical with three protons, 127 steps, 0.35 and 0.39 ms).
+template <bool EXT, int ECAP>
+__global__ void __launch_bounds__(kBlockRows, 1)
+    block_bounds64_kernel(const DevSystem sys, const BlockLayout B, const BlockRun R) {
+    using Vec = std::conditional_t<EXT, double2, double>;          // a state's part of a Lanczos vector
+    constexpr int XN = (EXT ? 2 : 1) * kBlockRows;            // the last slot takes what no one reads
+    __shared__ double s_coef[kMaxCoef];
+    __shared__ Vec s_x[2][XN + 1];
+    __shared__ double2 s_part[2][kBlockRows / 32];
+    __shared__ float s_al[kMaxLanczos], s_be[kMaxLanczos];
+    __shared__ float s_work[2][3][kMaxLanczos];
+    const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const BlockLane l = block_lane(B, tid);
+    block_coefficients(sys, R, o, s_coef);
+    double val[ECAP];
+    int col[ECAP];                                            // byte offsets
+    double2 dg = make_double2(0.0, 0.0);
+    {
+        const double sign = R.adjoint ? -1.0 : 1.0;
+        // four entries at a time: more FP64 sums in registers cost resident CTAs
+#pragma unroll
+        for (int i0 = 0; i0 < ECAP; i0 += 4) {
+            double v[4];
+            BlockLayout Bi = B;
+            Bi.src = B.src + (size_t)i0 * B.threads;
+            block_assemble<4>(sys, Bi, l.ew - i0, tid, s_coef, sign, v);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int i = i0 + q;
+                val[i] = v[q];
+                col[i] = i < l.ew ? B.col[i * B.threads + tid] * (int)sizeof(Vec) : 0;
+            }
+        }
+        if (l.state) dg = block_diagonal(sys, B.row_src[l.row], s_coef, sign);
+    }
+    int par = 0;
     // sum over the CTA; the slots alternate, so one barrier each
-    auto sum = [&](Real v) {
+    auto sum = [&](double v) {
 #pragma unroll
         for (int q = 16; q; q >>= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
         if (nwarps == 1) return v;
         if (lane == 0) s_part[par][warp].x = v;
         __syncthreads();
-        v = s_part[par][0].x;
-        for (int w = 1; w < nwarps; ++w) v += s_part[par][w].x;
+        v = lane < nwarps ? s_part[par][lane].x : 0.0;        // log2 of the warps' additions
+        for (int q = 1; q < nwarps; q *= 2) v += __shfl_xor_sync(0xffffffffu, v, q);
+        v = __shfl_sync(0xffffffffu, v, 0);
         par ^= 1;
         return v;
     };
     // largest of both components over the CTA
-    auto largest = [&](Pair v) {
+    auto largest = [&](double2 v) {
 #pragma unroll
         for (int q = 16; q; q >>= 1) {
-            const Real ux = __shfl_xor_sync(0xffffffffu, v.x, q), uy = __shfl_xor_sync(0xffffffffu, v.y, q);
+            const double ux = __shfl_xor_sync(0xffffffffu, v.x, q), uy = __shfl_xor_sync(0xffffffffu, v.y, q);
             v.x = ux > v.x ? ux : v.x;
             v.y = uy > v.y ? uy : v.y;
         }
@@ -370,49 +513,41 @@ __global__ void __launch_bounds__(kBlockRows, sizeof(Real) == 4 && ECAP <= 16 ? 
         if (lane == 0) s_part[par][warp] = v;
         __syncthreads();
         for (int w = 0; w < nwarps; ++w) {
-            const Pair u = s_part[par][w];
+            const double2 u = s_part[par][w];
             v.x = u.x > v.x ? u.x : v.x;
             v.y = u.y > v.y ? u.y : v.y;
         }
         par ^= 1;
         return v;
     };
-    auto join = [&](Real v) {                                 // sum over the parts of a row
+    auto join = [&](double v) {                                 // sum over the parts of a row
         for (int r = 0; r < l.rounds; ++r) {
-            const Real u = __shfl_xor_sync(0xffffffffu, v, 1 << r);
+            const double u = __shfl_xor_sync(0xffffffffu, v, 1 << r);
             if ((l.parts >> r) > 1) v += u;
         }
         return v;
     };
-    Real rad = 0;
+    double rad = 0;
 #pragma unroll
     for (int i = 0; i < ECAP; ++i)
-        if (!F64 || i < l.ew) rad += fabs(val[i]);
+        if (i < l.ew) rad += fabs(val[i]);
     rad = join(rad);
-    // float sums: 4e-6 of the row covers their rounding (FP64: the half-width's
-    // 1e-9 does)
-    const Real dgr = (Real)dg.x, slack = F64 ? (Real)0 : (Real)4e-6f * (fabs(dgr) + rad);
-    Pair ends;
-    ends.x = l.state ? dgr + rad + slack : (Real)-CUDART_INF_F;
-    ends.y = l.state ? -(dgr - rad - slack) : (Real)-CUDART_INF_F;
-    ends = largest(ends);
+    const double2 ends = largest(l.state ? make_double2(dg.x + rad, rad - dg.x) : make_double2(-CUDART_INF, -CUDART_INF));
     const double gmax = ends.x, gmin = -ends.y, mid = 0.5 * (gmax + gmin);
-    const Real dre = (Real)(dg.x - mid);
+    const double dre = dg.x - mid;
 
     Vec q_cur{}, q_prev{};
-    auto re = [](Vec &v) -> Real & { if constexpr (EXT) return v.x; else return v; };
+    auto re = [](Vec &v) -> double & { if constexpr (EXT) return v.x; else return v; };
     // over the real and, where there are any, the imaginary parts of two vectors
-    auto dot = [](const Vec &a, const Vec &b) -> Real {
+    auto dot = [](const Vec &a, const Vec &b) -> double {
         if constexpr (EXT) return a.x * b.x + a.y * b.y;
         else return a * b;
     };
-    if (l.state) re(q_cur) = (Real)(1.0f + 0.37f * __sinf(1.7f * (float)l.row + 0.3f));
+    if (l.state) re(q_cur) = (double)(1.0f + 0.37f * __sinf(1.7f * (float)l.row + 0.3f));
     re(q_cur) *= rsqrt(sum(re(q_cur) * re(q_cur)));
-    Real beta_prev = 0;
+    double beta_prev = 0;
     int m_eff = 0;
-    // FP32 also beyond n steps: its vectors lose their orthogonality on clustered
-    // spectra, and n steps then miss the ends (more only find them again)
-    const int lits = min(R.lanczos_its, F64 ? min(kMaxLanczos, B.n) : kMaxLanczos);
+    const int lits = min(R.lanczos_its, min(kMaxLanczos, B.n));
     const int slot = l.state ? l.row : XN, slot2 = l.state ? B.n + l.row : slot;
     for (int j = 0; j < lits; ++j) {
         Vec *x = s_x[j & 1];
@@ -428,7 +563,7 @@ __global__ void __launch_bounds__(kBlockRows, sizeof(Real) == 4 && ECAP <= 16 ? 
         const char *xb = reinterpret_cast<const char *>(x);
 #pragma unroll
         for (int i = 0; i < ECAP; ++i)
-            if (!F64 || i < l.ew) {
+            if (i < l.ew) {
                 const Vec xi = *reinterpret_cast<const Vec *>(xb + col[i]);
                 if constexpr (EXT) { y.x = fma(val[i], xi.x, y.x); y.y = fma(val[i], xi.y, y.y); }
                 else y = fma(val[i], xi, y);
@@ -442,16 +577,26 @@ __global__ void __launch_bounds__(kBlockRows, sizeof(Real) == 4 && ECAP <= 16 ? 
         } else {
             y += dre * q_cur - beta_prev * q_prev;
         }
-        const Real alpha = sum(dot(q_cur, y));
+        const double alpha = sum(dot(q_cur, y));
         if constexpr (EXT) { y.x -= alpha * q_cur.x; y.y -= alpha * q_cur.y; }
         else y -= alpha * q_cur;
         // beta from the residual itself: |w|^2 - alpha^2 would hide directions
         // that the start vector holds little of
-        const Real beta = sqrt(sum(dot(y, y)));
+        const double beta2 = sum(dot(y, y));
+        double beta, inv;
+        if (beta2 > 1e-30 && beta2 < 1e30) {
+            // a float's reciprocal root and one Newton step (to 5e-15): a third of the
+            // FP64 instructions of sqrt and a division, which were half of a step's
+            const double r = (double)rsqrtf((float)beta2);
+            inv = r * fma(-0.5 * beta2, r * r, 1.5);
+            beta = beta2 * inv;
+        } else {
+            beta = sqrt(beta2);
+            inv = 1.0 / beta;
+        }
         if (tid == 0) { s_al[j] = (float)alpha; s_be[j] = (float)beta; }
         m_eff = j + 1;
-        if (!(beta > (Real)1e-12 * (fabs(alpha) + (Real)1e-30))) break;      // invariant subspace
-        const Real inv = (Real)1 / beta;
+        if (!(beta > 1e-12 * (fabs(alpha) + 1e-30))) break;      // invariant subspace
         q_prev = q_cur;
         if constexpr (EXT) { q_cur.x = y.x * inv; q_cur.y = y.y * inv; }
         else q_cur = y * inv;

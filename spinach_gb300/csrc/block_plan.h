@@ -60,6 +60,16 @@ struct BlockCost {
     double latency = 0.0;
     int warps = 0;             // of one orientation's CTA
     int warps_per_sm = 16;     // resident, by registers
+    // a Lanczos step of the FP64 bounds on this layout, alike: one instruction (two
+    // with complex couplings) per entry and reduction step, and about 30 of its own
+    double bounds_issue = 0.0, bounds_latency = 0.0;
+    int bounds_warps = 0;
+    double bounds_time(double per_sm) const {
+        const double res = std::max(1.0, std::floor(16.0 / bounds_warps)), full = std::floor(per_sm / res);
+        const double rest = std::ceil(per_sm - full * res);
+        return full * std::max(bounds_latency, res * bounds_issue) +
+               (rest > 0.0 ? std::max(bounds_latency, rest * bounds_issue) : 0.0);
+    }
     // relative time of n orientations per SM: rounds of as many as fit, the last
     // with what is left
     double time(double per_sm) const {
@@ -88,7 +98,7 @@ inline size_t block_lane_count(const BlockPattern &P, int e) {
 
 // The layout on `warps` warps with at most e entries per lane; false if the
 // rows do not fit.
-inline bool block_lanes(const BlockPattern &P, int warps, int e, bool f64, bool damped, BlockLanes &L,
+inline bool block_lanes(const BlockPattern &P, int warps, int e, bool f64, bool damped, bool cplx, BlockLanes &L,
                         BlockCost &cost) {
     if (block_lane_count(P, e) > 32u * (size_t)warps) return false;
     const int T = 32 * warps, nr = P.n + P.nv;
@@ -129,9 +139,13 @@ inline bool block_lanes(const BlockPattern &P, int warps, int e, bool f64, bool 
     cost = BlockCost{};
     cost.warps = f64 ? 2 * warps : warps;
     cost.warps_per_sm = f64 ? 32 : 16;
-    double unit[4] = {0.0, 0.0, 0.0, 0.0};
+    double unit[4] = {0.0, 0.0, 0.0, 0.0}, bunit[4] = {0.0, 0.0, 0.0, 0.0};
+    cost.bounds_warps = warps;
     for (int w = 0; w < warps; ++w) {
         L.shape[w] = ew[w] | (rounds[w] << 8);
+        const double b = 64.0 * ((cplx ? 2.0 : 1.0) * (ew[w] + rounds[w]) + 30.0);
+        cost.bounds_issue += b / 4.0;
+        bunit[w % 4] += b;
         if (f64) {
             const double n = 64.0 * (ew[w] + rounds[w] + (damped ? 4.0 : 3.0));
             cost.issue += 2.0 * n / 4.0;
@@ -151,6 +165,7 @@ inline bool block_lanes(const BlockPattern &P, int warps, int e, bool f64, bool 
         }
     }
     for (double u : unit) cost.latency = std::max(cost.latency, u);
+    for (double u : bunit) cost.bounds_latency = std::max(cost.bounds_latency, u);
     cost.latency += f64 ? 200.0 : 120.0;
     if (cost.warps > 1) cost.latency += 30.0;
     return true;

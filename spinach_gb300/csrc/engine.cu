@@ -374,7 +374,7 @@ void build_plan(spx_handle *h, const std::vector<int> &rows, const std::vector<i
             if (w > spx::kBlockRows / 32) continue;
             spx::BlockLanes L;
             spx::BlockCost c;
-            if (block_lanes(P, w, e, p == 1, h->max_im_diag > 0.0, L, c)) {
+            if (block_lanes(P, w, e, p == 1, h->max_im_diag > 0.0, h->cplx, L, c)) {
                 lanes.push_back(std::move(L));
                 costs.push_back(c);
             }
@@ -883,7 +883,7 @@ struct Config {
     int traj_m = 1;                               // trajectory outputs: chunk length (1: none)
     bool traj = false;                            // the kernels with trajectory outputs
     // the coupled-state kernels (block.cuh), if they run: their layout and that
-    // of the spectral bounds (an FP32 layout in both precisions), chunk target, chunk cap, series cap, ladder steps and shared memory
+    // of the spectral bounds, chunk target, chunk cap, series cap, ladder steps and shared memory
     const BlockPlan::Layout *blk = nullptr, *blk_bounds = nullptr;
     double blk_x = 0.0;
     int blk_M = 0, blk_K = 0, blk_lev = 0;
@@ -1047,7 +1047,16 @@ bool configure_block(spx_handle *h, const BlockPlan &plan, int64_t n_orient, dou
     const size_t part = (h->smem_sm / (even + 1) + 256) & ~(size_t)15;
     c.blk_even = part > own ? std::max(c.blk_smem, part - own) : c.blk_smem;
     c.blk = best;
-    c.blk_bounds = f64 ? best_layout(plan.layouts[0], per_sm) : best;
+    c.blk_bounds = best;
+    if (f64) {
+        // the FP64 bounds run on any layout of at most kBlockMaxEntries a lane
+        c.blk_bounds = nullptr;
+        for (const auto &ls : plan.layouts)
+            for (const auto &l : ls)
+                if (l.ecap <= spx::kBlockMaxEntries &&
+                    (!c.blk_bounds || l.cost.bounds_time(per_sm) < c.blk_bounds->cost.bounds_time(per_sm)))
+                    c.blk_bounds = &l;
+    }
     c.blk_bounds_which = f64 ? 5 : 0;
     return true;
 }
