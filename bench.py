@@ -93,6 +93,14 @@ def coupled_nnz(L):
     return int(P[rows].nnz)
 
 
+def launch_shape(stats):
+    """What ran: the coupled states, or the whole system in its launch shape (the
+    statistics' threads and cluster describe that one either way)."""
+    if stats['coupled_dim']:
+        return {'coupled_states': stats['coupled_dim']}
+    return {'threads': stats['threads'], 'cluster': stats['cluster']}
+
+
 def profile_traffic(name='block_chebyshev_c1.md'):
     """Per-launch DRAM bytes of the propagation kernel from the committed ncu summary."""
     p = os.path.join(ROOT, 'profiles', name)
@@ -474,7 +482,7 @@ def run_gpu(args):
             'config': {'workload': WORKLOAD_TEXT[args.workload], 'fid_unit': FID_NOTE,
                        'l2': 'flushed between steps (256 MiB)',
                        'precision': args.precision, 'chunk_steps': stats['chunk_steps'],
-                       'series_terms_max': stats['max_terms'], 'threads': stats['threads'],
+                       'series_terms_max': stats['max_terms'], **launch_shape(stats),
                        'parallelism': f'orientations over CTAs; {world} rank(s), one grid block each'},
             'rel_err_vs_fp64_gpu': rel_err,
             'fp64_gpu': {'value': no / fp64_s, 'unit': UNIT, 'kernel_ms': r64.stats['kernel_ms']},
@@ -545,8 +553,7 @@ def c4_leg(device):
     out = {'workload': 'c4: e + 14N + 10 1H at 0.34 T, IK-1(3) dim 2736, T2e, 4000-orientation zcwn grid, '
                        '4096 steps of 1 ns', 'value': w.n_orient / t32, 'unit': UNIT,
            'rel_err_vs_fp64_gpu': _rel(r32.fid, r64.fid), 'fp64_gpu': {'value': w.n_orient / t64},
-           'kernel_ms': r32.stats['kernel_ms'], 'cluster': r32.stats['cluster'], 'threads': r32.stats['threads'],
-           'matvecs': r32.stats['matvecs']}
+           'kernel_ms': r32.stats['kernel_ms'], **launch_shape(r32.stats), 'matvecs': r32.stats['matvecs']}
     eng.close()
     return out
 
@@ -586,7 +593,7 @@ def mas_leg(device):
            'value': w.n_orient / res[E.FP32][0], 'unit': UNIT,
            'rel_err_vs_fp64_gpu': _rel(res[E.FP32][1].fid, res[E.FP64][1].fid),
            'fp64_gpu': {'value': w.n_orient / res[E.FP64][0]},
-           'kernel_ms': res[E.FP32][1].stats['kernel_ms'], 'cluster': res[E.FP32][1].stats['cluster'],
+           'kernel_ms': res[E.FP32][1].stats['kernel_ms'], **launch_shape(res[E.FP32][1].stats),
            'nnz': res[E.FP32][1].stats['nnz'], 'rotor_space_setup_s': t_fp,
            'floquet': {'workload': 'floquet.m: the same system, rate, axis, grid and steps, 17 Fourier '
                                    'components (dim 1088), upload + run',
@@ -594,7 +601,7 @@ def mas_leg(device):
                        'rel_err_vs_fp64_gpu': _rel(rfl[E.FP32][1].fid, rfl[E.FP64][1].fid),
                        'fp64_gpu': {'value': w.n_orient / rfl[E.FP64][0]},
                        'kernel_ms': rfl[E.FP32][1].stats['kernel_ms'],
-                       'cluster': rfl[E.FP32][1].stats['cluster'], 'nnz': rfl[E.FP32][1].stats['nnz'],
+                       **launch_shape(rfl[E.FP32][1].stats), 'nnz': rfl[E.FP32][1].stats['nnz'],
                        'setup_s': t_fl}}
     eng.close()
     return out

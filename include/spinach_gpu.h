@@ -136,7 +136,12 @@ typedef struct {
     int32_t coupled_dim;       /* states that couple to the coils, if the run was restricted
                                   to them (0: the whole system ran).  threads, cluster,
                                   smem_bytes, nnz and ell_entries describe the whole
-                                  system and its launch shape either way */
+                                  system and its launch shape either way.  Few states or
+                                  orientations may run by dense matrices: max_terms is then
+                                  16 (the degree of the exponential), chunk_steps the states
+                                  kept per orientation, matvecs counts the products of the
+                                  exponential's matrices by column, and the half-widths are
+                                  a bound on |L| */
     double fp32_powder_error;  /* the error those imply for the powder FID, two parts in
                                   quadrature: the checked orientations' running relative
                                   error weighted by the powder FID's intensity over time,
